@@ -246,3 +246,85 @@ def tolerance(case):
     if case["op"] == "fp4_scores":
         return {"rel": 1e-6, "max": 1e-5}               # exact group sums, added in fp32
     return {"rel": 1e-2, "max": 7e-2, "differ": 0.0}    # bf16 probabilities, partials and outputs
+
+
+def _attend(q, k, v, blocks, keep):
+    """softmax(q k^T / sqrt(D)) v of one list in 64 bits: q [g, n, D], k and v [nb, BLOCK, D], blocks [m], keep
+    [n, m * BLOCK] or None -> (o, lse)."""
+    kk, vv = (t[blocks].reshape(-1, D).double() for t in (k, v))
+    s = q.double() @ kk.T / math.sqrt(D)
+    if keep is not None:
+        s = s.masked_fill(~keep, -math.inf)
+    lse = s.logsumexp(-1)
+    return torch.exp(s - lse[..., None]) @ vv, lse
+
+
+def _exact_scores(s, case):
+    """Page scores of the ragged batch: decoded e2m1 codes and e4m3 scales, products and sums in 64 bits."""
+    table = torch.tensor([0, 0.5, 1, 1.5, 2, 3, 4, 6], dtype=torch.float64, device="cuda")
+    table = torch.cat([table, -table])
+
+    def decode(codes, scales):
+        pairs = torch.stack([codes & 15, codes >> 4], -1).flatten(-2)
+        return table[pairs.long()] * scales.to(torch.float64).repeat_interleave(16, -1)
+    q_lens, k_lens = _lengths(case)
+    hq, tiles, pages = case["hk"] * case["group"], -(-max(k_lens) // BLOCK), s["options"]["kv_indices"]
+    out = torch.full((hq, tiles, sum(q_lens)), -math.inf, dtype=torch.float64, device="cuda")
+    q0 = p0 = 0
+    for n, m in zip(q_lens, k_lens):
+        np_ = -(-m // BLOCK)
+        own = pages[p0:p0 + np_].long()
+        last = torch.arange(n, device="cuda") + (m - n if case["causal"] else m)      # last visible key of a query
+        for h in range(hq):
+            qd = decode(s["q"][q0:q0 + n, h], s["q_scale"][q0:q0 + n, h])
+            kd = decode(s["k"][own, h // case["group"]], s["k_scale"][own, h // case["group"]]).reshape(-1, D)
+            x = qd @ kd.T
+            col = torch.arange(np_ * BLOCK, device="cuda")
+            x = x.masked_fill((col[None] >= m) | (col[None] > last[:, None]), -math.inf)
+            out[h, :np_, q0:q0 + n] = x.view(n, np_, BLOCK).amax(-1).T
+        q0, p0 = q0 + n, p0 + np_
+    return out
+
+
+def exact(case, seed):
+    """The outputs of run() in 64 bits; None where the path selects its blocks itself (the ids are compared as they
+    are) and where it would take long."""
+    op = case["op"]
+    if op not in ("attention", "kv_centric", "kv_tokens", "fp4_scores") or work(case)["flops"] > 5e12:
+        return None
+    s = prepare(case, seed)
+    if op == "fp4_scores":
+        return _exact_scores(s, case)
+    b, hkv, g, nb = case["b"], case["hkv"], case["group"], case["nb"]
+    source = s["operator"] if op != "attention" else None
+    q, k, v = (source.q, source.k, source.v) if source else (s["q"], s["k"], s["v"])
+    ids, counts = (source.selected, None) if source else (s["ids"], s["counts"])
+    if case.get("q_token_major"):
+        q = q.transpose(1, 2)
+    sq = q.shape[2]
+    step = BLOCK
+    if op == "kv_tokens":
+        if 4.0 * b * hkv * g * sq * nb * BLOCK * D > 5e12:
+            return None
+        step = max(1, (1 << 27) // (g * nb * BLOCK))
+    out = torch.empty((b, hkv * g, sq, D), dtype=torch.float64, device="cuda")
+    lse = torch.empty((b, hkv * g, sq), dtype=torch.float64, device="cuda")
+    everything = torch.arange(nb, device="cuda")
+    lists = ids.long()
+    live = counts.tolist() if counts is not None else None
+    for i in range(b):
+        for h in range(hkv):
+            heads = slice(h * g, (h + 1) * g)
+            ki, vi = (t[i, h].view(nb, BLOCK, D) for t in (k, v))
+            for t in range(0, sq, step):
+                rows = slice(t, min(t + step, sq))
+                if op == "kv_tokens":
+                    mark = torch.zeros((rows.stop - t, nb), dtype=torch.bool, device="cuda")
+                    mark.scatter_(1, lists[i, h, rows], True)
+                    blocks, keep = everything, mark.repeat_interleave(BLOCK, 1)
+                else:
+                    blocks, keep = lists[i, h, t // BLOCK], None
+                    if live:
+                        blocks = blocks[:live[i][h][t // BLOCK]]
+                out[i, heads, rows], lse[i, heads, rows] = _attend(q[i, heads, rows], ki, vi, blocks, keep)
+    return out, lse
