@@ -193,6 +193,36 @@ __device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint64_t b, uint3
       : "memory");
 }
 
+// The same with operands in 128-byte-swizzled K-major / MN-major tiles given by the low words of their
+// descriptors (the high words are constants): fewer instructions on the issuing thread's path.
+template <uint32_t HI_A, uint32_t HI_B>
+__device__ __forceinline__ void mma_ss_lo(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      ".reg .b64 da, db;\n\t"
+      "mov.b64 da, {%1, %5};\n\t"
+      "mov.b64 db, {%2, %6};\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t"
+      "}" ::"r"(d),
+      "r"(a), "r"(b), "r"(idesc), "r"(accumulate), "n"(HI_A), "n"(HI_B)
+      : "memory");
+}
+template <uint32_t HI_B>
+__device__ __forceinline__ void mma_ts_lo(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      ".reg .b64 db;\n\t"
+      "mov.b64 db, {%2, %5};\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n\t"
+      "}" ::"r"(d),
+      "r"(a), "r"(b), "r"(idesc), "r"(accumulate), "n"(HI_B)
+      : "memory");
+}
+
 // 32 lanes x 32 consecutive 32-bit columns: thread t of the warp gets row t.
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
@@ -338,6 +368,12 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
       : "=f"(d.x), "=f"(d.y)
       : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
   return d;
+}
+// ties registers to a point of the program (after the wait that makes them valid)
+__device__ __forceinline__ void pin(uint32_t (&r)[32]) {
+#pragma unroll
+  for (int i = 0; i < 32; i += 8)
+    asm volatile("" : "+r"(r[i]), "+r"(r[i + 1]), "+r"(r[i + 2]), "+r"(r[i + 3]), "+r"(r[i + 4]), "+r"(r[i + 5]), "+r"(r[i + 6]), "+r"(r[i + 7]));
 }
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);

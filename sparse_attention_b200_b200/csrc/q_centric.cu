@@ -433,24 +433,28 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
     // S_q = Q_q K^T : 8 MMAs of K = 16 over two 64-column panels.
     auto issue_qk = [&](int q, uint32_t slot) {
       {
-        const uint64_t a0 = desc_sw128_kmajor(base + OFF_Q + q * TILE_BYTES);
-        const uint64_t b0 = desc_sw128_kmajor(base + OFF_RING + slot * TILE_BYTES);
+        // low descriptor words only: the issuing thread shares its scheduler with two softmax warps, so every
+        // instruction between "P is ready" and the MMA counts (64-bit descriptor arithmetic: 1-2 % slower)
+        const uint32_t a0 = (base + OFF_Q + q * TILE_BYTES) >> 4;
+        const uint32_t b0 = (base + OFF_RING + slot * TILE_BYTES) >> 4;
+        constexpr uint32_t HI = (1024u >> 4) | (1u << 14) | (2u << 29);
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) {
-          const uint64_t step = static_cast<uint64_t>((kk >> 2) * (PANEL_BYTES >> 4) + (kk & 3) * 2);
-          mma_ss(tmem + q * TILE, a0 + step, b0 + step, IDESC_QK, kk > 0);
+          const uint32_t step = (kk >> 2) * (PANEL_BYTES >> 4) + (kk & 3) * 2;
+          mma_ss_lo<HI, HI>(tmem + q * TILE, a0 + step, b0 + step, IDESC_QK, kk > 0);
         }
       }
     };
     // O_q (+)= P_q V : A from tensor memory (8 columns per K = 16), B = V MN-major.
     auto issue_pv_part = [&](int q, uint32_t slot, bool accumulate, int k0, int k1) {
       {
-        const uint64_t b0 = desc_sw128_mnmajor(base + OFF_RING + slot * TILE_BYTES, PANEL_BYTES, 1024);
+        const uint32_t b0 = ((base + OFF_RING + slot * TILE_BYTES) >> 4) | ((PANEL_BYTES >> 4) << 16);
+        constexpr uint32_t HI = (1024u >> 4) | (1u << 14) | (2u << 29);
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)
           if (kk >= k0 && kk < k1)
-            mma_ts(tmem + 256 + q * HEAD_DIM, tmem + q * TILE + kk * 8,
-                   b0 + static_cast<uint64_t>(kk * (2048 >> 4)), IDESC_PV, (accumulate || kk > 0) ? 1u : 0u);
+            mma_ts_lo<HI>(tmem + 256 + q * HEAD_DIM, tmem + q * TILE + kk * 8, b0 + kk * (2048 >> 4), IDESC_PV,
+                          (accumulate || kk > 0) ? 1u : 0u);
       }
     };
     uint32_t o_done[2] = {0, 0};   // items of each stream whose O went to the epilogue warps
@@ -642,17 +646,26 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
         tc_fence_after();
         uint32_t sv[4][32];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) tmem_ld32(t_s + c * 32, sv[c]);
+        for (int c = 0; c < 2; ++c) tmem_ld32(t_s + c * 32, sv[c]);
         tc_wait_ld();
-        // four independent running maxima, three-input max: 64 instructions per row
+        pin(sv[0]); pin(sv[1]);
+#pragma unroll
+        for (int c = 2; c < 4; ++c) tmem_ld32(t_s + c * 32, sv[c]);
+        // four independent running maxima, three-input max: 64 instructions per row. Those of the first half run
+        // while the second half is on its way (-1 to -3 % on the whole kernel, longest on short lists).
         float mx[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) mx[j] = -INFINITY;
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
+        for (int c = 0; c < 4; ++c) {
+          if (c == 2) {
+            tc_wait_ld();
+            pin(sv[2]); pin(sv[3]);
+          }
 #pragma unroll
           for (int j = 0; j < 32; j += 2)
             mx[(j >> 1) & 3] = max3(mx[(j >> 1) & 3], __uint_as_float(sv[c][j]), __uint_as_float(sv[c][j + 1]));
+        }
         float tile_max = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
         tile_max *= p.scale_log2;
         // Lazy rescale: keep a stale row max while the true max is less than
