@@ -305,7 +305,7 @@ int sparse_b200_indexer_summary(const void* q, const void* k, void* q_desc, void
   if (rc) return rc;
   rc = launch_summary_small(q_desc, k_desc, scores, block_idx, nullptr, batch, hq, hkv, sq / 128, skv / 128,
                             representatives, topk, static_cast<cudaStream_t>(stream));
-  if (rc != 1) return rc;            // small problem: cluster kernel, same ids and scores
+  if (rc != 1) return rc;            // small problem: row-tile kernel, same ids and scores
   return launch_summary_score_topk(q_desc, k_desc, scores, block_idx, batch, hq, hkv, sq / 128, skv / 128,
                                    representatives, topk, static_cast<cudaStream_t>(stream));
 }
@@ -325,14 +325,18 @@ int sparse_b200_indexer_summary_fast(const void* q, const void* k, void* q_desc,
   REQUIRE((reinterpret_cast<uintptr_t>(aux) & 3u) == 0 && aligned16(q_desc) && aligned16(k_desc), "misaligned workspace");
   rc = pool_both(q, q_desc, k, k_desc, batch, hq, hkv, sq, skv, representatives, stream);
   if (rc) return rc;
-  // small problems: the exact cluster kernel fills the GPU better than the tensor-core pre-filter
+  // small problems: the exact row-tile kernel fills the GPU better than the tensor-core pre-filter
   rc = launch_summary_small(q_desc, k_desc, nullptr, block_idx,
                             static_cast<int32_t*>(aux) + 2 * static_cast<long long>(batch) * hkv, batch, hq, hkv,
                             sq / 128, skv / 128, representatives, topk, static_cast<cudaStream_t>(stream));
   if (rc != 1) return rc;
   rc = launch_summary_select_tc(q_desc, k_desc, aux, block_idx, batch, hq, hkv, sq / 128, skv / 128, representatives,
                                 topk, static_cast<cudaStream_t>(stream));
-  if (rc == 1)      // not eligible for the tensor-core path: exact kernel, same ids
+  if (rc == 1)      // not eligible for the tensor-core path: exact kernels, same ids
+    rc = launch_summary_small(q_desc, k_desc, nullptr, block_idx,
+                              static_cast<int32_t*>(aux) + 2 * static_cast<long long>(batch) * hkv, batch, hq, hkv,
+                              sq / 128, skv / 128, representatives, topk, static_cast<cudaStream_t>(stream), true);
+  if (rc == 1)
     rc = launch_summary_score_topk(q_desc, k_desc, nullptr, block_idx, batch, hq, hkv, sq / 128, skv / 128,
                                    representatives, topk, static_cast<cudaStream_t>(stream));
   return rc;

@@ -7,13 +7,7 @@
 //                       sequential fp32 sum, so the descriptors are bit-identical with
 //                       pool_kernel, which keeps 16 lanes per descriptor and pays one
 //                       memory round trip per 8 tokens).
-//   score_cluster_kernel  a cluster of 8 CTAs per list (batch, KV head, query block).
-//                       Each CTA scores chunks of key descriptors against all query
-//                       descriptors of the list with a 4 x NKT register tile per thread
-//                       (dot products accumulate feature by feature in fp32, as in
-//                       score_topk_kernel), reduces to one score per KV block and writes
-//                       it into the shared memory of the cluster's first CTA, which runs
-//                       the top-k after a cluster barrier. No global workspace.
+//   score_rows_kernel   64 query descriptors (one or several lists of a KV head) per cluster of 1 - 8 CTAs, see there.
 // Same results as pool_blocks / descriptor_dot / reduce_topk
 // (indexers/r1_r4/gpu_ops.py:6-49): ids in score-descending order, ties to the lower id.
 #include "internal.h"
@@ -57,156 +51,270 @@ __global__ void __launch_bounds__(256) pool_small_kernel(const __nv_bfloat16* __
 }
 
 // ---------------------------------------------------------------- score + top-k
-constexpr int CLUSTER = 8;
+// A row tile is ROWS = 64 query descriptors: L lists (query blocks of one KV head) of MP descriptors each (MP = group
+// heads x R rounded up to a power of two, padding repeats a list's first descriptor: the maximum is unchanged). A
+// cluster of C CTAs (C = 1, 2, 4 or 8) shares the row tile: CTA `rank` scores the key chunks rank, rank + C, ... of
+// 64 descriptors, and owns the lists l with l % C == rank: every score goes straight into the owner's shared memory.
+// Bound by fp32 FMAs (the exact score is defined by fp32 sums in feature order): 4 x 4 register tile per thread, two
+// 16-byte shared-memory reads per 16 FMAs, the next chunk's bytes requested before the arithmetic of this one.
+constexpr int ROWS = 64, KD = 64;
+constexpr int SCORE_BYTES_MAX = 40 * 1024;
 
-// MPAD = padded number of query descriptors (group heads x R): 16, 32 or 64.
-// Thread (tq, tk) holds queries QT tq .. QT tq + QT - 1 and key descriptors NKT tk .. NKT tk + NKT - 1;
-// a chunk is KD = (256 / (MPAD / QT)) * NKT key descriptors (a multiple of 4, hence of R).
-template <int MPAD, int QT, int NKT>
-__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(256)
-score_cluster_kernel(const __nv_bfloat16* __restrict__ qd, const __nv_bfloat16* __restrict__ kd,
-                     float* __restrict__ scores_out, int32_t* __restrict__ ids_out,
-                     int32_t* __restrict__ fallback_counter, int hq, int hkv, int qt, int nt, int r, int topk) {
-  constexpr int TQ = MPAD / QT, TK = 256 / TQ, KD = TK * NKT;
-  static_assert(TQ <= 32 && (KD % 4) == 0, "query threads must fit a warp; chunks hold whole blocks");
+__device__ __forceinline__ unsigned score_key(float s) {      // order of the floats; both zeros are one value
+  const unsigned b = __float_as_uint(s + 0.f);
+  return b ^ ((b >> 31) ? 0xffffffffu : 0x80000000u);
+}
+
+// [feature][64] fp32 tile in shared memory. Odd 8-feature pieces are stored with bit 4 of the column flipped, so that
+// a warp which holds two neighbouring pieces of 16 rows (whole 32-byte sectors of global memory) stores without bank
+// conflicts.
+__device__ __forceinline__ void stage_piece(float* tile, int row, int c, const uint4& raw) {
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+  float* dst = tile + c * 8 * 64 + (row ^ ((c & 1) << 4));
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    const float2 f = __bfloat1622float2(h[p]);
+    dst[(2 * p) * 64] = f.x;
+    dst[(2 * p + 1) * 64] = f.y;
+  }
+}
+
+struct RowsParams {
+  const __nv_bfloat16 *qd, *kd;
+  float* scores_out;         // [lists][nt] or null
+  int32_t* ids;
+  int32_t* fallback_counter; // three words to reset, or null
+  int hq, hkv, qt, nt, r, topk;
+  int lists_per_cta, tiles_per_head, mp_log2;
+};
+
+// LPT = lists a thread's four rows belong to: 1 (MP >= 4), 2 (MP = 2) or 4 (MP = 1)
+template <int LPT>
+__global__ void __launch_bounds__(256) score_rows_kernel(const RowsParams p) {
   extern __shared__ __align__(16) float smem[];
-  float* q_s = smem;                         // [128][MPAD]
-  float* k_s = q_s + 128 * MPAD;             // [128][KD]
-  float* kbest = k_s + 128 * KD;             // [KD]
-  float* scores = kbest + KD;                // [nt]  (used in the cluster's first CTA)
-  float* scratch_f = scores + nt;            // [10]
-  int* scratch_i = reinterpret_cast<int*>(scratch_f + 10);
+  float* q_s = smem;                         // [128][ROWS]
+  float* k_s = q_s + 128 * ROWS;             // [128][KD]
+  float* scores = k_s + 128 * KD;            // [lists owned by this CTA][nt]
 
   cg::cluster_group cluster = cg::this_cluster();
-  const int rank = static_cast<int>(cluster.block_rank());
-  const int list = blockIdx.x / CLUSTER;     // (b * hkv + kvh) * qt + qtile
-  const int group = hq / hkv;
-  const int m_real = group * r;
-  const int qtile = list % qt;
-  const int bk = list / qt;
-  const int b = bk / hkv, kvh = bk - b * hkv;
+  const int rank = static_cast<int>(cluster.block_rank()), csize = static_cast<int>(cluster.num_blocks());
+  const int c_log2 = 31 - __clz(csize);
+  const int tile = blockIdx.x >> c_log2;
+  const int group = p.hq / p.hkv, m_real = group * p.r;
+  const int bk = tile / p.tiles_per_head;
+  const int b = bk / p.hkv, kvh = bk - b * p.hkv;
+  const int qtile0 = (tile - bk * p.tiles_per_head) * p.lists_per_cta;
+  const int lists = min(p.lists_per_cta, p.qt - qtile0);
+  const int n_keys = p.nt * p.r;
+  const int tid = threadIdx.x;
+  // staging role: 16-byte pieces piece0 + 2 i of row `srow` (i = 0 .. 3, both parities of a piece pair in a warp)
+  const int srow = (tid >> 1) & 63, piece0 = (tid & 1) | ((tid >> 7) << 3);
 
-  // query descriptors, transposed to [feature][descriptor]: thread <-> (descriptor, 16-byte piece)
-  for (int e = threadIdx.x; e < MPAD * 16; e += blockDim.x) {
-    const int m = e % MPAD, c = e / MPAD;
-    const int mm = m < m_real ? m : 0;       // padding repeats descriptor 0: the maximum is unchanged
-    const int g = mm / r, rq = mm - g * r;
-    const long long row = ((static_cast<long long>(b) * hq + kvh * group + g) * qt + qtile) * r + rq;
-    const uint4 raw = __ldg(reinterpret_cast<const uint4*>(qd + row * 128) + c);
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+  asm volatile("griddepcontrol.wait;" ::: "memory");      // the descriptors of the pooling kernel are visible from here
+  // every list is exact here: no fallback, no violated bound, no largest difference
+  if (p.fallback_counter && blockIdx.x == 0 && tid < 3) p.fallback_counter[tid] = 0;
+  const uint4* kbase = reinterpret_cast<const uint4*>(p.kd + static_cast<long long>(bk) * n_keys * 128);
+  uint4 raw[4];
+  auto fetch_keys = [&](int base) {
+    const bool live = base + srow < n_keys;
 #pragma unroll
-    for (int p = 0; p < 4; ++p) {
-      const float2 f = __bfloat1622float2(h[p]);
-      q_s[(c * 8 + 2 * p) * MPAD + m] = f.x;
-      q_s[(c * 8 + 2 * p + 1) * MPAD + m] = f.y;
-    }
+    for (int i = 0; i < 4; ++i)
+      raw[i] = live ? __ldg(kbase + static_cast<long long>(base + srow) * 16 + piece0 + 2 * i) : make_uint4(0u, 0u, 0u, 0u);
+  };
+  {
+    const int l = srow >> p.mp_log2, m = srow & ((1 << p.mp_log2) - 1);
+    const int mm = m < m_real ? m : 0;
+    const int g = mm / p.r, rq = mm - g * p.r;
+    const long long row = ((static_cast<long long>(b) * p.hq + kvh * group + g) * p.qt + qtile0 + (l < lists ? l : 0)) * p.r + rq;
+    const uint4* src = reinterpret_cast<const uint4*>(p.qd + row * 128);
+    uint4 qraw[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) qraw[i] = __ldg(src + piece0 + 2 * i);
+    fetch_keys(rank * KD);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) stage_piece(q_s, srow, piece0 + 2 * i, qraw[i]);
   }
-
-  if (fallback_counter && blockIdx.x == 0 && threadIdx.x == 0) *fallback_counter = 0;   // every list is exact here
-  cluster.sync();                              // all CTAs of the cluster run: their shared memory may be addressed
-  const int n_keys = nt * r;
-  const __nv_bfloat16* kbase = kd + static_cast<long long>(bk) * n_keys * 128;
-  float* leader_scores = cluster.map_shared_rank(scores, 0);
+  if (csize > 1) cluster.sync();               // all CTAs of the cluster run: their shared memory may be addressed
   const float scale = 0.08838834764831845f;   // fp32(128^-0.5)
-  const int tq = threadIdx.x % TQ, tk = threadIdx.x / TQ;
+  const int tq = tid & 15, tk = tid >> 4;
+  const int bpt = 4 / p.r;                     // KV blocks among a thread's four key descriptors
+  float* owner_scores[LPT];                    // where the scores of this thread's lists go (null: not a real list)
+#pragma unroll
+  for (int x = 0; x < LPT; ++x) {
+    const int l = (tq * 4 + x * (4 / LPT)) >> p.mp_log2;
+    const bool speaks = LPT > 1 || ((tq * 4) & ((1 << p.mp_log2) - 1)) == 0;
+    owner_scores[x] = speaks && l < lists ? cluster.map_shared_rank(scores, l & (csize - 1)) + (l >> c_log2) * p.nt : nullptr;
+  }
 
-  for (int base = rank * KD; base < n_keys; base += CLUSTER * KD) {
-    __syncthreads();                           // q_s staged (first pass) / k_s and kbest free again
-    // stage the chunk transposed: thread <-> (key descriptor, 16-byte piece); consecutive
-    // threads take consecutive descriptors, so the shared-memory stores do not conflict
-    for (int e = threadIdx.x; e < KD * 16; e += blockDim.x) {
-      const int kdi = e % KD, c = e / KD;
-      uint4 raw = make_uint4(0u, 0u, 0u, 0u);
-      if (base + kdi < n_keys) raw = __ldg(reinterpret_cast<const uint4*>(kbase + static_cast<long long>(base + kdi) * 128) + c);
-      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+  for (int base = rank * KD; base < n_keys; base += csize * KD) {
 #pragma unroll
-      for (int p = 0; p < 4; ++p) {
-        const float2 f = __bfloat1622float2(h[p]);
-        k_s[(c * 8 + 2 * p) * KD + kdi] = f.x;
-        k_s[(c * 8 + 2 * p + 1) * KD + kdi] = f.y;
+    for (int i = 0; i < 4; ++i) stage_piece(k_s, srow, piece0 + 2 * i, raw[i]);
+    __syncthreads();                           // tiles staged
+    if (base + csize * KD < n_keys) fetch_keys(base + csize * KD);
+    float acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+#pragma unroll 1
+    for (int d0 = 0; d0 < 128; d0 += 16) {
+#pragma unroll
+      for (int dd = 0; dd < 16; ++dd) {
+        const int flip = (dd >> 3) << 4;
+        const float4 qv = *reinterpret_cast<const float4*>(q_s + (d0 + dd) * 64 + ((tq * 4) ^ flip));
+        const float4 kv = *reinterpret_cast<const float4*>(k_s + (d0 + dd) * 64 + ((tk * 4) ^ flip));
+        const float qa[4] = {qv.x, qv.y, qv.z, qv.w}, ka[4] = {kv.x, kv.y, kv.z, kv.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(qa[i], ka[j], acc[i][j]);
       }
     }
-    __syncthreads();
-    float acc[QT][NKT];
+    // one score per (list, KV block): maximum over the list's rows and the block's R descriptors, then the scale
 #pragma unroll
-    for (int i = 0; i < QT; ++i)
+    for (int x = 0; x < LPT; ++x) {
+      float best[4];
 #pragma unroll
-      for (int j = 0; j < NKT; ++j) acc[i][j] = 0.f;
-#pragma unroll 8
-    for (int d = 0; d < 128; ++d) {
-      float qa[QT], kv[NKT];
+      for (int j = 0; j < 4; ++j) {
+        best[j] = acc[x * (4 / LPT)][j];
 #pragma unroll
-      for (int i = 0; i < QT; ++i) qa[i] = q_s[d * MPAD + tq * QT + i];
+        for (int i = 1; i < 4 / LPT; ++i) best[j] = fmaxf(best[j], acc[x * (4 / LPT) + i][j]);
+      }
+      if (p.r > 1) { best[0] = fmaxf(best[0], best[1]); best[2] = fmaxf(best[2], best[3]); }
+      if (p.r > 2) best[0] = fmaxf(best[0], best[2]);
+      if (LPT == 1) {
+        for (int dlt = 1; dlt < (1 << p.mp_log2) / 4; dlt <<= 1) {
 #pragma unroll
-      for (int j = 0; j < NKT; ++j) kv[j] = k_s[d * KD + tk * NKT + j];
+          for (int j = 0; j < 4; ++j) best[j] = fmaxf(best[j], __shfl_xor_sync(0xffffffffu, best[j], dlt));
+        }
+      }
+      if (owner_scores[x]) {
+        const int first = base + tk * 4;       // a multiple of R
+        float* dst = owner_scores[x] + first / p.r;
+        if (first < n_keys) dst[0] = best[0] * scale;
+        if (p.r == 1) {
 #pragma unroll
-      for (int i = 0; i < QT; ++i)
-#pragma unroll
-        for (int j = 0; j < NKT; ++j) acc[i][j] = fmaf(qa[i], kv[j], acc[i][j]);
-    }
-    // best over this thread's queries, then over the TQ threads that share the key descriptors
-#pragma unroll
-    for (int j = 0; j < NKT; ++j) {
-      float best = acc[0][j];
-#pragma unroll
-      for (int i = 1; i < QT; ++i) best = fmaxf(best, acc[i][j]);
-#pragma unroll
-      for (int dlt = 1; dlt < TQ; dlt <<= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, dlt));
-      if (tq == 0) kbest[tk * NKT + j] = best;
-    }
-    __syncthreads();
-    // one score per KV block: maximum over its R representatives, then the scale
-    for (int blk = threadIdx.x; blk * r < KD; blk += blockDim.x) {
-      const int first = base + blk * r;
-      if (first < n_keys) {
-        float best = kbest[blk * r];
-        for (int e = 1; e < r; ++e) best = fmaxf(best, kbest[blk * r + e]);
-        leader_scores[first / r] = best * scale;
+          for (int j = 1; j < 4; ++j)
+            if (first + j < n_keys) dst[j] = best[j] * scale;
+        } else if (p.r == 2) {
+          if (first + 2 < n_keys) dst[1] = best[2] * scale;
+        }
       }
     }
+    __syncthreads();                           // k_s free again
   }
-  cluster.sync();                              // every block's score is in the first CTA's shared memory
-  if (rank != 0) return;
-  if (scores_out)
-    for (int j = threadIdx.x; j < nt; j += blockDim.x) scores_out[static_cast<long long>(list) * nt + j] = scores[j];
-  // Few blocks: every score counts the scores that beat it (score descending, id ascending is
-  // a total order, so the counts are the ranks). NaN scores would break the order: then, and
-  // for long lists, the round-by-round arg-max is used.
-  bool plain = nt <= 1024;
-  if (plain) {
-    bool has_nan = false;
-    for (int j = threadIdx.x; j < nt; j += blockDim.x) has_nan |= scores[j] != scores[j];
-    plain = !__syncthreads_or(has_nan);
-  } else {
-    __syncthreads();
+  if (csize > 1) cluster.sync();               // every score is in its owner's shared memory
+  const int own = (lists - rank + csize - 1) >> c_log2;     // lists rank, rank + C, ... of the tile
+  if (own <= 0) return;
+  const long long list0 = static_cast<long long>(bk) * p.qt + qtile0 + rank;
+  bool has_nan = false;
+  for (int e = tid; e < own * p.nt; e += blockDim.x) {
+    const float v = scores[e];
+    has_nan |= v != v;
+    if (p.scores_out) {
+      const int l = e / p.nt;
+      p.scores_out[(list0 + static_cast<long long>(l) * csize) * p.nt + (e - l * p.nt)] = v;
+    }
   }
-  if (plain) {
-    for (int j = threadIdx.x; j < nt; j += blockDim.x) {
-      const float mine = scores[j];
-      int rank = 0;
-      for (int i = 0; i < nt; ++i) rank += better(scores[i], i, mine, j) ? 1 : 0;
-      if (rank < topk) ids_out[static_cast<long long>(list) * topk + rank] = j;
+  // (score descending, id ascending) is a total order unless a score is NaN: then, and for a large k of many blocks,
+  // rounds of block-wide arg-max.
+  has_nan = __syncthreads_or(has_nan);
+  if (!has_nan && p.nt <= 256 && (p.topk > 128 || ((own * p.nt + 255) >> 8) * p.nt <= 512 * ((own + 7) >> 3))) {
+    // Short lists: every score counts the scores that beat it, the count is its rank. The right-hand side is what
+    // the threshold search of a warp below takes in the same unit, scores read by a thread (64 lists of 256: 271 us
+    // by counting, 60 by searching, whole selector; 32 lists of 32: 20 and 25).
+    for (int e = tid; e < own * p.nt; e += blockDim.x) {
+      const int l = e / p.nt, j = e - l * p.nt;
+      const float* s = scores + l * p.nt;
+      const float mine = s[j];
+      int place = 0;
+#pragma unroll 4
+      for (int i = 0; i < p.nt; ++i) place += better(s[i], i, mine, j) ? 1 : 0;
+      if (place < p.topk) p.ids[(list0 + static_cast<long long>(l) * csize) * p.topk + place] = j;
     }
     return;
   }
-  block_topk(scores, nt, topk, ids_out + static_cast<long long>(list) * topk, scratch_f, scratch_i);
+  const int lane = tid & 31, warp = tid >> 5;
+  if (!has_nan && p.topk <= 128) {
+    // one warp per list: k-th largest score bit by bit, then ranks among the k that reach it
+    float* cand_s = q_s + warp * 256;
+    int* cand_i = reinterpret_cast<int*>(cand_s + 128);
+    for (int l = warp; l < own; l += 8) {
+      const float* s = scores + l * p.nt;
+      unsigned T = 0;
+      for (int bit = 31; bit >= 0; --bit) {
+        const unsigned trial = T | (1u << bit);
+        int cnt = 0;
+#pragma unroll 8
+        for (int j = lane; j < p.nt; j += 32) cnt += score_key(s[j]) >= trial ? 1 : 0;
+        cnt = __reduce_add_sync(0xffffffffu, cnt);
+        if (cnt >= p.topk) T = trial;
+        if (cnt == p.topk) break;              // exactly the wanted ones pass: `trial` separates as well as the k-th score
+      }
+      int above = 0;
+      for (int j = lane; j < p.nt; j += 32) above += score_key(s[j]) > T ? 1 : 0;
+      above = __reduce_add_sync(0xffffffffu, above);
+      const unsigned below = (1u << lane) - 1u;
+      int written = 0, ties = 0;
+      for (int j0 = 0; j0 < p.nt; j0 += 32) {
+        const int j = j0 + lane;
+        const unsigned u = j < p.nt ? score_key(s[j]) : 0u;
+        const bool eq = j < p.nt && u == T;
+        const unsigned eqs = __ballot_sync(0xffffffffu, eq);
+        const bool take = j < p.nt && (u > T || (eq && ties + __popc(eqs & below) < p.topk - above));
+        const unsigned takes = __ballot_sync(0xffffffffu, take);
+        if (take) {
+          const int pos = written + __popc(takes & below);
+          cand_s[pos] = s[j];
+          cand_i[pos] = j;
+        }
+        written += __popc(takes);
+        ties += __popc(eqs);
+      }
+      __syncwarp();
+      for (int c = lane; c < p.topk; c += 32) {
+        const float mine = cand_s[c];
+        const int id = cand_i[c];
+        int place = 0;
+#pragma unroll 4
+        for (int i = 0; i < p.topk; ++i) place += better(cand_s[i], cand_i[i], mine, id) ? 1 : 0;
+        p.ids[(list0 + static_cast<long long>(l) * csize) * p.topk + place] = id;
+      }
+      __syncwarp();
+    }
+    return;
+  }
+  float* scratch_f = k_s;
+  int* scratch_i = reinterpret_cast<int*>(k_s + 16);
+  for (int l = 0; l < own; ++l) {
+    block_topk(scores + l * p.nt, p.nt, p.topk, p.ids + (list0 + static_cast<long long>(l) * csize) * p.topk, scratch_f,
+               scratch_i);
+    __syncthreads();
+  }
 }
 
-template <int MPAD, int QT, int NKT>
-int launch_cluster(const __nv_bfloat16* qd, const __nv_bfloat16* kd, float* scores, int32_t* ids, int32_t* counter,
-                   int lists, int hq, int hkv, int qt, int nt, int r, int topk, DeviceCtx* ctx, int slot,
-                   cudaStream_t stream) {
-  constexpr int KD = (256 / (MPAD / QT)) * NKT;
-  const size_t smem = (128 * MPAD + 128 * KD + KD + nt + 10) * sizeof(float) + 16 * sizeof(int);
+template <int LPT>
+int launch_rows(const RowsParams& p, int grid, int csize, size_t smem, DeviceCtx* ctx, int slot, cudaStream_t stream) {
   if (!(ctx->small_attr & (1 << slot))) {
-    cudaError_t e = cudaFuncSetAttribute(score_cluster_kernel<MPAD, QT, NKT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         100 * 1024);
+    cudaError_t e = cudaFuncSetAttribute(score_rows_kernel<LPT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         2 * 32768 + SCORE_BYTES_MAX);
     if (e != cudaSuccess) return set_error(SB_ERR_CUDA, cudaGetErrorString(e));
     ctx->small_attr |= (1 << slot);
   }
-  score_cluster_kernel<MPAD, QT, NKT><<<lists * CLUSTER, 256, smem, stream>>>(qd, kd, scores, ids, counter, hq, hkv, qt,
-                                                                          nt, r, topk);
-  cudaError_t e = cudaGetLastError();
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(grid));
+  cfg.blockDim = dim3(256);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(csize);
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, score_rows_kernel<LPT>, p);
   return e == cudaSuccess ? SB_OK : set_error(SB_ERR_CUDA, cudaGetErrorString(e));
 }
 
@@ -233,20 +341,52 @@ int launch_pool_small_pair(const void* x, void* desc, long long num_desc, const 
   return e == cudaSuccess ? SB_OK : set_error(SB_ERR_CUDA, cudaGetErrorString(e));
 }
 
-// Returns 1 when the problem is not a small one (the caller then takes the other kernels).
+// Returns 1 when the problem is not a small one (the caller then takes the other kernels). force: whatever its size
+// (problems the tensor-core forms do not take: this kernel is several times faster than score_topk_kernel).
 int launch_summary_small(const void* qd, const void* kd, float* scores, int32_t* ids, int32_t* fallback_counter,
-                         int batch, int hq, int hkv, int qt, int nt, int r, int topk, cudaStream_t stream) {
+                         int batch, int hq, int hkv, int qt, int nt, int r, int topk, cudaStream_t stream, bool force) {
   DeviceCtx* ctx = device_ctx();
   if (!ctx) return SB_ERR_CUDA;
-  const long long lists = static_cast<long long>(batch) * hkv * qt;
   const int m = (hq / hkv) * r;
-  if (lists * CLUSTER > 8LL * ctx->sm_count || nt > 2048 || m > 64) return 1;
-  const __nv_bfloat16* q = static_cast<const __nv_bfloat16*>(qd);
-  const __nv_bfloat16* k = static_cast<const __nv_bfloat16*>(kd);
-  const int n = static_cast<int>(lists);
-  if (m <= 16) return launch_cluster<16, 1, 1>(q, k, scores, ids, fallback_counter, n, hq, hkv, qt, nt, r, topk, ctx, 0, stream);
-  if (m <= 32) return launch_cluster<32, 2, 2>(q, k, scores, ids, fallback_counter, n, hq, hkv, qt, nt, r, topk, ctx, 1, stream);
-  return launch_cluster<64, 4, 4>(q, k, scores, ids, fallback_counter, n, hq, hkv, qt, nt, r, topk, ctx, 2, stream);
+  if (nt > 2048 || m > ROWS) return 1;
+  int mp_log2 = 0;
+  while ((1 << mp_log2) < m) ++mp_log2;
+  int per_cta = ROWS >> mp_log2;
+  if (per_cta > qt) per_cta = qt;
+  const int chunks = (nt * r + KD - 1) / KD;
+  const long long heads = static_cast<long long>(batch) * hkv;
+  // The largest cluster that keeps every CTA resident at once (three 64 KiB CTAs per SM) and gives each a chunk; the
+  // scores of the lists a CTA owns must fit its share of shared memory.
+  int csize, tiles;
+  while (true) {
+    tiles = (qt + per_cta - 1) / per_cta;
+    csize = 8;
+    while (csize > 1 && (csize > chunks || heads * tiles * csize > 3LL * ctx->sm_count)) csize >>= 1;
+    if (static_cast<long long>((per_cta + csize - 1) / csize) * nt * 4 <= SCORE_BYTES_MAX) break;
+    per_cta = (per_cta + 1) / 2;
+  }
+  // Against the tensor-core forms (their selection phase costs about 16 us per round of eight lists whatever the
+  // length, a unit of 64 rows x 64 keys here about 5 us of an SM; select_summary with pooling, us, tensor-core form ->
+  // this one): below 16 descriptors per list those pack more than a round of lists into one CTA and leave most SMs
+  // idle (256 lists of 1 x 32 blocks 68 -> 20, 512 of 4 x 512 126 -> 58, 2048 of 1 x 256 271 -> 107); from 16 on only
+  // when the lists do not fill the GPU (64 lists of 64 x 512 key rows 42 -> 32, 128 of 16 x 1024 75 -> 61). Beyond four
+  // units per SM the tensor cores win (320 of 16 x 600: 62 against 70; 128 of 64 x 2048: 62 against 164).
+  if (!force && !((m < 16 || heads * qt <= ctx->sm_count) && heads * tiles * chunks <= 4LL * ctx->sm_count)) return 1;
+  RowsParams p{};
+  p.qd = static_cast<const __nv_bfloat16*>(qd);
+  p.kd = static_cast<const __nv_bfloat16*>(kd);
+  p.scores_out = scores;
+  p.ids = ids;
+  p.fallback_counter = fallback_counter;
+  p.hq = hq; p.hkv = hkv; p.qt = qt; p.nt = nt; p.r = r; p.topk = topk;
+  p.lists_per_cta = per_cta;
+  p.tiles_per_head = tiles;
+  p.mp_log2 = mp_log2;
+  const size_t smem = (128 * ROWS + 128 * KD) * sizeof(float) + static_cast<size_t>((per_cta + csize - 1) / csize) * nt * 4;
+  const int grid = static_cast<int>(heads) * tiles * csize;
+  if (mp_log2 == 0) return launch_rows<4>(p, grid, csize, smem, ctx, 0, stream);
+  if (mp_log2 == 1) return launch_rows<2>(p, grid, csize, smem, ctx, 1, stream);
+  return launch_rows<1>(p, grid, csize, smem, ctx, 2, stream);
 }
 
 }  // namespace sb

@@ -57,9 +57,11 @@ bool pool_small_eligible(long long num_desc);
 int launch_pool_small(const void* x, void* desc, long long num_desc, int tokens_per_desc, cudaStream_t stream);
 int launch_pool_small_pair(const void* x, void* desc, long long num_desc, const void* x2, void* desc2,
                            long long num_desc2, int tokens_per_desc, cudaStream_t stream);
-// returns 1 when the problem is not small; fallback_counter (may be null) is reset to 0
+// returns 1 when the problem is not small (force: when it cannot be run at all); the three words at fallback_counter
+// (may be null) are reset to 0
 int launch_summary_small(const void* qd, const void* kd, float* scores, int32_t* ids, int32_t* fallback_counter,
-                         int batch, int hq, int hkv, int qt, int nt, int r, int topk, cudaStream_t stream);
+                         int batch, int hq, int hkv, int qt, int nt, int r, int topk, cudaStream_t stream,
+                         bool force = false);
 // flagged_only: re-do only the lists whose first id is -1 (second pass after a pre-filter kernel)
 int launch_summary_score_topk(const void* qd, const void* kd, float* scores, int32_t* ids, int batch, int hq, int hkv,
                               int qt, int nt, int r, int topk, cudaStream_t stream, int flagged_only = 0);

@@ -307,6 +307,40 @@ def test_small_problem_selector_equals_the_exact_kernels(b, hkv, g, sq, skv, r, 
     assert torch.equal(staged.ids.cpu(), ref)
 
 
+@pytest.mark.parametrize("b,hkv,g,qb,nb,r,topk", [
+    (1, 8, 1, 33, 32, 1, 8),        # one descriptor per list: 64 lists in a row tile, the second tile nearly empty
+    (2, 3, 2, 40, 300, 1, 40),      # two per list; more than 256 blocks: threshold search
+    (1, 2, 3, 21, 65, 1, 65),       # three per list padded to four, every block selected
+    (1, 1, 3, 7, 129, 4, 129),      # twelve padded to sixteen, one key chunk more than a multiple, k > 128
+    (1, 1, 5, 3, 2048, 1, 64),      # the largest block count, chunks for a whole cluster
+    (1, 1, 16, 30, 70, 2, 1),       # 32 per list, two representatives, k = 1
+    (3, 1, 12, 60, 33, 4, 12),      # 48 padded to 64: a list fills the row tile; not a power of two, any size
+])
+@pytest.mark.parametrize("ties", [False, True])
+def test_row_tile_selector_equals_the_exact_kernels(b, hkv, g, qb, nb, r, topk, ties):
+    """Lists of 1 to 64 descriptors packed into row tiles of 64, shared by 1 to 8 CTAs: ids and scores bit for bit
+    against the staged exact kernels; with every third key block a copy of block 0 (equal scores, lower id first)."""
+    m = sp()
+    q, k, _ = gen.make_qkv(b, hkv * g, hkv, qb * 128, nb * 128, seed=37, k_block_offset=0.5)
+    if ties:
+        k = k.clone()
+        for blk in range(0, nb, 3):
+            k[:, :, blk * 128:(blk + 1) * 128] = k[:, :, :128]
+    qc, kc = q.cuda(), k.cuda()
+    staged = m.SummarySelector(qc, kc, r, topk=topk, keep_scores=True)
+    staged.prepare()
+    staged.score()
+    fused = m.SummarySelector(qc, kc, r, topk=topk, keep_scores=True)
+    fused.run()
+    fast = m.SummarySelector(qc, kc, r, topk=topk, keep_scores=False)
+    fast.run_fast()
+    torch.cuda.synchronize()
+    m.device_status()
+    assert torch.equal(fused.scores, staged.scores)
+    assert torch.equal(fused.ids, staged.ids)
+    assert torch.equal(fast.ids, staged.ids)
+
+
 def test_summary_selector_duplicate_scores_tie_to_lower_id():
     """Duplicate KV blocks give exactly equal scores: the lower id must come first."""
     m = sp()
