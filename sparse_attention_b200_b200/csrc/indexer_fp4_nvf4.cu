@@ -119,6 +119,12 @@ __device__ __forceinline__ int f2ord(float f) {
   const int i = __float_as_int(f);
   return i >= 0 ? i : i ^ 0x7fffffff;
 }
+// maximum of a warp's floats in one instruction; a NaN counts only when all are (as with fmaxf)
+__device__ __forceinline__ float warp_max(float v) {
+  float m;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(m) : "f"(v));
+  return m;
+}
 __device__ __forceinline__ float ord2f(int i) { return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff); }
 
 // Largest |dequantised element| and largest squared L2 norm over all key vectors -> stats[0], stats[1]
@@ -196,13 +202,18 @@ struct Geometry {
 };
 
 // ---------------------------------------------------------------- producer and MMA roles
-// Producer warp: query tile once, then key pages page0 + (t + rot) % wrap for t = 0 .. num_tiles - 1.
+// A page takes about 520 cycles of an SM with two CTAs on it (590 when the scales of page t + 3 were requested before
+// the proxy fence of page t, which then waited for them, and when the page maximum took five shuffles), against 128
+// cycles of MMAs: the hand-overs copy -> MMA -> accumulator -> epilogue bound it. One CTA per SM with three
+// accumulators and two to three threads issuing, the scales through tensor-memory stores, was no faster (510 to 840).
+// Producer warp: query tile once, then key pages page0 + (t + rot) % wrap for t = 0 .. num_tiles - 1 (num_tiles <= wrap,
+// rot < wrap).
 __device__ __forceinline__ void producer_role(const Geometry& g, const CUtensorMap* q_map, const CUtensorMap* k_map,
                                               uint32_t base, unsigned char* gbase, uint32_t bar0, const Guard& guard,
                                               int b, int h, int hk_idx, long long q_row0, int page0, int num_tiles,
                                               int rot, int wrap, int lane, int code0, volatile int* key_scale_max) {
   auto bar = [&](int i) { return bar0 + 8u * i; };
-  auto page_of = [&](int t) { return page0 + (t + rot) % wrap; };
+  auto page_of = [&](int t) { return page0 + (t + rot >= wrap ? t + rot - wrap : t + rot); };
   auto key_row = [&](int pg) { return ((static_cast<long long>(b) * g.tiles + pg) * g.hk + hk_idx) * 128; };
   if (lane == 0) {
     mbar_expect_tx(bar(B_FULL), CODE_BYTES);
@@ -236,10 +247,11 @@ __device__ __forceinline__ void producer_role(const Geometry& g, const CUtensorM
     store_scale_chunks(gbase + OFF_A + s * STAGE_BYTES + CODE_BYTES, regs, lane);
 #pragma unroll
     for (int i = 0; i < 4; ++i) seen = max_scale_bytes(max_scale_bytes(seen, regs.r[i].x), regs.r[i].y);
-    if (t + 3 < num_tiles) regs = load_scales(g.ks + key_row(page_of(t + 3)) * 8, 8, lane);
     fence_async_smem();
     __syncwarp();
     if (lane == 0) mbar_arrive(bar(A_FULL + s));
+    // after the fence, which would wait for them
+    if (t + 3 < num_tiles) regs = load_scales(g.ks + key_row(page_of(t + 3)) * 8, 8, lane);
     return true;
   };
   for (int t = 0; ok && t < num_tiles; t += 3) {
@@ -428,10 +440,9 @@ fp4_nv_select_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
           m5[jj] = max3(__uint_as_float(v[c][3 * jj]), __uint_as_float(v[c][3 * jj + 1]), __uint_as_float(v[c][3 * jj + 2]));
         m4[c] = fmaxf(max3(m5[0], m5[1], m5[2]), max3(m5[3], m5[4], __uint_as_float(v[c][15])));
       }
-      float m = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
-#pragma unroll
-      for (int d = 16; d > 0; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
-      if (lane == 0) atomicMax(&scores[(t + rot) % num_tiles], f2ord(m));
+      const float m = warp_max(fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])));
+      const int at = t + rot >= num_tiles ? t + rot - num_tiles : t + rot;
+      if (lane == 0) atomicMax(&scores[at], f2ord(m));
     }
   }
   tc_fence_before();
@@ -673,7 +684,8 @@ fp4_nv_prune_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
   const Geometry& g = p.g;
   unsigned char* aux = gbase + PR_OFF_AUX;
   const uint32_t bar0 = base + PR_OFF_AUX;
-  // tmem base, abort flag, L1 bits, largest key scale byte, largest approximate value of a page [3 slots], queue length
+  // tmem base, abort flag, L1 bits, largest key scale byte, largest approximate value of a page [3 slots], queue length,
+  // largest |approximate - exact| / delta (float bits)
   volatile int* misc = reinterpret_cast<volatile int*>(aux + 128);
   int* queue = reinterpret_cast<int*>(gbase + PR_OFF_QUEUE);
   float* queue_apx = reinterpret_cast<float*>(gbase + PR_OFF_APX);
@@ -703,6 +715,7 @@ fp4_nv_prune_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
     misc[3] = 0;
     for (int i = 4; i < 7; ++i) misc[i] = INT_MIN;
     misc[7] = 0;
+    misc[8] = 0;
     for (int i = 0; i < A_STAGES; ++i) {
       mbar_init(bar(A_FULL + i), 2);
       mbar_init(bar(A_EMPTY + i), 1);
@@ -769,7 +782,7 @@ fp4_nv_prune_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
                                     g.ks + (page * 128 + krow) * 8);
       if (e == e) atomicMax(res + t, f2ord(e));
       const float diff = fabsf(apx - e);
-      if (delta > 0.f) atomicMax(p.stats + 4, __float_as_int(diff / delta));
+      if (delta > 0.f) atomicMax(const_cast<int*>(misc + 8), __float_as_int(diff / delta));
       if (!(diff <= delta) && e == e) {
         redo[t] = 1;
         atomicAdd(p.violations, 1);
@@ -803,9 +816,7 @@ fp4_nv_prune_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
           m4[c] = fmaxf(max3(m5[0], m5[1], m5[2]), max3(m5[3], m5[4], __uint_as_float(v[c][15])));
         }
         mine = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
-        float m = mine;
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
+        const float m = warp_max(mine);
         if (lane == 0) atomicMax(const_cast<int*>(misc + slot), f2ord(m));
       }
       meet();
@@ -850,6 +861,7 @@ fp4_nv_prune_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
       evaluate(e >> 14, (e >> 7) & 127, e & 127, queue_apx[i]);
     }
     meet();
+    if (threadIdx.x == 0 && misc[8] > 0) atomicMax(p.stats + 4, misc[8]);      // one global atomic per CTA
     // a pair whose bound was violated: every one of its 16384 elements, exactly (256 threads)
     for (int t = 0; t < num_tiles; ++t) {
       if (!redo[t]) continue;
@@ -937,6 +949,8 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int group = p.hq / p.hk;
 
+  // nothing to score: the grid must still not be complete before the fill kernel is
+  auto leave = [] { asm volatile("griddepcontrol.wait;" ::: "memory"); };
   int h0, qtile, b, hk_idx, heads_here = 1;
   if (PACKED) {
     const int head_block = blockIdx.x % p.head_blocks;
@@ -955,12 +969,12 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
   }
   const int q_begin = p.cu_q[b], q_len = p.cu_q[b + 1] - q_begin;
   const int k_len = p.cu_k[b + 1] - p.cu_k[b];
-  if (q_begin < 0 || qtile * 128 >= q_len || k_len <= 0) return;      // block-uniform
+  if (q_begin < 0 || qtile * 128 >= q_len || k_len <= 0) return leave();      // block-uniform
   const int page_begin = p.cu_pages[b];
-  if (page_begin < 0) return;
+  if (page_begin < 0) return leave();
   int pages = min(min((k_len + 127) >> 7, p.tiles_out), p.cu_pages[b + 1] - page_begin);
   const int rows_live = min(min(PACKED ? QS_PACK_Q : 128, q_len - qtile * 128), p.total_q - q_begin - qtile * 128);
-  if (rows_live <= 0) return;
+  if (rows_live <= 0) return leave();
   const int offset = p.causal ? (p.qo_offset ? p.qo_offset[b] : k_len - q_len) : 0;
   if (p.causal) {          // pages past the last live query's horizon stay -inf
     const long long horizon = static_cast<long long>(qtile) * 128 + rows_live - 1 + offset;
@@ -968,7 +982,7 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
   }
   const int page0 = blockIdx.y * p.pages_per_cta;
   const int num_tiles = min(p.pages_per_cta, pages - page0);
-  if (num_tiles <= 0) return;
+  if (num_tiles <= 0) return leave();
   // row r of the CTA -> query position inside the request, head, alive?
   auto row_query = [&](int r) { return PACKED ? (r >> 4) : qtile * 128 + r; };
   auto row_head = [&](int r) { return PACKED ? h0 + (r & (QS_PACK_HEADS - 1)) : h0; };
@@ -1047,10 +1061,11 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
         tma_load_2d(base + OFF_A + s * STAGE_BYTES, &k_map, 0, static_cast<int>(key_row(t)), bar_(A_FULL + s));
       }
       store_scale_chunks(gbase + OFF_A + s * STAGE_BYTES + CODE_BYTES, regs, lane);
-      if (t + 3 < num_tiles) regs = load_scales(p.ks + key_row(t + 3) * 8, 8, lane);
       fence_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_(A_FULL + s));
+      // after the fence, which would wait for them
+      if (t + 3 < num_tiles) regs = load_scales(p.ks + key_row(t + 3) * 8, 8, lane);
       return true;
     };
     for (int t = 0; ok && t < num_tiles; t += 3) {
@@ -1097,6 +1112,9 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
     __syncwarp();
   } else {
     // ----------------------------------------------------------- epilogue: one lane = one query row
+    // The fill kernel before this one on the stream has written its -inf (scoring begins under it: everything else here
+    // only reads the inputs, and those were complete before the fill kernel began).
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
     const int r = warp * 32 + lane;
     const bool alive = row_alive(r);
@@ -1154,10 +1172,18 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
   }
 }
 
+// -inf everywhere; 16-byte stores from the first aligned element on
 __global__ void __launch_bounds__(256) fill_neg_inf_kernel(float* out, long long n) {
-  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-       i += static_cast<long long>(gridDim.x) * blockDim.x)
-    out[i] = -INFINITY;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const long long head = min(n, static_cast<long long>((16u - (reinterpret_cast<uintptr_t>(out) & 15u)) & 15u) >> 2);
+  const long long gid = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
+  const long long n4 = (n - head) >> 2;
+  float4* body = reinterpret_cast<float4*>(out + head);
+  const float4 v = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+  for (long long i = gid; i < n4; i += stride) body[i] = v;
+  if (gid < head) out[gid] = -INFINITY;
+  if (gid < n - head - 4 * n4) out[head + 4 * n4 + gid] = -INFINITY;
 }
 
 }  // namespace fnv
@@ -1289,8 +1315,8 @@ int launch_fp4_scores_varlen_nv(const void* qp, const void* qs, const void* kp, 
                                  : static_cast<long long>(batch) * p.qt_max * hq;
   if (items > 0x7fffffffLL) return set_error(SB_ERR_INVALID, "too many (request, query tile, head) items");
   const long long n = static_cast<long long>(hq) * p.tiles_out * total_q;
-  const long long fill_blocks = std::min<long long>((n + 255) / 256, 32LL * ctx->sm_count);
-  fill_neg_inf_kernel<<<static_cast<unsigned>(fill_blocks > 0 ? fill_blocks : 1), 256, 0, stream>>>(out, n);
+  const long long fill_blocks = std::min<long long>((n / 4 + 255) / 256 + 1, 8LL * ctx->sm_count);
+  fill_neg_inf_kernel<<<static_cast<unsigned>(fill_blocks), 256, 0, stream>>>(out, n);
   if (items == 0 || p.tiles_out == 0) return SB_OK;
   // enough CTAs to fill the GPU twice over, as long a run of pages per CTA as that allows (the query tile is
   // loaded once per CTA)
@@ -1326,11 +1352,18 @@ int launch_fp4_scores_varlen_nv(const void* qp, const void* qs, const void* kp, 
     if (e != cudaSuccess) return set_error(SB_ERR_CUDA, cudaGetErrorString(e));
     ctx->tc_attr |= (1 << 12);
   }
-  if (packed)
-    fp4_nv_query_scores_kernel<true><<<grid, QS_THREADS, smem, stream>>>(qm, km, p);
-  else
-    fp4_nv_query_scores_kernel<false><<<grid, QS_THREADS, smem, stream>>>(qm, km, p);
-  cudaError_t e = cudaGetLastError();
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(QS_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, packed ? fp4_nv_query_scores_kernel<true> : fp4_nv_query_scores_kernel<false>,
+                                     qm, km, p);
   return e == cudaSuccess ? SB_OK : set_error(SB_ERR_CUDA, cudaGetErrorString(e));
 }
 
