@@ -293,6 +293,11 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = static_cast<uint32_t>(misc[0]);
+  // Launched as a programmatic dependent: the setup above overlaps the tail of the kernel before it on the stream
+  // (often the one that selects this one's blocks); nothing of it is read before this wait. The next dependent launch
+  // (the merge of the last round, or another call) may be set up under this kernel in the same way.
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   float* stats = reinterpret_cast<float*>(gbase + OFF_STATS);
   // tensor memory columns: S0 0..127, S1 128..255, O0 256..383, O1 384..511.
   // P (bf16 pairs) overwrites columns 0..63 of its S.
@@ -1032,20 +1037,22 @@ int launch_q_centric(const QCentricArgs& a, cudaStream_t stream) {
     if (e != cudaSuccess) return set_error(SB_ERR_CUDA, cudaGetErrorString(e));
     configured = 1;
   }
-  kernel<<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(qm, km, vm, om, omt, p, ScatterOff{});
-  cudaError_t e = cudaGetLastError();
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(NUM_THREADS);
+  cfg.dynamicSmemBytes = SMEM_BYTES;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, qm, km, vm, om, omt, p, ScatterOff{});
   if (e != cudaSuccess) return set_error(SB_ERR_CUDA, cudaGetErrorString(e));
   if (tail_out) {
-    cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((p.num_items - p.tail_first) * 32);
     cfg.blockDim = dim3(128);
     cfg.dynamicSmemBytes = 0;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
     const __nv_bfloat16* tail_in = tail_out;
     e = cudaLaunchKernelEx(&cfg, tail_merge_kernel, p, tail_in);
     if (e != cudaSuccess) return set_error(SB_ERR_CUDA, cudaGetErrorString(e));
