@@ -303,9 +303,10 @@ int sparse_b200_indexer_summary(const void* q, const void* k, void* q_desc, void
   if (rc) return rc;
   rc = pool_both(q, q_desc, k, k_desc, batch, hq, hkv, sq, skv, representatives, stream);
   if (rc) return rc;
+  // exact scores are wanted of every block: the row-tile kernel whatever the size, up to its block count
   rc = launch_summary_small(q_desc, k_desc, scores, block_idx, nullptr, batch, hq, hkv, sq / 128, skv / 128,
-                            representatives, topk, static_cast<cudaStream_t>(stream));
-  if (rc != 1) return rc;            // small problem: row-tile kernel, same ids and scores
+                            representatives, topk, static_cast<cudaStream_t>(stream), true);
+  if (rc != 1) return rc;
   return launch_summary_score_topk(q_desc, k_desc, scores, block_idx, batch, hq, hkv, sq / 128, skv / 128,
                                    representatives, topk, static_cast<cudaStream_t>(stream));
 }
