@@ -134,8 +134,9 @@ int sparse_b200_q_centric(const void* q, const void* k, const void* v, const int
 int64_t sparse_b200_q_centric_workspace_bytes(void) {
   DeviceCtx* ctx = device_ctx();
   if (!ctx) return SB_ERR_CUDA;
-  // at most one piece per CTA in the balanced round: two streams of 128 rows, bf16 O + fp32 LSE
-  return static_cast<int64_t>(ctx->sm_count) * 2 * 128 * (128 * 2 + 4) + 512;
+  // at most one piece per CTA in the balanced round: two streams of 128 rows, O (fp32 in launches of less than a round,
+  // else bf16) + fp32 LSE
+  return static_cast<int64_t>(ctx->sm_count) * 2 * 128 * (128 * 4 + 4) + 512;
 }
 
 int sparse_b200_q_centric_ws(const void* q, const void* k, const void* v, const int32_t* block_idx,

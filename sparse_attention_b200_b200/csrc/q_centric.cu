@@ -48,6 +48,7 @@ constexpr int SOFTMAX_REGS = 176;
 constexpr int EPI_REGS = 64;
 constexpr int CTRL_REGS = 96;        // MMA issuer, TMA producer, idle warps
 constexpr int TMEM_COLS = 512;
+constexpr int SMALL_PARTS = 16;      // pieces of an item in a launch of less than a round
 constexpr float RESCALE_LOG2 = 8.0f;   // keep a stale row max while it lags by < 2^8
 
 // shared memory map (offsets from a 1024-aligned base)
@@ -85,9 +86,10 @@ struct Params {
   int group, qt, pair_mode;
   int items_per_seg, num_items;
   float scale_log2;
-  // Tail balancing (single-segment bf16 launches with a workspace): the items of the last, partly
+  // Tail balancing (single-segment launches with bf16 output and a workspace): the items of the last, partly
   // filled round (index >= tail_first) are cut into tail_parts pieces of their lists; piece v writes a
-  // normalised partial (O, LSE) into the workspace and tail_merge_kernel combines the pieces.
+  // normalised partial (O, LSE) into the workspace and tail_merge_kernel combines the pieces. When the whole launch
+  // is less than a round, tail_first is 0 and the partials are fp32.
   // num_virtual = items as the roles see them; without balancing tail_first = num_virtual = num_items.
   int tail_first, tail_parts, num_virtual;
   float* tail_lse;         // [pieces * 2 * 128]
@@ -871,52 +873,62 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
 // out = sum_r exp(L_r - L) O_r / sum_r exp(L_r - L), L = logsumexp_r L_r, pieces in order; a piece with
 // L_r = -inf (empty share of the list) has weight 0 whatever it holds. Launched as a programmatic
 // dependent of the attention kernel: its prologue overlaps that kernel's tail.
-__global__ void __launch_bounds__(128) tail_merge_kernel(const Params p, const __nv_bfloat16* __restrict__ tail_out) {
+// T: type of the partials, MAXP: bound on the pieces of an item.
+template <typename T, int MAXP>
+__global__ void __launch_bounds__(128) tail_merge_kernel(const Params p, const T* __restrict__ tail_out) {
   const int t = blockIdx.x >> 5, q = (blockIdx.x >> 4) & 1;
   Params real = p;
   real.tail_first = p.num_items;                 // decode the item itself, not a piece of it
   Stream s[2];
-  decode_item(real, p.tail_first + t, s);
   asm volatile("griddepcontrol.wait;" ::: "memory");      // the attention kernel's stores are visible from here on
+  decode_item(real, p.tail_first + t, s);
   if (!s[q].valid) return;
   const int part16 = threadIdx.x & 15;
-  {
-    const int row = (blockIdx.x & 15) * 8 + (threadIdx.x >> 4);
-    float L[4], maximum = -INFINITY;
+  const int row = (blockIdx.x & 15) * 8 + (threadIdx.x >> 4);
+  float L[MAXP], maximum = -INFINITY;
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      L[r] = -INFINITY;
-      if (r < p.tail_parts) L[r] = p.tail_lse[(static_cast<long long>(t * p.tail_parts + r) * 2 + q) * TILE + row];
-      maximum = fmaxf(maximum, L[r]);
-    }
-    float w[4], denom = 0.f;
+  for (int r = 0; r < MAXP; ++r) {
+    L[r] = -INFINITY;
+    if (r < p.tail_parts) L[r] = p.tail_lse[(static_cast<long long>(t * p.tail_parts + r) * 2 + q) * TILE + row];
+  }
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      w[r] = (r < p.tail_parts && L[r] > -INFINITY) ? expf(L[r] - maximum) : 0.f;
-      denom += w[r];
-    }
-    const float inv = denom > 0.f ? 1.f / denom : 0.f;
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  for (int r = 0; r < MAXP; ++r) maximum = fmaxf(maximum, L[r]);
+  float denom = 0.f;
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      if (r < p.tail_parts && w[r] > 0.f) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(
-            tail_out + ((static_cast<long long>(t * p.tail_parts + r) * 2 + q) * TILE + row) * HEAD_DIM + part16 * 8);
+  for (int r = 0; r < MAXP; ++r) {
+    L[r] = L[r] == -INFINITY ? -1.f : expf(L[r] - maximum);    // the weight from here on; an empty piece has none
+    if (!(L[r] < 0.f)) denom += L[r];                          // (a NaN counts: the row is NaN without the split, too)
+  }
+  const float inv = denom != 0.f ? 1.f / denom : 0.f;
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int r = 0; r < MAXP; ++r) {
+    if (r < p.tail_parts && !(L[r] < 0.f)) {
+      const T* src = tail_out + ((static_cast<long long>(t * p.tail_parts + r) * 2 + q) * TILE + row) * HEAD_DIM + part16 * 8;
+      float f[8];
+      if constexpr (sizeof(T) == 4) {
+        const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + 4);
+        f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w;
+        f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+      } else {
+        const uint4 raw = *reinterpret_cast<const uint4*>(src);
         const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float2 f = __bfloat1622float2(h[e]);
-          acc[2 * e] = fmaf(w[r], f.x, acc[2 * e]);
-          acc[2 * e + 1] = fmaf(w[r], f.y, acc[2 * e + 1]);
+          const float2 v = __bfloat1622float2(h[e]);
+          f[2 * e] = v.x;
+          f[2 * e + 1] = v.y;
         }
       }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[e] = fmaf(L[r], f[e], acc[e]);
     }
-    const long long orow = s[q].out_row + row;
-    *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(p.out) + orow * HEAD_DIM + part16 * 8) =
-        make_uint4(pack_bf16x2(acc[0] * inv, acc[1] * inv), pack_bf16x2(acc[2] * inv, acc[3] * inv),
-                   pack_bf16x2(acc[4] * inv, acc[5] * inv), pack_bf16x2(acc[6] * inv, acc[7] * inv));
-    if (part16 == 0 && p.lse) p.lse[orow] = denom > 0.f ? maximum + logf(denom) : -INFINITY;
   }
+  const long long orow = s[q].out_row + row;
+  *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(p.out) + orow * HEAD_DIM + part16 * 8) =
+      make_uint4(pack_bf16x2(acc[0] * inv, acc[1] * inv), pack_bf16x2(acc[2] * inv, acc[3] * inv),
+                 pack_bf16x2(acc[4] * inv, acc[5] * inv), pack_bf16x2(acc[6] * inv, acc[7] * inv));
+  if (part16 == 0 && p.lse) p.lse[orow] = denom != 0.f ? maximum + logf(denom) : -INFINITY;
 }
 
 // ------------------------------------------------------------------ host side
@@ -961,7 +973,7 @@ int launch_q_centric(const QCentricArgs& a, cudaStream_t stream) {
                                 : a.batch * a.hq * ((p.qt + 1) / 2);
   p.num_items = p.items_per_seg * a.nseg;
   p.scale_log2 = 1.4426950408889634f / sqrtf(static_cast<float>(HEAD_DIM));
-  const int grid = p.num_items < ctx->sm_count ? p.num_items : ctx->sm_count;
+  int grid = p.num_items < ctx->sm_count ? p.num_items : ctx->sm_count;
 
   // Tail balancing. With few rounds of items per CTA the last, partly filled round costs a whole
   // round: when at most half of the CTAs would work in it, its items are cut into 2-4 pieces (as
@@ -970,7 +982,8 @@ int launch_q_centric(const QCentricArgs& a, cudaStream_t stream) {
   p.tail_first = p.num_virtual = p.num_items;
   p.tail_parts = 1;
   p.tail_lse = nullptr;
-  __nv_bfloat16* tail_out = nullptr;
+  void* tail_out = nullptr;
+  bool tail_f32 = false;
   const int rounds = p.num_items / grid, rem = p.num_items - rounds * grid;
   if (a.tail_ws && a.owners <= 1 && a.nseg == 1 && !a.out_f32 && rem > 0 && 2 * rem <= grid && rounds >= 1 && rounds <= 8 && a.topk >= 8) {
     int parts = grid / rem;
@@ -985,8 +998,32 @@ int launch_q_centric(const QCentricArgs& a, cudaStream_t stream) {
       p.tail_first = p.num_items - rem;
       p.tail_parts = parts;
       p.num_virtual = p.tail_first + rem * parts;
-      tail_out = static_cast<__nv_bfloat16*>(a.tail_ws);
+      tail_out = a.tail_ws;
       p.tail_lse = reinterpret_cast<float*>(static_cast<unsigned char*>(a.tail_ws) + ((rows * HEAD_DIM * 2 + 255) & ~255LL));
+    }
+  }
+
+  // Less than one round: the SMs without an item take pieces of the others' lists, up to SMALL_PARTS per item, at least
+  // two blocks each. The partials are fp32 here (the output of these calls was rounded once before, and still is).
+  // Worth it when the blocks saved (1.7 us each) outweigh the fp32 partials and the merge, 10 to 15 us. Measured in a
+  // CUDA graph, plain -> split, us: 4 items of 64 blocks 110.6 -> 24.0 (16 pieces), 12 of 16 35.1 -> 21.4 (8 pieces),
+  // 32 of 32 59.6 -> 32.0 (4 pieces); below the line 32 items of 8 20.0 -> 21.3, 72 of 16 33.9 -> 35.2, 74 of 8
+  // 20.6 -> 28.5.
+  if (a.tail_ws && a.owners <= 1 && a.nseg == 1 && !a.out_f32 && 2 * p.num_items <= ctx->sm_count && a.topk >= 4) {
+    int parts = ctx->sm_count / p.num_items;
+    if (parts > SMALL_PARTS) parts = SMALL_PARTS;
+    if (parts > a.topk / 2) parts = a.topk / 2;
+    const long long rows = static_cast<long long>(p.num_items) * parts * 2 * TILE;
+    const long long need = rows * (HEAD_DIM * 4 + 4);
+    const bool pays = 1.7f * static_cast<float>(a.topk - (a.topk + parts - 1) / parts) >= 16.f;
+    if (pays && need <= a.tail_bytes && (reinterpret_cast<uintptr_t>(a.tail_ws) & 15u) == 0) {
+      p.tail_first = 0;
+      p.tail_parts = parts;
+      p.num_virtual = p.num_items * parts;
+      tail_out = a.tail_ws;
+      tail_f32 = true;
+      p.tail_lse = static_cast<float*>(a.tail_ws) + rows * HEAD_DIM;
+      grid = p.num_virtual;
     }
   }
 
@@ -997,7 +1034,7 @@ int launch_q_centric(const QCentricArgs& a, cudaStream_t stream) {
       encode_out_map(&om, a.out, static_cast<uint64_t>(a.nseg) * a.batch * a.hq * a.sq, a.out_f32 != 0))
     return set_error(SB_ERR_CUDA, "cuTensorMapEncodeTiled failed for q/k/v/out");
   omt = om;
-  if (tail_out && encode_out_map(&omt, tail_out, static_cast<uint64_t>(p.num_virtual - p.tail_first) * 2 * TILE, false))
+  if (tail_out && encode_out_map(&omt, tail_out, static_cast<uint64_t>(p.num_virtual - p.tail_first) * 2 * TILE, tail_f32))
     return set_error(SB_ERR_CUDA, "cuTensorMapEncodeTiled failed for the tail workspace");
 
   if (a.owners > 1) {
@@ -1030,8 +1067,11 @@ int launch_q_centric(const QCentricArgs& a, cudaStream_t stream) {
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? SB_OK : set_error(SB_ERR_CUDA, cudaGetErrorString(e));
   }
-  auto kernel = a.out_f32 ? q_centric_kernel<true, ScatterOff> : q_centric_kernel<false, ScatterOff>;
-  int& configured = a.out_f32 ? ctx->qc_attr_f32 : ctx->qc_attr_bf16;
+  // (when the whole launch writes fp32 partials, the kernel is the fp32 one although the output is bf16: an empty list
+  // is then an empty piece of a tail item, whose rows only the merge writes)
+  const bool f32 = a.out_f32 || tail_f32;
+  auto kernel = f32 ? q_centric_kernel<true, ScatterOff> : q_centric_kernel<false, ScatterOff>;
+  int& configured = f32 ? ctx->qc_attr_f32 : ctx->qc_attr_bf16;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     if (e != cudaSuccess) return set_error(SB_ERR_CUDA, cudaGetErrorString(e));
@@ -1053,8 +1093,8 @@ int launch_q_centric(const QCentricArgs& a, cudaStream_t stream) {
     cfg.gridDim = dim3((p.num_items - p.tail_first) * 32);
     cfg.blockDim = dim3(128);
     cfg.dynamicSmemBytes = 0;
-    const __nv_bfloat16* tail_in = tail_out;
-    e = cudaLaunchKernelEx(&cfg, tail_merge_kernel, p, tail_in);
+    e = tail_f32 ? cudaLaunchKernelEx(&cfg, tail_merge_kernel<float, SMALL_PARTS>, p, static_cast<const float*>(tail_out))
+                 : cudaLaunchKernelEx(&cfg, tail_merge_kernel<__nv_bfloat16, 4>, p, static_cast<const __nv_bfloat16*>(tail_out));
     if (e != cudaSuccess) return set_error(SB_ERR_CUDA, cudaGetErrorString(e));
   }
   return SB_OK;

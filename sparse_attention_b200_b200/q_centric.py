@@ -57,7 +57,8 @@ _WORKSPACES = {}
 
 
 def _workspace(device):
-    """Scratch of the balanced last round, one per (device, stream): allocated at the first call."""
+    """Scratch of the balanced last round and of split small launches (20 MB), one per (device, stream): allocated at
+    the first call."""
     key = (device.index, torch.cuda.current_stream(device).cuda_stream)
     ws = _WORKSPACES.get(key)
     if ws is None:

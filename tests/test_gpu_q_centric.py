@@ -301,3 +301,50 @@ def test_balanced_last_round_matches_the_plain_call(shape, topk, counts_kind):
     assert torch.all((bal_lse[fin] - plain_lse[fin]).abs() <= 2e-6 * plain_lse[fin].abs().clamp_min(1.0))
     ref_o, ref_l = oracle.gather_attention(q, k, v, ids, counts)
     check(bal, bal_lse, ref_o, ref_l)
+
+
+@pytest.mark.parametrize("shape,topk,counts_kind", [
+    ((1, 2, 1, 128, 8192), 64, None),          # one pair item: 16 pieces of 4 blocks
+    ((1, 3, 1, 384, 2048), 16, None),          # split mode, odd number of query blocks: a stream without a tile
+    ((2, 1, 1, 384, 4096), 16, "ragged"),      # lists of 0 to 16 blocks: empty lists and empty pieces
+    ((1, 4, 2, 2304, 2304), 18, "ragged"),     # 36 items: four pieces
+    ((1, 8, 1, 2304, 4096), 32, None),         # 72 items: two pieces
+    ((1, 8, 1, 2304, 1024), 8, None),          # 72 items, not worth a split: the plain launch
+])
+@pytest.mark.parametrize("nan", [False, True])
+def test_launch_of_less_than_a_round_matches_the_plain_call(shape, topk, counts_kind, nan):
+    """With a workspace and at most half as many items as SMs, every item is cut into pieces with fp32 partials: same
+    result as the plain call up to the rounding of the bf16 probabilities and outputs, LSE to fp32 rounding, inside the
+    oracle tolerance; rows that are NaN without the split stay NaN."""
+    m = sp()
+    b, hq, hkv, sq, skv = shape
+    q, k, v = gen.make_qkv(b, hq, hkv, sq, skv, seed=13, k_block_offset=0.5)
+    ids = gen.make_ids(b, hkv, sq // 128, skv // 128, topk, 5, "unsorted")
+    counts = None
+    if counts_kind == "ragged":
+        counts = (torch.arange(b * hkv * (sq // 128)) * 7 % (topk + 1)).to(torch.int32).reshape(b, hkv, sq // 128)
+    if nan:
+        q = q.clone()
+        q[:, 0, 5] = float("nan")
+    qc, kc, vc, ic = q.cuda(), k.cuda(), v.cuda(), ids.cuda()
+    cc = None if counts is None else counts.cuda()
+    plain = torch.full(q.shape, 7.0, dtype=torch.bfloat16, device="cuda")
+    plain_lse = torch.full(q.shape[:3], 7.0, device="cuda")
+    m.attention_out(qc, kc, vc, ic, plain, cc, plain_lse, balance=False)
+    split = torch.full_like(plain, 9.0)
+    split_lse = torch.full_like(plain_lse, 9.0)
+    m.attention_out(qc, kc, vc, ic, split, cc, split_lse, balance=True)
+    torch.cuda.synchronize()
+    m.device_status()
+    assert torch.equal(split.isnan(), plain.isnan()) and torch.equal(split_lse.isnan(), plain_lse.isnan())
+    fin = torch.isfinite(plain.float())
+    diff = (split.float() - plain.float())[fin].abs()
+    # Both calls round every probability to bf16 (relative error 2^-9 each, relative to different running maxima) and
+    # the output once: |difference| <= 2 * 2^-9 * (sum p |v| + |o|) <= 2^-8 * (max |v| + |o|).
+    assert torch.all(diff <= 2.0 ** -8 * (v.float().abs().max().item() + plain.float()[fin].abs()))
+    lfin = torch.isfinite(plain_lse)
+    assert torch.equal(torch.isneginf(split_lse), torch.isneginf(plain_lse))
+    assert torch.all((split_lse[lfin] - plain_lse[lfin]).abs() <= 2e-6 * plain_lse[lfin].abs().clamp_min(1.0))
+    if not nan:
+        ref_o, ref_l = oracle.gather_attention(q, k, v, ids, counts)
+        check(split, split_lse, ref_o, ref_l)
