@@ -6,7 +6,7 @@
 //   warp 12       TMA producer: the 256 query descriptors of the unit (B operand, one buffer)
 //                 and the key descriptor tiles (A operand, ring of two 32 KiB slots);
 //   warp 13       MMA issuer: tcgen05 M128 N256 K16 x 8 per key tile into one of two 256-column
-//                 TMEM accumulators (N = 256: 167 cycles per instruction against 2 x 116 at N = 128);
+//                 TMEM accumulators (N = 256: half the instructions and hand-overs of N = 128);
 //   warps 0-7     epilogue: lane = key descriptor, warp >> 2 = half of the 256 columns; max over
 //                 a list's 32 columns and over the R rows of a KV block -> approximate block
 //                 scores, written to one of two CHUNK buffers (16 key tiles) in shared memory;
