@@ -170,15 +170,16 @@ __global__ void __launch_bounds__(256) score_rows_kernel(const RowsParams p) {
           for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(qa[i], ka[j], acc[i][j]);
       }
     }
-    // one score per (list, KV block): maximum over the list's rows and the block's R descriptors, then the scale
+    // one score per (list, KV block): maximum over the list's rows and the block's R descriptors, then the scale. As in
+    // the exact kernel the maximum starts at -inf: a NaN product never wins, and no score is NaN.
 #pragma unroll
     for (int x = 0; x < LPT; ++x) {
       float best[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        best[j] = acc[x * (4 / LPT)][j];
+        best[j] = -CUDART_INF_F;
 #pragma unroll
-        for (int i = 1; i < 4 / LPT; ++i) best[j] = fmaxf(best[j], acc[x * (4 / LPT) + i][j]);
+        for (int i = 0; i < 4 / LPT; ++i) best[j] = fmaxf(best[j], acc[x * (4 / LPT) + i][j]);
       }
       if (p.r > 1) { best[0] = fmaxf(best[0], best[1]); best[2] = fmaxf(best[2], best[3]); }
       if (p.r > 2) best[0] = fmaxf(best[0], best[2]);
@@ -207,19 +208,13 @@ __global__ void __launch_bounds__(256) score_rows_kernel(const RowsParams p) {
   const int own = (lists - rank + csize - 1) >> c_log2;     // lists rank, rank + C, ... of the tile
   if (own <= 0) return;
   const long long list0 = static_cast<long long>(bk) * p.qt + qtile0 + rank;
-  bool has_nan = false;
-  for (int e = tid; e < own * p.nt; e += blockDim.x) {
-    const float v = scores[e];
-    has_nan |= v != v;
-    if (p.scores_out) {
+  if (p.scores_out)
+    for (int e = tid; e < own * p.nt; e += blockDim.x) {
       const int l = e / p.nt;
-      p.scores_out[(list0 + static_cast<long long>(l) * csize) * p.nt + (e - l * p.nt)] = v;
+      p.scores_out[(list0 + static_cast<long long>(l) * csize) * p.nt + (e - l * p.nt)] = scores[e];
     }
-  }
-  // (score descending, id ascending) is a total order unless a score is NaN: then, and for a large k of many blocks,
-  // rounds of block-wide arg-max.
-  has_nan = __syncthreads_or(has_nan);
-  if (!has_nan && p.nt <= 256 && (p.topk > 128 || ((own * p.nt + 255) >> 8) * p.nt <= 512 * ((own + 7) >> 3))) {
+  // (score descending, id ascending) is a total order: no score is NaN
+  if (p.nt <= 256 && (p.topk > 128 || ((own * p.nt + 255) >> 8) * p.nt <= 512 * ((own + 7) >> 3))) {
     // Short lists: every score counts the scores that beat it, the count is its rank. The right-hand side is what
     // the threshold search of a warp below takes in the same unit, scores read by a thread (64 lists of 256: 271 us
     // by counting, 60 by searching, whole selector; 32 lists of 32: 20 and 25).
@@ -235,7 +230,7 @@ __global__ void __launch_bounds__(256) score_rows_kernel(const RowsParams p) {
     return;
   }
   const int lane = tid & 31, warp = tid >> 5;
-  if (!has_nan && p.topk <= 128) {
+  if (p.topk <= 128) {
     // one warp per list: k-th largest score bit by bit, then ranks among the k that reach it
     float* cand_s = q_s + warp * 256;
     int* cand_i = reinterpret_cast<int*>(cand_s + 128);
@@ -284,6 +279,7 @@ __global__ void __launch_bounds__(256) score_rows_kernel(const RowsParams p) {
     }
     return;
   }
+  __syncthreads();                             // scores read out before block_topk retires entries
   float* scratch_f = k_s;
   int* scratch_i = reinterpret_cast<int*>(k_s + 16);
   for (int l = 0; l < own; ++l) {

@@ -341,6 +341,42 @@ def test_row_tile_selector_equals_the_exact_kernels(b, hkv, g, qb, nb, r, topk, 
     assert torch.equal(fast.ids, staged.ids)
 
 
+@pytest.mark.parametrize("b,hkv,g,qb,nb,r,topk", [
+    (1, 2, 1, 80, 33, 1, 33),        # 160 lists of one descriptor, every block selected
+    (1, 1, 2, 150, 300, 2, 40),      # four descriptors, threshold search
+    (1, 1, 3, 152, 40, 1, 40),       # group of three: no tensor-core form
+    (2, 1, 16, 8, 40, 4, 40),        # 64 descriptors, few lists
+    (1, 1, 1, 4, 600, 1, 600),       # k > 128 of more than 256 blocks
+])
+def test_selector_with_nan_keys_and_queries_equals_the_exact_kernel(b, hkv, g, qb, nb, r, topk):
+    """A NaN product never is a maximum: a block without any other product scores -inf and keeps an id of its own,
+    whichever kernel scores it."""
+    m = sp()
+    q, k, _ = gen.make_qkv(b, hkv * g, hkv, qb * 128, nb * 128, seed=43, k_block_offset=0.5)
+    k = k.clone()
+    for blk in (0, 3, nb - 1):
+        k[:, :, blk * 128:(blk + 1) * 128] = float("nan")           # no descriptor of the block is a number
+    k[:, :, 5 * 128 + 7, 3] = float("nan")                          # one of its R descriptors is not
+    q = q.clone()
+    q[:, 0, 128] = float("nan")                                     # one head (R = 1: the whole row) of the second list
+    qc, kc = q.cuda(), k.cuda()
+    staged = m.SummarySelector(qc, kc, r, topk=topk, keep_scores=True)
+    staged.prepare()
+    staged.score()
+    fused = m.SummarySelector(qc, kc, r, topk=topk, keep_scores=True)
+    fused.run()
+    fast = m.SummarySelector(qc, kc, r, topk=topk, keep_scores=False)
+    fast.run_fast()
+    torch.cuda.synchronize()
+    m.device_status()
+    assert not staged.scores.isnan().any()
+    assert torch.isneginf(staged.scores[:, :, 0, 0]).all()
+    assert torch.equal(fused.scores, staged.scores)
+    assert torch.equal(fused.ids, staged.ids)
+    assert torch.equal(fast.ids, staged.ids)
+    assert all(len(set(row)) == topk for row in fused.ids.flatten(0, 2).tolist())
+
+
 def test_summary_selector_duplicate_scores_tie_to_lower_id():
     """Duplicate KV blocks give exactly equal scores: the lower id must come first."""
     m = sp()
