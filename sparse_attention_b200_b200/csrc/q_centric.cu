@@ -27,6 +27,7 @@
 // by the KV-centric operator and the cross-GPU KV split.
 #include "ptx.cuh"
 #include "internal.h"
+#include <cfloat>
 
 namespace sb {
 namespace qc {
@@ -679,7 +680,9 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
         // 2^RESCALE_LOG2 above it (P stays finite in bf16, the sum in fp32).
         float factor = 1.0f;
         if (i == 0) {
-          row_max = tile_max;
+          // finite, so that scores of -inf have weight 0 in the first block of a list (or of a piece of it), as they
+          // have in every later one
+          row_max = fmaxf(tile_max, -FLT_MAX);
         } else if (tile_max - row_max > RESCALE_LOG2) {
           factor = ex2_approx(row_max - tile_max);
           row_max = tile_max;
@@ -871,7 +874,7 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
 // dependent round trips to memory (LSEs, then partial rows), so the kernel's time is that latency
 // plus its launch, whatever the row count.
 // out = sum_r exp(L_r - L) O_r / sum_r exp(L_r - L), L = logsumexp_r L_r, pieces in order; a piece with
-// L_r = -inf (empty share of the list) has weight 0 whatever it holds. Launched as a programmatic
+// L_r = -inf (empty share of the list, or only scores of -inf) has weight 0 whatever it holds. Launched as a programmatic
 // dependent of the attention kernel: its prologue overlaps that kernel's tail.
 // T: type of the partials, MAXP: bound on the pieces of an item.
 template <typename T, int MAXP>
@@ -899,7 +902,8 @@ __global__ void __launch_bounds__(128) tail_merge_kernel(const Params p, const T
     L[r] = L[r] == -INFINITY ? -1.f : expf(L[r] - maximum);    // the weight from here on; an empty piece has none
     if (!(L[r] < 0.f)) denom += L[r];                          // (a NaN counts: the row is NaN without the split, too)
   }
-  const float inv = denom != 0.f ? 1.f / denom : 0.f;
+  // no piece has a weight: 0 for an empty list; a row whose scores are all -inf is NaN, as it is without the split
+  const float inv = denom != 0.f ? 1.f / denom : (s[q].count > 0 ? NAN : 0.f);
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
   for (int r = 0; r < MAXP; ++r) {

@@ -348,3 +348,46 @@ def test_launch_of_less_than_a_round_matches_the_plain_call(shape, topk, counts_
     if not nan:
         ref_o, ref_l = oracle.gather_attention(q, k, v, ids, counts)
         check(split, split_lse, ref_o, ref_l)
+
+
+@pytest.mark.parametrize("shape,topk", [
+    ((1, 6, 3, 128, 8192), 64),           # three pair items in 16 pieces of four blocks each
+    ((1, 3, 1, 384, 2048), 16),           # split mode, a stream without a tile
+    ((1, 10, 5, 4096, 2048), 16),         # one round and twelve items: the pieces of a balanced last round
+])
+def test_blocks_of_minus_infinite_scores_have_no_weight(shape, topk):
+    """Keys whose scores are all -inf (first feature -inf against a positive query feature) take no part in the softmax,
+    wherever they stand: as the whole of a piece of a list, as its first block, as any other. A row with no other keys
+    is NaN with LSE -inf, split or not."""
+    m = sp()
+    b, hq, hkv, sq, skv = shape
+    q, k, v = gen.make_qkv(b, hq, hkv, sq, skv, seed=17, k_block_offset=0.5)
+    nt, qt = skv // 128, sq // 128
+    q, k = q.clone(), k.clone()
+    q[..., 0] = 1.0
+    masked = torch.zeros(nt, dtype=torch.bool)
+    masked[: nt // 4] = True              # ascending lists: whole pieces at the start ...
+    masked[nt // 2::3] = True             # ... and blocks here and there
+    k.view(b, hkv, nt, 128, 128)[:, :, masked, :, 0] = -float("inf")
+    ids = torch.arange(topk, dtype=torch.int32).mul(nt).div(topk, rounding_mode="floor").expand(b, hkv, qt, topk).contiguous()
+    ids[:, 0, 0] = ids[:, -1, -1] = torch.where(masked)[0][:1].int()     # lists of masked blocks only
+    kept = ~masked[ids.long()]
+    counts = kept.sum(-1).to(torch.int32)
+    kept_ids = torch.zeros_like(ids)
+    for i in range(b):
+        for h in range(hkv):
+            for t in range(qt):
+                live = ids[i, h, t][kept[i, h, t]]
+                kept_ids[i, h, t, :len(live)] = live
+    ref_o, ref_l = oracle.gather_attention(q, k, v, kept_ids, counts)
+    none = (counts == 0).repeat_interleave(hq // hkv, 1).repeat_interleave(128, 2)
+    assert none.any() and not none.all()
+    qc, kc, vc, ic = q.cuda(), k.cuda(), v.cuda(), ids.cuda()
+    for balance in (False, True):
+        out = torch.full(q.shape, 7.0, dtype=torch.bfloat16, device="cuda")
+        lse = torch.full(q.shape[:3], 7.0, device="cuda")
+        m.attention_out(qc, kc, vc, ic, out, None, lse, balance=balance)
+        torch.cuda.synchronize()
+        m.device_status()
+        assert out.cpu()[none].isnan().all() and torch.isneginf(lse.cpu()[none]).all()
+        check(out.cpu()[~none], lse.cpu()[~none], ref_o[~none], ref_l[~none])
