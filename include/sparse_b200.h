@@ -69,8 +69,8 @@ int sparse_b200_q_centric(const void* q, const void* k, const void* v, const int
  * items per SM and the last round would keep at most half of the SMs busy, the items of that round are
  * cut into 2-4 pieces of their lists, the pieces write normalised partials into the workspace and a small
  * kernel merges them (the log-sum-exp merge of sparse_b200_combine). Results of those rows may differ
- * from the unbalanced call in the last bf16 bit; everything else is identical. A launch with at most half as many
- * items as SMs is split in the same way as a whole: up to 16 pieces per list, fp32 partials. workspace == NULL is
+ * from the unbalanced call in the last bf16 bit; everything else is identical. A launch without counts that has at most half
+ * as many items as SMs is split in the same way as a whole: up to 16 pieces per list, fp32 partials. workspace == NULL is
  * sparse_b200_q_centric, and with a workspace too small for a split the call runs without it. No counterpart in
  * the reference (its kernels take no workspace). */
 int64_t sparse_b200_q_centric_workspace_bytes(void);

@@ -1008,12 +1008,14 @@ int launch_q_centric(const QCentricArgs& a, cudaStream_t stream) {
   }
 
   // Less than one round: the SMs without an item take pieces of the others' lists, up to SMALL_PARTS per item, at least
-  // two blocks each. The partials are fp32 here (the output of these calls was rounded once before, and still is).
+  // two blocks each. Only where every list is as long as the capacity: with counts the host cannot tell how much of a
+  // list is live, and short ones would pay for the partials and save nothing (lists of 64 with 4 live blocks, us, plain ->
+  // split: 12 items 13.9 -> 19.3, 74 items 15.3 -> 24.4). The partials are fp32 here (the output of these calls was rounded once before, and still is).
   // Worth it when the blocks saved (1.7 us each) outweigh the fp32 partials and the merge, 10 to 15 us. Measured in a
   // CUDA graph, plain -> split, us: 4 items of 64 blocks 110.6 -> 24.0 (16 pieces), 12 of 16 35.1 -> 21.4 (8 pieces),
   // 32 of 32 59.6 -> 32.0 (4 pieces); below the line 32 items of 8 20.0 -> 21.3, 72 of 16 33.9 -> 35.2, 74 of 8
   // 20.6 -> 28.5.
-  if (a.tail_ws && a.owners <= 1 && a.nseg == 1 && !a.out_f32 && 2 * p.num_items <= ctx->sm_count && a.topk >= 4) {
+  if (a.tail_ws && a.owners <= 1 && a.nseg == 1 && !a.out_f32 && !a.block_count && 2 * p.num_items <= ctx->sm_count && a.topk >= 4) {
     int parts = ctx->sm_count / p.num_items;
     if (parts > SMALL_PARTS) parts = SMALL_PARTS;
     if (parts > a.topk / 2) parts = a.topk / 2;

@@ -391,3 +391,17 @@ def test_blocks_of_minus_infinite_scores_have_no_weight(shape, topk):
         m.device_status()
         assert out.cpu()[none].isnan().all() and torch.isneginf(lse.cpu()[none]).all()
         check(out.cpu()[~none], lse.cpu()[~none], ref_o[~none], ref_l[~none])
+
+
+def test_small_launch_with_counts_is_not_split():
+    """How much of a list is live stands on the device: with counts a launch of less than a round runs as the plain
+    call does, bit for bit, and the same lists without counts are split (other bits somewhere)."""
+    m = sp()
+    q, k, v = (t.cuda() for t in gen.make_qkv(1, 4, 2, 384, 8192, seed=19, k_block_offset=0.5))
+    ids = gen.make_ids(1, 2, 3, 64, 64, 5, "unsorted").cuda()
+    for counts in (torch.full((1, 2, 3), 2, dtype=torch.int32, device="cuda"), None):
+        plain, out = torch.empty_like(q), torch.empty_like(q)
+        m.attention_out(q, k, v, ids, plain, counts, balance=False)
+        m.attention_out(q, k, v, ids, out, counts)
+        assert torch.equal(plain, out) == (counts is not None)
+    m.device_status()
