@@ -1008,20 +1008,22 @@ int launch_q_centric(const QCentricArgs& a, cudaStream_t stream) {
   }
 
   // Less than one round: the SMs without an item take pieces of the others' lists, up to SMALL_PARTS per item, at least
-  // two blocks each. Only where every list is as long as the capacity: with counts the host cannot tell how much of a
-  // list is live, and short ones would pay for the partials and save nothing (lists of 64 with 4 live blocks, us, plain ->
-  // split: 12 items 13.9 -> 19.3, 74 items 15.3 -> 24.4). The partials are fp32 here (the output of these calls was rounded once before, and still is).
-  // Worth it when the blocks saved (1.7 us each) outweigh the fp32 partials and the merge, 10 to 15 us. Measured in a
-  // CUDA graph, plain -> split, us: 4 items of 64 blocks 110.6 -> 24.0 (16 pieces), 12 of 16 35.1 -> 21.4 (8 pieces),
-  // 32 of 32 59.6 -> 32.0 (4 pieces); below the line 32 items of 8 20.0 -> 21.3, 72 of 16 33.9 -> 35.2, 74 of 8
-  // 20.6 -> 28.5.
+  // two blocks each. The partials are fp32 here (the output of these calls was rounded once before, and still is).
+  // Only where every list is as long as the capacity: with counts the host cannot tell how much of a list is live, and
+  // short ones would pay for the partials and save nothing (lists of 64 with 4 live blocks, us, plain -> split: 12 items
+  // 13.9 -> 19.3, 74 items 15.3 -> 24.4).
+  // Worth it when the blocks saved (1.7 us each) outweigh the fp32 partials and the merge: measured about 8 us + 0.18 us
+  // per item. In a CUDA graph, plain -> split, us: 4 items of 64 blocks 115 -> 24 (16 pieces), 12 of 16 34 -> 21 (8),
+  // 32 of 32 62 -> 37, 37 of 16 35 -> 27 (4), 49 of 24 49 -> 40 (3), 74 of 32 64 -> 58 (2); below the line 74 of 20
+  // 42 -> 46, 74 of 24 49 -> 50, 32 of 8 20.0 -> 21.3.
   if (a.tail_ws && a.owners <= 1 && a.nseg == 1 && !a.out_f32 && !a.block_count && 2 * p.num_items <= ctx->sm_count && a.topk >= 4) {
     int parts = ctx->sm_count / p.num_items;
     if (parts > SMALL_PARTS) parts = SMALL_PARTS;
     if (parts > a.topk / 2) parts = a.topk / 2;
     const long long rows = static_cast<long long>(p.num_items) * parts * 2 * TILE;
     const long long need = rows * (HEAD_DIM * 4 + 4);
-    const bool pays = 1.7f * static_cast<float>(a.topk - (a.topk + parts - 1) / parts) >= 16.f;
+    const float saved = 1.7f * static_cast<float>(a.topk - (a.topk + parts - 1) / parts);
+    const bool pays = saved >= 16.f && saved >= 10.f + 0.18f * static_cast<float>(p.num_items);
     if (pays && need <= a.tail_bytes && (reinterpret_cast<uintptr_t>(a.tail_ws) & 15u) == 0) {
       p.tail_first = 0;
       p.tail_parts = parts;
@@ -1073,8 +1075,8 @@ int launch_q_centric(const QCentricArgs& a, cudaStream_t stream) {
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? SB_OK : set_error(SB_ERR_CUDA, cudaGetErrorString(e));
   }
-  // (when the whole launch writes fp32 partials, the kernel is the fp32 one although the output is bf16: an empty list
-  // is then an empty piece of a tail item, whose rows only the merge writes)
+  // (when the whole launch writes fp32 partials, the kernel is the fp32 one although the output is bf16: only the merge
+  // writes output rows then)
   const bool f32 = a.out_f32 || tail_f32;
   auto kernel = f32 ? q_centric_kernel<true, ScatterOff> : q_centric_kernel<false, ScatterOff>;
   int& configured = f32 ? ctx->qc_attr_f32 : ctx->qc_attr_bf16;

@@ -405,3 +405,19 @@ def test_small_launch_with_counts_is_not_split():
         m.attention_out(q, k, v, ids, out, counts)
         assert torch.equal(plain, out) == (counts is not None)
     m.device_status()
+
+
+@pytest.mark.parametrize("items,topk,split", [(74, 20, False), (74, 24, False), (74, 32, True), (37, 16, True), (37, 13, False), (1, 64, True)])
+def test_small_launch_split_rule(items, topk, split):
+    """Both sides of the line where the blocks saved outweigh partials and merge, which cost more with more items: a
+    launch that is not split has the bits of the plain call."""
+    m = sp()
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the sizes are for 148 SMs")
+    q, k, v = (t.cuda() for t in gen.make_qkv(1, 2 * items, items, 128, topk * 128, seed=23, k_block_offset=0.5))
+    ids = gen.make_ids(1, items, 1, topk, topk, 7, "unsorted").cuda()
+    plain, out = torch.empty_like(q), torch.empty_like(q)
+    m.attention_out(q, k, v, ids, plain, balance=False)
+    m.attention_out(q, k, v, ids, out)
+    assert torch.equal(plain, out) != split
+    m.device_status()
