@@ -63,16 +63,20 @@ int sparse_b200_q_centric(const void* q, const void* k, const void* v, const int
                           const int32_t* block_count, void* out, float* lse, int batch, int hq, int hkv,
                           int sq, int skv, int topk, void* stream);
 
-/* sparse_b200_q_centric with a caller-provided scratch buffer (sparse_b200_q_centric_workspace_bytes()
- * bytes on the current device, 16-byte aligned, private to the call while it runs). With it the kernel
- * balances its last round of work items: when a launch is a few rounds of (query block, head pair)
- * items per SM and the last round would keep at most half of the SMs busy, the items of that round are
- * cut into 2-4 pieces of their lists, the pieces write normalised partials into the workspace and a small
- * kernel merges them (the log-sum-exp merge of sparse_b200_combine). Results of those rows may differ
- * from the unbalanced call in the last bf16 bit; everything else is identical. A launch without counts that has at most half
- * as many items as SMs is split in the same way as a whole: up to 16 pieces per list, fp32 partials. workspace == NULL is
- * sparse_b200_q_centric, and with a workspace too small for a split the call runs without it. No counterpart in
- * the reference (its kernels take no workspace). */
+/* sparse_b200_q_centric with a caller-provided scratch buffer (16-byte aligned, private to the call while it
+ * runs, graph replays included). With it the kernel balances its last round of work items: when a launch is a few
+ * rounds of (query block, head pair) items per SM and the last round would keep at most half of the SMs busy, the
+ * items of that round are cut into 2-4 pieces of their lists, the pieces write normalised partials into the
+ * workspace and a small kernel merges them (the log-sum-exp merge of sparse_b200_combine). A launch without counts
+ * that has at most half as many items as SMs is split in the same way as a whole where the blocks saved outweigh
+ * the merge: up to 16 pieces per list, fp32 partials. A piece rounds its probabilities to bf16 against a running
+ * maximum of its own, and the partials of a last round are bf16, so split rows differ from the plain call within
+ * the rounding of bf16 probabilities; all others are identical. workspace == NULL is sparse_b200_q_centric, and
+ * with a workspace too small for a split the call runs without it.
+ * sparse_b200_q_centric_split_bytes: the bytes that a call of these sizes uses (0: it is not split);
+ * sparse_b200_q_centric_workspace_bytes: enough for every call on the current device, about 20 MB.
+ * No counterpart in the reference (its kernels take no workspace). */
+int64_t sparse_b200_q_centric_split_bytes(int batch, int hq, int hkv, int sq, int topk, int has_counts);
 int64_t sparse_b200_q_centric_workspace_bytes(void);
 int sparse_b200_q_centric_ws(const void* q, const void* k, const void* v, const int32_t* block_idx,
                              const int32_t* block_count, void* out, float* lse, void* workspace,

@@ -139,6 +139,15 @@ int64_t sparse_b200_q_centric_workspace_bytes(void) {
   return static_cast<int64_t>(ctx->sm_count) * 2 * 128 * (128 * 4 + 4) + 512;
 }
 
+int64_t sparse_b200_q_centric_split_bytes(int batch, int hq, int hkv, int sq, int topk, int has_counts) {
+  REQUIRE(batch > 0 && hkv > 0 && hq >= hkv && hq % hkv == 0 && sq >= 128 && sq % 128 == 0 && topk > 0,
+          "sizes as in sparse_b200_q_centric");
+  REQUIRE(static_cast<long long>(batch) * hq * sq < (1LL << 31), "flattened Q row count must fit int32");
+  DeviceCtx* ctx = device_ctx();
+  if (!ctx) return SB_ERR_CUDA;
+  return q_centric_split_bytes(batch, hq, hkv, sq, topk, has_counts != 0, ctx->sm_count);
+}
+
 int sparse_b200_q_centric_ws(const void* q, const void* k, const void* v, const int32_t* block_idx,
                              const int32_t* block_count, void* out, float* lse, void* workspace,
                              int64_t workspace_bytes, int batch, int hq, int hkv, int sq, int skv, int topk,

@@ -45,6 +45,8 @@ struct QCentricArgs {
   float* const* owner_lse = nullptr;
 };
 int launch_q_centric(const QCentricArgs& a, cudaStream_t stream);
+// scratch that a launch with these sizes splits its lists into (0: it does not)
+long long q_centric_split_bytes(int batch, int hq, int hkv, int sq, int topk, bool counts, int sm_count);
 
 int launch_combine(const void* partial, int partial_is_f32, const float* lses, void* out, float* out_lse,
                    long long rows, int ranks, long long p_stride_rank, long long p_stride_row,

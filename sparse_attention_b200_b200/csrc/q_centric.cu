@@ -955,7 +955,69 @@ static int encode_rows_map(CUtensorMap* map, const void* ptr, uint64_t rows) {
                       steps, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
 }
 
+// Which items of a launch are cut into pieces of their lists (parts == 1: none), and the scratch the pieces need.
+struct SplitPlan {
+  int first = 0, parts = 1;
+  bool f32 = false;
+  long long rows = 0, bytes = 0;     // bytes: O, rounded up to 256, then the LSEs
+};
+
+static SplitPlan plan_split(int num_items, int topk, bool counts, int sm_count) {
+  SplitPlan s;
+  const int grid = num_items < sm_count ? num_items : sm_count;
+  // Tail balancing. With few rounds of items per CTA the last, partly filled round costs a whole
+  // round: when at most half of the CTAs would work in it, its items are cut into 2-4 pieces (as
+  // many as idle CTAs allow), so that the round takes a half to a quarter of the time, and a small
+  // kernel merges the pieces.
+  const int rounds = num_items / grid, rem = num_items - rounds * grid;
+  if (rem > 0 && 2 * rem <= grid && rounds <= 8 && topk >= 8) {
+    int parts = grid / rem;
+    if (parts > 4) parts = 4;
+    if (parts > topk / 4) parts = topk / 4;      // at least four blocks per piece
+    // worth it when the blocks a CTA no longer walks (about 1.7 us each, measured) outweigh the merge
+    // (launch + the partials' round trip through memory: about 4 us + 0.1 us per tail item)
+    if (parts >= 2 && 1.7f * static_cast<float>(topk - topk / parts) >= 4.f + 0.1f * static_cast<float>(rem)) {
+      s.first = num_items - rem;
+      s.parts = parts;
+    }
+  }
+  // Less than one round: the SMs without an item take pieces of the others' lists, up to SMALL_PARTS per item, at least
+  // two blocks each. The partials are fp32 here (the output of these calls was rounded once before, and still is).
+  // Only where every list is as long as the capacity: with counts the host cannot tell how much of a list is live, and
+  // short ones would pay for the partials and save nothing (lists of 64 with 4 live blocks, us, plain -> split: 12 items
+  // 13.9 -> 19.3, 74 items 15.3 -> 24.4).
+  // Worth it when the blocks saved (1.7 us each) outweigh the fp32 partials and the merge: measured about 8 us + 0.18 us
+  // per item. In a CUDA graph, plain -> split, us: 4 items of 64 blocks 115 -> 24 (16 pieces), 12 of 16 34 -> 21 (8),
+  // 32 of 32 62 -> 37, 37 of 16 35 -> 27 (4), 49 of 24 49 -> 40 (3), 74 of 32 64 -> 58 (2); below the line 74 of 20
+  // 42 -> 46, 74 of 24 49 -> 50, 32 of 8 20.0 -> 21.3.
+  if (!counts && 2 * num_items <= sm_count && topk >= 4) {
+    int parts = sm_count / num_items;
+    if (parts > SMALL_PARTS) parts = SMALL_PARTS;
+    if (parts > topk / 2) parts = topk / 2;
+    const float saved = 1.7f * static_cast<float>(topk - (topk + parts - 1) / parts);
+    if (saved >= 16.f && saved >= 10.f + 0.18f * static_cast<float>(num_items)) {
+      s.parts = parts;
+      s.f32 = true;
+    }
+  }
+  if (s.parts > 1) {
+    s.rows = static_cast<long long>(num_items - s.first) * s.parts * 2 * TILE;
+    s.bytes = ((s.rows * HEAD_DIM * (s.f32 ? 4 : 2) + 255) & ~255LL) + s.rows * 4;
+  }
+  return s;
+}
+
+// items of one segment (see decode_item)
+static int segment_items(int batch, int hq, int hkv, int qt) {
+  const int group = hq / hkv;
+  return group % 2 == 0 ? batch * hkv * qt * (group / 2) : batch * hq * ((qt + 1) / 2);
+}
+
 }  // namespace qc
+
+long long q_centric_split_bytes(int batch, int hq, int hkv, int sq, int topk, bool counts, int sm_count) {
+  return qc::plan_split(qc::segment_items(batch, hq, hkv, sq / qc::TILE), topk, counts, sm_count).bytes;
+}
 
 int launch_q_centric(const QCentricArgs& a, cudaStream_t stream) {
   using namespace qc;
@@ -973,65 +1035,27 @@ int launch_q_centric(const QCentricArgs& a, cudaStream_t stream) {
   p.group = group;
   p.qt = a.sq / TILE;
   p.pair_mode = (group % 2 == 0) ? 1 : 0;
-  p.items_per_seg = p.pair_mode ? a.batch * a.hkv * p.qt * (group / 2)
-                                : a.batch * a.hq * ((p.qt + 1) / 2);
+  p.items_per_seg = segment_items(a.batch, a.hq, a.hkv, p.qt);
   p.num_items = p.items_per_seg * a.nseg;
   p.scale_log2 = 1.4426950408889634f / sqrtf(static_cast<float>(HEAD_DIM));
   int grid = p.num_items < ctx->sm_count ? p.num_items : ctx->sm_count;
 
-  // Tail balancing. With few rounds of items per CTA the last, partly filled round costs a whole
-  // round: when at most half of the CTAs would work in it, its items are cut into 2-4 pieces (as
-  // many as idle CTAs allow), so that the round takes a half to a quarter of the time, and a small
-  // kernel merges the pieces. Needs a workspace; single-segment bf16 launches only.
+  // single-segment bf16 launches with a workspace that the pieces fit
   p.tail_first = p.num_virtual = p.num_items;
   p.tail_parts = 1;
   p.tail_lse = nullptr;
   void* tail_out = nullptr;
   bool tail_f32 = false;
-  const int rounds = p.num_items / grid, rem = p.num_items - rounds * grid;
-  if (a.tail_ws && a.owners <= 1 && a.nseg == 1 && !a.out_f32 && rem > 0 && 2 * rem <= grid && rounds >= 1 && rounds <= 8 && a.topk >= 8) {
-    int parts = grid / rem;
-    if (parts > 4) parts = 4;
-    if (parts > a.topk / 4) parts = a.topk / 4;  // at least four blocks per piece
-    const long long rows = static_cast<long long>(rem) * parts * 2 * TILE;
-    const long long need = rows * (HEAD_DIM * 2 + 4) + 256;
-    // worth it when the blocks a CTA no longer walks (about 1.7 us each, measured) outweigh the merge
-    // (launch + the partials' round trip through memory: about 4 us + 0.1 us per tail item)
-    const bool pays = parts >= 2 && 1.7f * static_cast<float>(a.topk - a.topk / parts) >= 4.f + 0.1f * static_cast<float>(rem);
-    if (pays && need <= a.tail_bytes && (reinterpret_cast<uintptr_t>(a.tail_ws) & 15u) == 0) {
-      p.tail_first = p.num_items - rem;
-      p.tail_parts = parts;
-      p.num_virtual = p.tail_first + rem * parts;
+  if (a.tail_ws && a.owners <= 1 && a.nseg == 1 && !a.out_f32 && (reinterpret_cast<uintptr_t>(a.tail_ws) & 15u) == 0) {
+    const SplitPlan s = plan_split(p.num_items, a.topk, a.block_count != nullptr, ctx->sm_count);
+    if (s.parts > 1 && s.bytes <= a.tail_bytes) {
+      p.tail_first = s.first;
+      p.tail_parts = s.parts;
+      p.num_virtual = s.first + (p.num_items - s.first) * s.parts;
       tail_out = a.tail_ws;
-      p.tail_lse = reinterpret_cast<float*>(static_cast<unsigned char*>(a.tail_ws) + ((rows * HEAD_DIM * 2 + 255) & ~255LL));
-    }
-  }
-
-  // Less than one round: the SMs without an item take pieces of the others' lists, up to SMALL_PARTS per item, at least
-  // two blocks each. The partials are fp32 here (the output of these calls was rounded once before, and still is).
-  // Only where every list is as long as the capacity: with counts the host cannot tell how much of a list is live, and
-  // short ones would pay for the partials and save nothing (lists of 64 with 4 live blocks, us, plain -> split: 12 items
-  // 13.9 -> 19.3, 74 items 15.3 -> 24.4).
-  // Worth it when the blocks saved (1.7 us each) outweigh the fp32 partials and the merge: measured about 8 us + 0.18 us
-  // per item. In a CUDA graph, plain -> split, us: 4 items of 64 blocks 115 -> 24 (16 pieces), 12 of 16 34 -> 21 (8),
-  // 32 of 32 62 -> 37, 37 of 16 35 -> 27 (4), 49 of 24 49 -> 40 (3), 74 of 32 64 -> 58 (2); below the line 74 of 20
-  // 42 -> 46, 74 of 24 49 -> 50, 32 of 8 20.0 -> 21.3.
-  if (a.tail_ws && a.owners <= 1 && a.nseg == 1 && !a.out_f32 && !a.block_count && 2 * p.num_items <= ctx->sm_count && a.topk >= 4) {
-    int parts = ctx->sm_count / p.num_items;
-    if (parts > SMALL_PARTS) parts = SMALL_PARTS;
-    if (parts > a.topk / 2) parts = a.topk / 2;
-    const long long rows = static_cast<long long>(p.num_items) * parts * 2 * TILE;
-    const long long need = rows * (HEAD_DIM * 4 + 4);
-    const float saved = 1.7f * static_cast<float>(a.topk - (a.topk + parts - 1) / parts);
-    const bool pays = saved >= 16.f && saved >= 10.f + 0.18f * static_cast<float>(p.num_items);
-    if (pays && need <= a.tail_bytes && (reinterpret_cast<uintptr_t>(a.tail_ws) & 15u) == 0) {
-      p.tail_first = 0;
-      p.tail_parts = parts;
-      p.num_virtual = p.num_items * parts;
-      tail_out = a.tail_ws;
-      tail_f32 = true;
-      p.tail_lse = static_cast<float*>(a.tail_ws) + rows * HEAD_DIM;
-      grid = p.num_virtual;
+      tail_f32 = s.f32;
+      p.tail_lse = reinterpret_cast<float*>(static_cast<unsigned char*>(a.tail_ws) + (s.bytes - s.rows * 4));
+      if (s.f32) grid = p.num_virtual;
     }
   }
 

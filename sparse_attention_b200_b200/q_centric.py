@@ -4,6 +4,7 @@ attention/q_centric/progression_attention.cpp:19-125 `attention` / `attention_ou
 bound to the C ABI. Same argument meaning and the same rejected inputs; adds
 the optional `counts` and `lse` arguments."""
 import ctypes
+import functools
 
 import torch
 
@@ -53,42 +54,39 @@ def _validate(q, k, v, ids, out=None, counts=None, lse=None):
         bad("lse must be contiguous float32 [B,Hq,Sq] on q's device")
 
 
-_WORKSPACES = {}
-
-
-def _workspace(device):
-    """Scratch of the balanced last round and of split small launches (20 MB), one per (device, stream): allocated at
-    the first call."""
-    key = (device.index, torch.cuda.current_stream(device).cuda_stream)
-    ws = _WORKSPACES.get(key)
-    if ws is None:
-        import ctypes
-        fn = _lib.lib().sparse_b200_q_centric_workspace_bytes
-        fn.restype = ctypes.c_int64
-        with torch.cuda.device(device):
-            ws = torch.empty(int(fn()), dtype=torch.uint8, device=device)
-        _WORKSPACES[key] = ws
-    return ws
+@functools.lru_cache(maxsize=1024)
+def _split_bytes(device, b, hq, hkv, sq, topk, counts):
+    """Scratch that a call of these sizes splits its lists into on the device of that index; 0 where it does not."""
+    fn = _lib.lib().sparse_b200_q_centric_split_bytes
+    fn.restype = ctypes.c_int64
+    with torch.cuda.device(device):
+        n = int(fn(b, hq, hkv, sq, topk, int(counts)))
+    if n < 0 and n != _lib.ERR_INVALID:
+        _lib.check(n)
+    return max(n, 0)                             # the call itself rejects sizes that it does not take
 
 
 def attention_out(q, k, v, ids, out, counts=None, lse=None, balance=True):
-    """out <- block-sparse attention on the current stream. balance: let the kernel split the work items of a
-    last, partly filled round (a per-stream scratch buffer is allocated at the first call; no allocation
-    afterwards); False is the plain entry, which never allocates."""
+    """out <- block-sparse attention on the current stream. balance: let the kernel split the lists of a last, partly
+    filled round of work items, or of a launch that leaves most SMs idle. The scratch of such a call (at most 20 MB) is
+    its own, from torch's caching allocator: calls of several threads and streams do not meet in it, and inside
+    torch.cuda.graph it belongs to the graph. False is the plain entry, which never allocates (a capture that bypasses
+    torch's allocator needs it)."""
     _validate(q, k, v, ids, out, counts, lse)
     b, hq, sq, _ = q.shape
     hkv, skv = k.shape[1:3]
+    topk = int(ids.shape[3])
     with torch.cuda.device(q.device):
-        if not balance:
+        need = _split_bytes(q.device.index, b, hq, hkv, sq, topk, counts is not None) if balance else 0
+        if not need:
             _lib.check(_lib.lib().sparse_b200_q_centric(
                 _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(ids), _lib.ptr(counts), _lib.ptr(out), _lib.ptr(lse),
-                b, hq, hkv, sq, skv, int(ids.shape[3]), _lib.current_stream()))
+                b, hq, hkv, sq, skv, topk, _lib.current_stream()))
             return
-        import ctypes
-        ws = _workspace(q.device)
+        ws = torch.empty(need, dtype=torch.uint8, device=q.device)
         _lib.check(_lib.lib().sparse_b200_q_centric_ws(
             _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(ids), _lib.ptr(counts), _lib.ptr(out), _lib.ptr(lse),
-            _lib.ptr(ws), ctypes.c_int64(ws.numel()), b, hq, hkv, sq, skv, int(ids.shape[3]), _lib.current_stream()))
+            _lib.ptr(ws), ctypes.c_int64(need), b, hq, hkv, sq, skv, topk, _lib.current_stream()))
 
 
 def attention(q, k, v, ids, counts=None, return_lse=False):

@@ -16,8 +16,9 @@ operator is not registered yet, attention/q_centric/progression.py:29-36):
       in storage of its own next to the grouped list it hands back.
 
 Each operator validates like the reference (RuntimeError on rejected inputs), runs on the current
-CUDA stream of the tensors' device, allocates only where the reference's does (`attention`,
-`tile_topk`), and is capturable in a CUDA graph. Nothing here is needed by the package itself.
+CUDA stream of the tensors' device, allocates results only where the reference's does (`attention`,
+`tile_topk`; split attention calls take scratch from torch's caching allocator), and is capturable
+in a CUDA graph. Nothing here is needed by the package itself.
 """
 import ctypes
 

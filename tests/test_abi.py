@@ -48,3 +48,6 @@ def test_invalid_arguments_return_error_codes_without_a_gpu():
     assert rc == _lib.ERR_INVALID
     rc = lib.sparse_b200_q_centric(one, one, one, one, None, ctypes.c_void_p(8192), None, 1, 8, 8, 256, 256, 3, None)
     assert rc == _lib.ERR_INVALID and b"exceed" in lib.sparse_b200_last_error()
+    for bad in ((0, 8, 8, 256, 4, 0), (1, 8, 3, 256, 4, 0), (1, 8, 8, 200, 4, 0), (1, 8, 8, 256, 0, 0)):
+        lib.sparse_b200_q_centric_split_bytes.restype = ctypes.c_int64
+        assert lib.sparse_b200_q_centric_split_bytes(*bad) == _lib.ERR_INVALID

@@ -421,3 +421,40 @@ def test_small_launch_split_rule(items, topk, split):
     m.attention_out(q, k, v, ids, out)
     assert torch.equal(plain, out) != split
     m.device_status()
+
+
+def test_split_calls_share_no_scratch():
+    """Two graphs captured one after the other on the same stream and replayed at the same time on two, with launches
+    that are split into pieces: every output stays that of the plain call. (32 CTAs each: both graphs fit the GPU.)"""
+    m = sp()
+    b, hq, hkv, sq, skv, topk, calls = 1, 4, 2, 128, 8192, 64, 20
+    graphs, want, outs, keep = [], [], [], []
+    for seed in (1, 2):
+        q, k, v = (t.cuda() for t in gen.make_qkv(b, hq, hkv, sq, skv, seed=seed, k_block_offset=0.5))
+        ids = gen.make_ids(b, hkv, 1, skv // 128, topk, seed, "unsorted").cuda()
+        plain = torch.empty_like(q)
+        m.attention_out(q, k, v, ids, plain, balance=False)
+        out = torch.empty((calls, *q.shape), dtype=q.dtype, device="cuda")
+        m.attention_out(q, k, v, ids, out[0])
+        torch.cuda.synchronize()
+        assert not torch.equal(out[0], plain)            # the call is split: other bits
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            for i in range(calls):
+                m.attention_out(q, k, v, ids, out[i])
+        graphs.append(g)
+        want.append(out[0].clone())
+        outs.append(out)
+        keep.append((q, k, v, ids))
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    for _ in range(10):
+        for out in outs:
+            out.zero_()
+        torch.cuda.synchronize()
+        for g, s in zip(graphs, streams):
+            with torch.cuda.stream(s):
+                g.replay()
+        torch.cuda.synchronize()
+        for out, w in zip(outs, want):
+            assert torch.equal(out, w.expand_as(out))
+    m.device_status()
