@@ -297,10 +297,8 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
   tc_fence_after();
   const uint32_t tmem = static_cast<uint32_t>(misc[0]);
   // Launched as a programmatic dependent: the setup above overlaps the tail of the kernel before it on the stream
-  // (often the one that selects this one's blocks); nothing of it is read before this wait. The next dependent launch
-  // (the merge of the last round, or another call) may be set up under this kernel in the same way.
+  // (often the one that selects this one's blocks); nothing of it is read before this wait.
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   float* stats = reinterpret_cast<float*>(gbase + OFF_STATS);
   // tensor memory columns: S0 0..127, S1 128..255, O0 256..383, O1 384..511.
   // P (bf16 pairs) overwrites columns 0..63 of its S.
@@ -410,6 +408,9 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
       for (int q = 0; q < 2; ++q)
         if (qloads[q] > 0) mbar_wait_drain(bar(BAR_Q_FULL + q), (qloads[q] - 1) & 1);
     }
+    // The next dependent launch (the merge of split lists, or another call) may be set up under the rest of this kernel:
+    // from here on, not from the start, because its CTAs wait on the SMs that a small launch leaves to other streams.
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   } else if (warp == MMA_WARP) {
     // ------------------------------------------------------------- MMA issuer (one thread)
     if (lane == 0) {

@@ -458,3 +458,38 @@ def test_split_calls_share_no_scratch():
         for out, w in zip(outs, want):
             assert torch.equal(out, w.expand_as(out))
     m.device_status()
+
+
+def test_a_waiting_attention_call_leaves_the_idle_sms_to_other_streams():
+    """Stream 1 runs one long work item (one SM) and then a call that fills the GPU; stream 2 a short call. The second
+    call of stream 1 may be set up under the first one's tail, but must not hold the other SMs while that runs: the
+    short call is done long before the long item."""
+    m = sp()
+
+    def call(hkv, nb, topk, seed):
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        q = torch.randn((1, 2 * hkv, 128, 128), device="cuda", generator=g).to(torch.bfloat16)
+        k = torch.randn((1, hkv, nb * 128, 128), device="cuda", generator=g).to(torch.bfloat16)
+        v = torch.randn((1, hkv, nb * 128, 128), device="cuda", generator=g).to(torch.bfloat16)
+        ids = torch.arange(topk, dtype=torch.int32, device="cuda").expand(1, hkv, 1, topk).contiguous()
+        out = torch.empty_like(q)
+        return lambda: m.attention_out(q, k, v, ids, out, balance=False)
+
+    long_item, filling, short = call(1, 2048, 2048, 1), call(148, 2, 2, 2), call(148, 2, 2, 3)
+    s1, s2 = torch.cuda.Stream(), torch.cuda.Stream()
+    for _ in range(2):                          # once to warm up
+        start, end1, end2 = (torch.cuda.Event(enable_timing=True) for _ in range(3))
+        torch.cuda.synchronize()
+        with torch.cuda.stream(s1):
+            start.record()
+            long_item()
+            filling()
+            end1.record()
+        with torch.cuda.stream(s2):
+            short()
+            end2.record()
+        torch.cuda.synchronize()
+    whole, other = start.elapsed_time(end1), start.elapsed_time(end2)
+    assert whole > 2.0                          # 2048 blocks at 1.7 us
+    assert other < 0.5 * whole, (other, whole)
+    m.device_status()
