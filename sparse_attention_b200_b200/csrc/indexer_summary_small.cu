@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(256) score_rows_kernel(const RowsParams p) {
       p.scores_out[(list0 + static_cast<long long>(l) * csize) * p.nt + (e - l * p.nt)] = scores[e];
     }
   // (score descending, id ascending) is a total order: no score is NaN
-  if (p.nt <= 256 && (p.topk > 128 || ((own * p.nt + 255) >> 8) * p.nt <= 512 * ((own + 7) >> 3))) {
+  if (p.nt <= 256 && ((own * p.nt + 255) >> 8) * p.nt <= 512 * ((own + 7) >> 3)) {
     // Short lists: every score counts the scores that beat it, the count is its rank. The right-hand side is what
     // the threshold search of a warp below takes in the same unit, scores read by a thread (64 lists of 256: 271 us
     // by counting, 60 by searching, whole selector; 32 lists of 32: 20 and 25).
@@ -279,12 +279,39 @@ __global__ void __launch_bounds__(256) score_rows_kernel(const RowsParams p) {
     }
     return;
   }
-  __syncthreads();                             // scores read out before block_topk retires entries
-  float* scratch_f = k_s;
-  int* scratch_i = reinterpret_cast<int*>(k_s + 16);
-  for (int l = 0; l < own; ++l) {
-    block_topk(scores + l * p.nt, p.nt, p.topk, p.ids + (list0 + static_cast<long long>(l) * csize) * p.topk, scratch_f,
-               scratch_i);
+  // k > 128: the lists are sorted, as many at a time as fit the tiles' 64 KiB (8192 keys; bitonic, 64-bit keys of score
+  // and inverted id, so that the order is score descending, id ascending; padding sorts last). Rounds of block-wide
+  // arg-max, k per list and list after list, took 1320 us for 64 lists of 512 with k = 256, this 44 (whole selector).
+  unsigned long long* keys = reinterpret_cast<unsigned long long*>(q_s);
+  int p_log2 = 1;
+  while ((1 << p_log2) < p.nt) ++p_log2;
+  const int batch = 8192 >> p_log2, half = 1 << (p_log2 - 1);
+  for (int l0 = 0; l0 < own; l0 += batch) {
+    const int nl = min(batch, own - l0);
+    for (int e = tid; e < nl << p_log2; e += blockDim.x) {
+      const int l = e >> p_log2, j = e & (2 * half - 1);
+      keys[e] = j < p.nt ? (static_cast<unsigned long long>(score_key(scores[(l0 + l) * p.nt + j])) << 32) | (0xffffffffu - j) : 0ull;
+    }
+    __syncthreads();
+    for (int k = 1; k <= p_log2; ++k) {
+      for (int d = k - 1; d >= 0; --d) {
+        for (int c = tid; c < nl * half; c += blockDim.x) {
+          const int i = ((c >> d) << (d + 1)) | (c & ((1 << d) - 1));      // bit d clear; i + 2^d is its partner
+          const bool descending = k == p_log2 || ((i >> k) & 1) == 0;
+          const unsigned long long x = keys[i], y = keys[i + (1 << d)];
+          if ((x < y) == descending) {
+            keys[i] = y;
+            keys[i + (1 << d)] = x;
+          }
+        }
+        __syncthreads();
+      }
+    }
+    for (int e = tid; e < nl * p.topk; e += blockDim.x) {
+      const int l = e / p.topk, place = e - l * p.topk;
+      p.ids[(list0 + static_cast<long long>(l0 + l) * csize) * p.topk + place] =
+          static_cast<int32_t>(0xffffffffu - static_cast<unsigned>(keys[(l << p_log2) + place]));
+    }
     __syncthreads();
   }
 }

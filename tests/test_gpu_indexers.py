@@ -315,6 +315,11 @@ def test_small_problem_selector_equals_the_exact_kernels(b, hkv, g, sq, skv, r, 
     (1, 1, 5, 3, 2048, 1, 64),      # the largest block count, chunks for a whole cluster
     (1, 1, 16, 30, 70, 2, 1),       # 32 per list, two representatives, k = 1
     (3, 1, 12, 60, 33, 4, 12),      # 48 padded to 64: a list fills the row tile; not a power of two, any size
+    (1, 1, 1, 70, 512, 1, 256),     # k > 128, sorted: several lists per CTA in one batch
+    (1, 4, 1, 64, 300, 1, 140),     # more than one batch of lists per CTA, padded to 512
+    (1, 1, 4, 20, 1025, 1, 700),    # padded to 2048
+    (1, 1, 1, 40, 2048, 1, 2048),   # the largest block count, every block
+    (1, 2, 3, 150, 200, 1, 129),    # at most 256 blocks, too many lists for counting
 ])
 @pytest.mark.parametrize("ties", [False, True])
 def test_row_tile_selector_equals_the_exact_kernels(b, hkv, g, qb, nb, r, topk, ties):
