@@ -1,5 +1,6 @@
-// R1 / R4 summary selector for SMALL problems (few lists, few KV blocks): the same
-// arithmetic as indexer_summary.cu, cut so that a problem of 64 lists fills the GPU.
+// R1 / R4 summary selector for problems that do not fill the GPU, and for every problem of up to 2048 KV blocks whose
+// scores are wanted or that the tensor-core forms refuse: the arithmetic of indexer_summary.cu, cut so that a problem of
+// 64 lists fills the GPU.
 //
 //   pool_small_kernel   one CTA per descriptor: the 128/R token rows (contiguous in
 //                       memory) are fetched into shared memory in ONE round trip by all
@@ -7,7 +8,7 @@
 //                       sequential fp32 sum, so the descriptors are bit-identical with
 //                       pool_kernel, which keeps 16 lanes per descriptor and pays one
 //                       memory round trip per 8 tokens).
-//   score_rows_kernel   64 query descriptors (one or several lists of a KV head) per cluster of 1 - 8 CTAs, see there.
+//   score_rows_kernel   16 to 64 query descriptors (one or several lists of a KV head) per cluster of 1 - 8 CTAs.
 // Same results as pool_blocks / descriptor_dot / reduce_topk
 // (indexers/r1_r4/gpu_ops.py:6-49): ids in score-descending order, ties to the lower id.
 #include "internal.h"
@@ -51,31 +52,34 @@ __global__ void __launch_bounds__(256) pool_small_kernel(const __nv_bfloat16* __
 }
 
 // ---------------------------------------------------------------- score + top-k
-// A row tile is ROWS = 64 query descriptors: L lists (query blocks of one KV head) of MP descriptors each (MP = group
-// heads x R rounded up to a power of two, padding repeats a list's first descriptor: the maximum is unchanged). A
-// cluster of C CTAs (C = 1, 2, 4 or 8) shares the row tile: CTA `rank` scores the key chunks rank, rank + C, ... of
-// 64 descriptors, and owns the lists l with l % C == rank: every score goes straight into the owner's shared memory.
-// Bound by fp32 FMAs (the exact score is defined by fp32 sums in feature order): 4 x 4 register tile per thread, two
-// 16-byte shared-memory reads per 16 FMAs, the next chunk's bytes requested before the arithmetic of this one.
-constexpr int ROWS = 64, KD = 64;
+// A row tile is ROWS = 16 QT query descriptors (QT = 1, 2 or 4): L lists (query blocks of one KV head) of MP descriptors
+// each (MP = group heads x R rounded up to a power of two, padding repeats a list's first descriptor: the maximum is
+// unchanged). A cluster of C CTAs (C = 1, 2, 4 or 8) shares the row tile: CTA `rank` scores the key chunks rank,
+// rank + C, ... of 64 descriptors, and owns the lists l with l % C == rank: every score goes straight into the owner's
+// shared memory. Bound by fp32 FMAs (the exact score is defined by fp32 sums in feature order): QT x 4 register tile per
+// thread, two shared-memory reads of up to 16 bytes per 4 QT FMAs, the next chunk's bytes requested before the arithmetic
+// of this one. QT, L and C are chosen by plan_rows().
+constexpr int KD = 64;
 constexpr int SCORE_BYTES_MAX = 40 * 1024;
+constexpr size_t SMEM_PER_SM = 228 * 1024;       // of which 1 KiB per CTA is the system's
 
 __device__ __forceinline__ unsigned score_key(float s) {      // order of the floats; both zeros are one value
   const unsigned b = __float_as_uint(s + 0.f);
   return b ^ ((b >> 31) ? 0xffffffffu : 0x80000000u);
 }
 
-// [feature][64] fp32 tile in shared memory. Odd 8-feature pieces are stored with bit 4 of the column flipped, so that
-// a warp which holds two neighbouring pieces of 16 rows (whole 32-byte sectors of global memory) stores without bank
-// conflicts.
+// [feature][ROWS] fp32 tile in shared memory. Odd 8-feature pieces are stored with bit 4 of the column flipped (tiles of
+// at least 32 columns), so that a warp which holds two neighbouring pieces of 16 rows (whole 32-byte sectors of global
+// memory) stores without bank conflicts.
+template <int ROWS>
 __device__ __forceinline__ void stage_piece(float* tile, int row, int c, const uint4& raw) {
   const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
-  float* dst = tile + c * 8 * 64 + (row ^ ((c & 1) << 4));
+  float* dst = tile + c * 8 * ROWS + (ROWS > 16 ? row ^ ((c & 1) << 4) : row);
 #pragma unroll
   for (int p = 0; p < 4; ++p) {
     const float2 f = __bfloat1622float2(h[p]);
-    dst[(2 * p) * 64] = f.x;
-    dst[(2 * p + 1) * 64] = f.y;
+    dst[(2 * p) * ROWS] = f.x;
+    dst[(2 * p + 1) * ROWS] = f.y;
   }
 }
 
@@ -88,9 +92,10 @@ struct RowsParams {
   int lists_per_cta, tiles_per_head, mp_log2;
 };
 
-// LPT = lists a thread's four rows belong to: 1 (MP >= 4), 2 (MP = 2) or 4 (MP = 1)
-template <int LPT>
+// QT = rows per thread, LPT = lists that they belong to: 1 (MP >= QT) or QT / MP
+template <int QT, int LPT>
 __global__ void __launch_bounds__(256) score_rows_kernel(const RowsParams p) {
+  constexpr int ROWS = 16 * QT;
   extern __shared__ __align__(16) float smem[];
   float* q_s = smem;                         // [128][ROWS]
   float* k_s = q_s + 128 * ROWS;             // [128][KD]
@@ -107,8 +112,10 @@ __global__ void __launch_bounds__(256) score_rows_kernel(const RowsParams p) {
   const int lists = min(p.lists_per_cta, p.qt - qtile0);
   const int n_keys = p.nt * p.r;
   const int tid = threadIdx.x;
-  // staging role: 16-byte pieces piece0 + 2 i of row `srow` (i = 0 .. 3, both parities of a piece pair in a warp)
+  // staging role: 16-byte pieces piece0 + 2 i of row `srow` (i = 0 .. 3, both parities of a piece pair in a warp); for
+  // the queries QT pieces qpiece0 + 2 i of row `qrow`
   const int srow = (tid >> 1) & 63, piece0 = (tid & 1) | ((tid >> 7) << 3);
+  const int qrow = (tid >> 1) & (ROWS - 1), qpiece0 = (tid & 1) | (tid / (2 * ROWS)) * (2 * QT);
 
   asm volatile("griddepcontrol.wait;" ::: "memory");      // the descriptors of the pooling kernel are visible from here
   // every list is exact here: no fallback, no violated bound, no largest difference
@@ -122,50 +129,60 @@ __global__ void __launch_bounds__(256) score_rows_kernel(const RowsParams p) {
       raw[i] = live ? __ldg(kbase + static_cast<long long>(base + srow) * 16 + piece0 + 2 * i) : make_uint4(0u, 0u, 0u, 0u);
   };
   {
-    const int l = srow >> p.mp_log2, m = srow & ((1 << p.mp_log2) - 1);
+    const int l = qrow >> p.mp_log2, m = qrow & ((1 << p.mp_log2) - 1);
     const int mm = m < m_real ? m : 0;
     const int g = mm / p.r, rq = mm - g * p.r;
     const long long row = ((static_cast<long long>(b) * p.hq + kvh * group + g) * p.qt + qtile0 + (l < lists ? l : 0)) * p.r + rq;
     const uint4* src = reinterpret_cast<const uint4*>(p.qd + row * 128);
-    uint4 qraw[4];
+    uint4 qraw[QT];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) qraw[i] = __ldg(src + piece0 + 2 * i);
+    for (int i = 0; i < QT; ++i) qraw[i] = __ldg(src + qpiece0 + 2 * i);
     fetch_keys(rank * KD);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) stage_piece(q_s, srow, piece0 + 2 * i, qraw[i]);
+    for (int i = 0; i < QT; ++i) stage_piece<ROWS>(q_s, qrow, qpiece0 + 2 * i, qraw[i]);
   }
   if (csize > 1) cluster.sync();               // all CTAs of the cluster run: their shared memory may be addressed
   const float scale = 0.08838834764831845f;   // fp32(128^-0.5)
   const int tq = tid & 15, tk = tid >> 4;
-  const int bpt = 4 / p.r;                     // KV blocks among a thread's four key descriptors
   float* owner_scores[LPT];                    // where the scores of this thread's lists go (null: not a real list)
 #pragma unroll
   for (int x = 0; x < LPT; ++x) {
-    const int l = (tq * 4 + x * (4 / LPT)) >> p.mp_log2;
-    const bool speaks = LPT > 1 || ((tq * 4) & ((1 << p.mp_log2) - 1)) == 0;
+    const int l = (tq * QT + x * (QT / LPT)) >> p.mp_log2;
+    const bool speaks = LPT > 1 || ((tq * QT) & ((1 << p.mp_log2) - 1)) == 0;
     owner_scores[x] = speaks && l < lists ? cluster.map_shared_rank(scores, l & (csize - 1)) + (l >> c_log2) * p.nt : nullptr;
   }
 
   for (int base = rank * KD; base < n_keys; base += csize * KD) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) stage_piece(k_s, srow, piece0 + 2 * i, raw[i]);
+    for (int i = 0; i < 4; ++i) stage_piece<KD>(k_s, srow, piece0 + 2 * i, raw[i]);
     __syncthreads();                           // tiles staged
     if (base + csize * KD < n_keys) fetch_keys(base + csize * KD);
-    float acc[4][4];
+    float acc[QT][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < QT; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    const int features = base + (tid >> 5) * 8 < n_keys ? 128 : 0;      // a warp's eight keys may all be padding
 #pragma unroll 1
-    for (int d0 = 0; d0 < 128; d0 += 16) {
+    for (int d0 = 0; d0 < features; d0 += 16) {
 #pragma unroll
       for (int dd = 0; dd < 16; ++dd) {
         const int flip = (dd >> 3) << 4;
-        const float4 qv = *reinterpret_cast<const float4*>(q_s + (d0 + dd) * 64 + ((tq * 4) ^ flip));
         const float4 kv = *reinterpret_cast<const float4*>(k_s + (d0 + dd) * 64 + ((tk * 4) ^ flip));
-        const float qa[4] = {qv.x, qv.y, qv.z, qv.w}, ka[4] = {kv.x, kv.y, kv.z, kv.w};
+        const float ka[4] = {kv.x, kv.y, kv.z, kv.w};
+        const float* qsrc = q_s + (d0 + dd) * ROWS + (QT > 1 ? (tq * QT) ^ flip : tq);
+        float qa[QT];
+        if constexpr (QT == 4) {
+          const float4 qv = *reinterpret_cast<const float4*>(qsrc);
+          qa[0] = qv.x; qa[1] = qv.y; qa[2] = qv.z; qa[3] = qv.w;
+        } else if constexpr (QT == 2) {
+          const float2 qv = *reinterpret_cast<const float2*>(qsrc);
+          qa[0] = qv.x; qa[1] = qv.y;
+        } else {
+          qa[0] = *qsrc;
+        }
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < QT; ++i)
 #pragma unroll
           for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(qa[i], ka[j], acc[i][j]);
       }
@@ -179,12 +196,12 @@ __global__ void __launch_bounds__(256) score_rows_kernel(const RowsParams p) {
       for (int j = 0; j < 4; ++j) {
         best[j] = -CUDART_INF_F;
 #pragma unroll
-        for (int i = 0; i < 4 / LPT; ++i) best[j] = fmaxf(best[j], acc[x * (4 / LPT) + i][j]);
+        for (int i = 0; i < QT / LPT; ++i) best[j] = fmaxf(best[j], acc[x * (QT / LPT) + i][j]);
       }
       if (p.r > 1) { best[0] = fmaxf(best[0], best[1]); best[2] = fmaxf(best[2], best[3]); }
       if (p.r > 2) best[0] = fmaxf(best[0], best[2]);
       if (LPT == 1) {
-        for (int dlt = 1; dlt < (1 << p.mp_log2) / 4; dlt <<= 1) {
+        for (int dlt = 1; dlt < (1 << p.mp_log2) / QT; dlt <<= 1) {
 #pragma unroll
           for (int j = 0; j < 4; ++j) best[j] = fmaxf(best[j], __shfl_xor_sync(0xffffffffu, best[j], dlt));
         }
@@ -279,13 +296,13 @@ __global__ void __launch_bounds__(256) score_rows_kernel(const RowsParams p) {
     }
     return;
   }
-  // k > 128: the lists are sorted, as many at a time as fit the tiles' 64 KiB (8192 keys; bitonic, 64-bit keys of score
-  // and inverted id, so that the order is score descending, id ascending; padding sorts last). Rounds of block-wide
+  // k > 128: the lists are sorted, as many at a time as fit the tiles' 40 to 64 KiB (bitonic, 64-bit keys of score and
+  // inverted id, so that the order is score descending, id ascending; padding sorts last). Rounds of block-wide
   // arg-max, k per list and list after list, took 1320 us for 64 lists of 512 with k = 256, this 44 (whole selector).
   unsigned long long* keys = reinterpret_cast<unsigned long long*>(q_s);
   int p_log2 = 1;
   while ((1 << p_log2) < p.nt) ++p_log2;
-  const int batch = 8192 >> p_log2, half = 1 << (p_log2 - 1);
+  const int batch = ((128 * ROWS + 128 * KD) / 2) >> p_log2, half = 1 << (p_log2 - 1);
   for (int l0 = 0; l0 < own; l0 += batch) {
     const int nl = min(batch, own - l0);
     for (int e = tid; e < nl << p_log2; e += blockDim.x) {
@@ -316,11 +333,11 @@ __global__ void __launch_bounds__(256) score_rows_kernel(const RowsParams p) {
   }
 }
 
-template <int LPT>
+template <int QT, int LPT>
 int launch_rows(const RowsParams& p, int grid, int csize, size_t smem, DeviceCtx* ctx, int slot, cudaStream_t stream) {
   if (!(ctx->small_attr & (1 << slot))) {
-    cudaError_t e = cudaFuncSetAttribute(score_rows_kernel<LPT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         2 * 32768 + SCORE_BYTES_MAX);
+    cudaError_t e = cudaFuncSetAttribute(score_rows_kernel<QT, LPT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (QT * 16 + KD) * 512 + SCORE_BYTES_MAX);
     if (e != cudaSuccess) return set_error(SB_ERR_CUDA, cudaGetErrorString(e));
     ctx->small_attr |= (1 << slot);
   }
@@ -337,8 +354,74 @@ int launch_rows(const RowsParams& p, int grid, int csize, size_t smem, DeviceCtx
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, score_rows_kernel<LPT>, p);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, score_rows_kernel<QT, LPT>, p);
   return e == cudaSuccess ? SB_OK : set_error(SB_ERR_CUDA, cudaGetErrorString(e));
+}
+
+struct RowsPlan {
+  int lists, tiles, csize, qt;       // lists per row tile, row tiles per KV head, cluster size, rows per thread
+  size_t smem;
+};
+
+// How the lists of a KV head are cut into row tiles and how many CTAs share one: the cheapest by an estimate in cycles of
+// an SM. Few lists are spread over the SMs in smaller tiles; many are packed, as far as the scores of the lists that a CTA
+// owns fit its share of shared memory, which for long lists takes a large cluster. Whole selector with scores, us, always
+// 64-row tiles packed as densely as the rows hold -> this: 64 lists of 1 x 128 descriptors, which ran on two CTAs,
+// 49.9 -> 11.5; 16 of 1 x 64 16.9 -> 9.6; 4 of 1 x 8 11.6 -> 8.1; 2048 of 1 x 2048, five lists to a tile, 662 -> 161;
+// 1024 of 8 x 8192 2237 -> 1948. (A cluster of 8 CTAs per list and 16 descriptors, which was used for up to 148 lists before
+// the row tiles, took 15.1, 10.7 and 9.1 us for the first three; on a few lists of 65 to 128 keys it was 1 us faster.)
+RowsPlan plan_rows(long long heads, int qt, int nt, int r, int topk, int mp_log2, int sm_count) {
+  const int chunks = (nt * r + KD - 1) / KD;
+  const float nf = static_cast<float>(nt);
+  float sort_stage = 0.f, stages = 0.f;        // k > 128: cycles per list and stage beside others, number of stages
+  int p_log2 = 1;
+  while ((1 << p_log2) < nt) ++p_log2;
+  stages = 0.5f * p_log2 * (p_log2 + 1);
+  sort_stage = 25.f * (1 << p_log2) / 512.f;
+  const float search = 1300.f + 5.2f * nf + 0.25f * static_cast<float>(topk) * static_cast<float>(topk);
+  RowsPlan best{};
+  float best_cost = 0.f;
+  int full = 64 >> mp_log2;
+  if (full > qt) full = qt;
+  for (int n = full;; n = (n + 1) / 2) {
+    const int tiles = (qt + n - 1) / n, lists = (qt + tiles - 1) / tiles;
+    const int rows = lists << mp_log2, per_thread = rows <= 16 ? 1 : rows <= 32 ? 2 : 4;
+    for (int c = 8; c >= 1; c >>= 1) {
+      const int own = (lists + c - 1) / c;
+      if ((c > 1 && c / 2 >= chunks) || own * nt * 4 > SCORE_BYTES_MAX) continue;
+      const size_t smem = static_cast<size_t>(16 * per_thread + KD) * 512 + static_cast<size_t>(own) * nt * 4;
+      const long long ctas = heads * tiles * c;
+      const int resident = static_cast<int>(SMEM_PER_SM / (smem + 1024)) < 4 ? static_cast<int>(SMEM_PER_SM / (smem + 1024)) : 4;
+      const long long slots = static_cast<long long>(resident) * sm_count;
+      const float waves = static_cast<float>((ctas + slots - 1) / slots);
+      const float load = static_cast<float>((ctas + sm_count - 1) / sm_count);       // CTAs of an SM in all
+      // a chunk: bound by shared-memory reads, 8, 6 or 5 wavefronts per warp and feature; slower for a CTA by itself
+      float chunk = per_thread == 1 ? 5200.f : per_thread == 2 ? 6200.f : 8200.f;
+      if (ctas <= sm_count) chunk *= 1.17f;
+      // clusters of a second wave wait until all their slots are free
+      if (ctas > slots) chunk *= c == 8 ? 1.25f : c == 4 ? 1.2f : c == 2 ? 1.1f : 1.f;
+      const float share = static_cast<float>(lists) / static_cast<float>(c);
+      float alone, among;                      // ranking: of the busiest CTA by itself, of the average one beside others
+      if (nt <= 256 && ((own * nt + 255) >> 8) * nt <= 512 * ((own + 7) >> 3)) {
+        alone = static_cast<float>((own * nt + 255) >> 8) * nf * 10.f;
+        among = share * nf * nf * (10.f / 256.f);
+      } else if (topk <= 128) {
+        alone = search * (own > 5 ? 0.2f * static_cast<float>(own) : 1.f);
+        among = search * 0.2f * share;
+      } else {
+        alone = stages * (own * sort_stage > 80.f ? own * sort_stage : 80.f);
+        among = stages * share * sort_stage;
+      }
+      const float ranking = alone > load * among ? alone : load * among;
+      const float cost = waves * (c > 1 ? 3300.f : 2500.f) + load * chunk * static_cast<float>((chunks + c - 1) / c) + ranking;
+      if (best.lists == 0 || cost < best_cost) {
+        best = RowsPlan{lists, tiles, c, per_thread, smem};
+        best_cost = cost;
+      }
+    }
+    if (n == 1) break;
+  }
+  return best;
 }
 
 }  // namespace
@@ -371,30 +454,22 @@ int launch_summary_small(const void* qd, const void* kd, float* scores, int32_t*
   DeviceCtx* ctx = device_ctx();
   if (!ctx) return SB_ERR_CUDA;
   const int m = (hq / hkv) * r;
-  if (nt > 2048 || m > ROWS) return 1;
+  if (nt > 2048 || m > 64) return 1;
   int mp_log2 = 0;
   while ((1 << mp_log2) < m) ++mp_log2;
-  int per_cta = ROWS >> mp_log2;
-  if (per_cta > qt) per_cta = qt;
-  const int chunks = (nt * r + KD - 1) / KD;
   const long long heads = static_cast<long long>(batch) * hkv;
-  // The largest cluster that keeps every CTA resident at once (three 64 KiB CTAs per SM) and gives each a chunk; the
-  // scores of the lists a CTA owns must fit its share of shared memory.
-  int csize, tiles;
-  while (true) {
-    tiles = (qt + per_cta - 1) / per_cta;
-    csize = 8;
-    while (csize > 1 && (csize > chunks || heads * tiles * csize > 3LL * ctx->sm_count)) csize >>= 1;
-    if (static_cast<long long>((per_cta + csize - 1) / csize) * nt * 4 <= SCORE_BYTES_MAX) break;
-    per_cta = (per_cta + 1) / 2;
-  }
+  // 64 x 64 units of the problem: lists packed as densely as a cluster of 8 allows
+  int packed = 64 >> mp_log2;
+  if (packed > 8 * (SCORE_BYTES_MAX / (4 * nt))) packed = 8 * (SCORE_BYTES_MAX / (4 * nt));
+  const long long units = heads * ((qt + packed - 1) / packed) * ((nt * r + KD - 1) / KD);
   // Against the tensor-core forms (their selection phase costs about 16 us per round of eight lists whatever the
   // length, a unit of 64 rows x 64 keys here about 5 us of an SM; select_summary with pooling, us, tensor-core form ->
   // this one): below 16 descriptors per list those pack more than a round of lists into one CTA and leave most SMs
   // idle (256 lists of 1 x 32 blocks 68 -> 20, 512 of 4 x 512 126 -> 58, 2048 of 1 x 256 271 -> 107); from 16 on only
   // when the lists do not fill the GPU (64 lists of 64 x 512 key rows 42 -> 32, 128 of 16 x 1024 75 -> 61). Beyond four
   // units per SM the tensor cores win (320 of 16 x 600: 62 against 70; 128 of 64 x 2048: 62 against 164).
-  if (!force && !((m < 16 || heads * qt <= ctx->sm_count) && heads * tiles * chunks <= 4LL * ctx->sm_count)) return 1;
+  if (!force && !((m < 16 || heads * qt <= ctx->sm_count) && units <= 4LL * ctx->sm_count)) return 1;
+  const RowsPlan plan = plan_rows(heads, qt, nt, r, topk, mp_log2, ctx->sm_count);
   RowsParams p{};
   p.qd = static_cast<const __nv_bfloat16*>(qd);
   p.kd = static_cast<const __nv_bfloat16*>(kd);
@@ -402,14 +477,16 @@ int launch_summary_small(const void* qd, const void* kd, float* scores, int32_t*
   p.ids = ids;
   p.fallback_counter = fallback_counter;
   p.hq = hq; p.hkv = hkv; p.qt = qt; p.nt = nt; p.r = r; p.topk = topk;
-  p.lists_per_cta = per_cta;
-  p.tiles_per_head = tiles;
+  p.lists_per_cta = plan.lists;
+  p.tiles_per_head = plan.tiles;
   p.mp_log2 = mp_log2;
-  const size_t smem = (128 * ROWS + 128 * KD) * sizeof(float) + static_cast<size_t>((per_cta + csize - 1) / csize) * nt * 4;
-  const int grid = static_cast<int>(heads) * tiles * csize;
-  if (mp_log2 == 0) return launch_rows<4>(p, grid, csize, smem, ctx, 0, stream);
-  if (mp_log2 == 1) return launch_rows<2>(p, grid, csize, smem, ctx, 1, stream);
-  return launch_rows<1>(p, grid, csize, smem, ctx, 2, stream);
+  const int grid = static_cast<int>(heads) * plan.tiles * plan.csize;
+  if (plan.qt == 1) return launch_rows<1, 1>(p, grid, plan.csize, plan.smem, ctx, 0, stream);
+  if (plan.qt == 2 && mp_log2 == 0) return launch_rows<2, 2>(p, grid, plan.csize, plan.smem, ctx, 1, stream);
+  if (plan.qt == 2) return launch_rows<2, 1>(p, grid, plan.csize, plan.smem, ctx, 2, stream);
+  if (mp_log2 == 0) return launch_rows<4, 4>(p, grid, plan.csize, plan.smem, ctx, 3, stream);
+  if (mp_log2 == 1) return launch_rows<4, 2>(p, grid, plan.csize, plan.smem, ctx, 4, stream);
+  return launch_rows<4, 1>(p, grid, plan.csize, plan.smem, ctx, 5, stream);
 }
 
 }  // namespace sb

@@ -320,6 +320,10 @@ def test_small_problem_selector_equals_the_exact_kernels(b, hkv, g, sq, skv, r, 
     (1, 1, 4, 20, 1025, 1, 700),    # padded to 2048
     (1, 1, 1, 40, 2048, 1, 2048),   # the largest block count, every block
     (1, 2, 3, 150, 200, 1, 129),    # at most 256 blocks, too many lists for counting
+    (1, 1, 1, 1000, 300, 1, 5),     # many lists of one descriptor: four to a thread
+    (1, 1, 2, 500, 301, 1, 7),      # two to a thread
+    (1, 2, 1, 16, 128, 1, 8),       # few lists spread over small row tiles: one row per thread
+    (1, 1, 3, 5, 20, 4, 3),         # the same, three chunks for four CTAs of a cluster
 ])
 @pytest.mark.parametrize("ties", [False, True])
 def test_row_tile_selector_equals_the_exact_kernels(b, hkv, g, qb, nb, r, topk, ties):
