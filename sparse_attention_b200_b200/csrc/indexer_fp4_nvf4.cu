@@ -1317,6 +1317,8 @@ int launch_fp4_scores_varlen_nv(const void* qp, const void* qs, const void* kp, 
   const long long n = static_cast<long long>(hq) * p.tiles_out * total_q;
   const long long fill_blocks = std::min<long long>((n / 4 + 255) / 256 + 1, 8LL * ctx->sm_count);
   fill_neg_inf_kernel<<<static_cast<unsigned>(fill_blocks), 256, 0, stream>>>(out, n);
+  const cudaError_t filled = cudaGetLastError();
+  if (filled != cudaSuccess) return set_error(SB_ERR_CUDA, cudaGetErrorString(filled));
   if (items == 0 || p.tiles_out == 0) return SB_OK;
   // enough CTAs to fill the GPU twice over, as long a run of pages per CTA as that allows (the query tile is
   // loaded once per CTA)
