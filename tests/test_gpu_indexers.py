@@ -79,7 +79,7 @@ def test_summary_selector_bit_exact(shape):
 
 @pytest.mark.parametrize("shape", [
     # B, Hq, Hkv, Sq, Skv, R, topk, k offset
-    (1, 8, 8, 4096, 4096, 1, 8, 0.5),        # configuration 1 (GR = 1, candidates = 24 of 32)
+    (1, 8, 8, 4096, 4096, 1, 8, 0.5),        # one descriptor per list, 32 blocks (row tiles)
     (2, 16, 2, 1024, 8192, 4, 32, 0.5),      # group 8, R4 (GR = 32)
     (1, 16, 1, 512, 16384, 4, 64, 0.5),      # group 16, R4 (GR = 64), top-64 of 128
     (1, 4, 2, 256, 1024, 2, 8, 0.0),         # GR = 4, top-k == all blocks
@@ -88,6 +88,8 @@ def test_summary_selector_bit_exact(shape):
     (1, 6, 2, 256, 2048, 4, 5, 0.0),         # group 3: not eligible, exact kernel behind the same entry
 ])
 def test_summary_selector_tensor_core_path_bit_exact(shape):
+    """The entry that chooses between row tiles, pre-filter and exact kernels by size, against the oracle. (That the
+    pre-filter itself ran is asserted by the tests of few descriptors, long lists and the persistent form below.)"""
     b, hq, hkv, sq, skv, r, topk, off = shape
     m = sp()
     q, k, _ = gen.make_qkv(b, hq, hkv, sq, skv, seed=19, k_block_offset=off)
@@ -104,8 +106,8 @@ def test_summary_selector_tensor_core_path_ties_and_constant_inputs():
     """Exact ties cannot be proven safe by the pre-filter: those lists must take the
     exact fallback and still come out with the lower block id first."""
     m = sp()
-    # 160 lists (more than one per SM, so the tensor-core path is taken, not the small-problem
-    # cluster kernel) of 64 blocks > 32 candidates
+    # 160 lists (more than one per SM) of 16 descriptors: the tensor-core path, not the row-tile kernel; 64 blocks > 32
+    # candidates
     q = torch.zeros((1, 4, 160 * 128, 128), dtype=torch.bfloat16)
     k = torch.zeros((1, 1, 8192, 128), dtype=torch.bfloat16)
     sel = m.SummarySelector(q.cuda(), k.cuda(), 4, topk=16, keep_scores=False)
@@ -160,6 +162,43 @@ def test_summary_selector_tensor_core_path_long_lists(shape):
     ref = oracle.summary_select(q, k, r, topk)[3]
     assert torch.equal(ids.cpu(), ref)
     print("lists that fell back to exact scoring:", sel.fallback_lists())
+
+
+@pytest.mark.parametrize("hkv,g,qb,nb,r,topk", [
+    (8, 1, 320, 1024, 1, 8),          # one descriptor per list
+    (4, 2, 320, 1024, 1, 16),         # two
+    (4, 2, 320, 600, 2, 16),          # four, two of them from R
+    (2, 2, 160, 700, 4, 16),          # eight
+])
+@pytest.mark.parametrize("near", [False, True])
+def test_summary_selector_tensor_core_path_few_descriptors(hkv, g, qb, nb, r, topk, near):
+    """Lists of fewer than 16 descriptors take the pre-filter where their row tiles would be more than four 64 x 64 units
+    per SM; near: twenty blocks at the top are copies of one block with one token scaled (differences that the
+    approximate scores cannot order). Ids equal those of the staged exact kernel, every re-scored candidate is inside
+    the error bound."""
+    m = sp()
+    gen_ = torch.Generator(device="cuda").manual_seed(53)
+    q = (torch.randn((1, hkv * g, qb * 128, 128), device="cuda", generator=gen_) + (0.5 if near else 0.0)).to(torch.bfloat16)
+    k = torch.randn((1, hkv, nb, 128, 128), device="cuda", generator=gen_) * (0.2 if near else 1.0)
+    k += 0.5 * torch.randn((1, hkv, nb, 1, 128), device="cuda", generator=gen_) * (0.0 if near else 1.0)
+    if near:
+        k[:, :, :20] = k[:, :, :1] + 1.0
+        k[:, :, :20, 5] *= 1.0 + 0.01 * torch.arange(20, device="cuda").view(20, 1)
+    k = k.to(torch.bfloat16).view(1, hkv, nb * 128, 128)
+    fast = m.SummarySelector(q, k, r, topk=topk, keep_scores=False)
+    ids = fast.run_fast().clone()
+    exact = m.SummarySelector(q, k, r, topk=topk, keep_scores=False)
+    exact.prepare()
+    exact.score()
+    torch.cuda.synchronize()
+    m.device_status()
+    assert float(fast.aux[:hkv].view(torch.float32).min()) > 0      # the key abs-max only the tensor-core path writes
+    assert torch.equal(ids, exact.ids)
+    violations, ratio = fast.bound_stats()
+    assert violations == 0
+    if near:
+        assert ratio > 0                                            # some candidates were re-scored exactly
+    print("lists that fell back to exact scoring:", fast.fallback_lists(), "max |approx - exact| / delta:", ratio)
 
 
 @pytest.mark.parametrize("shape", [
@@ -248,8 +287,8 @@ def test_summary_selector_persistent_form_adversarial_score_order(order):
     print(order, "lists that fell back to exact scoring:", fast.fallback_lists())
 
 
-@pytest.mark.parametrize("r", [1, 4])
-def test_summary_selector_tensor_core_path_near_ties(r):
+@pytest.mark.parametrize("r,nt", [(1, 2112), (4, 64)])       # four descriptors per list: row tiles up to 2048 blocks
+def test_summary_selector_tensor_core_path_near_ties(r, nt):
     """A cluster of almost equal blocks at the top of every list (copies of one block, some
     exact, some with one feature nudged): their approximate scores cannot order them, so the
     pre-filter must re-score exactly these and still agree with the oracle id for id, while
@@ -257,7 +296,7 @@ def test_summary_selector_tensor_core_path_near_ties(r):
     m = sp()
     g = torch.Generator().manual_seed(77)
     q = (torch.randn((1, 4, 160 * 128, 128), generator=g) + 0.5).to(torch.bfloat16)   # 160 lists: not a small problem
-    k = (0.2 * torch.randn((1, 1, 8192, 128), generator=g)).to(torch.bfloat16)
+    k = (0.2 * torch.randn((1, 1, nt * 128, 128), generator=g)).to(torch.bfloat16)
     base = (k[:, :, :128].float() + 1.0).to(torch.bfloat16)
     for blk in range(20):
         k[:, :, blk * 128:(blk + 1) * 128] = base
@@ -269,6 +308,8 @@ def test_summary_selector_tensor_core_path_near_ties(r):
     ref = oracle.summary_select(q, k, r, 32)[3]
     assert torch.equal(ids, ref)
     assert set(ids[0, 0, 0, :20].tolist()) == set(range(20))
+    assert float(sel.aux[:1].view(torch.float32)) > 0     # the key abs-max only the tensor-core path writes
+    assert sel.bound_stats()[0] == 0 and sel.bound_stats()[1] > 0     # candidates were re-scored, inside the bound
     assert sel.fallback_lists() <= 8                 # the near ties are settled by re-scoring, not by the fallback
     print("lists that fell back to exact scoring:", sel.fallback_lists())
 
@@ -281,7 +322,7 @@ def test_summary_selector_tensor_core_path_near_ties(r):
     (1, 4, 4, 256, 1024, 4, 8),
 ])
 def test_small_problem_selector_equals_the_exact_kernels(b, hkv, g, sq, skv, r, topk):
-    """The cluster kernel for small problems (taken by run() and run_fast()) against the
+    """The row-tile kernel for small problems (taken by run() and run_fast()) against the
     staged exact kernels (prepare() + score()): descriptors, scores and ids bit for bit,
     and ids against the CPU oracle."""
     m = sp()

@@ -306,15 +306,15 @@ def test_balanced_last_round_matches_the_plain_call(shape, topk, counts_kind):
 @pytest.mark.parametrize("shape,topk,counts_kind", [
     ((1, 2, 1, 128, 8192), 64, None),          # one pair item: 16 pieces of 4 blocks
     ((1, 3, 1, 384, 2048), 16, None),          # split mode, odd number of query blocks: a stream without a tile
-    ((2, 1, 1, 384, 4096), 16, "ragged"),      # lists of 0 to 16 blocks: empty lists and empty pieces
-    ((1, 4, 2, 2304, 2304), 18, "ragged"),     # 36 items: four pieces
+    ((2, 1, 1, 384, 4096), 16, "ragged"),      # lists of 0 to 16 blocks: with counts the plain launch
+    ((1, 4, 2, 2304, 2304), 18, "ragged"),     # 36 items, the same
     ((1, 8, 1, 2304, 4096), 32, None),         # 72 items: two pieces
     ((1, 8, 1, 2304, 1024), 8, None),          # 72 items, not worth a split: the plain launch
 ])
 @pytest.mark.parametrize("nan", [False, True])
 def test_launch_of_less_than_a_round_matches_the_plain_call(shape, topk, counts_kind, nan):
-    """With a workspace and at most half as many items as SMs, every item is cut into pieces with fp32 partials: same
-    result as the plain call up to the rounding of the bf16 probabilities and outputs, LSE to fp32 rounding, inside the
+    """With a workspace, no counts and at most half as many items as SMs, every item is cut into pieces with fp32
+    partials (which launches are split, and the weights of the pieces, are asserted by the next test): same result as the plain call up to the rounding of the bf16 probabilities and outputs, LSE to fp32 rounding, inside the
     oracle tolerance; rows that are NaN without the split stay NaN."""
     m = sp()
     b, hq, hkv, sq, skv = shape
@@ -348,6 +348,48 @@ def test_launch_of_less_than_a_round_matches_the_plain_call(shape, topk, counts_
     if not nan:
         ref_o, ref_l = oracle.gather_attention(q, k, v, ids, counts)
         check(split, split_lse, ref_o, ref_l)
+
+
+@pytest.mark.parametrize("shape,topk,counts_kind,pieces", [
+    ((1, 2, 1, 128, 8192), 64, None, True),          # one pair item: 16 pieces of 4 blocks
+    ((1, 3, 1, 384, 2048), 16, None, True),          # split mode, odd number of query blocks: a stream without a tile
+    ((1, 4, 2, 2304, 2304), 18, None, True),         # 36 items: four pieces, not all of the same length
+    ((1, 8, 1, 2304, 4096), 32, None, True),         # 72 items: two pieces
+    ((2, 1, 1, 384, 4096), 16, "ragged", False),     # counts, empty lists among them: the plain launch
+    ((1, 8, 1, 2304, 1024), 8, None, False),         # 72 items, not worth a split: the plain launch
+])
+def test_pieces_of_small_launches_have_their_weights(shape, topk, counts_kind, pieces):
+    """Every key block's values have a mean of their own, so that a wrong weight of a piece shows: the error of a tile
+    against the fp32 oracle is that of the plain call. A launch that is not split has the plain call's bits."""
+    m = sp()
+    b, hq, hkv, sq, skv = shape
+    q, k, v = gen.make_qkv(b, hq, hkv, sq, skv, seed=13, k_block_offset=0.5)
+    means = torch.randn((b, hkv, skv // 128, 1, 128), generator=torch.Generator().manual_seed(29)) * 4.0
+    v = (v.float().view(b, hkv, skv // 128, 128, 128) + means).view(b, hkv, skv, 128).to(torch.bfloat16)
+    ids = gen.make_ids(b, hkv, sq // 128, skv // 128, topk, 5, "unsorted")
+    counts = None
+    if counts_kind == "ragged":
+        counts = (torch.arange(b * hkv * (sq // 128)) * 7 % (topk + 1)).to(torch.int32).reshape(b, hkv, sq // 128)
+    qc, kc, vc, ic = q.cuda(), k.cuda(), v.cuda(), ids.cuda()
+    cc = None if counts is None else counts.cuda()
+    plain, split = torch.empty_like(qc), torch.empty_like(qc)
+    m.attention_out(qc, kc, vc, ic, plain, cc, balance=False)
+    m.attention_out(qc, kc, vc, ic, split, cc, balance=True)
+    torch.cuda.synchronize()
+    m.device_status()
+    # every 128-row tile goes through the merge, or none does
+    differs = (split != plain).reshape(b, hq, sq // 128, -1).any(-1)
+    assert torch.equal(differs, torch.full_like(differs, pieces))
+    ref, _ = oracle.gather_attention(q, k, v, ids, counts)
+
+    def rms(x):
+        return x.reshape(b, hq, sq // 128, -1).square().mean(-1).sqrt()
+    plain_err, split_err = rms(plain.float().cpu() - ref), rms(split.float().cpu() - ref)
+    # Both calls round every probability to bf16 once (against different running maxima) and the output once; partials
+    # and weights are fp32. So the errors are of one size, 1.25 for the sampling of a tile's 16384 values; one piece of
+    # 16 left out is 200 times that. The output's rounding is 2^-9 / sqrt(3) of it, the probabilities' about a fifth.
+    assert torch.all(split_err <= 1.25 * plain_err)
+    assert torch.all(plain_err <= 2.0 ** -8 * rms(ref))
 
 
 @pytest.mark.parametrize("shape,topk", [
