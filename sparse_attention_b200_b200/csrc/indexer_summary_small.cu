@@ -56,9 +56,10 @@ __global__ void __launch_bounds__(256) pool_small_kernel(const __nv_bfloat16* __
 // each (MP = group heads x R rounded up to a power of two, padding repeats a list's first descriptor: the maximum is
 // unchanged). A cluster of C CTAs (C = 1, 2, 4 or 8) shares the row tile: CTA `rank` scores the key chunks rank,
 // rank + C, ... of 64 descriptors, and owns the lists l with l % C == rank: every score goes straight into the owner's
-// shared memory. Bound by fp32 FMAs (the exact score is defined by fp32 sums in feature order): QT x 4 register tile per
-// thread, two shared-memory reads of up to 16 bytes per 4 QT FMAs, the next chunk's bytes requested before the arithmetic
-// of this one. QT, L and C are chosen by plan_rows().
+// shared memory. QT x 4 register tile per thread, the next chunk's bytes requested before the arithmetic of this one
+// (the exact score is defined by fp32 sums in feature order). Bound by shared-memory reads: the two of a thread and
+// feature are 8, 6 or 5 wavefronts of a warp (QT = 4, 2, 1), 8192 cycles per chunk at QT = 4 against 4096 of FMAs; 1024
+// lists of 64 x 8192 take 8130 (3790 us). QT, L and C are chosen by plan_rows().
 constexpr int KD = 64;
 constexpr int SCORE_BYTES_MAX = 40 * 1024;
 constexpr size_t SMEM_PER_SM = 228 * 1024;       // of which 1 KiB per CTA is the system's
@@ -233,8 +234,8 @@ __global__ void __launch_bounds__(256) score_rows_kernel(const RowsParams p) {
   // (score descending, id ascending) is a total order: no score is NaN
   if (p.nt <= 256 && ((own * p.nt + 255) >> 8) * p.nt <= 512 * ((own + 7) >> 3)) {
     // Short lists: every score counts the scores that beat it, the count is its rank. The right-hand side is what
-    // the threshold search of a warp below takes in the same unit, scores read by a thread (64 lists of 256: 271 us
-    // by counting, 60 by searching, whole selector; 32 lists of 32: 20 and 25).
+    // the threshold search of a warp below takes in the same unit, scores read by a thread (whole selector, us, with as
+    // many lists in a CTA: 64 lists of 256 271 by counting, 60 by searching; 32 lists of 32 20 and 25).
     for (int e = tid; e < own * p.nt; e += blockDim.x) {
       const int l = e / p.nt, j = e - l * p.nt;
       const float* s = scores + l * p.nt;
@@ -298,7 +299,8 @@ __global__ void __launch_bounds__(256) score_rows_kernel(const RowsParams p) {
   }
   // k > 128: the lists are sorted, as many at a time as fit the tiles' 40 to 64 KiB (bitonic, 64-bit keys of score and
   // inverted id, so that the order is score descending, id ascending; padding sorts last). Rounds of block-wide
-  // arg-max, k per list and list after list, took 1320 us for 64 lists of 512 with k = 256, this 44 (whole selector).
+  // arg-max, k per list and list after list, took 1320 us for 64 lists of 512 with k = 256, this 44 with 64 lists to a
+  // tile and 20 with 14 (whole selector).
   unsigned long long* keys = reinterpret_cast<unsigned long long*>(q_s);
   int p_log2 = 1;
   while ((1 << p_log2) < p.nt) ++p_log2;
@@ -447,8 +449,10 @@ int launch_pool_small_pair(const void* x, void* desc, long long num_desc, const 
   return e == cudaSuccess ? SB_OK : set_error(SB_ERR_CUDA, cudaGetErrorString(e));
 }
 
-// Returns 1 when the problem is not a small one (the caller then takes the other kernels). force: whatever its size
-// (problems the tensor-core forms do not take: this kernel is several times faster than score_topk_kernel).
+// Returns 1 when the problem is not a small one (the caller then takes the other kernels). force: whatever its size, up
+// to 2048 blocks (scores wanted, or problems the tensor-core forms do not take). Against score_topk_kernel, us, that one ->
+// this: 512 lists of 4 x 512 89 -> 69, 2048 of 1 x 2048 420 -> 161, 1024 of 64 x 8192 5370 -> 3790; the worst of 530 random
+// problems 202 of 16 x 342 55 -> 61.
 int launch_summary_small(const void* qd, const void* kd, float* scores, int32_t* ids, int32_t* fallback_counter,
                          int batch, int hq, int hkv, int qt, int nt, int r, int topk, cudaStream_t stream, bool force) {
   DeviceCtx* ctx = device_ctx();
@@ -465,9 +469,9 @@ int launch_summary_small(const void* qd, const void* kd, float* scores, int32_t*
   // Against the tensor-core forms (their selection phase costs about 16 us per round of eight lists whatever the
   // length, a unit of 64 rows x 64 keys here about 5 us of an SM; select_summary with pooling, us, tensor-core form ->
   // this one): below 16 descriptors per list those pack more than a round of lists into one CTA and leave most SMs
-  // idle (256 lists of 1 x 32 blocks 68 -> 20, 512 of 4 x 512 126 -> 58, 2048 of 1 x 256 271 -> 107); from 16 on only
-  // when the lists do not fill the GPU (64 lists of 64 x 512 key rows 42 -> 32, 128 of 16 x 1024 75 -> 61). Beyond four
-  // units per SM the tensor cores win (320 of 16 x 600: 62 against 70; 128 of 64 x 2048: 62 against 164).
+  // idle (256 lists of 1 x 32 blocks 65 -> 10, 512 of 4 x 512 131 -> 68, 2048 of 1 x 256 269 -> 56); from 16 on only
+  // when the lists do not fill the GPU (64 lists of 64 x 512 key rows 42 -> 32, 128 of 16 x 1024 75 -> 67). Beyond four
+  // units per SM the tensor cores win (320 of 16 x 600: 85 against 100; 128 of 64 x 2048: 62 against 167).
   if (!force && !((m < 16 || heads * qt <= ctx->sm_count) && units <= 4LL * ctx->sm_count)) return 1;
   const RowsPlan plan = plan_rows(heads, qt, nt, r, topk, mp_log2, ctx->sm_count);
   RowsParams p{};
