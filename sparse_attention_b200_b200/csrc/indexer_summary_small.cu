@@ -451,8 +451,8 @@ int launch_pool_small_pair(const void* x, void* desc, long long num_desc, const 
 
 // Returns 1 when the problem is not a small one (the caller then takes the other kernels). force: whatever its size, up
 // to 2048 blocks (scores wanted, or problems the tensor-core forms do not take). Against score_topk_kernel, us, that one ->
-// this: 512 lists of 4 x 512 89 -> 69, 2048 of 1 x 2048 420 -> 161, 1024 of 64 x 8192 5370 -> 3790; the worst of 530 random
-// problems 202 of 16 x 342 55 -> 61.
+// this: 512 lists of 4 x 512 89 -> 69, 2048 of 1 x 2048 420 -> 161, 1024 of 64 x 8192 5370 -> 3790; behind it only on
+// problems of a few microseconds (262 of 4 x 136 with k = 1 16.8 -> 21.3, 202 of 16 x 342 55 -> 61 were the worst of 680).
 int launch_summary_small(const void* qd, const void* kd, float* scores, int32_t* ids, int32_t* fallback_counter,
                          int batch, int hq, int hkv, int qt, int nt, int r, int topk, cudaStream_t stream, bool force) {
   DeviceCtx* ctx = device_ctx();
