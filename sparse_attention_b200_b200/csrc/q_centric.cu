@@ -662,8 +662,8 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
 #pragma unroll
         for (int c = 2; c < 4; ++c) tmem_ld32(t_s + c * 32, sv[c]);
         // four independent running maxima, three-input max: 64 instructions per row. Those of the first half run
-        // while the second half is on its way: 1 Mi-token group 34.2 -> 34.05 ms, KV-centric case 33.87 -> 33.71,
-        // but 32-head 32 Ki sequence 1118 -> 1129 us.
+        // while the second half is on its way: within 1.2 % either way (1 Mi-token group 35.26 -> 34.84 ms, 32-head 32 Ki
+        // sequence 1142 -> 1153 us, 16 heads over 16 Ki keys 133.6 -> 134.1, KV-centric case 34.10 -> 34.20 ms).
         float mx[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) mx[j] = -INFINITY;
