@@ -91,6 +91,40 @@ __device__ __forceinline__ bool mbar_wait_limited(uint32_t bar, uint32_t parity,
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const Guard& g, int code) {
   return mbar_wait_limited(bar, parity, g, code, WAIT_LIMIT_CYCLES);
 }
+// The same wait by a whole converged warp, which stays converged: every lane gets the same answer. (One lane that waits
+// and a shuffle of its answer is slower.)
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, const Guard& g, int code) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  const long long t0 = clock64();
+  int spins = 0;
+  while (true) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    if ((++spins & 31) == 0) {
+      const bool late = clock64() - t0 > WAIT_LIMIT_CYCLES;
+      if (__any_sync(0xffffffffu, late || *g.abort_flag)) {
+        if (late) {
+          *g.abort_flag = 1;
+          atomicCAS(g.status, 0, code);
+        }
+        __syncwarp();
+        return false;
+      }
+    }
+  }
+}
+// One lane of a converged warp. tcgen05 instructions of an `if (elect_one())` block take their operands from uniform
+// registers: an MMA issues in 14 cycles, against 54 in a block of `if (lane == 0)`, and up to eight of them queue.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "}"
+      : "=r"(p));
+  return p != 0;
+}
 // Quiet bounded wait used while draining after an abort (ignores the flag).
 __device__ __forceinline__ void mbar_wait_drain(uint32_t bar, uint32_t parity) {
   const long long t0 = clock64();

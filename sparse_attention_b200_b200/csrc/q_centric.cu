@@ -9,9 +9,8 @@
 //     head, each with its own list and its own K/V tiles.
 // Roles (four warpgroups, 512 threads): warps 0-3 softmax of stream 0, warps 4-7
 // softmax of stream 1, warps 8-11 epilogue (read O out of tensor memory, normalise,
-// TMA-store; the softmax warps go straight on to the next item), one thread of warp 12
-// issues tcgen05 MMAs (waits, issue and commits in a single thread keep the
-// P-ready -> MMA-issue latency short), warp 13 issues TMA loads. After the setup
+// TMA-store; the softmax warps go straight on to the next item), warp 12 waits as
+// a whole and its elected lane issues tcgen05 MMAs and commits, warp 13 issues TMA loads. After the setup
 // barrier setmaxnreg moves registers from the last two warpgroups to the softmax warps.
 // K/V tiles selected by block index are gathered by TMA into a ring of 32 KiB
 // shared-memory slots; S = QK^T and O += PV accumulate in tensor memory
@@ -412,8 +411,14 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
     // from here on, not from the start, because its CTAs wait on the SMs that a small launch leaves to other streams.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   } else if (warp == MMA_WARP) {
-    // ------------------------------------------------------------- MMA issuer (one thread)
-    if (lane == 0) {
+    // ------------------------------------------------------------- MMA issuer (elected lane of a converged warp)
+    // Waits by the whole warp, issue and commits by its elected lane: an MMA issues in 14 cycles and up to eight of them
+    // queue, against 54 cycles under `if (lane == 0)`, where the lane itself set the pace (PV + next QK 940 of the 1620
+    // cycles of a stream's half step). Cycles of a (tile, two streams) step 3335 -> 3100 on the 1 Mi-token group (34.3 -> 33.8
+    // ms only: its clock falls as the step gets shorter, the power cap sets the time), 3940 -> 3590 on the 32-head
+    // 32 Ki sequence (1135 -> 1108 us). K is awaited after PV has been issued, not before: with half of the ring per stream in
+    // split mode it often is the last to arrive (4800 cycles).
+    const bool lead = elect_one();
     constexpr uint32_t IDESC_QK = idesc_bf16(TILE, TILE, false);
     constexpr uint32_t IDESC_PV = idesc_bf16(TILE, HEAD_DIM, true);
     uint32_t taken = 0;            // ring tiles consumed so far
@@ -422,29 +427,27 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
     bool ok = true;
     auto acquire = [&](uint32_t& slot) -> bool {
       slot = taken % RING;
-      bool w = mbar_wait(bar(BAR_KV_FULL + slot), (taken / RING) & 1, guard, 0x200 + slot);
+      const bool w = mbar_wait_warp(bar(BAR_KV_FULL + slot), (taken / RING) & 1, guard, 0x200 + slot);
       ++taken;
       tc_fence_after();
       return w;
     };
     auto wait_q = [&](int q) -> bool {
-      bool w = mbar_wait(bar(BAR_Q_FULL + q), qtaken[q] & 1, guard, 0x210 + q);
+      const bool w = mbar_wait_warp(bar(BAR_Q_FULL + q), qtaken[q] & 1, guard, 0x210 + q);
       ++qtaken[q];
       tc_fence_after();
       return w;
     };
     auto wait_p = [&](int q) -> bool {
-      bool w = mbar_wait(bar(BAR_P_FULL + q), pphase[q], guard, 0x220 + q);
+      const bool w = mbar_wait_warp(bar(BAR_P_FULL + q), pphase[q], guard, 0x220 + q);
       pphase[q] ^= 1;
       tc_fence_after();
       return w;
     };
     // S_q = Q_q K^T : 8 MMAs of K = 16 over two 64-column panels.
     auto issue_qk = [&](int q, uint32_t slot) {
-      {
-        // low descriptor words only: the issuing thread shares its scheduler with two softmax warps, so every
-        // instruction between "P is ready" and the MMA counts (64-bit descriptor arithmetic: 16 heads over 16 Ki keys
-        // 125.7 -> 130.6 us, 1 Mi-token group 34.1 -> 35.4 ms, 32-head 32 Ki sequence the same)
+      if (lead) {
+        // low descriptor words only: 64-bit descriptor arithmetic is more instructions on the issuing lane's path
         const uint32_t a0 = (base + OFF_Q + q * TILE_BYTES) >> 4;
         const uint32_t b0 = (base + OFF_RING + slot * TILE_BYTES) >> 4;
         constexpr uint32_t HI = (1024u >> 4) | (1u << 14) | (2u << 29);
@@ -453,11 +456,12 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
           const uint32_t step = (kk >> 2) * (PANEL_BYTES >> 4) + (kk & 3) * 2;
           mma_ss_lo<HI, HI>(tmem + q * TILE, a0 + step, b0 + step, IDESC_QK, kk > 0);
         }
+        tc_commit(bar(BAR_S_FULL + q));
       }
     };
     // O_q (+)= P_q V : A from tensor memory (8 columns per K = 16), B = V MN-major.
     auto issue_pv_part = [&](int q, uint32_t slot, bool accumulate, int k0, int k1) {
-      {
+      if (lead) {
         const uint32_t b0 = ((base + OFF_RING + slot * TILE_BYTES) >> 4) | ((PANEL_BYTES >> 4) << 16);
         constexpr uint32_t HI = (1024u >> 4) | (1u << 14) | (2u << 29);
 #pragma unroll
@@ -474,7 +478,7 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
     uint32_t hphase[2] = {0, 0};
     auto pv = [&](int q, uint32_t slot, bool accumulate) -> bool {
       if (p.pair_mode) {
-        if (!mbar_wait(bar(BAR_P_HALF + q), hphase[q], guard, 0x230 + q)) return false;
+        if (!mbar_wait_warp(bar(BAR_P_HALF + q), hphase[q], guard, 0x230 + q)) return false;
         hphase[q] ^= 1;
         tc_fence_after();
       } else if (!wait_p(q)) {
@@ -482,7 +486,7 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
       }
       if (!accumulate && o_done[q] > 0) {
         // the first PV of an item overwrites O: the previous item's O must have been read out
-        if (!mbar_wait(bar(BAR_O_EMPTY + q), (o_done[q] - 1) & 1, guard, 0x240 + q)) return false;
+        if (!mbar_wait_warp(bar(BAR_O_EMPTY + q), (o_done[q] - 1) & 1, guard, 0x240 + q)) return false;
         tc_fence_after();
       }
       if (p.pair_mode) {
@@ -494,8 +498,8 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
       }
       return true;
     };
-    auto commit_o = [&](int q) { tc_commit(bar(BAR_O_FULL + q)); ++o_done[q]; };
-    auto commit = [&](int b) { tc_commit(bar(b)); };
+    auto commit = [&](int b) { if (lead) tc_commit(bar(b)); };
+    auto commit_o = [&](int q) { commit(BAR_O_FULL + q); ++o_done[q]; };
 
     bool primed[2] = {false, false};
     int cnt[2] = {0, 0}, ncnt[2] = {0, 0};
@@ -513,8 +517,8 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
         if (!was_primed) {
           ok = wait_q(0) && wait_q(1) && acquire(kslot);
           if (!ok) break;
-          issue_qk(0, kslot); commit(BAR_S_FULL + 0);
-          issue_qk(1, kslot); commit(BAR_S_FULL + 1);
+          issue_qk(0, kslot);
+          issue_qk(1, kslot);
           commit(BAR_KV_EMPTY + kslot);
           if (n == 1) { commit(BAR_Q_EMPTY + 0); commit(BAR_Q_EMPTY + 1); }
         }
@@ -526,20 +530,20 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
           if (more) {
             ok = acquire(kslot);
             if (!ok) break;
-            issue_qk(0, kslot); commit(BAR_S_FULL + 0);
+            issue_qk(0, kslot);
           } else {
             commit_o(0);
             if (prime) {              // first QK of the next item, stream 0
               ok = wait_q(0) && acquire(kslot);
               if (!ok) break;
-              issue_qk(0, kslot); commit(BAR_S_FULL + 0);
+              issue_qk(0, kslot);
             }
           }
           ok = pv(1, vslot, i > 0);
           if (!ok) break;
           commit(BAR_KV_EMPTY + vslot);
           if (more) {
-            issue_qk(1, kslot); commit(BAR_S_FULL + 1);
+            issue_qk(1, kslot);
             commit(BAR_KV_EMPTY + kslot);
             if (i + 2 == n) { commit(BAR_Q_EMPTY + 0); commit(BAR_Q_EMPTY + 1); }
           } else {
@@ -547,7 +551,7 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
             if (prime) {              // and stream 1, same K tile
               ok = wait_q(1);
               if (!ok) break;
-              issue_qk(1, kslot); commit(BAR_S_FULL + 1);
+              issue_qk(1, kslot);
               commit(BAR_KV_EMPTY + kslot);
               if (ncnt[0] == 1) { commit(BAR_Q_EMPTY + 0); commit(BAR_Q_EMPTY + 1); }
               primed[0] = primed[1] = true;
@@ -561,7 +565,7 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
           if (cnt[q] > 0 && !was_primed[q]) {
             ok = wait_q(q) && acquire(kslot);
             if (!ok) break;
-            issue_qk(q, kslot); commit(BAR_S_FULL + q);
+            issue_qk(q, kslot);
             commit(BAR_KV_EMPTY + kslot);
             if (cnt[q] == 1) commit(BAR_Q_EMPTY + q);
           }
@@ -575,7 +579,7 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
               if (i + 1 < cnt[q]) {
                 ok = acquire(kslot);
                 if (!ok) break;
-                issue_qk(q, kslot); commit(BAR_S_FULL + q);
+                issue_qk(q, kslot);
                 commit(BAR_KV_EMPTY + kslot);
                 if (i + 2 == cnt[q]) commit(BAR_Q_EMPTY + q);
               } else {
@@ -583,7 +587,7 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
                 if (has_next && ncnt[q] > 0) {     // first QK of this stream's next item
                   ok = wait_q(q) && acquire(kslot);
                   if (!ok) break;
-                  issue_qk(q, kslot); commit(BAR_S_FULL + q);
+                  issue_qk(q, kslot);
                   commit(BAR_KV_EMPTY + kslot);
                   if (ncnt[q] == 1) commit(BAR_Q_EMPTY + q);
                   primed[q] = true;
@@ -591,7 +595,6 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
               }
             }
       }
-    }
     }
     __syncwarp();
   }
