@@ -202,10 +202,12 @@ struct Geometry {
 };
 
 // ---------------------------------------------------------------- producer and MMA roles
-// A page takes about 520 cycles of an SM with two CTAs on it (590 when the scales of page t + 3 were requested before
+// A page takes about 450 cycles of an SM with two CTAs on it (520 when one lane issued under `if (lane == 0)` instead of the
+// elected lane of a converged warp, see elect_one(); 590 when the scales of page t + 3 were requested before
 // the proxy fence of page t, which then waited for them, and when the page maximum took five shuffles), against 128
 // cycles of MMAs: the hand-overs copy -> MMA -> accumulator -> epilogue bound it. One CTA per SM with three
-// accumulators and two to three threads issuing, the scales through tensor-memory stores, was no faster (510 to 840).
+// accumulators and two to three threads issuing, the scales through tensor-memory stores, was no faster (510 to 840); nor are
+// three accumulators of 64 columns in a CTA, now that issuing is cheap (450, and 48 -> 56 us on a ragged prefill batch).
 // Producer warp: query tile once, then key pages page0 + (t + rot) % wrap for t = 0 .. num_tiles - 1 (num_tiles <= wrap,
 // rot < wrap).
 __device__ __forceinline__ void producer_role(const Geometry& g, const CUtensorMap* q_map, const CUtensorMap* k_map,
@@ -270,7 +272,7 @@ __device__ __forceinline__ void producer_role(const Geometry& g, const CUtensorM
       mbar_wait_drain(bar(A_FULL + t % A_STAGES), (t / A_STAGES) & 1);
 }
 
-// MMA thread: page t against the whole query tile into accumulator t % ACC_STAGES. The key scales of
+// MMA warp: page t against the whole query tile into accumulator t % ACC_STAGES. The key scales of
 // page t go to slot t & 1, copied as soon as the page has landed: the slot was last read by the MMAs of
 // page t - 2, which had completed (their accumulator had been read out and released) before the MMAs
 // of page t - 1 were issued; this holds for one or two accumulators.
@@ -279,30 +281,37 @@ __device__ __forceinline__ void mma_role(uint32_t base, uint32_t bar0, uint32_t 
                                          int code0) {
   auto bar = [&](int i) { return bar0 + 8u * i; };
   constexpr uint32_t IDESC = idesc_nvf4(128, 128);
-  if (!mbar_wait(bar(B_FULL), 0, guard, code0)) return;
+  const bool lead = elect_one();
+  if (!mbar_wait_warp(bar(B_FULL), 0, guard, code0)) return;
   tc_fence_after();
-  tmem_cp_scales(tmem + TM_SFB, desc_scale_chunk(base + OFF_B + CODE_BYTES));
-  tmem_cp_scales(tmem + TM_SFB + 4, desc_scale_chunk(base + OFF_B + CODE_BYTES + 512));
+  if (lead) {
+    tmem_cp_scales(tmem + TM_SFB, desc_scale_chunk(base + OFF_B + CODE_BYTES));
+    tmem_cp_scales(tmem + TM_SFB + 4, desc_scale_chunk(base + OFF_B + CODE_BYTES + 512));
+  }
   const uint64_t b0 = desc_sw64_kmajor(base + OFF_B);
   for (int t = 0; t < num_tiles; ++t) {
     const int s = t % A_STAGES, st = t % ACC_STAGES;
-    if (!mbar_wait(bar(A_FULL + s), (t / A_STAGES) & 1, guard, code0 + 1 + s)) return;
+    if (!mbar_wait_warp(bar(A_FULL + s), (t / A_STAGES) & 1, guard, code0 + 1 + s)) return;
     tc_fence_after();
     // the scale copy does not touch the accumulator: it goes out before the accumulator hand-over is awaited
     const uint64_t a0 = desc_sw64_kmajor(base + OFF_A + s * STAGE_BYTES);
     const uint32_t sfa = tmem + TM_SFA + (t & 1) * 8;
-    tmem_cp_scales(sfa, desc_scale_chunk(base + OFF_A + s * STAGE_BYTES + CODE_BYTES));
-    tmem_cp_scales(sfa + 4, desc_scale_chunk(base + OFF_A + s * STAGE_BYTES + CODE_BYTES + 512));
+    if (lead) {
+      tmem_cp_scales(sfa, desc_scale_chunk(base + OFF_A + s * STAGE_BYTES + CODE_BYTES));
+      tmem_cp_scales(sfa + 4, desc_scale_chunk(base + OFF_A + s * STAGE_BYTES + CODE_BYTES + 512));
+    }
     if (t >= ACC_STAGES) {
-      if (!mbar_wait(bar(ACC_EMPTY + st), ((t / ACC_STAGES) - 1) & 1, guard, code0 + 8 + st)) return;
+      if (!mbar_wait_warp(bar(ACC_EMPTY + st), ((t / ACC_STAGES) - 1) & 1, guard, code0 + 8 + st)) return;
       tc_fence_after();
     }
-    // second K = 64: 32 bytes further along every row, its scales in the next four columns
+    if (lead) {
+      // second K = 64: 32 bytes further along every row, its scales in the next four columns
 #pragma unroll
-    for (int kh = 0; kh < 2; ++kh)
-      mma_nvf4(tmem + TM_ACC + st * 128, a0 + kh * 2, b0 + kh * 2, IDESC, sfa + kh * 4, tmem + TM_SFB + kh * 4, kh);
-    tc_commit(bar(ACC_FULL + st));
-    tc_commit(bar(A_EMPTY + s));
+      for (int kh = 0; kh < 2; ++kh)
+        mma_nvf4(tmem + TM_ACC + st * 128, a0 + kh * 2, b0 + kh * 2, IDESC, sfa + kh * 4, tmem + TM_SFB + kh * 4, kh);
+      tc_commit(bar(ACC_FULL + st));
+      tc_commit(bar(A_EMPTY + s));
+    }
   }
 }
 
@@ -355,7 +364,7 @@ struct Params {
 // overlaps the tensor-core scoring of the other): approximate tile scores of every key
 // page on the tensor cores, then candidate selection and exact re-scoring.
 // Warps 0-7 epilogue (lane quarter = warp & 3, query half = warp >> 2), warp 8 producer,
-// warp 9 MMA issue (one thread).
+// warp 9 MMA issue (its elected lane).
 __global__ void __launch_bounds__(NUM_THREADS, 2)
 fp4_nv_select_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map, const Params p) {
   extern __shared__ unsigned char smem_raw[];
@@ -410,7 +419,7 @@ fp4_nv_select_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
     producer_role(g, &q_map, &k_map, base, gbase, bar0, guard, b, h, hk_idx, q_row0, 0, num_tiles, rot, num_tiles, lane,
                   0x500, nullptr);
   } else if (warp == MMA_WARP) {
-    if (lane == 0) mma_role(base, bar0, tmem, guard, num_tiles, 0x510);
+    mma_role(base, bar0, tmem, guard, num_tiles, 0x510);
     __syncwarp();
   } else {
     // epilogue: thread = key row of the page, this warp's 64-query half of the tile
@@ -744,7 +753,7 @@ fp4_nv_prune_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
     producer_role(g, &q_map, &k_map, base, gbase, bar0, guard, b, h, hk_idx, q_row0, page0, num_tiles, 0, num_tiles, lane,
                   0x580, nullptr);
   } else if (warp == MMA_WARP) {
-    if (lane == 0) mma_role(base, bar0, tmem, guard, num_tiles, 0x590);
+    mma_role(base, bar0, tmem, guard, num_tiles, 0x590);
     __syncwarp();
   } else {
     // epilogue: thread = key row of the page, this warp's 64-query half of the tile
@@ -1077,30 +1086,35 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
       for (int t = max(0, num_tiles - A_STAGES); t < num_tiles; ++t)
         mbar_wait_drain(bar_(A_FULL + t % A_STAGES), (t / A_STAGES) & 1);
   } else if (warp == 5) {
-    // ----------------------------------------------------------- MMA issue (one thread)
-    if (lane == 0) {
-      constexpr uint32_t IDESC = idesc_nvf4(128, 128);
-      bool ok = mbar_wait(bar(B_FULL), 0, guard, 0x610);
-      if (ok) {
-        tc_fence_after();
-        const uint32_t sfq = tmem + TM_SFB;          // query scales: the A operand here
+    // ----------------------------------------------------------- MMA issue (elected lane of a converged warp)
+    constexpr uint32_t IDESC = idesc_nvf4(128, 128);
+    const bool lead = elect_one();
+    bool ok = mbar_wait_warp(bar(B_FULL), 0, guard, 0x610);
+    if (ok) {
+      tc_fence_after();
+      const uint32_t sfq = tmem + TM_SFB;          // query scales: the A operand here
+      if (lead) {
         tmem_cp_scales(sfq, desc_scale_chunk(base + OFF_B + CODE_BYTES));
         tmem_cp_scales(sfq + 4, desc_scale_chunk(base + OFF_B + CODE_BYTES + 512));
-        const uint64_t a0 = desc_sw64_kmajor(base + OFF_B);
-        for (int t = 0; ok && t < num_tiles; ++t) {
-          const int s = t % A_STAGES;
-          ok = mbar_wait(bar(A_FULL + s), (t / A_STAGES) & 1, guard, 0x611 + s);
-          if (!ok) break;
-          tc_fence_after();
-          const uint64_t b0 = desc_sw64_kmajor(base + OFF_A + s * STAGE_BYTES);
-          const uint32_t sfk = tmem + TM_SFA + (t & 1) * 8;
+      }
+      const uint64_t a0 = desc_sw64_kmajor(base + OFF_B);
+      for (int t = 0; t < num_tiles; ++t) {
+        const int s = t % A_STAGES;
+        ok = mbar_wait_warp(bar(A_FULL + s), (t / A_STAGES) & 1, guard, 0x611 + s);
+        if (!ok) break;
+        tc_fence_after();
+        const uint64_t b0 = desc_sw64_kmajor(base + OFF_A + s * STAGE_BYTES);
+        const uint32_t sfk = tmem + TM_SFA + (t & 1) * 8;
+        if (lead) {
           tmem_cp_scales(sfk, desc_scale_chunk(base + OFF_A + s * STAGE_BYTES + CODE_BYTES));
           tmem_cp_scales(sfk + 4, desc_scale_chunk(base + OFF_A + s * STAGE_BYTES + CODE_BYTES + 512));
-          if (t >= 1) {
-            ok = mbar_wait(bar(ACC_EMPTY), (t - 1) & 1, guard, 0x618);
-            if (!ok) break;
-            tc_fence_after();
-          }
+        }
+        if (t >= 1) {
+          ok = mbar_wait_warp(bar(ACC_EMPTY), (t - 1) & 1, guard, 0x618);
+          if (!ok) break;
+          tc_fence_after();
+        }
+        if (lead) {
 #pragma unroll
           for (int kh = 0; kh < 2; ++kh)
             mma_nvf4(tmem + TM_ACC, a0 + kh * 2, b0 + kh * 2, IDESC, sfq + kh * 4, sfk + kh * 4, kh);
