@@ -118,11 +118,19 @@ int sparse_b200_split_kv_segments(const int32_t* block_idx, const int32_t* block
                                   int32_t* seg_block_count, int32_t* error_word, int batch, int hkv, int q_blocks,
                                   int topk, int kv_blocks, int nseg, void* stream);
 
+/* Main and merge of a KV-centric operator with a single KV range in one launch: its bf16 partial is the output. Lists
+ * as sparse_b200_split_kv_segments writes them for nseg = 1. A row without any weight (an empty list, or only scores of
+ * -inf) is 0 with LSE -inf, as sparse_b200_combine leaves it. lse may be NULL. */
+int sparse_b200_kv_centric_single(const void* q, const void* k, const void* v, const int32_t* seg_block_idx,
+                                  const int32_t* seg_block_count, void* out, float* lse, int batch, int hq, int hkv,
+                                  int sq, int skv, int topk, void* stream);
+
 /* Whole KV-centric operator = metadata + main + combine on one stream, the
  * sequence of Prepared.run() (attention/kv_centric/optimization_round11/api11.py:85-92).
  * KV ranges are processed outer; each (query block, KV range) yields one partial
  * (O, LSE), merged per query. `workspace` (device, 256-byte aligned) must hold
- * sparse_b200_kv_centric_workspace_bytes(...) bytes; nothing is allocated. */
+ * sparse_b200_kv_centric_workspace_bytes(...) bytes; nothing is allocated. With nseg = 1 and bf16 partials the single
+ * partial goes straight to out. */
 int64_t sparse_b200_kv_centric_workspace_bytes(int batch, int hq, int hkv, int sq, int topk, int nseg,
                                                int partial_is_f32);
 int sparse_b200_kv_centric(const void* q, const void* k, const void* v, const int32_t* block_idx,

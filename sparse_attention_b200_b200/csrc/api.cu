@@ -187,6 +187,17 @@ int sparse_b200_q_centric_partial(const void* q, const void* k, const void* v, c
   return launch_q_centric(a, static_cast<cudaStream_t>(stream));
 }
 
+int sparse_b200_kv_centric_single(const void* q, const void* k, const void* v, const int32_t* seg_block_idx,
+                                  const int32_t* seg_block_count, void* out, float* lse, int batch, int hq, int hkv,
+                                  int sq, int skv, int topk, void* stream) {
+  int rc = check_attention(q, k, v, seg_block_idx, out, batch, hq, hkv, sq, skv, topk, 1);
+  if (rc) return rc;
+  REQUIRE(seg_block_count, "segment counts are required");
+  QCentricArgs a{q, k, v, seg_block_idx, seg_block_count, out, lse, batch, hq, hkv, sq, skv, topk, 1, 0};
+  a.dead_zero = true;
+  return launch_q_centric(a, static_cast<cudaStream_t>(stream));
+}
+
 int sparse_b200_combine(const void* partial, int partial_is_f32, const float* partial_lse, void* out, float* out_lse,
                         int64_t rows, int ranks, int rank_major, void* stream) {
   REQUIRE(partial && partial_lse && out, "partial, partial_lse and out must be non-null device pointers");
@@ -250,6 +261,8 @@ int sparse_b200_kv_centric(const void* q, const void* k, const void* v, const in
   rc = launch_split_segments(block_idx, block_count, seg_ids, seg_counts, err, static_cast<long long>(lists), topk,
                              skv / 128, nseg, st);
   if (rc) return rc;
+  if (nseg == 1 && !partial_is_f32)      // one bf16 partial is the output
+    return sparse_b200_kv_centric_single(q, k, v, seg_ids, seg_counts, out, lse, batch, hq, hkv, sq, skv, topk, stream);
   QCentricArgs a{q, k, v, seg_ids, seg_counts, partial, plse, batch, hq, hkv, sq, skv, topk, nseg,
                  partial_is_f32 ? 1 : 0};
   rc = launch_q_centric(a, st);

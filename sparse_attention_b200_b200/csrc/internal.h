@@ -43,6 +43,7 @@ struct QCentricArgs {
   int owners = 1;
   void* const* owner_out = nullptr;
   float* const* owner_lse = nullptr;
+  bool dead_zero = false;       // bf16: a row without any weight is 0 with LSE -inf, as the merge of partials leaves it (not NaN)
 };
 int launch_q_centric(const QCentricArgs& a, cudaStream_t stream);
 // scratch that a launch with these sizes splits its lists into (0: it does not)

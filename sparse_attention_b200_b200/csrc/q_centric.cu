@@ -93,6 +93,7 @@ struct Params {
   // num_virtual = items as the roles see them; without balancing tail_first = num_virtual = num_items.
   int tail_first, tail_parts, num_virtual;
   float* tail_lse;         // [pieces * 2 * 128]
+  int dead_zero;           // rows without any weight are 0 (see QCentricArgs)
 };
 
 struct Stream {
@@ -751,7 +752,7 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
       }
       __syncwarp();
       if (lane == 0) *handed_ptr = handed + 1;
-      stats[q * TILE + row_in_tile] = 1.0f / row_sum;
+      stats[q * TILE + row_in_tile] = p.dead_zero && row_sum == 0.f ? 0.f : 1.0f / row_sum;
       if constexpr (SCATTER) {
         long long tile_row = s[q].out_row;
         const int slice = slice_of(sc, tile_row);
@@ -834,11 +835,16 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
             }
           }
         } else {
+          const bool dead = p.dead_zero && inv == 0.f;
 #pragma unroll
           for (int cc = 0; cc < 4; ++cc) {
             uint32_t ov[32];
             tmem_ld32(t_o + cc * 32, ov);
             tc_wait_ld();
+            if (dead) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) ov[j] = 0u;
+            }
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               const uint4 val = make_uint4(
@@ -1044,6 +1050,7 @@ int launch_q_centric(const QCentricArgs& a, cudaStream_t stream) {
   p.items_per_seg = segment_items(a.batch, a.hq, a.hkv, p.qt);
   p.num_items = p.items_per_seg * a.nseg;
   p.scale_log2 = 1.4426950408889634f / sqrtf(static_cast<float>(HEAD_DIM));
+  p.dead_zero = a.dead_zero ? 1 : 0;
   int grid = p.num_items < ctx->sm_count ? p.num_items : ctx->sm_count;
 
   // single-segment bf16 launches with a workspace that the pieces fit

@@ -199,3 +199,48 @@ def test_many_items_per_cta_with_short_segment_lists(hq, hkv, partial):
     m.device_status()
     assert (o2.float() - out.float()).abs().max().item() <= 2e-2
     assert torch.all((l2 - lse).abs() <= 1e-3 * lse.abs().clamp_min(1.0))
+
+
+@pytest.mark.parametrize("b,hkv,g,qb,nb,topk,with_counts,nseg", [
+    (2, 2, 4, 40, 12, 8, False, 1),       # more than a round of items: one range, straight to the output
+    (1, 3, 3, 51, 9, 5, True, 1),         # odd group, odd tile count, ragged and empty lists
+    (1, 1, 2, 1, 64, 32, False, 4),       # one item: ranges fill the chip
+    (1, 2, 1, 3, 2, 1, False, 1),         # fewer blocks than ranges
+])
+def test_default_ranges(b, hkv, g, qb, nb, topk, with_counts, nseg):
+    """The operator without a number of ranges: its choice, its result against the oracle and against two ranges, every
+    partial slot written; rows whose scores are all -inf are 0 with LSE -inf however many ranges there are."""
+    m = sp()
+    q, k, v = gen.make_qkv(b, hkv * g, hkv, qb * 128, nb * 128, seed=7 * qb + g)
+    ids = gen.make_ids(b, hkv, qb, nb, topk, 3 + qb, "unsorted")
+    counts = torch.randint(0, topk + 1, (b, hkv, qb), generator=torch.Generator().manual_seed(5)).int() if with_counts else None
+    dev = [None if t is None else t.cuda() for t in (q, k, v, ids, counts)]
+    p = m.Prepared(*dev)
+    assert p.nseg == nseg
+    p.poison()
+    out, lse = p.run()
+    two = m.Prepared(*dev, nseg=min(2, nb), partial="f32")
+    out2, lse2 = two.run()
+    torch.cuda.synchronize()
+    m.device_status()
+    p.audit()
+    assert torch.isfinite(out.float()).all() and torch.isfinite(p.partial.float()).all() and not torch.isnan(p.lses).any()
+    torch.testing.assert_close(out.float(), out2.float(), atol=0.02, rtol=0.02)
+    torch.testing.assert_close(lse, lse2, atol=0.002, rtol=0.0002)
+    if counts is None:
+        close(out, lse, *oracle.gather_attention(q, k, v, ids))
+    else:
+        empty = (counts == 0).repeat_interleave(g, 1).repeat_interleave(128, 2)
+        assert empty.any() and (out.cpu()[empty] == 0).all() and torch.isinf(lse.cpu()[empty]).all()
+    one, _ = m.kv_centric_attention(*dev)
+    assert torch.equal(one.view(torch.int16), out.view(torch.int16))
+    if nseg == 1:                          # the stages by hand leave the same
+        want = lse.clone()
+        p.poison()
+        p.metadata(), p.main(), p.combine()
+        assert torch.equal(one.view(torch.int16), p.out.view(torch.int16)) and torch.equal(p.out_lse, want)
+    q[..., 0], k[..., 0] = 1, float("-inf")
+    for n in (None, min(2, nb)):
+        dead = m.Prepared(q.cuda(), k.cuda(), dev[2], dev[3], dev[4], nseg=n)
+        out, lse = dead.run()
+        assert (out == 0).all() and (lse == float("-inf")).all()
