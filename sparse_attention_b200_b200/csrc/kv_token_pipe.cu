@@ -10,7 +10,7 @@
 //                G heads} of Q per 64-column panel, straight into the 128-byte-swizzled
 //                operand tile of a four-slot ring (Q rows mostly come from HBM: four
 //                tasks of loads in flight cover that latency)
-//   warp 12      one thread issues QK(j), then PV(j-1) of the other stream (tcgen05, TMEM)
+//   warp 12      its elected lane issues QK(j), then PV(j-1) of the other stream (tcgen05, TMEM)
 //   warps 0-3 / 4-7   softmax of stream 0 / 1 over the single block, P (bf16) back into S,
 //                1/row-sum to shared memory, LSE to global memory
 //   warps 8-11   epilogue: O out of tensor memory, normalise, stage, and one 4-D TMA store
@@ -19,6 +19,9 @@
 // Same computation as kv_tma11_ops::main_kernel
 // (attention/kv_centric/optimization_round11/tma11_kernel.cu:97-390) for any TopK, with q
 // head-major [B,Hq,Sq,128], partials [B,Hq,Sq,TopK,128] bf16 and LSE [B,Hq,Sq,TopK].
+// Bound by the issue of its lone warps and by the writes of the partials: eight 4 Ki sequences of 16 heads, 32 blocks, 16
+// of them per token, 895 -> 718 us (2.1 GB of partials: 330 us at the copy rate) since task records and ids are fetched
+// ahead (895 -> 755), found by counters instead of divisions, and MMAs issued by an elected lane (755 -> 718).
 // Rows of a tile beyond the task's query count keep whatever the buffer held: every row
 // of S, P and O depends on its own Q row only, and those rows are never stored.
 #include <algorithm>
@@ -34,10 +37,11 @@ constexpr int NUM_THREADS = 512;
 constexpr int EPI_WARP0 = 8;
 constexpr int MMA_WARP = 12;
 constexpr int LOAD_WARP = 13;
-// register budgets per thread after the setup barrier: 128 * (2 * 176 + 64 + 96) = 65536
-constexpr int SOFTMAX_REGS = 176;
+// register budgets per thread after the setup barrier: 128 * (2 * 192 + 64 + 64) = 65536 (176 for the softmax warps
+// leave them 25 spilled words: main stage of eight 4 Ki sequences 718 -> 985 us)
+constexpr int SOFTMAX_REGS = 192;
 constexpr int EPI_REGS = 64;
-constexpr int CTRL_REGS = 96;
+constexpr int CTRL_REGS = 64;
 
 constexpr int QRING = 4;
 constexpr int OFF_Q = 0;                               // [QRING] Q tiles
@@ -77,10 +81,27 @@ struct Params {
 // K/V reload per CTA and segment.
 struct Walk {
   int total, seg, per, count;   // tasks, tasks per segment, tasks per CTA and segment, slots to visit
-  __device__ __forceinline__ int task(int i) const {      // -1: nothing in this slot
-    const int ph = i / per, j = static_cast<int>(blockIdx.x) * per + (i - ph * per);
-    const long long t = static_cast<long long>(ph) * seg + j;
-    return (j < seg && t < total) ? static_cast<int>(t) : -1;
+};
+
+// A role's place in the walk: task records are fetched slot by slot. (Counters: with the slot's segment and place found by
+// division, every role spent a thousand cycles per task on index arithmetic, a lone warp issuing it.)
+struct Cursor {
+  int left, at, first, base;    // slots left, slot within the segment's share, share's first task, segment's first task
+  __device__ __forceinline__ explicit Cursor(const Walk& w)
+      : left(w.count), at(0), first(static_cast<int>(blockIdx.x) * w.per), base(0) {}
+  // record of the next slot's task; count 0 where the slot is empty or the walk is over
+  __device__ __forceinline__ int4 fetch(const int32_t* tasks, const Walk& w) {
+    int4 raw = make_int4(0, 0, 0, 0);
+    if (left > 0) {
+      --left;
+      const int j = first + at;
+      if (j < w.seg && base + j < w.total) raw = __ldg(reinterpret_cast<const int4*>(tasks) + base + j);
+      if (++at == w.per) {
+        at = 0;
+        base += w.seg;
+      }
+    }
+    return raw;
   }
 };
 
@@ -89,15 +110,19 @@ struct Task {
   bool valid;
 };
 
-__device__ __forceinline__ Task read_task(const Params& p, const Walk& walk, int i) {
-  const int t = i < walk.count ? walk.task(i) : -1;
-  if (t < 0) return Task{0, 0, 0, 0, false};
-  const int4 raw = *reinterpret_cast<const int4*>(p.tasks + static_cast<long long>(t) * 4);
+// Task records are fetched two tasks, query ids and ranks one task before their use, and only looked at then: a record and
+// the ids it points to are two dependent trips to memory, which every role had waited for in every task.
+__device__ __forceinline__ Task decode_task(const Params& p, const int4& raw) {
   Task k;
   k.group = raw.x; k.block = raw.y; k.start = raw.z; k.count = raw.w;
   k.valid = k.group >= 0 && k.group < p.batch * p.hkv && k.block >= 0 && k.block < p.skv / 128 && k.start >= 0 &&
             k.count > 0 && k.count <= (128 >> p.group_log2) && static_cast<long long>(k.start) + k.count <= p.edges;
   return k;
+}
+
+// query id (and rank) of query `tl` of a task, as they are in memory; the caller checks them
+__device__ __forceinline__ int fetch_id(const int32_t* ids, const Task& k, int tl) {
+  return k.valid && tl < k.count ? __ldg(ids + k.start + tl) : -1;
 }
 
 // 3-D tile load {x, y, z}
@@ -184,28 +209,24 @@ kv_token_pipe_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
     uint32_t n = 0;                 // valid tasks so far
     int loads = 0;                  // K/V block loads so far
     int cur_group = -1, cur_block = -1;
+    int b = 0, kvh = 0;             // batch and KV head of cur_group
     bool ok = true;
-    // the query ids of a task are fetched one task ahead
-    auto fetch_qi = [&](const Task& k) -> int {
-      int qi = -1;
-      if (k.valid && lane < k.count) {
-        qi = p.qids[k.start + lane];
-        if (qi < 0 || qi >= p.sq) qi = -1;
-      }
-      return qi;
-    };
-    Task k = read_task(p, walk, t_begin);
-    int qi = fetch_qi(k);
+    Cursor cursor(walk);
+    Task k = decode_task(p, cursor.fetch(p.tasks, walk));
+    int4 raw = cursor.fetch(p.tasks, walk);
+    int qi = fetch_id(p.qids, k, lane);
     for (int t = t_begin; ok && t < t_end; ++t) {
       const Task cur = k;
-      const int cur_qi = qi;
-      k = read_task(p, walk, t + 1);
-      qi = fetch_qi(k);
+      const int cur_qi = qi >= 0 && qi < p.sq ? qi : -1;
+      k = decode_task(p, raw);
+      raw = cursor.fetch(p.tasks, walk);
+      qi = fetch_id(p.qids, k, lane);
       if (!cur.valid) continue;
       const uint32_t slot = n % QRING, use = n / QRING;
       ++n;
       if (cur.group != cur_group || cur.block != cur_block) {
         cur_group = cur.group; cur_block = cur.block;
+        b = cur.group / p.hkv; kvh = cur.group - b * p.hkv;
         if (loads > 0) {
           bool w = mbar_wait(bar(KV_EMPTY), (loads - 1) & 1, guard, 0x700);
           ok = __all_sync(0xffffffffu, w);
@@ -231,7 +252,6 @@ kv_token_pipe_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
       if (lane == 0) mbar_expect_tx(bar(Q_FULL + slot), static_cast<uint32_t>(__popc(live)) * G * 256u);
       __syncwarp();
       if (cur_qi >= 0) {
-        const int b = cur.group / p.hkv, kvh = cur.group - b * p.hkv;
         const uint32_t dst = base + OFF_Q + slot * TILE_BYTES + lane * G * 128;
         // head-major q: {column, token, batch * Hq + head}; token-major q: {column, head, batch * Sq + token}
         const int y = p.q_token_major ? kvh * G : cur_qi;
@@ -247,8 +267,9 @@ kv_token_pipe_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
       if (loads > 0) mbar_wait_drain(bar(KV_FULL), (loads - 1) & 1);
     }
   } else if (warp == MMA_WARP) {
-    // ------------------------------------------------------------- MMA issuer (one thread)
-    if (lane == 0) {
+    // ------------------------------------------------------------- MMA issuer (elected lane of a converged warp)
+    {
+      const bool lead = elect_one();
       constexpr uint32_t IDESC_QK = idesc_bf16(128, 128, false);
       constexpr uint32_t IDESC_PV = idesc_bf16(128, 128, true);
       uint32_t n = 0;
@@ -258,21 +279,25 @@ kv_token_pipe_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
       // O_{s} = P_{s} V of the task numbered m (stream m & 1)
       auto issue_pv = [&](uint32_t m) -> bool {
         const uint32_t s = m & 1, u = m >> 1;
-        if (!mbar_wait(bar(P_FULL + s), u & 1, guard, 0x720 + s)) return false;
-        if (u > 0 && !mbar_wait(bar(O_EMPTY + s), (u - 1) & 1, guard, 0x730 + s)) return false;
+        if (!mbar_wait_warp(bar(P_FULL + s), u & 1, guard, 0x720 + s)) return false;
+        if (u > 0 && !mbar_wait_warp(bar(O_EMPTY + s), (u - 1) & 1, guard, 0x730 + s)) return false;
         tc_fence_after();
-        const uint64_t b0 = desc_sw128_mnmajor(base + OFF_KV + TILE_BYTES, PANEL_BYTES, 1024);
+        if (lead) {
+          constexpr uint32_t HI = (1024u >> 4) | (1u << 14) | (2u << 29);
+          const uint32_t b0 = ((base + OFF_KV + TILE_BYTES) >> 4) | ((PANEL_BYTES >> 4) << 16);
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          mma_ts(tmem + 256 + s * 128, tmem + s * 128 + kk * 8, b0 + static_cast<uint64_t>(kk * (2048 >> 4)),
-                 IDESC_PV, kk > 0 ? 1u : 0u);
-        tc_commit(bar(O_FULL + s));
+          for (int kk = 0; kk < 8; ++kk)
+            mma_ts_lo<HI>(tmem + 256 + s * 128, tmem + s * 128 + kk * 8, b0 + kk * (2048 >> 4), IDESC_PV, kk > 0 ? 1u : 0u);
+          tc_commit(bar(O_FULL + s));
+        }
         return true;
       };
-      Task k = read_task(p, walk, t_begin);
+      Cursor cursor(walk);
+      int4 raw = cursor.fetch(p.tasks, walk), raw2 = cursor.fetch(p.tasks, walk);
       for (int t = t_begin; ok && t < t_end; ++t) {
-        const Task cur = k;
-        k = read_task(p, walk, t + 1);                        // fetched one task ahead of its use
+        const Task cur = decode_task(p, raw);
+        raw = raw2;
+        raw2 = cursor.fetch(p.tasks, walk);
         if (!cur.valid) continue;
         const uint32_t s = n & 1, slot = n % QRING, use = n / QRING;
         if (cur.group != cur_group || cur.block != cur_block) {
@@ -283,25 +308,25 @@ kv_token_pipe_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
             pv_pending = false;
             if (!ok) break;
           }
-          if (loads > 0) tc_commit(bar(KV_EMPTY));
-          ok = mbar_wait(bar(KV_FULL), loads & 1, guard, 0x740);
+          if (loads > 0 && lead) tc_commit(bar(KV_EMPTY));
+          ok = mbar_wait_warp(bar(KV_FULL), loads & 1, guard, 0x740);
           ++loads;
           if (!ok) break;
         }
-        ok = mbar_wait(bar(Q_FULL + slot), use & 1, guard, 0x750 + slot);
+        ok = mbar_wait_warp(bar(Q_FULL + slot), use & 1, guard, 0x750 + slot);
         if (!ok) break;
         tc_fence_after();
-        {
-          const uint64_t a0 = desc_sw128_kmajor(base + OFF_Q + slot * TILE_BYTES);
-          const uint64_t b0 = desc_sw128_kmajor(base + OFF_KV);
+        if (lead) {
+          constexpr uint32_t HI = (1024u >> 4) | (1u << 14) | (2u << 29);
+          const uint32_t a0 = (base + OFF_Q + slot * TILE_BYTES) >> 4, b0 = (base + OFF_KV) >> 4;
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk) {
-            const uint64_t step = static_cast<uint64_t>((kk >> 2) * (PANEL_BYTES >> 4) + (kk & 3) * 2);
-            mma_ss(tmem + s * 128, a0 + step, b0 + step, IDESC_QK, kk > 0);
+            const uint32_t step = (kk >> 2) * (PANEL_BYTES >> 4) + (kk & 3) * 2;
+            mma_ss_lo<HI, HI>(tmem + s * 128, a0 + step, b0 + step, IDESC_QK, kk > 0);
           }
+          tc_commit(bar(S_FULL + s));
+          tc_commit(bar(Q_EMPTY + slot));
         }
-        tc_commit(bar(S_FULL + s));
-        tc_commit(bar(Q_EMPTY + slot));
         if (pv_pending) {
           ok = issue_pv(n - 1);
           if (!ok) break;
@@ -322,23 +347,31 @@ kv_token_pipe_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
     const uint32_t t_s = tmem + lane_base + s * 128;
     uint32_t n = 0;
     bool ok = true;
+    const int tl = row >> p.group_log2, g = row & (G - 1);
+    int group = -1, head_row = 0;                             // this row's (batch, head) in group `group`
+    Cursor cursor(walk);
+    Task next = decode_task(p, cursor.fetch(p.tasks, walk));
+    int4 raw = cursor.fetch(p.tasks, walk);
+    int qi = fetch_id(p.qids, next, tl), rank = fetch_id(p.ranks, next, tl);
     for (int t = t_begin; ok && t < t_end; ++t) {
-      const Task k = read_task(p, walk, t);
+      const Task k = next;
+      const int cur_qi = qi, cur_rank = rank;
+      next = decode_task(p, raw);
+      raw = cursor.fetch(p.tasks, walk);
+      qi = fetch_id(p.qids, next, tl);
+      rank = fetch_id(p.ranks, next, tl);
       if (!k.valid) continue;
       const uint32_t mine = (n & 1) == s, u = n >> 1;
       ++n;
       if (!mine) continue;
-      // where this row's LSE goes (fetched before the scores are ready)
-      long long lse_at = -1;
-      {
-        const int tl = row >> p.group_log2, g = row & (G - 1);
-        if (tl < k.count) {
-          const int qi = p.qids[k.start + tl], rank = p.ranks[k.start + tl];
-          if (qi >= 0 && qi < p.sq && rank >= 0 && rank < p.topk) {
-            const int b = k.group / p.hkv, kvh = k.group - b * p.hkv;
-            lse_at = ((static_cast<long long>(b) * p.hq + kvh * G + g) * p.sq + qi) * p.topk + rank;
-          }
+      long long lse_at = -1;                                  // where this row's LSE goes
+      if (cur_qi >= 0 && cur_qi < p.sq && cur_rank >= 0 && cur_rank < p.topk) {
+        if (k.group != group) {
+          group = k.group;
+          const int b = group / p.hkv;
+          head_row = b * p.hq + (group - b * p.hkv) * G + g;
         }
+        lse_at = (static_cast<long long>(head_row) * p.sq + cur_qi) * p.topk + cur_rank;
       }
       bool w = mbar_wait(bar(S_FULL + s), u & 1, guard, 0x760 + s);
       ok = __all_sync(0xffffffffu, w);
@@ -396,20 +429,28 @@ kv_token_pipe_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
     const int per_warp = 32 >> p.group_log2;       // queries whose heads this warp holds
     uint32_t n = 0;
     bool ok = true;
+    // lane l < per_warp owns query quarter * per_warp + l of the task
+    const int tl = lane < per_warp ? quarter * per_warp + lane : 128;
+    int group = -1, b = 0, kvh = 0;                           // batch and KV head of group `group`
+    Cursor cursor(walk);
+    Task next = decode_task(p, cursor.fetch(p.tasks, walk));
+    int4 raw = cursor.fetch(p.tasks, walk);
+    int qi_next = fetch_id(p.qids, next, tl), rank_next = fetch_id(p.ranks, next, tl);
     for (int t = t_begin; ok && t < t_end; ++t) {
-      const Task k = read_task(p, walk, t);
+      const Task k = next;
+      int qi = qi_next, rank = rank_next;
+      next = decode_task(p, raw);
+      raw = cursor.fetch(p.tasks, walk);
+      qi_next = fetch_id(p.qids, next, tl);
+      rank_next = fetch_id(p.ranks, next, tl);
       if (!k.valid) continue;
       const uint32_t s = n & 1, u = n >> 1;
       ++n;
-      // lane l < per_warp owns query quarter * per_warp + l of the task
-      int qi = -1, rank = -1;
-      {
-        const int tl = quarter * per_warp + lane;
-        if (lane < per_warp && tl < k.count) {
-          qi = p.qids[k.start + tl];
-          rank = p.ranks[k.start + tl];
-          if (qi < 0 || qi >= p.sq || rank < 0 || rank >= p.topk) qi = rank = -1;
-        }
+      if (qi < 0 || qi >= p.sq || rank < 0 || rank >= p.topk) qi = rank = -1;
+      if (k.group != group) {
+        group = k.group;
+        b = group / p.hkv;
+        kvh = group - b * p.hkv;
       }
       bool w = mbar_wait(bar(STATS_FULL + s), u & 1, guard, 0x780 + s);
       w = mbar_wait(bar(O_FULL + s), u & 1, guard, 0x790 + s) && w;
@@ -424,7 +465,7 @@ kv_token_pipe_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
         // fp32 partials: lane = row (query lane / G, head lane % G) writes its 512 bytes from tensor memory
         const int owner = lane >> p.group_log2, g = lane & (G - 1);
         const int row_q = __shfl_sync(0xffffffffu, qi, owner), row_rank = __shfl_sync(0xffffffffu, rank, owner);
-        const int b = k.group / p.hkv, head = (k.group - b * p.hkv) * G + g;
+        const int head = kvh * G + g;
         const long long row =
             p.partial_token_major
                 ? ((static_cast<long long>(b) * p.sq + row_q) * p.topk + row_rank) * p.hq + head
@@ -471,7 +512,6 @@ kv_token_pipe_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
       fence_async_smem();
       __syncwarp();
       if (qi >= 0) {
-        const int b = k.group / p.hkv, kvh = k.group - b * p.hkv;
         const uint32_t src = stage + lane * G * 128;
         if (p.partial_token_major) {              // box {64 columns, G heads, 1 rank, 1 token}
           tma_store_4d(&o_map, 0, kvh * G, rank, b * p.sq + qi, src);
