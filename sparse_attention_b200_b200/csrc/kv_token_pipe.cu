@@ -21,7 +21,9 @@
 // head-major [B,Hq,Sq,128], partials [B,Hq,Sq,TopK,128] bf16 and LSE [B,Hq,Sq,TopK].
 // Bound by the issue of its lone warps and by the writes of the partials: eight 4 Ki sequences of 16 heads, 32 blocks, 16
 // of them per token, 895 -> 718 us (2.1 GB of partials: 330 us at the copy rate) since task records and ids are fetched
-// ahead (895 -> 755), found by counters instead of divisions, and MMAs issued by an elected lane (755 -> 718).
+// ahead (895 -> 755), found by counters instead of divisions, and MMAs issued by an elected lane (755 -> 718). With fp32
+// partials 2520 -> 1200 us since their rows are staged and stored by TMA, too (16 bytes of every row per store instruction
+// before: half a sector each).
 // Rows of a tile beyond the task's query count keep whatever the buffer held: every row
 // of S, P and O depends on its own Q row only, and those rows are never stored.
 #include <algorithm>
@@ -69,7 +71,6 @@ struct Params {
   int phases;                   // upper bound on the number of passes over the task list (see Walk)
   int q_token_major;            // q is [B, Sq, Hq, 128]: the G heads of a token are one dense box
   int partial_token_major;      // partials are [B, Sq, TopK, Hq, 128] (the reference's token-major operators)
-  float* partial_f32;           // non-null: fp32 partials (the reference's fp32 controls), written with plain stores
   float scale_log2;
 };
 
@@ -140,7 +141,7 @@ __device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, int x, int 
                : "memory");
 }
 
-template <bool F32>      // fp32 partials (plain stores) instead of bf16 (staged, TMA stores)
+template <bool F32>      // fp32 partials instead of bf16
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 kv_token_pipe_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
                      const __grid_constant__ CUtensorMap v_map, const __grid_constant__ CUtensorMap o_map,
@@ -462,30 +463,40 @@ kv_token_pipe_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
       if (lane == 0) mbar_arrive(bar(STATS_EMPTY + s));
       const uint32_t t_o = tmem + lane_base + 256 + s * 128;
       if constexpr (F32) {
-        // fp32 partials: lane = row (query lane / G, head lane % G) writes its 512 bytes from tensor memory
-        const int owner = lane >> p.group_log2, g = lane & (G - 1);
-        const int row_q = __shfl_sync(0xffffffffu, qi, owner), row_rank = __shfl_sync(0xffffffffu, rank, owner);
-        const int head = kvh * G + g;
-        const long long row =
-            p.partial_token_major
-                ? ((static_cast<long long>(b) * p.sq + row_q) * p.topk + row_rank) * p.hq + head
-                : ((static_cast<long long>(b) * p.hq + head) * p.sq + row_q) * p.topk + row_rank;
-        float4* dst = reinterpret_cast<float4*>(p.partial_f32 + (row_q >= 0 ? row : 0) * 128);
+        // fp32 partials: 512 bytes per row, two rounds of two 128-byte boxes
+        const uint32_t src = stage + lane * G * 128;
 #pragma unroll 1
-        for (int cc = 0; cc < 8; ++cc) {
-          uint32_t ov[16];
-          tmem_ld16(t_o + cc * 16, ov);
-          tc_wait_ld();
-          if (row_q >= 0) {
+        for (int half = 0; half < 2; ++half) {
+          bulk_wait_read0();                         // this lane's earlier stores have left the staging tile
+          __syncwarp();
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-              dst[cc * 4 + j] = make_float4(__uint_as_float(ov[4 * j]) * inv, __uint_as_float(ov[4 * j + 1]) * inv,
-                                            __uint_as_float(ov[4 * j + 2]) * inv, __uint_as_float(ov[4 * j + 3]) * inv);
+          for (int cc = 0; cc < 2; ++cc) {
+            uint32_t ov[32];
+            tmem_ld32(t_o + half * 64 + cc * 32, ov);
+            tc_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              *reinterpret_cast<float4*>(stage_g + cc * 4096 + lane * 128 + ((j ^ (lane & 7)) << 4)) =
+                  make_float4(__uint_as_float(ov[4 * j]) * inv, __uint_as_float(ov[4 * j + 1]) * inv,
+                              __uint_as_float(ov[4 * j + 2]) * inv, __uint_as_float(ov[4 * j + 3]) * inv);
+          }
+          if (half == 1) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(O_EMPTY + s));
+          }
+          fence_async_smem();
+          __syncwarp();
+          if (qi >= 0) {
+#pragma unroll
+            for (int cc = 0; cc < 2; ++cc) {
+              const int x = half * 64 + cc * 32;
+              if (p.partial_token_major) tma_store_4d(&o_map, x, kvh * G, rank, b * p.sq + qi, src + cc * 4096);
+              else tma_store_4d(&o_map, x, rank, qi, b * p.hq + kvh * G, src + cc * 4096);
+            }
+            bulk_commit();
           }
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(O_EMPTY + s));
         continue;
       }
       bulk_wait_read0();                             // this lane's earlier stores have left the staging tile
@@ -558,7 +569,7 @@ int launch_kv_token_pipe(const void* q, const void* k, const void* v, const int3
   p.scale_log2 = 1.4426950408889634f / sqrtf(128.0f);
   p.q_token_major = q_token_major & 1;
   p.partial_token_major = (q_token_major >> 1) & 1;
-  p.partial_f32 = (q_token_major & 4) ? static_cast<float*>(partial) : nullptr;
+  const bool f32 = (q_token_major & 4) != 0;
   q_token_major &= 1;
   // one segment per 24 MB of Q: the Q rows a segment gathers then stay within L2
   const long long q_bytes = static_cast<long long>(batch) * hq * sq * 256;
@@ -606,21 +617,24 @@ int launch_kv_token_pipe(const void* q, const void* k, const void* v, const int3
       strides[2] = static_cast<cuuint64_t>(topk) * hq * 256;
       box[1] = static_cast<cuuint32_t>(group); box[3] = 1;
     }
-    // (fp32 partials are written with plain stores: the map is encoded over the same base and never used)
-    if (encode_tiled(&om, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, partial, dims, strides, box, ones,
+    if (f32) {                 // 128-byte boxes of 32 fp32 columns
+      for (cuuint64_t& stride : strides) stride *= 2;
+      box[0] = 32;
+    }
+    if (encode_tiled(&om, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, partial, dims, strides, box, ones,
                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE))
       return set_error(SB_ERR_CUDA, "cuTensorMapEncodeTiled failed for the partial outputs");
   }
-  const int slot = p.partial_f32 ? 18 : 10;
+  const int slot = f32 ? 18 : 10;
   if (!(ctx->tc_attr & (1 << slot))) {
-    cudaError_t e = p.partial_f32 ? cudaFuncSetAttribute(kv_token_pipe_kernel<true>,
+    cudaError_t e = f32 ? cudaFuncSetAttribute(kv_token_pipe_kernel<true>,
                                                          cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES)
                                   : cudaFuncSetAttribute(kv_token_pipe_kernel<false>,
                                                          cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     if (e != cudaSuccess) return set_error(SB_ERR_CUDA, cudaGetErrorString(e));
     ctx->tc_attr |= (1 << slot);
   }
-  if (p.partial_f32)
+  if (f32)
     kv_token_pipe_kernel<true><<<ctx->sm_count, NUM_THREADS, SMEM_BYTES, stream>>>(qm, km, vm, om, p);
   else
     kv_token_pipe_kernel<false><<<ctx->sm_count, NUM_THREADS, SMEM_BYTES, stream>>>(qm, km, vm, om, p);
