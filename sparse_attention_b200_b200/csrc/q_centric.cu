@@ -43,10 +43,12 @@ constexpr int NUM_THREADS = 512;     // four warpgroups: softmax 0, softmax 1, e
 constexpr int EPI_WARP0 = 8;         // warps 8..11: warp w serves tensor-memory lanes 32 * (w % 4) ..
 constexpr int MMA_WARP = 12;
 constexpr int LOAD_WARP = 13;
-// register budgets per thread after the setup barrier (setmaxnreg); 128 * (2 * 176 + 64 + 96) = 65536
-constexpr int SOFTMAX_REGS = 176;
+// register budgets per thread after the setup barrier (setmaxnreg); 128 * (2 * 192 + 64 + 64) = 65536. At 176 / 64 / 96 the
+// softmax warps spill six words: 1 Mi-token group 34.2 -> 33.6 ms, KV-centric case 30.0 -> 29.7, 16 heads over 16 Ki keys
+// 124.6 -> 123.9 us, 32 heads at 32 Ki 1118 -> 1112 without (medians of three interleaved runs)
+constexpr int SOFTMAX_REGS = 192;
 constexpr int EPI_REGS = 64;
-constexpr int CTRL_REGS = 96;        // MMA issuer, TMA producer, idle warps
+constexpr int CTRL_REGS = 64;        // MMA issuer, TMA producer, idle warps
 constexpr int TMEM_COLS = 512;
 constexpr int SMALL_PARTS = 16;      // pieces of an item in a launch of less than a round
 constexpr float RESCALE_LOG2 = 8.0f;   // keep a stale row max while it lags by < 2^8
