@@ -609,10 +609,10 @@ fp4_nv_select_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
 // tensor cores give every dot within delta of its exact value, so only the elements whose
 // approximate value reaches (largest approximate value - 2 delta) can hold the exact maximum:
 // any other element is below the exact value of the approximate arg-max. Those few elements
-// (usually one) are evaluated with the canonical arithmetic (integer group sums, scaled and
-// added in group order) straight from the codes in global memory. Same scores, bit for bit,
-// as fp4_score_mma_kernel, which evaluates all 16384 elements of a pair exactly. Every
-// evaluated element is also compared with its approximate value: a difference above delta is
+// (usually one) are queued with the other fifteen of their group of columns and evaluated at the end with the
+// canonical arithmetic (integer group sums, scaled and added in group order) straight from the codes in global
+// memory. Same scores, bit for bit, as fp4_score_mma_kernel, which evaluates all 16384 elements of a pair exactly.
+// The exact maximum of every evaluated group is also compared with its approximate one: a difference above delta is
 // counted and the pair is re-done by evaluating all of its elements.
 struct PruneParams {
   Geometry g;
@@ -671,10 +671,10 @@ __device__ __forceinline__ float fp4_exact_dot(const uint8_t* __restrict__ q_cod
   return acc;
 }
 
-constexpr int PR_QCAP = 2048;                // queued elements per CTA
+constexpr int PR_QCAP = 2048;                // queued groups of elements per CTA
 constexpr int PR_OFF_AUX = OFF_CAND;         // barriers (128 bytes), misc (128 bytes)
-constexpr int PR_OFF_QUEUE = PR_OFF_AUX + 256;            // [PR_QCAP] elements waiting for their exact value
-constexpr int PR_OFF_APX = PR_OFF_QUEUE + PR_QCAP * 4;     // [PR_QCAP] their approximate values
+constexpr int PR_OFF_QUEUE = PR_OFF_AUX + 256;            // [PR_QCAP] groups waiting for their exact values
+constexpr int PR_OFF_APX = PR_OFF_QUEUE + PR_QCAP * 4;     // [PR_QCAP] their largest approximate values
 constexpr int PR_OFF_RES = PR_OFF_APX + PR_QCAP * 4;       // [pages per CTA] exact maxima as ordered ints
                                                            // then [pages per CTA] flags: pair to be re-done in full
 
@@ -767,10 +767,18 @@ fp4_nv_prune_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
     {
       // largest scale among this CTA's key pages: 64 threads per page, 16 bytes each
       uint32_t seen = 0;
-      for (int t = threadIdx.x >> 6; t < num_tiles; t += 4) {
-        const long long page = (static_cast<long long>(b) * g.tiles + page0 + t) * g.hk + hk_idx;
-        const uint4 w = __ldg(reinterpret_cast<const uint4*>(g.ks + page * 1024) + (threadIdx.x & 63));
-        seen = max_scale_bytes(max_scale_bytes(max_scale_bytes(max_scale_bytes(seen, w.x), w.y), w.z), w.w);
+      for (int t0 = threadIdx.x >> 6; t0 < num_tiles; t0 += 32) {     // eight pages' loads in flight
+        uint4 w[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int t = t0 + 4 * i;
+          const long long page = (static_cast<long long>(b) * g.tiles + page0 + t) * g.hk + hk_idx;
+          w[i] = make_uint4(0u, 0u, 0u, 0u);
+          if (t < num_tiles) w[i] = __ldg(reinterpret_cast<const uint4*>(g.ks + page * 1024) + (threadIdx.x & 63));
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          seen = max_scale_bytes(max_scale_bytes(max_scale_bytes(max_scale_bytes(seen, w[i].x), w[i].y), w[i].z), w[i].w);
       }
       uint32_t m = top_byte(seen);
 #pragma unroll
@@ -783,20 +791,6 @@ fp4_nv_prune_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const int half = warp >> 2;
     const int key_row = (warp & 3) * 32 + lane;
-    // exact value of element (page t of this CTA, key row, query column) into the page's maximum
-    auto evaluate = [&](int t, int krow, int col, float apx) {
-      const long long page = (static_cast<long long>(b) * g.tiles + page0 + t) * g.hk + hk_idx;
-      const long long qrow = (q_row0 + col) * g.hidx + h;
-      const float e = fp4_exact_dot(g.qp + qrow * 64, g.qs + qrow * 8, g.kp + (page * 128 + krow) * 64,
-                                    g.ks + (page * 128 + krow) * 8);
-      if (e == e) atomicMax(res + t, f2ord(e));
-      const float diff = fabsf(apx - e);
-      if (delta > 0.f) atomicMax(const_cast<int*>(misc + 8), __float_as_int(diff / delta));
-      if (!(diff <= delta) && e == e) {
-        redo[t] = 1;
-        atomicAdd(p.violations, 1);
-      }
-    };
     bool ok = true;
     for (int t = 0; t < num_tiles; ++t) {
       const int st = t % ACC_STAGES, slot = 4 + t % 3;
@@ -805,7 +799,7 @@ fp4_nv_prune_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
         ok = __all_sync(0xffffffffu, w);
       }
       uint32_t v[4][16];
-      float mine = -INFINITY;
+      float m4[4], mine = -INFINITY;
       if (ok) {
         tc_fence_after();
         const uint32_t t_acc = tmem + lane_base + TM_ACC + st * 128 + half * 64;
@@ -815,7 +809,6 @@ fp4_nv_prune_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(ACC_EMPTY + st));
-        float m4[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           float m5[5];
@@ -834,40 +827,50 @@ fp4_nv_prune_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
       if (threadIdx.x == 0 && t > 0) misc[4 + (t - 1) % 3] = INT_MIN;
       if (ok) {
         const float thr = ord2f(misc[slot]) - two;
-        if (!(mine < thr)) {                 // this key row holds at least one element that may be the maximum
-          unsigned long long mask = 0ull;
+        // Groups of sixteen columns of this key row that hold an element that may be the maximum. Everyone waits for this
+        // at the page's next meeting, and a lone lane does it: the column is left to the evaluation (looking for it here,
+        // with its approximate value, took the lane longer than the page took everyone: 1070 cycles of an SM per page).
+        if (!(mine < thr)) {
 #pragma unroll
           for (int c = 0; c < 4; ++c)
-#pragma unroll
-            for (int jj = 0; jj < 16; ++jj)
-              if (!(__uint_as_float(v[c][jj]) < thr)) mask |= 1ull << (c * 16 + jj);
-          while (mask) {
-            const int bit = __ffsll(static_cast<long long>(mask)) - 1;
-            mask &= mask - 1;
-            const int col = half * 64 + bit;
-            float apx = 0.f;                 // v[bit / 16][bit % 16] without a dynamically indexed register array
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-#pragma unroll
-              for (int jj = 0; jj < 16; ++jj)
-                if (c * 16 + jj == bit) apx = __uint_as_float(v[c][jj]);
-            const int at = atomicAdd(const_cast<int*>(misc + 7), 1);
-            if (at < PR_QCAP) {
-              queue[at] = (t << 14) | (key_row << 7) | col;
-              queue_apx[at] = apx;
-            } else {
-              evaluate(t, key_row, col, apx);  // queue full (masses of ties): pay for it here
+            if (!(m4[c] < thr)) {
+              const int at = atomicAdd(const_cast<int*>(misc + 7), 1);
+              if (at < PR_QCAP) {
+                queue[at] = (t << 10) | (key_row << 3) | (half * 4 + c);
+                queue_apx[at] = m4[c];
+              } else {
+                redo[t] = 1;                 // queue full (masses of ties): the page is re-done below
+              }
             }
-          }
         }
       }
     }
     meet();
-    // the queued elements, one per thread at a time, then the scores of this CTA's pages
+    // the queued groups, sixteen threads each: exact values of the group's elements into the page's maximum
     const int queued = min(misc[7], PR_QCAP);
-    for (int i = threadIdx.x; i < queued; i += 256) {
-      const int e = queue[i];
-      evaluate(e >> 14, (e >> 7) & 127, e & 127, queue_apx[i]);
+    for (int i = static_cast<int>(threadIdx.x) >> 4; i < ((queued + 15) & ~15); i += 16) {
+      const bool live = i < queued;
+      const int e = live ? queue[i] : 0, t = e >> 10, krow = (e >> 3) & 127;
+      float m = -INFINITY;
+      if (live) {
+        const long long page = (static_cast<long long>(b) * g.tiles + page0 + t) * g.hk + hk_idx;
+        const long long qrow = (q_row0 + (e & 7) * 16 + (threadIdx.x & 15)) * g.hidx + h;
+        const float x = fp4_exact_dot(g.qp + qrow * 64, g.qs + qrow * 8, g.kp + (page * 128 + krow) * 64,
+                                      g.ks + (page * 128 + krow) * 8);
+        if (x == x) m = x;
+      }
+#pragma unroll
+      for (int d = 8; d > 0; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
+      if (live && (threadIdx.x & 15) == 0 && m > -INFINITY) {
+        atomicMax(res + t, f2ord(m));
+        // the largest value of a group, exact and approximate, differ by at most delta, as its elements do
+        const float diff = fabsf(queue_apx[i] - m);
+        if (delta > 0.f) atomicMax(const_cast<int*>(misc + 8), __float_as_int(diff / delta));
+        if (!(diff <= delta)) {
+          redo[t] = 1;
+          atomicAdd(p.violations, 1);
+        }
+      }
     }
     meet();
     if (threadIdx.x == 0 && misc[8] > 0) atomicMax(p.stats + 4, misc[8]);      // one global atomic per CTA
