@@ -202,12 +202,13 @@ struct Geometry {
 };
 
 // ---------------------------------------------------------------- producer and MMA roles
-// A page takes about 450 cycles of an SM with two CTAs on it (520 when one lane issued under `if (lane == 0)` instead of the
-// elected lane of a converged warp, see elect_one(); 590 when the scales of page t + 3 were requested before
-// the proxy fence of page t, which then waited for them, and when the page maximum took five shuffles), against 128
-// cycles of MMAs: the hand-overs copy -> MMA -> accumulator -> epilogue bound it. One CTA per SM with three
-// accumulators and two to three threads issuing, the scales through tensor-memory stores, was no faster (510 to 840); nor are
-// three accumulators of 64 columns in a CTA, now that issuing is cheap (450, and 48 -> 56 us on a ragged prefill batch).
+// A page takes about 440 cycles of an SM with two CTAs on it, against 128 cycles of MMAs: the serial work of lone warps
+// (waits, scale copies, hand-overs) bounds it, in the producer, the MMA warp and the epilogue alike: leaving out any one of
+// maxima, accumulator reads, TMA copies or scale stores changes nothing. 450 when the producer fenced its scale stores for the
+// async proxy (a fence takes 300 cycles, and waits for the loads in flight; now the MMA warp does it, when a page
+// has landed), 520 when one lane issued under `if (lane == 0)`, see elect_one(). No faster: one CTA per SM with three
+// accumulators and one to four producer warps (540 to 720), two or three producer warps per CTA here (450), three
+// accumulators of 64 columns per CTA (450).
 // Producer warp: query tile once, then key pages page0 + (t + rot) % wrap for t = 0 .. num_tiles - 1 (num_tiles <= wrap,
 // rot < wrap).
 __device__ __forceinline__ void producer_role(const Geometry& g, const CUtensorMap* q_map, const CUtensorMap* k_map,
@@ -249,10 +250,8 @@ __device__ __forceinline__ void producer_role(const Geometry& g, const CUtensorM
     store_scale_chunks(gbase + OFF_A + s * STAGE_BYTES + CODE_BYTES, regs, lane);
 #pragma unroll
     for (int i = 0; i < 4; ++i) seen = max_scale_bytes(max_scale_bytes(seen, regs.r[i].x), regs.r[i].y);
-    fence_async_smem();
     __syncwarp();
     if (lane == 0) mbar_arrive(bar(A_FULL + s));
-    // after the fence, which would wait for them
     if (t + 3 < num_tiles) regs = load_scales(g.ks + key_row(page_of(t + 3)) * 8, 8, lane);
     return true;
   };
@@ -292,6 +291,7 @@ __device__ __forceinline__ void mma_role(uint32_t base, uint32_t bar0, uint32_t 
   for (int t = 0; t < num_tiles; ++t) {
     const int s = t % A_STAGES, st = t % ACC_STAGES;
     if (!mbar_wait_warp(bar(A_FULL + s), (t / A_STAGES) & 1, guard, code0 + 1 + s)) return;
+    fence_async_smem();              // the producer's scale stores, for the copies below
     tc_fence_after();
     // the scale copy does not touch the accumulator: it goes out before the accumulator hand-over is awaited
     const uint64_t a0 = desc_sw64_kmajor(base + OFF_A + s * STAGE_BYTES);
@@ -1073,10 +1073,8 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
         tma_load_2d(base + OFF_A + s * STAGE_BYTES, &k_map, 0, static_cast<int>(key_row(t)), bar_(A_FULL + s));
       }
       store_scale_chunks(gbase + OFF_A + s * STAGE_BYTES + CODE_BYTES, regs, lane);
-      fence_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_(A_FULL + s));
-      // after the fence, which would wait for them
       if (t + 3 < num_tiles) regs = load_scales(p.ks + key_row(t + 3) * 8, 8, lane);
       return true;
     };
@@ -1105,6 +1103,7 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
         const int s = t % A_STAGES;
         ok = mbar_wait_warp(bar(A_FULL + s), (t / A_STAGES) & 1, guard, 0x611 + s);
         if (!ok) break;
+        fence_async_smem();            // the producer's scale stores, for the copies below
         tc_fence_after();
         const uint64_t b0 = desc_sw64_kmajor(base + OFF_A + s * STAGE_BYTES);
         const uint32_t sfk = tmem + TM_SFA + (t & 1) * 8;
