@@ -127,6 +127,14 @@ __device__ __forceinline__ float warp_max(float v) {
 }
 __device__ __forceinline__ float ord2f(int i) { return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff); }
 
+// 8 bytes of global memory to shared memory, asynchronously; groups of a thread's copies and a wait for all but the newest N
+__device__ __forceinline__ void cp_async8(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
 // Largest |dequantised element| and largest squared L2 norm over all key vectors -> stats[0], stats[1]
 // (zeroed by the caller). Sixteen adjacent threads hold one row.
 __global__ void __launch_bounds__(256) key_stats_kernel(const uint8_t* __restrict__ codes, const uint8_t* __restrict__ scales,
@@ -933,19 +941,168 @@ static bool aligned(const void* p, uintptr_t a) { return (reinterpret_cast<uintp
 // reference's gate for this output is rtol 1e-4 / atol 1e-3, benchmarks/ch4_selectors/harness.py:33-42).
 // Here the QUERY tile is the M operand (one tensor-memory lane = one query, so the maximum over the keys of a
 // page is a maximum along a lane) and the key pages stream through as the N operand.
-// One CTA per (request, query tile, head) -- or, packed (decode batches), per (request, KV head, block of 16
-// group heads) with rows = (query, head) pairs -- and chunk of pages. Warps 0-3 epilogue (lane quarter = warp),
-// warp 4 producer, warp 5 MMA issue (one thread). 192 threads, 152 tensor-memory columns: two CTAs per SM.
+// An item is a (request, query tile, head) -- or, packed (decode batches), a (request, KV head, block of 16 group heads)
+// with rows = (query, head) pairs; its pages are the visible ones of its request. The pages of all items, one after
+// the other, are cut into equal runs, one per CTA: two CTAs per SM (160 tensor-memory columns each) stay for the whole
+// launch, whatever the lengths, which only the device knows. With a CTA per (item, 16 to 64 pages) the last round was
+// nearly empty and every CTA paid its start (descriptors, first loads: 4000 cycles) for 16 pages of 1000.
+// Warps 0-3 epilogue (lane quarter = warp), warp 4 copies the codes, warp 6 brings the scales, warp 5 issues the MMAs (its
+// elected lane).
 struct QueryScoreParams {
   const uint8_t *qp, *qs, *kp, *ks;
   const int32_t *cu_q, *cu_k, *cu_pages, *kv_indices, *qo_offset;
   float* out;                          // [Hq, tiles_out, total_q], pre-filled with -inf
   int* status;
-  int batch, hq, hk, total_q, total_pages, qt_max, tiles_out, pages_per_cta, causal, head_blocks;
+  int batch, hq, hk, total_q, total_pages, qt_max, tiles_out, causal;
+  int group, subs;                     // query heads of a KV head; items of a KV head (heads, or blocks of 16 of them)
 };
-constexpr int QS_THREADS = 192;
+constexpr int QS_THREADS = 224;
 constexpr int QS_PACK_Q = 8, QS_PACK_HEADS = 16;
-constexpr int QS_OFF_AUX = OFF_CAND;   // barriers (128 bytes), misc (64 bytes)
+constexpr int QS_STAGES = 8;           // pages in flight
+constexpr int QS_AHEAD = 4;            // pages whose scales are on their way to their staging ring
+constexpr int QS_OFF_Q = QS_STAGES * STAGE_BYTES;          // two query tiles: codes + scales
+constexpr int QS_OFF_RAW = QS_OFF_Q + 2 * STAGE_BYTES;     // staging ring: the scales of a page as they are in memory
+constexpr int QS_OFF_AUX = QS_OFF_RAW + QS_AHEAD * SF_BYTES;   // barriers, misc (64 bytes)
+enum { QS_K_FULL = 0, QS_K_EMPTY = QS_STAGES, QS_Q_FULL = 2 * QS_STAGES, QS_Q_EMPTY = QS_Q_FULL + 2,
+       QS_ACC_FULL = QS_Q_EMPTY + 2, QS_ACC_EMPTY, QS_BARS };
+constexpr int QS_BAR_BYTES = (QS_BARS * 8 + 63) & ~63;
+constexpr int QS_SMEM = QS_OFF_AUX + QS_BAR_BYTES + 64 + 1024;
+// tensor memory: the accumulator, two slots of key scales, two of query scales
+constexpr int QS_SFK = 128, QS_SFQ = 144;
+static_assert(QS_SFQ + 16 <= TM_COLS, "tensor memory map");
+
+// What a request means for the scorer; qtiles is 0 where there is nothing to score.
+struct Request {
+  int q_begin, q_len, q_rows, k_len, page_begin, pages, offset, qtiles;     // q_rows: query rows that exist in q
+  template <bool PACKED>
+  static __device__ __forceinline__ Request load(const QueryScoreParams& p, int b) {
+    Request r;
+    r.q_begin = p.cu_q[b];
+    r.q_len = p.cu_q[b + 1] - r.q_begin;
+    r.k_len = p.cu_k[b + 1] - p.cu_k[b];
+    r.page_begin = p.cu_pages[b];
+    r.pages = min(min((r.k_len + 127) >> 7, p.tiles_out), p.cu_pages[b + 1] - r.page_begin);
+    r.q_rows = min(r.q_len, p.total_q - r.q_begin);
+    if (PACKED) r.q_rows = min(r.q_rows, QS_PACK_Q);
+    r.offset = p.causal ? (p.qo_offset ? p.qo_offset[b] : r.k_len - r.q_len) : 0;
+    const bool nothing = r.q_begin < 0 || r.q_rows <= 0 || r.k_len <= 0 || r.page_begin < 0 || r.pages <= 0;
+    r.qtiles = nothing ? 0 : min((r.q_rows + 127) >> 7, p.qt_max);
+    return r;
+  }
+  // pages that query tile j sees: up to its last live query's horizon
+  __device__ __forceinline__ int visible(const QueryScoreParams& p, int j) const {
+    if (!p.causal) return pages;
+    const long long horizon = min(static_cast<long long>(j) * 128 + 128, static_cast<long long>(q_rows)) - 1 + offset;
+    return horizon < 0 ? 0 : static_cast<int>(min(static_cast<long long>(pages), (horizon >> 7) + 1));
+  }
+  // sum of visible() over all tiles: a full tile j sees max(0, min(pages, j + c)), c = ((127 + offset) >> 7) + 1
+  __device__ __forceinline__ long long total(const QueryScoreParams& p) const {
+    if (qtiles == 0) return 0;
+    const long long n = qtiles - 1, last = visible(p, qtiles - 1);
+    if (!p.causal) return n * pages + last;
+    const long long c = ((127LL + offset) >> 7) + 1;
+    const long long a = min(n, max(0LL, 1 - c)), sat = min(n, max(a, pages - c));    // tiles from a on see some, from sat all
+    return (a + sat - 1 + 2 * c) * (sat - a) / 2 + (n - sat) * pages + last;
+  }
+};
+
+// A role's place in the CTA's run of pages: the same items in the same order in every role.
+template <bool PACKED>
+struct ScoreWalk {
+  int left;                      // pages of the run from the current item's `page` on
+  int b, j, kvh, sub;            // item: request, query tile, KV head, query head or head block of it
+  int page, end;                 // next page, visible pages of the item
+  Request r;
+  __device__ __forceinline__ ScoreWalk(const QueryScoreParams& p, volatile const int* start)
+      : left(start[5]), b(start[0]), j(start[1]), kvh(start[2]), sub(start[3]), page(start[4]) {
+    r = Request::load<PACKED>(p, b);
+    end = r.visible(p, j);
+  }
+  // pages of the run in the current item
+  __device__ __forceinline__ int count() const { return min(left, end - page); }
+  __device__ __forceinline__ void next(const QueryScoreParams& p) {
+    left -= count();
+    page = 0;
+    if (left <= 0 || ++sub < p.subs) return;
+    sub = 0;
+    if (++kvh < p.hk) return;
+    kvh = 0;
+    do {
+      ++j;
+      while (j >= r.qtiles) {
+        if (++b >= p.batch) {
+          left = 0;
+          return;
+        }
+        r = Request::load<PACKED>(p, b);
+        j = 0;
+      }
+      end = r.visible(p, j);
+    } while (end == 0);
+  }
+  __device__ __forceinline__ int head0(const QueryScoreParams& p) const {      // head of row 0
+    return kvh * p.group + (PACKED ? sub * QS_PACK_HEADS : sub);
+  }
+};
+
+// Where the run of this CTA begins: request, query tile, KV head, item of it, page; number of pages (0: nothing). One warp.
+template <bool PACKED>
+__device__ __forceinline__ void find_run(const QueryScoreParams& p, volatile int* start, int lane) {
+  const int heads = p.hk * p.subs;
+  auto scan = [&](long long v) {
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const long long o = __shfl_up_sync(0xffffffffu, v, d);
+      if (lane >= d) v += o;
+    }
+    return v;
+  };
+  long long total = 0;
+  for (int b0 = 0; b0 < p.batch; b0 += 32) {
+    const int b = b0 + lane;
+    total += __shfl_sync(0xffffffffu, scan(b < p.batch ? heads * Request::load<PACKED>(p, b).total(p) : 0LL), 31);
+  }
+  const long long per = max(2LL, (total + gridDim.x - 1) / gridDim.x), first = per * blockIdx.x;
+  if (first >= total) {
+    if (lane == 0) start[5] = 0;
+    return;
+  }
+  long long before = 0;                      // pages of the requests before the current ones
+  for (int b0 = 0; b0 < p.batch; b0 += 32) {
+    const int b = b0 + lane;
+    const long long mine = b < p.batch ? heads * Request::load<PACKED>(p, b).total(p) : 0LL;
+    const long long upto = before + scan(mine);
+    const unsigned hit = __ballot_sync(0xffffffffu, upto > first);
+    if (hit == 0) {
+      before = __shfl_sync(0xffffffffu, upto, 31);
+      continue;
+    }
+    const int at = __ffs(hit) - 1;
+    const Request r = Request::load<PACKED>(p, b0 + at);
+    long long rest = first - __shfl_sync(0xffffffffu, upto - mine, at);
+    for (int j0 = 0; j0 < r.qtiles; j0 += 32) {
+      const int j = j0 + lane;
+      const long long pages = j < r.qtiles ? r.visible(p, j) : 0, sum = scan(pages * heads);
+      const unsigned in = __ballot_sync(0xffffffffu, sum > rest);
+      if (in == 0) {
+        rest -= __shfl_sync(0xffffffffu, sum, 31);
+        continue;
+      }
+      if (lane == __ffs(in) - 1) {
+        const long long local = rest - (sum - pages * heads);
+        start[0] = b0 + at;
+        start[1] = j;
+        const int h = static_cast<int>(local / pages), kvh = h / p.subs;
+        start[2] = kvh;
+        start[3] = h - kvh * p.subs;
+        start[4] = static_cast<int>(local - h * pages);
+        start[5] = static_cast<int>(min(per, total - first));
+      }
+      return;
+    }
+    return;
+  }
+}
 
 template <bool PACKED>
 __global__ void __launch_bounds__(QS_THREADS, 2)
@@ -956,64 +1113,26 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
   const uint32_t base = (raw + 1023u) & ~1023u;
   unsigned char* gbase = smem_raw + (base - raw);
   const uint32_t bar0 = base + QS_OFF_AUX;
-  volatile int* misc = reinterpret_cast<volatile int*>(gbase + QS_OFF_AUX + 128);   // tmem base, abort
+  volatile int* misc = reinterpret_cast<volatile int*>(gbase + QS_OFF_AUX + QS_BAR_BYTES);   // tmem base, abort, start of the run
   auto bar = [&](int i) { return bar0 + 8u * i; };
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int group = p.hq / p.hk;
-
-  // nothing to score: the grid must still not be complete before the fill kernel is
-  auto leave = [] { asm volatile("griddepcontrol.wait;" ::: "memory"); };
-  int h0, qtile, b, hk_idx, heads_here = 1;
-  if (PACKED) {
-    const int head_block = blockIdx.x % p.head_blocks;
-    const int rest = blockIdx.x / p.head_blocks;
-    hk_idx = rest % p.hk;
-    b = rest / p.hk;
-    qtile = 0;
-    h0 = hk_idx * group + head_block * QS_PACK_HEADS;
-    heads_here = min(QS_PACK_HEADS, group - head_block * QS_PACK_HEADS);
-  } else {
-    h0 = blockIdx.x % p.hq;
-    const int rest = blockIdx.x / p.hq;
-    qtile = rest % p.qt_max;
-    b = rest / p.qt_max;
-    hk_idx = h0 / group;
-  }
-  const int q_begin = p.cu_q[b], q_len = p.cu_q[b + 1] - q_begin;
-  const int k_len = p.cu_k[b + 1] - p.cu_k[b];
-  if (q_begin < 0 || qtile * 128 >= q_len || k_len <= 0) return leave();      // block-uniform
-  const int page_begin = p.cu_pages[b];
-  if (page_begin < 0) return leave();
-  int pages = min(min((k_len + 127) >> 7, p.tiles_out), p.cu_pages[b + 1] - page_begin);
-  const int rows_live = min(min(PACKED ? QS_PACK_Q : 128, q_len - qtile * 128), p.total_q - q_begin - qtile * 128);
-  if (rows_live <= 0) return leave();
-  const int offset = p.causal ? (p.qo_offset ? p.qo_offset[b] : k_len - q_len) : 0;
-  if (p.causal) {          // pages past the last live query's horizon stay -inf
-    const long long horizon = static_cast<long long>(qtile) * 128 + rows_live - 1 + offset;
-    pages = horizon < 0 ? 0 : min(pages, static_cast<int>(horizon >> 7) + 1);
-  }
-  const int page0 = blockIdx.y * p.pages_per_cta;
-  const int num_tiles = min(p.pages_per_cta, pages - page0);
-  if (num_tiles <= 0) return leave();
-  // row r of the CTA -> query position inside the request, head, alive?
-  auto row_query = [&](int r) { return PACKED ? (r >> 4) : qtile * 128 + r; };
-  auto row_head = [&](int r) { return PACKED ? h0 + (r & (QS_PACK_HEADS - 1)) : h0; };
-  auto row_alive = [&](int r) {
-    return PACKED ? ((r & (QS_PACK_HEADS - 1)) < heads_here && (r >> 4) < rows_live) : r < rows_live;
-  };
   Guard guard{misc + 1, p.status};
 
   if (threadIdx.x == 0) {
     misc[1] = 0;
-    for (int i = 0; i < A_STAGES; ++i) {
-      mbar_init(bar(A_FULL + i), 2);
-      mbar_init(bar(A_EMPTY + i), 1);
+    for (int i = 0; i < QS_STAGES; ++i) {
+      mbar_init(bar(QS_K_FULL + i), 2);          // the TMA transaction of the codes + the producer warp's scale stores
+      mbar_init(bar(QS_K_EMPTY + i), 1);
     }
-    mbar_init(bar(ACC_FULL), 1);
-    mbar_init(bar(ACC_EMPTY), 4);
-    mbar_init(bar(B_FULL), 2);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bar(QS_Q_FULL + i), 2);
+      mbar_init(bar(QS_Q_EMPTY + i), 1);
+    }
+    mbar_init(bar(QS_ACC_FULL), 1);
+    mbar_init(bar(QS_ACC_EMPTY), 4);
     fence_mbar_init();
   }
+  if (warp == 4) find_run<PACKED>(p, misc + 2, lane);
   if (warp == 5) {
     tmem_alloc(smem_u32(const_cast<int*>(misc)), TM_COLS);
     tmem_relinquish();
@@ -1022,107 +1141,170 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = static_cast<uint32_t>(misc[0]);
-  // physical page of logical page pg, or -1 when the table entry is out of range (the page stays -inf)
-  auto phys_page = [&](int pg) {
-    const int ph = __ldg(p.kv_indices + page_begin + pg);
-    return (ph < 0 || ph >= p.total_pages) ? -1 : ph;
-  };
+  const int total = misc[7];
 
+  if (total > 0) {
   if (warp == 4) {
-    // ----------------------------------------------------------- producer
-    auto bar_ = bar;
-    if (lane == 0) {
-      mbar_expect_tx(bar_(B_FULL), CODE_BYTES);
-      if (PACKED)      // box {64 bytes, 16 heads, 8 queries}: row = query * 16 + head
-        tma_load_3d(base + OFF_B, &q_map, 0, h0, q_begin, bar_(B_FULL));
-      else             // box {64 bytes, 1 head, 128 queries}
-        tma_load_3d(base + OFF_B, &q_map, 0, h0, q_begin + qtile * 128, bar_(B_FULL));
-    }
-    {
-      ScaleRegs s;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int r = lane + 32 * i;
-        s.r[i] = make_uint2(0u, 0u);
-        if (row_alive(r))
-          s.r[i] = __ldg(reinterpret_cast<const uint2*>(
-              p.qs + ((static_cast<long long>(q_begin) + row_query(r)) * p.hq + row_head(r)) * 8));
+    // ----------------------------------------------------------- codes (TMA); page ids 32 at a time
+    ScoreWalk<PACKED> walk(p, misc + 2);
+    int items = 0, left = 0, pg = 0, ids = 0;     // items begun, pages left in the current one
+    int pushed = 0;
+    bool ok = true;
+    for (int t = 0; t < total; ++t) {
+      if (left == 0 || (pg & 31) == 0) {
+        const int i = ((left == 0 ? walk.page : pg) & ~31) + lane;
+        ids = i < walk.r.pages ? __ldg(p.kv_indices + walk.r.page_begin + i) : 0;
       }
-      store_scale_chunks(gbase + OFF_B + CODE_BYTES, s, lane);
-      fence_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar_(B_FULL));
+      if (left == 0) {
+        const int slot = items & 1;
+        if (items >= 2) ok = mbar_wait_warp(bar(QS_Q_EMPTY + slot), ((items >> 1) - 1) & 1, guard, 0x630 + slot);
+        if (!ok) break;
+        ++items;
+        if (lane == 0) {
+          mbar_expect_tx(bar(QS_Q_FULL + slot), CODE_BYTES);
+          // packed: box {64 bytes, 16 heads, 8 queries}, row = query * 16 + head; else box {64 bytes, 1 head, 128 queries}
+          tma_load_3d(base + QS_OFF_Q + slot * STAGE_BYTES, &q_map, 0, walk.head0(p), walk.r.q_begin + walk.j * 128,
+                      bar(QS_Q_FULL + slot));
+        }
+        left = walk.count();
+        pg = walk.page;
+      }
+      const int s = t % QS_STAGES, use = t / QS_STAGES;
+      if (use > 0) ok = mbar_wait_warp(bar(QS_K_EMPTY + s), (use - 1) & 1, guard, 0x600 + s);
+      if (!ok) break;
+      const int ph = __shfl_sync(0xffffffffu, ids, pg & 31);
+      if (lane == 0) {
+        mbar_expect_tx(bar(QS_K_FULL + s), CODE_BYTES);
+        tma_load_2d(base + OFF_A + s * STAGE_BYTES, &k_map, 0, ((ph < 0 || ph >= p.total_pages ? 0 : ph) * p.hk + walk.kvh) * 128,
+                    bar(QS_K_FULL + s));
+      }
+      ++pushed;
+      ++pg;
+      if (--left == 0) walk.next(p);
     }
-    auto key_row = [&](int t) {
-      const int ph = phys_page(page0 + t);
-      return (static_cast<long long>(ph < 0 ? 0 : ph) * p.hk + hk_idx) * 128;
+    if (!ok) {
+      // let copies in flight land before the CTA gives up its shared memory
+      for (int t = max(0, pushed - QS_STAGES); t < pushed; ++t)
+        mbar_wait_drain(bar(QS_K_FULL + t % QS_STAGES), (t / QS_STAGES) & 1);
+      for (int i = max(0, items - 2); i < items; ++i) mbar_wait_drain(bar(QS_Q_FULL + (i & 1)), (i >> 1) & 1);
+    }
+  } else if (warp == 6) {
+    // ----------------------------------------------------------- scales: staged QS_AHEAD pages ahead, then re-ordered
+    // (asynchronous copies, not loads into registers: those need the loop unrolled over the pages in flight, and its
+    // instructions alone, fetched for the first time, took 7000 cycles before the first page)
+    ScoreWalk<PACKED> ahead_walk(p, misc + 2), walk(p, misc + 2);
+    int ids = 0, ahead_left = 0, ahead_pg = 0;    // of the walk ahead: 32 page ids, pages left in its item, next page
+    auto raw = [&](int t) { return QS_OFF_RAW + (t % QS_AHEAD) * SF_BYTES + lane * 8; };
+    auto fetch = [&](int t) {                     // rows lane, lane + 32, .. of page t; one group per page
+      if (t < total) {
+        const bool first = ahead_left == 0;
+        if (first) {
+          ahead_left = ahead_walk.count();
+          ahead_pg = ahead_walk.page;
+        }
+        if (first || (ahead_pg & 31) == 0) {
+          const int i = (ahead_pg & ~31) + lane;
+          ids = i < ahead_walk.r.pages ? __ldg(p.kv_indices + ahead_walk.r.page_begin + i) : 0;
+        }
+        const int ph = __shfl_sync(0xffffffffu, ids, ahead_pg & 31);
+        const long long row = ((ph < 0 || ph >= p.total_pages ? 0 : ph) * p.hk + ahead_walk.kvh) * 128LL;
+        const uint8_t* src = p.ks + row * 8 + lane * 8;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) cp_async8(base + raw(t) + i * 256, src + i * 256);
+        ++ahead_pg;
+        if (--ahead_left == 0) ahead_walk.next(p);
+      }
+      cp_async_commit();
     };
     bool ok = true;
-    ScaleRegs ahead[3];
+#pragma unroll 1
+    for (int t = 0; t < QS_AHEAD; ++t) fetch(t);
+    int items = 0, left = 0;
+#pragma unroll 1
+    for (int t = 0; t < total; ++t) {
+      if (left == 0) {
+        const int slot = items & 1;
+        const int h0 = walk.head0(p), q0 = walk.j * 128;
+        const int rows_live = walk.r.q_rows - q0, heads_here = PACKED ? p.group - walk.sub * QS_PACK_HEADS : 1;
+        ScaleRegs s;
 #pragma unroll
-    for (int i = 0; i < 3; ++i)
-      if (i < num_tiles) ahead[i] = load_scales(p.ks + key_row(i) * 8, 8, lane);
-    auto step = [&](int t, ScaleRegs& regs) -> bool {
-      const int s = t % A_STAGES, use = t / A_STAGES;
-      if (use > 0) {
-        bool w = mbar_wait(bar_(A_EMPTY + s), (use - 1) & 1, guard, 0x600 + s);
-        if (!__all_sync(0xffffffffu, w)) return false;
+        for (int i = 0; i < 4; ++i) {
+          const int r = lane + 32 * i, q = PACKED ? r >> 4 : r, h = PACKED ? r & (QS_PACK_HEADS - 1) : 0;
+          s.r[i] = make_uint2(0u, 0u);
+          if (q < rows_live && h < heads_here)
+            s.r[i] = __ldg(reinterpret_cast<const uint2*>(
+                p.qs + ((static_cast<long long>(walk.r.q_begin) + q0 + q) * p.hq + h0 + h) * 8));
+        }
+        if (items >= 2) ok = mbar_wait_warp(bar(QS_Q_EMPTY + slot), ((items >> 1) - 1) & 1, guard, 0x634 + slot);
+        if (!ok) break;
+        ++items;
+        store_scale_chunks(gbase + QS_OFF_Q + slot * STAGE_BYTES + CODE_BYTES, s, lane);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(QS_Q_FULL + slot));
+        left = walk.count();
       }
-      if (lane == 0) {
-        mbar_expect_tx(bar_(A_FULL + s), CODE_BYTES);
-        tma_load_2d(base + OFF_A + s * STAGE_BYTES, &k_map, 0, static_cast<int>(key_row(t)), bar_(A_FULL + s));
-      }
+      const int s = t % QS_STAGES, use = t / QS_STAGES;
+      if (use > 0) ok = mbar_wait_warp(bar(QS_K_EMPTY + s), (use - 1) & 1, guard, 0x608 + s);
+      if (!ok) break;
+      cp_async_wait<QS_AHEAD - 1>();              // this lane's rows of page t have landed
+      ScaleRegs regs;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) regs.r[i] = *reinterpret_cast<const uint2*>(gbase + raw(t) + i * 256);
       store_scale_chunks(gbase + OFF_A + s * STAGE_BYTES + CODE_BYTES, regs, lane);
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar_(A_FULL + s));
-      if (t + 3 < num_tiles) regs = load_scales(p.ks + key_row(t + 3) * 8, 8, lane);
-      return true;
-    };
-    for (int t = 0; ok && t < num_tiles; t += 3) {
-      ok = step(t, ahead[0]);
-      if (ok && t + 1 < num_tiles) ok = step(t + 1, ahead[1]);
-      if (ok && t + 2 < num_tiles) ok = step(t + 2, ahead[2]);
+      if (lane == 0) mbar_arrive(bar(QS_K_FULL + s));
+      fetch(t + QS_AHEAD);
+      if (--left == 0) walk.next(p);
     }
-    if (!ok)
-      for (int t = max(0, num_tiles - A_STAGES); t < num_tiles; ++t)
-        mbar_wait_drain(bar_(A_FULL + t % A_STAGES), (t / A_STAGES) & 1);
+    cp_async_wait<0>();
   } else if (warp == 5) {
     // ----------------------------------------------------------- MMA issue (elected lane of a converged warp)
     constexpr uint32_t IDESC = idesc_nvf4(128, 128);
     const bool lead = elect_one();
-    bool ok = mbar_wait_warp(bar(B_FULL), 0, guard, 0x610);
-    if (ok) {
-      tc_fence_after();
-      const uint32_t sfq = tmem + TM_SFB;          // query scales: the A operand here
-      if (lead) {
-        tmem_cp_scales(sfq, desc_scale_chunk(base + OFF_B + CODE_BYTES));
-        tmem_cp_scales(sfq + 4, desc_scale_chunk(base + OFF_B + CODE_BYTES + 512));
-      }
-      const uint64_t a0 = desc_sw64_kmajor(base + OFF_B);
-      for (int t = 0; t < num_tiles; ++t) {
-        const int s = t % A_STAGES;
-        ok = mbar_wait_warp(bar(A_FULL + s), (t / A_STAGES) & 1, guard, 0x611 + s);
+    ScoreWalk<PACKED> walk(p, misc + 2);
+    bool ok = true;
+    int items = 0, left = 0;
+    for (int t = 0; t < total; ++t) {
+      const int slot = (items - (left ? 1 : 0)) & 1;       // of the current item's query tile
+      const uint32_t q_tile = base + QS_OFF_Q + slot * STAGE_BYTES;
+      const uint32_t sfq = tmem + QS_SFQ + slot * 8;       // query scales: the A operand here
+      if (left == 0) {
+        ok = mbar_wait_warp(bar(QS_Q_FULL + slot), (items >> 1) & 1, guard, 0x610 + slot);
         if (!ok) break;
         fence_async_smem();            // the producer's scale stores, for the copies below
         tc_fence_after();
-        const uint64_t b0 = desc_sw64_kmajor(base + OFF_A + s * STAGE_BYTES);
-        const uint32_t sfk = tmem + TM_SFA + (t & 1) * 8;
         if (lead) {
-          tmem_cp_scales(sfk, desc_scale_chunk(base + OFF_A + s * STAGE_BYTES + CODE_BYTES));
-          tmem_cp_scales(sfk + 4, desc_scale_chunk(base + OFF_A + s * STAGE_BYTES + CODE_BYTES + 512));
+          tmem_cp_scales(sfq, desc_scale_chunk(q_tile + CODE_BYTES));
+          tmem_cp_scales(sfq + 4, desc_scale_chunk(q_tile + CODE_BYTES + 512));
         }
-        if (t >= 1) {
-          ok = mbar_wait_warp(bar(ACC_EMPTY), (t - 1) & 1, guard, 0x618);
-          if (!ok) break;
-          tc_fence_after();
-        }
-        if (lead) {
+        ++items;
+        left = walk.count();
+        walk.next(p);
+      }
+      const int s = t % QS_STAGES;
+      ok = mbar_wait_warp(bar(QS_K_FULL + s), (t / QS_STAGES) & 1, guard, 0x612 + s);
+      if (!ok) break;
+      fence_async_smem();              // the producer's scale stores, for the copies below
+      tc_fence_after();
+      const uint64_t a0 = desc_sw64_kmajor(q_tile), b0 = desc_sw64_kmajor(base + OFF_A + s * STAGE_BYTES);
+      const uint32_t sfk = tmem + QS_SFK + (t & 1) * 8;
+      if (lead) {
+        tmem_cp_scales(sfk, desc_scale_chunk(base + OFF_A + s * STAGE_BYTES + CODE_BYTES));
+        tmem_cp_scales(sfk + 4, desc_scale_chunk(base + OFF_A + s * STAGE_BYTES + CODE_BYTES + 512));
+      }
+      if (t >= 1) {
+        ok = mbar_wait_warp(bar(QS_ACC_EMPTY), (t - 1) & 1, guard, 0x61a);
+        if (!ok) break;
+        tc_fence_after();
+      }
+      --left;
+      if (lead) {
 #pragma unroll
-          for (int kh = 0; kh < 2; ++kh)
-            mma_nvf4(tmem + TM_ACC, a0 + kh * 2, b0 + kh * 2, IDESC, sfq + kh * 4, sfk + kh * 4, kh);
-          tc_commit(bar(ACC_FULL));
-          tc_commit(bar(A_EMPTY + s));
-        }
+        for (int kh = 0; kh < 2; ++kh)
+          mma_nvf4(tmem + TM_ACC, a0 + kh * 2, b0 + kh * 2, IDESC, sfq + kh * 4, sfk + kh * 4, kh);
+        tc_commit(bar(QS_ACC_FULL));
+        tc_commit(bar(QS_K_EMPTY + s));
+        if (left == 0) tc_commit(bar(QS_Q_EMPTY + slot));
       }
     }
     __syncwarp();
@@ -1132,53 +1314,64 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
     // only reads the inputs, and those were complete before the fill kernel began).
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
-    const int r = warp * 32 + lane;
-    const bool alive = row_alive(r);
-    const int qi = row_query(r);
-    float* dst = p.out + (static_cast<long long>(row_head(r)) * p.tiles_out) * p.total_q + q_begin + qi;
-    // last visible key of this query (inclusive), relative to the request
-    const long long last_key = p.causal ? min(static_cast<long long>(k_len) - 1, static_cast<long long>(qi) + offset)
-                                        : static_cast<long long>(k_len) - 1;
+    const int row = warp * 32 + lane;
+    ScoreWalk<PACKED> walk(p, misc + 2);
     bool ok = true;
-    for (int t = 0; ok && t < num_tiles; ++t) {
-      bool w = mbar_wait(bar(ACC_FULL), t & 1, guard, 0x620);
-      ok = __all_sync(0xffffffffu, w);
-      if (!ok) break;
-      tc_fence_after();
-      const int pg = page0 + t;
-      const long long visible = last_key - static_cast<long long>(pg) * 128 + 1;     // visible keys of this page
-      float m = -INFINITY;
+    int t = 0;
+    while (ok && walk.left > 0) {
+      const int qi = PACKED ? row >> 4 : walk.j * 128 + row, head = PACKED ? row & (QS_PACK_HEADS - 1) : 0;
+      const int h0 = walk.head0(p);
+      const bool alive = qi < walk.r.q_rows && (!PACKED || walk.sub * QS_PACK_HEADS + head < p.group);
+      float* dst = p.out + static_cast<long long>(h0 + head) * p.tiles_out * p.total_q + walk.r.q_begin + qi;
+      // last visible key of this query (inclusive), relative to the request
+      const long long last_key = p.causal ? min(static_cast<long long>(walk.r.k_len) - 1, static_cast<long long>(qi) + walk.r.offset)
+                                          : static_cast<long long>(walk.r.k_len) - 1;
+      const int stop = walk.page + walk.count();
+      for (int pg = walk.page; pg < stop; ++pg, ++t) {
+        const int ph = __ldg(p.kv_indices + walk.r.page_begin + pg);      // (the page stays -inf where it is out of range)
+        bool w = mbar_wait(bar(QS_ACC_FULL), t & 1, guard, 0x620);
+        ok = __all_sync(0xffffffffu, w);
+        if (!ok) break;
+        tc_fence_after();
+        const long long visible = last_key - static_cast<long long>(pg) * 128 + 1;     // visible keys of this page
+        float m = -INFINITY;
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint32_t v[4][16];
+        for (int half = 0; half < 2; ++half) {
+          uint32_t v[4][16];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) tmem_ld16(tmem + lane_base + TM_ACC + half * 64 + c * 16, v[c]);
-        tc_wait_ld();
-        if (half == 1) {
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar(ACC_EMPTY));
-        }
-        if (visible >= (half + 1) * 64) {
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            float m5[5];
-#pragma unroll
-            for (int jj = 0; jj < 5; ++jj)
-              m5[jj] = max3(__uint_as_float(v[c][3 * jj]), __uint_as_float(v[c][3 * jj + 1]), __uint_as_float(v[c][3 * jj + 2]));
-            m = fmaxf(m, fmaxf(max3(m5[0], m5[1], m5[2]), max3(m5[3], m5[4], __uint_as_float(v[c][15]))));
+          for (int c = 0; c < 4; ++c) tmem_ld16(tmem + lane_base + TM_ACC + half * 64 + c * 16, v[c]);
+          tc_wait_ld();
+          if (half == 1) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(QS_ACC_EMPTY));
           }
-        } else if (visible > half * 64) {
-          const int n = static_cast<int>(visible) - half * 64;           // 1 .. 63 visible columns of this half
+          if (visible >= (half + 1) * 64) {
 #pragma unroll
-          for (int c = 0; c < 4; ++c)
+            for (int c = 0; c < 4; ++c) {
+              float m5[5];
 #pragma unroll
-            for (int jj = 0; jj < 16; ++jj)
-              if (c * 16 + jj < n) m = fmaxf(m, __uint_as_float(v[c][jj]));
+              for (int jj = 0; jj < 5; ++jj)
+                m5[jj] = max3(__uint_as_float(v[c][3 * jj]), __uint_as_float(v[c][3 * jj + 1]), __uint_as_float(v[c][3 * jj + 2]));
+              m = fmaxf(m, fmaxf(max3(m5[0], m5[1], m5[2]), max3(m5[3], m5[4], __uint_as_float(v[c][15]))));
+            }
+          } else if (visible > half * 64) {
+            const int n = static_cast<int>(visible) - half * 64;           // 1 .. 63 visible columns of this half
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+#pragma unroll
+              for (int jj = 0; jj < 16; ++jj)
+                if (c * 16 + jj < n) m = fmaxf(m, __uint_as_float(v[c][jj]));
+          }
         }
+        if (alive && ph >= 0 && ph < p.total_pages) dst[static_cast<long long>(pg) * p.total_q] = m;
       }
-      if (alive && phys_page(pg) >= 0) dst[static_cast<long long>(pg) * p.total_q] = m;
+      walk.next(p);
     }
+  }
+  } else {
+    // nothing to score: the grid must still not be complete before the fill kernel is
+    asm volatile("griddepcontrol.wait;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
@@ -1326,8 +1519,9 @@ int launch_fp4_scores_varlen_nv(const void* qp, const void* qs, const void* kp, 
   p.tiles_out = (max_seqlen_k + 127) / 128;
   p.causal = causal;
   const bool packed = max_seqlen_q <= QS_PACK_Q && hq / hk > 1;
-  p.head_blocks = (hq / hk + QS_PACK_HEADS - 1) / QS_PACK_HEADS;
-  const long long items = packed ? static_cast<long long>(batch) * hk * p.head_blocks
+  p.group = hq / hk;
+  p.subs = packed ? (p.group + QS_PACK_HEADS - 1) / QS_PACK_HEADS : p.group;
+  const long long items = packed ? static_cast<long long>(batch) * hk * p.subs
                                  : static_cast<long long>(batch) * p.qt_max * hq;
   if (items > 0x7fffffffLL) return set_error(SB_ERR_INVALID, "too many (request, query tile, head) items");
   const long long n = static_cast<long long>(hq) * p.tiles_out * total_q;
@@ -1336,13 +1530,9 @@ int launch_fp4_scores_varlen_nv(const void* qp, const void* qs, const void* kp, 
   const cudaError_t filled = cudaGetLastError();
   if (filled != cudaSuccess) return set_error(SB_ERR_CUDA, cudaGetErrorString(filled));
   if (items == 0 || p.tiles_out == 0) return SB_OK;
-  // enough CTAs to fill the GPU twice over, as long a run of pages per CTA as that allows (the query tile is
-  // loaded once per CTA)
-  int ppc = 64;
-  while (ppc > 2 && ((p.tiles_out + ppc - 1) / ppc) * items < 4LL * ctx->sm_count) ppc >>= 1;
-  p.pages_per_cta = ppc;
-  const dim3 grid(static_cast<unsigned>(items), static_cast<unsigned>((p.tiles_out + ppc - 1) / ppc));
-  if (grid.y > 65535) return set_error(SB_ERR_INVALID, "too many KV pages per request");
+  // two CTAs per SM, at least two pages each
+  const long long most = (items * p.tiles_out + 1) / 2;
+  const dim3 grid(static_cast<unsigned>(std::min<long long>(2LL * ctx->sm_count, most)));
   CUtensorMap qm, km;
   {
     const cuuint64_t dims[3] = {64, static_cast<cuuint64_t>(hq), static_cast<cuuint64_t>(total_q)};
@@ -1362,18 +1552,17 @@ int launch_fp4_scores_varlen_nv(const void* qp, const void* qs, const void* kp, 
                      CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B))
       return set_error(SB_ERR_CUDA, "cuTensorMapEncodeTiled failed for the key codes");
   }
-  const size_t smem = QS_OFF_AUX + 256 + 1024;
   if (!(ctx->tc_attr & (1 << 12))) {
-    cudaError_t e = cudaFuncSetAttribute(fp4_nv_query_scores_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536);
+    cudaError_t e = cudaFuncSetAttribute(fp4_nv_query_scores_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, QS_SMEM);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(fp4_nv_query_scores_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536);
+      e = cudaFuncSetAttribute(fp4_nv_query_scores_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, QS_SMEM);
     if (e != cudaSuccess) return set_error(SB_ERR_CUDA, cudaGetErrorString(e));
     ctx->tc_attr |= (1 << 12);
   }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(QS_THREADS);
-  cfg.dynamicSmemBytes = smem;
+  cfg.dynamicSmemBytes = QS_SMEM;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -798,6 +798,43 @@ def test_fp4_varlen_scores_against_the_reference_scorer(causal):
     m.device_status()
 
 
+@pytest.mark.parametrize("requests,hq,hk,q_hi,k_hi,causal,offsets", [
+    (1, 1, 1, 1, 100, False, False),           # one page: one CTA has a run, the others none
+    (3, 6, 2, 300, 700, True, False),          # heads of a group and query tiles follow each other within a run
+    (70, 3, 3, 40, 900, True, True),           # more requests than a warp has lanes, some of them empty
+    (45, 40, 2, 8, 1500, True, False),         # packed rows, two blocks of heads per KV head
+    (33, 16, 1, 5, 6000, False, False),        # packed, more than 32 pages per item
+    (2, 2, 1, 4500, 5200, True, True),         # more than 32 query tiles
+])
+def test_fp4_varlen_runs_of_pages(requests, hq, hk, q_hi, k_hi, causal, offsets):
+    """The tensor-core scorer cuts the pages of all (request, tile, head) items into equal runs on the device: against the
+    exact scorer, which takes item by item. Same -inf pattern; finite scores within the bound on the tensor core's sums,
+    2^-18 of (largest L1 norm of a query) x (largest key element), at most 128 * 6 * 6 * the largest scales."""
+    m = sp()
+    rng = np.random.RandomState(requests * 31 + hq)
+    q_lens = [int(x) for x in rng.randint(1, q_hi + 1, requests)]
+    k_lens = [int(x) for x in rng.randint(1, k_hi + 1, requests)]
+    if requests > 2:
+        q_lens[1] = 0                          # nothing to score
+        k_lens[2] = 1
+    qp, qs, kp, ks, cu_q, cu_k, cu_p, kv_idx = _varlen_case(5 + requests, hq, hk, q_lens, k_lens)
+    if requests > 1:
+        kv_idx[0] = kp.shape[0] + 3            # out of range: that page stays -inf
+    dev = [t.cuda() for t in (qp, kp, qs, ks, cu_q, cu_k, cu_p)]
+    kw = dict(max_seqlen_q=max(q_lens), max_seqlen_k=max(k_lens), kv_indices=kv_idx.cuda(), causal=causal)
+    if offsets:
+        kw["qo_offset"] = torch.from_numpy(rng.randint(-100, 600, requests).astype(np.int32)).cuda()
+    exact = m.fp4_block_scores_varlen(*dev, **kw)
+    for _ in range(2):
+        fast = m.fp4_block_scores_varlen(*dev, exact=False, **kw)
+        torch.cuda.synchronize()
+        m.device_status()
+        assert torch.equal(torch.isinf(exact), torch.isinf(fast))
+        fin = torch.isfinite(exact)
+        scale = max(float(qs.float().max()) * float(ks.float().max()), 1.0)
+        assert (exact[fin] - fast[fin]).abs().max().item() <= 128 * 36 * scale * 2.0 ** -18
+
+
 def test_fp4_scores_varlen_inconsistent_lengths_stay_in_bounds():
     """max_seqlen_k smaller than one request's key length, a page table shorter than the key
     length claims, and cu_seqlens_q that runs past total_q: the kernel must skip what does not fit.
