@@ -39,7 +39,7 @@ namespace fnv {
 constexpr int CODE_BYTES = 128 * 64;              // one operand tile: 128 rows of 64 bytes of codes
 constexpr int SF_BYTES = 1024;                    // its scales: two 512-byte chunks (features 0-63, 64-127)
 constexpr int STAGE_BYTES = CODE_BYTES + SF_BYTES;
-constexpr int A_STAGES = 4;
+constexpr int A_STAGES = 6;
 constexpr int C_MAX = 192;
 constexpr int NUM_THREADS = 320;
 constexpr int TMA_WARP = 8, MMA_WARP = 9;
@@ -55,7 +55,9 @@ constexpr int ACC_STAGES = 1;                     // accumulators of 128 columns
 
 constexpr int OFF_A = 0;
 constexpr int OFF_B = A_STAGES * STAGE_BYTES;     // query tile: codes + scales
-constexpr int OFF_CAND = OFF_B + STAGE_BYTES;     // candidate arrays of the selection phase
+constexpr int RAW_STAGES = 4;                     // pages whose scales are on their way
+constexpr int OFF_RAW = OFF_B + STAGE_BYTES;      // staging ring: the scales of a page as they are in memory
+constexpr int OFF_CAND = OFF_RAW + RAW_STAGES * SF_BYTES;   // candidate arrays of the selection phase
 constexpr int OFF_SCORES = OFF_CAND + 4 * C_MAX * 4;
 // the selection phase re-uses [0, OFF_CAND) for int8 rows and fp32 scales of a query tile and a key page
 static_assert(2 * 128 * FP4_ROW_WORDS * 4 + 2 * 128 * 8 * 4 <= OFF_CAND, "staging area of the exact scorer does not fit");
@@ -210,19 +212,19 @@ struct Geometry {
 };
 
 // ---------------------------------------------------------------- producer and MMA roles
-// A page takes about 440 cycles of an SM with two CTAs on it, against 128 cycles of MMAs: the serial work of lone warps
+// A page takes about 430 cycles of an SM with two CTAs on it, against 128 cycles of MMAs: the serial work of lone warps
 // (waits, scale copies, hand-overs) bounds it, in the producer, the MMA warp and the epilogue alike: leaving out any one of
-// maxima, accumulator reads, TMA copies or scale stores changes nothing. 450 when the producer fenced its scale stores for the
-// async proxy (a fence takes 300 cycles, and waits for the loads in flight; now the MMA warp does it, when a page
-// has landed), 520 when one lane issued under `if (lane == 0)`, see elect_one(). No faster: one CTA per SM with three
-// accumulators and one to four producer warps (540 to 720), two or three producer warps per CTA here (450), three
-// accumulators of 64 columns per CTA (450).
+// maxima, accumulator reads, TMA copies or scale stores changes nothing. 440 when the producer loaded the scales into
+// registers, in a loop unrolled over the pages in flight, 450 when it also fenced its scale stores for the async proxy (a fence
+// takes 300 cycles, and waits for the loads in flight; now the MMA warp does it, when a page has landed), 520 when one lane
+// issued under `if (lane == 0)`, see elect_one(). No faster: one CTA per SM with three accumulators and one to four producer
+// warps (540 to 720), two or three producer warps per CTA here (450), three accumulators of 64 columns per CTA (450).
 // Producer warp: query tile once, then key pages page0 + (t + rot) % wrap for t = 0 .. num_tiles - 1 (num_tiles <= wrap,
 // rot < wrap).
 __device__ __forceinline__ void producer_role(const Geometry& g, const CUtensorMap* q_map, const CUtensorMap* k_map,
                                               uint32_t base, unsigned char* gbase, uint32_t bar0, const Guard& guard,
                                               int b, int h, int hk_idx, long long q_row0, int page0, int num_tiles,
-                                              int rot, int wrap, int lane, int code0, volatile int* key_scale_max) {
+                                              int rot, int wrap, int lane, int code0) {
   auto bar = [&](int i) { return bar0 + 8u * i; };
   auto page_of = [&](int t) { return page0 + (t + rot >= wrap ? t + rot - wrap : t + rot); };
   auto key_row = [&](int pg) { return ((static_cast<long long>(b) * g.tiles + pg) * g.hk + hk_idx) * 128; };
@@ -237,43 +239,39 @@ __device__ __forceinline__ void producer_role(const Geometry& g, const CUtensorM
     __syncwarp();
     if (lane == 0) mbar_arrive(bar(B_FULL));
   }
-  // The scales of a page come through registers: requested three pages ahead, so that the producer
-  // never waits a full global-memory latency per page.
-  bool ok = true;
-  uint32_t seen = 0;                 // bytewise maximum of the key scales that went through this warp
-  ScaleRegs ahead[3];
+  // The scales of a page are staged RAW_STAGES pages ahead by asynchronous copies, a lane its rows lane, lane + 32, .., and
+  // re-ordered from there. (Loads into registers need the loop unrolled over the pages in flight.)
+  auto raw = [&](int t) { return OFF_RAW + (t % RAW_STAGES) * SF_BYTES + lane * 8; };
+  auto fetch = [&](int t) {
+    if (t < num_tiles) {
+      const uint8_t* src = g.ks + key_row(page_of(t)) * 8 + lane * 8;
 #pragma unroll
-  for (int i = 0; i < 3; ++i)
-    if (i < num_tiles) ahead[i] = load_scales(g.ks + key_row(page_of(i)) * 8, 8, lane);
-  auto step = [&](int t, ScaleRegs& regs) -> bool {
-    const int s = t % A_STAGES, use = t / A_STAGES;
-    if (use > 0) {
-      bool w = mbar_wait(bar(A_EMPTY + s), (use - 1) & 1, guard, code0 + s);
-      if (!__all_sync(0xffffffffu, w)) return false;
+      for (int i = 0; i < 4; ++i) cp_async8(base + raw(t) + i * 256, src + i * 256);
     }
+    cp_async_commit();
+  };
+#pragma unroll 1
+  for (int t = 0; t < RAW_STAGES; ++t) fetch(t);
+  bool ok = true;
+#pragma unroll 1
+  for (int t = 0; t < num_tiles; ++t) {
+    const int s = t % A_STAGES, use = t / A_STAGES;
+    if (use > 0) ok = mbar_wait_warp(bar(A_EMPTY + s), (use - 1) & 1, guard, code0 + s);
+    if (!ok) break;
     if (lane == 0) {
       mbar_expect_tx(bar(A_FULL + s), CODE_BYTES);
       tma_load_2d(base + OFF_A + s * STAGE_BYTES, k_map, 0, static_cast<int>(key_row(page_of(t))), bar(A_FULL + s));
     }
-    store_scale_chunks(gbase + OFF_A + s * STAGE_BYTES + CODE_BYTES, regs, lane);
+    cp_async_wait<RAW_STAGES - 1>();
+    ScaleRegs regs;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) seen = max_scale_bytes(max_scale_bytes(seen, regs.r[i].x), regs.r[i].y);
+    for (int i = 0; i < 4; ++i) regs.r[i] = *reinterpret_cast<const uint2*>(gbase + raw(t) + i * 256);
+    store_scale_chunks(gbase + OFF_A + s * STAGE_BYTES + CODE_BYTES, regs, lane);
     __syncwarp();
     if (lane == 0) mbar_arrive(bar(A_FULL + s));
-    if (t + 3 < num_tiles) regs = load_scales(g.ks + key_row(page_of(t + 3)) * 8, 8, lane);
-    return true;
-  };
-  for (int t = 0; ok && t < num_tiles; t += 3) {
-    ok = step(t, ahead[0]);
-    if (ok && t + 1 < num_tiles) ok = step(t + 1, ahead[1]);
-    if (ok && t + 2 < num_tiles) ok = step(t + 2, ahead[2]);
+    fetch(t + RAW_STAGES);
   }
-  if (key_scale_max) {
-    uint32_t m = top_byte(seen);
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, d));
-    if (lane == 0) *key_scale_max = static_cast<int>(m);
-  }
+  cp_async_wait<0>();
   if (!ok)
     for (int t = max(0, num_tiles - A_STAGES); t < num_tiles; ++t)
       mbar_wait_drain(bar(A_FULL + t % A_STAGES), (t / A_STAGES) & 1);
@@ -425,7 +423,7 @@ fp4_nv_select_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
 
   if (warp == TMA_WARP) {
     producer_role(g, &q_map, &k_map, base, gbase, bar0, guard, b, h, hk_idx, q_row0, 0, num_tiles, rot, num_tiles, lane,
-                  0x500, nullptr);
+                  0x500);
   } else if (warp == MMA_WARP) {
     mma_role(base, bar0, tmem, guard, num_tiles, 0x510);
     __syncwarp();
@@ -759,7 +757,7 @@ fp4_nv_prune_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
 
   if (warp == TMA_WARP) {
     producer_role(g, &q_map, &k_map, base, gbase, bar0, guard, b, h, hk_idx, q_row0, page0, num_tiles, 0, num_tiles, lane,
-                  0x580, nullptr);
+                  0x580);
   } else if (warp == MMA_WARP) {
     mma_role(base, bar0, tmem, guard, num_tiles, 0x590);
     __syncwarp();
