@@ -6,6 +6,8 @@ Differences the block-list contract brings: selections are per query BLOCK
 ([B,Hkv,Sq/128,TopK], any TopK) and q stays head-major [B,Hq,Sq,128]; the
 reverse index is by KV range (nseg ranges) instead of by single block, so the
 partial buffers are nseg x the output instead of TopK x (none with a single range)."""
+import functools
+
 import torch
 
 from . import _lib
@@ -32,6 +34,11 @@ def default_segments(kv_blocks, topk, items=None, rows=0, sm_count=148):
     return min((n for n in (1, 2, 4) if n <= min(kv_blocks, topk)), key=cost, default=1)
 
 
+@functools.lru_cache(maxsize=None)
+def _sm_count(device):
+    return torch.cuda.get_device_properties(device).multi_processor_count
+
+
 def _default_ranges(q, k, topk, partial):
     b, hq, sq, _ = q.shape
     hkv, blocks = k.shape[1], k.shape[2] // 128
@@ -39,8 +46,7 @@ def _default_ranges(q, k, topk, partial):
         return default_segments(blocks, topk)
     group, qb = hq // hkv, sq // 128
     items = b * hkv * qb * (group // 2) if group % 2 == 0 else b * hq * ((qb + 1) // 2)
-    return default_segments(blocks, topk, items, b * hq * sq,
-                            torch.cuda.get_device_properties(q.device).multi_processor_count)
+    return default_segments(blocks, topk, items, b * hq * sq, _sm_count(q.device.index))
 
 
 class Prepared:
