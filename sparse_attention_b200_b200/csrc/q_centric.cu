@@ -78,6 +78,21 @@ constexpr int OFF_MISC = OFF_BAR + NUM_BARS * 8;   // tmem base (4 B), abort fla
 constexpr int SMEM_BYTES = OFF_MISC + 48 + 1024;   // + slack for manual 1024 alignment
 static_assert(SMEM_BYTES <= 227 * 1024, "shared memory map exceeds the per-CTA limit");
 
+// Division of 0 <= n < 2^31 by a number that the host knows: one wide multiplication and a shift (exact: the multiplier
+// exceeds 2^(31 + s) / d by less than one, 2^s >= d). Every role places its items by half a dozen divisions, and a role's first
+// one stands before the first loads.
+struct FastDiv {
+  uint32_t mul, shift;
+  __host__ static FastDiv by(int d) {
+    uint32_t s = 0;
+    while ((1ll << s) < d) ++s;
+    return {static_cast<uint32_t>(((1ull << (31 + s)) + d - 1) / d), 31 + s};
+  }
+  __device__ __forceinline__ int operator()(int n) const {
+    return static_cast<int>((static_cast<unsigned long long>(static_cast<uint32_t>(n)) * mul) >> shift);
+  }
+};
+
 struct Params {
   const int32_t* ids;      // [nseg, B, Hkv, Qt, topk]
   const int32_t* counts;   // [nseg, B, Hkv, Qt] or nullptr (= topk everywhere)
@@ -96,6 +111,7 @@ struct Params {
   int tail_first, tail_parts, num_virtual;
   float* tail_lse;         // [pieces * 2 * 128]
   int dead_zero;           // rows without any weight are 0 (see QCentricArgs)
+  FastDiv by_parts, by_seg, by_pairs, by_qt, by_hkv, by_qpairs, by_hq, by_group;
 };
 
 struct Stream {
@@ -108,23 +124,22 @@ struct Stream {
   bool tail;           // a piece of a tail item: out_row is a row of the workspace
 };
 
-__device__ __forceinline__ void decode_item(const Params& p, int virt, Stream (&s)[2]) {
+// pair_mode: p.pair_mode, a constant where the kernel's instantiation knows it
+__device__ __forceinline__ void decode_item(const Params& p, bool pair_mode, int virt, Stream (&s)[2]) {
   int item = virt, part = 0;
   const bool tail = virt >= p.tail_first;
   if (tail) {
     const int t = virt - p.tail_first;
-    item = p.tail_first + t / p.tail_parts;
-    part = t - (t / p.tail_parts) * p.tail_parts;
+    const int whole = p.by_parts(t);
+    item = p.tail_first + whole;
+    part = t - whole * p.tail_parts;
   }
-  const int seg = item / p.items_per_seg;
+  const int seg = p.by_seg(item);
   const int local = item - seg * p.items_per_seg;
-  if (p.pair_mode) {
-    const int pairs = p.group >> 1;
-    const int pair = local % pairs;
-    const int t = local / pairs;
-    const int qtile = t % p.qt;
-    const int bk = t / p.qt;            // batch * Hkv + kv head
-    const int b = bk / p.hkv, kvh = bk - b * p.hkv;
+  if (pair_mode) {
+    const int t = p.by_pairs(local), pair = local - t * (p.group >> 1);
+    const int bk = p.by_qt(t), qtile = t - bk * p.qt;      // bk: batch * Hkv + kv head
+    const int b = p.by_hkv(bk), kvh = bk - b * p.hkv;
     const long long row = (static_cast<long long>(seg) * p.batch * p.hkv + bk) * p.qt + qtile;
     const int cnt = p.counts ? p.counts[row] : p.topk;
 #pragma unroll
@@ -140,10 +155,9 @@ __device__ __forceinline__ void decode_item(const Params& p, int virt, Stream (&
     }
   } else {
     const int qpairs = (p.qt + 1) >> 1;
-    const int qp = local % qpairs;
-    const int bh = local / qpairs;      // batch * Hq + head
-    const int b = bh / p.hq, head = bh - b * p.hq;
-    const int kvh = head / p.group;
+    const int bh = p.by_qpairs(local), qp = local - bh * qpairs;      // bh: batch * Hq + head
+    const int b = p.by_hq(bh), head = bh - b * p.hq;
+    const int kvh = p.by_group(head);
     const int bk = b * p.hkv + kvh;
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
@@ -164,7 +178,7 @@ __device__ __forceinline__ void decode_item(const Params& p, int virt, Stream (&
     s[q].count = min(max(s[q].count, 0), p.topk);
     s[q].tail = tail;
     if (tail) {                                  // this piece's share of the list, its rows in the workspace
-      const int lo = part * s[q].count / p.tail_parts, hi = (part + 1) * s[q].count / p.tail_parts;
+      const int lo = p.by_parts(part * s[q].count), hi = p.by_parts((part + 1) * s[q].count);
       s[q].list += lo;
       s[q].count = hi - lo;
       s[q].out_row = (static_cast<long long>(virt - p.tail_first) * 2 + q) * TILE;
@@ -174,34 +188,35 @@ __device__ __forceinline__ void decode_item(const Params& p, int virt, Stream (&
 
 // Live list lengths of the two streams of an item: all the MMA issuer needs to know
 // (it keeps few registers so that its wait -> issue path stays free of spills).
-__device__ __forceinline__ void item_counts(const Params& p, int virt, int (&cnt)[2]) {
+__device__ __forceinline__ void item_counts(const Params& p, bool pair_mode, int virt, int (&cnt)[2]) {
   int item = virt, part = 0;
   const bool tail = virt >= p.tail_first;
   if (tail) {
     const int t = virt - p.tail_first;
-    item = p.tail_first + t / p.tail_parts;
-    part = t - (t / p.tail_parts) * p.tail_parts;
+    const int whole = p.by_parts(t);
+    item = p.tail_first + whole;
+    part = t - whole * p.tail_parts;
   }
-  const int seg = item / p.items_per_seg;
+  const int seg = p.by_seg(item);
   const int local = item - seg * p.items_per_seg;
-  if (p.pair_mode) {
+  if (pair_mode) {
     int c = p.topk;
     if (p.counts) {
-      const int t = local / (p.group >> 1);          // (batch * Hkv + kv head) * Qt + query tile
+      const int t = p.by_pairs(local);               // (batch * Hkv + kv head) * Qt + query tile
       c = p.counts[static_cast<long long>(seg) * p.batch * p.hkv * p.qt + t];
     }
     cnt[0] = cnt[1] = min(max(c, 0), p.topk);
   } else {
     const int qpairs = (p.qt + 1) >> 1;
-    const int bh = local / qpairs;
+    const int bh = p.by_qpairs(local);
     const int qp = local - bh * qpairs;
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
       const int qtile = 2 * qp + q;
       int c = qtile < p.qt ? p.topk : 0;
       if (p.counts && qtile < p.qt) {
-        const int b = bh / p.hq, head = bh - b * p.hq;
-        const int bk = b * p.hkv + head / p.group;
+        const int b = p.by_hq(bh), head = bh - b * p.hq;
+        const int bk = b * p.hkv + p.by_group(head);
         c = p.counts[(static_cast<long long>(seg) * p.batch * p.hkv + bk) * p.qt + qtile];
       }
       cnt[q] = min(max(c, 0), p.topk);
@@ -209,7 +224,7 @@ __device__ __forceinline__ void item_counts(const Params& p, int virt, int (&cnt
   }
   if (tail) {
 #pragma unroll
-    for (int q = 0; q < 2; ++q) cnt[q] = (part + 1) * cnt[q] / p.tail_parts - part * cnt[q] / p.tail_parts;
+    for (int q = 0; q < 2; ++q) cnt[q] = p.by_parts((part + 1) * cnt[q]) - p.by_parts(part * cnt[q]);
   }
 }
 
@@ -246,7 +261,12 @@ __device__ __forceinline__ int slice_of(const ScatterOn& sc, long long& out_row)
 }
 __device__ __forceinline__ int slice_of(const ScatterOff&, long long&) { return 0; }
 
-template <bool OUT_F32, typename Scatter>
+// PAIR: pair mode (see the head of this file). An instantiation of its own for each mode: the roles' loops hold one mode's
+// code, and no branch on it (with a load of the parameter that the issuer has no register to keep) stands between a wait and
+// its MMAs. With FastDiv, which alone made the compiler reload more (all cases 3-12 % slower): 16 heads over 16 Ki keys
+// 126 -> 115.5 us, 32 heads at 32 Ki 1106 -> 1080 us, 1 Mi-token group 33.3 -> 32.7 ms, R1 selection + attention of a
+// 4 Ki prompt 35.1 -> 33.0 us.
+template <bool OUT_F32, bool PAIR, typename Scatter>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
                  const __grid_constant__ CUtensorMap v_map, const __grid_constant__ CUtensorMap o_map,
@@ -348,12 +368,12 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
     bool primed[2] = {false, false};
     for (int item = blockIdx.x; ok && item < p.num_virtual; item += gridDim.x) {
       Stream s[2], nx[2];
-      decode_item(p, item, s);
+      decode_item(p, PAIR, item, s);
       const bool has_next = item + static_cast<int>(gridDim.x) < p.num_virtual;
-      if (has_next) decode_item(p, item + gridDim.x, nx);
+      if (has_next) decode_item(p, PAIR, item + gridDim.x, nx);
       IdCursor kc[2], vc[2], nc[2];
       kc[0].cached = kc[1].cached = vc[0].cached = vc[1].cached = nc[0].cached = nc[1].cached = 0;
-      if (p.pair_mode) {
+      if constexpr (PAIR) {
         const int n = s[0].count;
         const bool was_primed = primed[0];
         primed[0] = primed[1] = false;
@@ -480,7 +500,7 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
     // in-order issuer costs more than the early start gains, +3 %).
     uint32_t hphase[2] = {0, 0};
     auto pv = [&](int q, uint32_t slot, bool accumulate) -> bool {
-      if (p.pair_mode) {
+      if (PAIR) {
         if (!mbar_wait_warp(bar(BAR_P_HALF + q), hphase[q], guard, 0x230 + q)) return false;
         hphase[q] ^= 1;
         tc_fence_after();
@@ -492,7 +512,7 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
         if (!mbar_wait_warp(bar(BAR_O_EMPTY + q), (o_done[q] - 1) & 1, guard, 0x240 + q)) return false;
         tc_fence_after();
       }
-      if (p.pair_mode) {
+      if (PAIR) {
         issue_pv_part(q, slot, accumulate, 0, 6);
         if (!wait_p(q)) return false;
         issue_pv_part(q, slot, accumulate, 6, 8);
@@ -506,13 +526,13 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
 
     bool primed[2] = {false, false};
     int cnt[2] = {0, 0}, ncnt[2] = {0, 0};
-    if (static_cast<int>(blockIdx.x) < p.num_virtual) item_counts(p, blockIdx.x, ncnt);
+    if (static_cast<int>(blockIdx.x) < p.num_virtual) item_counts(p, PAIR, blockIdx.x, ncnt);
     for (int item = blockIdx.x; ok && item < p.num_virtual; item += gridDim.x) {
       cnt[0] = ncnt[0]; cnt[1] = ncnt[1];
       const bool has_next = item + static_cast<int>(gridDim.x) < p.num_virtual;
-      if (has_next) item_counts(p, item + gridDim.x, ncnt);
+      if (has_next) item_counts(p, PAIR, item + gridDim.x, ncnt);
       uint32_t kslot = 0, vslot = 0;
-      if (p.pair_mode) {
+      if constexpr (PAIR) {
         const int n = cnt[0];
         const bool was_primed = primed[0];
         primed[0] = primed[1] = false;
@@ -618,7 +638,7 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
     bool ok = true;
     for (int item = blockIdx.x; ok && item < p.num_virtual; item += gridDim.x) {
       Stream s[2];
-      decode_item(p, item, s);
+      decode_item(p, PAIR, item, s);
       const Stream& me = s[q];
       if (!me.valid) continue;
       // (scatter launches look their destination up where they store, after the loop: nothing more to keep in
@@ -729,7 +749,7 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
             pk[j] = pack_bf16x2(e.x, e.y);
           }
           tmem_st16(t_s + c * 16, pk);
-          if (c == 2 && p.pair_mode) {
+          if (c == 2 && PAIR) {
             tc_wait_st();
             tc_fence_before();
             __syncwarp();
@@ -779,7 +799,7 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
     bool ok = true;
     for (int item = blockIdx.x; ok && item < p.num_virtual; item += gridDim.x) {
       Stream s[2];
-      decode_item(p, item, s);
+      decode_item(p, PAIR, item, s);
 #pragma unroll 1
       for (int q = 0; ok && q < 2; ++q) {
         const Stream& me = s[q];
@@ -898,7 +918,7 @@ __global__ void __launch_bounds__(128) tail_merge_kernel(const Params p, const T
   real.tail_first = p.num_items;                 // decode the item itself, not a piece of it
   Stream s[2];
   asm volatile("griddepcontrol.wait;" ::: "memory");      // the attention kernel's stores are visible from here on
-  decode_item(real, p.tail_first + t, s);
+  decode_item(real, p.pair_mode != 0, p.tail_first + t, s);
   if (!s[q].valid) return;
   const int part16 = threadIdx.x & 15;
   const int row = (blockIdx.x & 15) * 8 + (threadIdx.x >> 4);
@@ -1074,6 +1094,15 @@ int launch_q_centric(const QCentricArgs& a, cudaStream_t stream) {
     }
   }
 
+  p.by_parts = FastDiv::by(p.tail_parts);
+  p.by_seg = FastDiv::by(p.items_per_seg);
+  p.by_pairs = FastDiv::by(p.pair_mode ? group / 2 : 1);
+  p.by_qt = FastDiv::by(p.qt);
+  p.by_hkv = FastDiv::by(a.hkv);
+  p.by_qpairs = FastDiv::by((p.qt + 1) / 2);
+  p.by_hq = FastDiv::by(a.hq);
+  p.by_group = FastDiv::by(group);
+
   CUtensorMap qm, km, vm, om, omt;
   if (encode_rows_map(&qm, a.q, static_cast<uint64_t>(a.batch) * a.hq * a.sq) ||
       encode_rows_map(&km, a.k, static_cast<uint64_t>(a.batch) * a.hkv * a.skv) ||
@@ -1104,25 +1133,28 @@ int launch_q_centric(const QCentricArgs& a, cudaStream_t stream) {
       if (encode_out_map(&sc.m[j - 1], a.owner_out[j], static_cast<uint64_t>(rows / a.owners), false))
         return set_error(SB_ERR_CUDA, "cuTensorMapEncodeTiled failed for a slice's destination");
     }
-    if (!(ctx->tc_attr & (1 << 19))) {
-      cudaError_t e = cudaFuncSetAttribute(q_centric_kernel<false, ScatterOn>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    auto kernel = p.pair_mode ? q_centric_kernel<false, true, ScatterOn> : q_centric_kernel<false, false, ScatterOn>;
+    const int configured = p.pair_mode ? 1 << 20 : 1 << 19;
+    if (!(ctx->tc_attr & configured)) {
+      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
       if (e != cudaSuccess) return set_error(SB_ERR_CUDA, cudaGetErrorString(e));
-      ctx->tc_attr |= (1 << 19);
+      ctx->tc_attr |= configured;
     }
-    q_centric_kernel<false, ScatterOn><<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(qm, km, vm, om, om, p, sc);
+    kernel<<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(qm, km, vm, om, om, p, sc);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? SB_OK : set_error(SB_ERR_CUDA, cudaGetErrorString(e));
   }
   // (when the whole launch writes fp32 partials, the kernel is the fp32 one although the output is bf16: only the merge
   // writes output rows then)
   const bool f32 = a.out_f32 || tail_f32;
-  auto kernel = f32 ? q_centric_kernel<true, ScatterOff> : q_centric_kernel<false, ScatterOff>;
-  int& configured = f32 ? ctx->qc_attr_f32 : ctx->qc_attr_bf16;
-  if (!configured) {
+  auto kernel = f32 ? (p.pair_mode ? q_centric_kernel<true, true, ScatterOff> : q_centric_kernel<true, false, ScatterOff>)
+                    : (p.pair_mode ? q_centric_kernel<false, true, ScatterOff> : q_centric_kernel<false, false, ScatterOff>);
+  int& configured = f32 ? ctx->qc_attr_f32 : ctx->qc_attr_bf16;      // one bit per mode
+  const int mode = 1 << p.pair_mode;
+  if (!(configured & mode)) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     if (e != cudaSuccess) return set_error(SB_ERR_CUDA, cudaGetErrorString(e));
-    configured = 1;
+    configured |= mode;
   }
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
