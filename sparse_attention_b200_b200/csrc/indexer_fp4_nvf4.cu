@@ -8,7 +8,7 @@
 // instructions cover the 128 features. The scales of a 128-row tile are re-ordered by the producer
 // warp into the 512-byte "32 x (4 row groups x 4 scales)" chunks the instruction reads
 // (byte (r % 32) * 16 + (r / 32) * 4 + j = scale j of row r) and copied to tensor memory with
-// tcgen05.cp.32x128b.warpx4 by the MMA thread. One 128 x 128 accumulator, two key-scale slots and the
+// tcgen05.cp.32x128b.warpx4 by the elected lane of the MMA warp. One 128 x 128 accumulator, two key-scale slots and the
 // query scales take 152 tensor-memory columns (256 allocated), so two CTAs share an SM and the
 // epilogue of one runs under the MMAs of the other. (N = 64 halves of the query tile with three
 // accumulators per CTA were measured slower: an M128 N64 K64 instruction takes nearly as long as
