@@ -12,9 +12,11 @@
 // Same results as pool_blocks / descriptor_dot / reduce_topk
 // (indexers/r1_r4/gpu_ops.py:6-49): ids in score-descending order, ties to the lower id.
 #include "internal.h"
+#include "ptx.cuh"
 #include "topk.cuh"
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
+#include <type_traits>
 
 namespace sb {
 namespace {
@@ -55,11 +57,17 @@ __global__ void __launch_bounds__(256) pool_small_kernel(const __nv_bfloat16* __
 // A row tile is ROWS = 16 QT query descriptors (QT = 1, 2 or 4): L lists (query blocks of one KV head) of MP descriptors
 // each (MP = group heads x R rounded up to a power of two, padding repeats a list's first descriptor: the maximum is
 // unchanged). A cluster of C CTAs (C = 1, 2, 4 or 8) shares the row tile: CTA `rank` scores the key chunks rank,
-// rank + C, ... of 64 descriptors, and owns the lists l with l % C == rank: every score goes straight into the owner's
-// shared memory. QT x 4 register tile per thread, the next chunk's bytes requested before the arithmetic of this one
-// (the exact score is defined by fp32 sums in feature order). Bound by shared-memory reads: the two of a thread and
-// feature are 8, 6 or 5 wavefronts of a warp (QT = 4, 2, 1), 8192 cycles per chunk at QT = 4 against 4096 of FMAs; 1024
-// lists of 64 x 8192 take 8130 (3790 us). QT, L and C are chosen by plan_rows().
+// rank + C, ... of 64 KG descriptors, and owns the lists l with l % C == rank: every score goes straight into the owner's
+// shared memory. QT x 4 KG register tile per thread, the next chunk's bytes requested before the arithmetic of this one (the
+// exact score is defined by fp32 sums in feature order). The tiles stay bf16 in shared memory, two features to a word, and are
+// widened by the reader: half the bytes of fp32 tiles, whose reads (8 wavefronts of a warp and feature for 4 x 4) bounded the
+// loop at 8192 cycles per 64 x 64 unit against 4096 of FMAs. Products go two keys at a time through fma.rn.f32x2 (each half
+// is fmaf), the same sums with half the instructions; KG = 2 (64 rows x 128 keys, 4 x 8 per thread) shares the widened
+// queries among twice the keys. Now bound by the FMA pipe (60 % of its cycles busy, its throttle the largest stall; shared
+// memory 39 %). Whole selector, us, fp32 4 x 4 -> this: 1024 lists of 64 x 8192 3790 -> 3390, 128 of 64 x 2048 166 -> 152,
+// 64 of 64 x 512 29.6 -> 28.1. 4 x 8 with scalar FMAs took 3811; with fp32 keys 3309, but 96 KiB of shared memory: 512 lists
+// of 1 x 2048 332 us instead of 310, and sorts of 1024 x 2048 361 instead of 243; 4 x 4 with packed FMAs 4062. QT, KG, L and
+// C are chosen by plan_rows().
 constexpr int KD = 64;
 constexpr int SCORE_BYTES_MAX = 40 * 1024;
 constexpr size_t SMEM_PER_SM = 228 * 1024;       // of which 1 KiB per CTA is the system's
@@ -69,19 +77,22 @@ __device__ __forceinline__ unsigned score_key(float s) {      // order of the fl
   return b ^ ((b >> 31) ? 0xffffffffu : 0x80000000u);
 }
 
-// [feature][ROWS] fp32 tile in shared memory. Odd 8-feature pieces are stored with bit 4 of the column flipped (tiles of
-// at least 32 columns), so that a warp which holds two neighbouring pieces of 16 rows (whole 32-byte sectors of global
-// memory) stores without bank conflicts.
+// [feature pair][ROWS] words of two bf16 in shared memory. Odd 8-feature pieces are stored with bit 4 of the column flipped
+// (tiles of at least 32 columns), so that a warp which holds two neighbouring pieces of 16 rows (whole 32-byte sectors of
+// global memory) stores without bank conflicts.
 template <int ROWS>
-__device__ __forceinline__ void stage_piece(float* tile, int row, int c, const uint4& raw) {
-  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
-  float* dst = tile + c * 8 * ROWS + (ROWS > 16 ? row ^ ((c & 1) << 4) : row);
-#pragma unroll
-  for (int p = 0; p < 4; ++p) {
-    const float2 f = __bfloat1622float2(h[p]);
-    dst[(2 * p) * ROWS] = f.x;
-    dst[(2 * p + 1) * ROWS] = f.y;
-  }
+__device__ __forceinline__ void stage_piece(uint32_t* tile, int row, int c, const uint4& raw) {
+  uint32_t* dst = tile + c * 4 * ROWS + (ROWS > 16 ? row ^ ((c & 1) << 4) : row);
+  dst[0] = raw.x;
+  dst[ROWS] = raw.y;
+  dst[2 * ROWS] = raw.z;
+  dst[3 * ROWS] = raw.w;
+}
+
+// feature F (0 or 1) of a pair of bf16
+template <int F>
+__device__ __forceinline__ float feature(uint32_t pair) {
+  return __uint_as_float(F ? pair & 0xffff0000u : pair << 16);
 }
 
 struct RowsParams {
@@ -91,16 +102,17 @@ struct RowsParams {
   int32_t* fallback_counter; // three words to reset, or null
   int hq, hkv, qt, nt, r, topk;
   int lists_per_cta, tiles_per_head, mp_log2;
+  int tile_words;            // words of shared memory before the scores
 };
 
-// QT = rows per thread, LPT = lists that they belong to: 1 (MP >= QT) or QT / MP
-template <int QT, int LPT>
-__global__ void __launch_bounds__(256) score_rows_kernel(const RowsParams p) {
-  constexpr int ROWS = 16 * QT;
+// QT = rows per thread, LPT = lists that they belong to: 1 (MP >= QT) or QT / MP, KG = groups of 64 keys in a chunk
+template <int QT, int LPT, int KG>
+__global__ void __launch_bounds__(256, QT < 4 ? 4 : KG == 1 ? 3 : 2) score_rows_kernel(const RowsParams p) {
+  constexpr int ROWS = 16 * QT, KEYS = KD * KG;
   extern __shared__ __align__(16) float smem[];
-  float* q_s = smem;                         // [128][ROWS]
-  float* k_s = q_s + 128 * ROWS;             // [128][KD]
-  float* scores = k_s + 128 * KD;            // [lists owned by this CTA][nt]
+  uint32_t* q_s = reinterpret_cast<uint32_t*>(smem);      // [64][ROWS]
+  uint32_t* k_s = q_s + 64 * ROWS;           // [KG][64][KD]
+  float* scores = smem + p.tile_words;       // [lists owned by this CTA][nt]
 
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = static_cast<int>(cluster.block_rank()), csize = static_cast<int>(cluster.num_blocks());
@@ -122,12 +134,15 @@ __global__ void __launch_bounds__(256) score_rows_kernel(const RowsParams p) {
   // every list is exact here: no fallback, no violated bound, no largest difference
   if (p.fallback_counter && blockIdx.x == 0 && tid < 3) p.fallback_counter[tid] = 0;
   const uint4* kbase = reinterpret_cast<const uint4*>(p.kd + static_cast<long long>(bk) * n_keys * 128);
-  uint4 raw[4];
+  uint4 raw[KG][4];
   auto fetch_keys = [&](int base) {
-    const bool live = base + srow < n_keys;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-      raw[i] = live ? __ldg(kbase + static_cast<long long>(base + srow) * 16 + piece0 + 2 * i) : make_uint4(0u, 0u, 0u, 0u);
+    for (int g = 0; g < KG; ++g) {
+      const int key = base + g * KD + srow;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        raw[g][i] = key < n_keys ? __ldg(kbase + static_cast<long long>(key) * 16 + piece0 + 2 * i) : make_uint4(0u, 0u, 0u, 0u);
+    }
   };
   {
     const int l = qrow >> p.mp_log2, m = qrow & ((1 << p.mp_log2) - 1);
@@ -138,7 +153,7 @@ __global__ void __launch_bounds__(256) score_rows_kernel(const RowsParams p) {
     uint4 qraw[QT];
 #pragma unroll
     for (int i = 0; i < QT; ++i) qraw[i] = __ldg(src + qpiece0 + 2 * i);
-    fetch_keys(rank * KD);
+    fetch_keys(rank * KEYS);
 #pragma unroll
     for (int i = 0; i < QT; ++i) stage_piece<ROWS>(q_s, qrow, qpiece0 + 2 * i, qraw[i]);
   }
@@ -153,70 +168,97 @@ __global__ void __launch_bounds__(256) score_rows_kernel(const RowsParams p) {
     owner_scores[x] = speaks && l < lists ? cluster.map_shared_rank(scores, l & (csize - 1)) + (l >> c_log2) * p.nt : nullptr;
   }
 
-  for (int base = rank * KD; base < n_keys; base += csize * KD) {
+  for (int base = rank * KEYS; base < n_keys; base += csize * KEYS) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) stage_piece<KD>(k_s, srow, piece0 + 2 * i, raw[i]);
+    for (int g = 0; g < KG; ++g)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) stage_piece<KD>(k_s + g * 64 * KD, srow, piece0 + 2 * i, raw[g][i]);
     __syncthreads();                           // tiles staged
-    if (base + csize * KD < n_keys) fetch_keys(base + csize * KD);
-    float acc[QT][4];
+    if (base + csize * KEYS < n_keys) fetch_keys(base + csize * KEYS);
+    unsigned long long acc[QT][2 * KG];        // two neighbouring keys each
 #pragma unroll
     for (int i = 0; i < QT; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-    const int features = base + (tid >> 5) * 8 < n_keys ? 128 : 0;      // a warp's eight keys may all be padding
+      for (int j = 0; j < 2 * KG; ++j) acc[i][j] = 0ull;
+    const int pairs = base + (tid >> 5) * 8 < n_keys ? 64 : 0;          // a warp's keys may all be padding
 #pragma unroll 1
-    for (int d0 = 0; d0 < features; d0 += 16) {
+    for (int d0 = 0; d0 < pairs; d0 += 8) {
 #pragma unroll
-      for (int dd = 0; dd < 16; ++dd) {
-        const int flip = (dd >> 3) << 4;
-        const float4 kv = *reinterpret_cast<const float4*>(k_s + (d0 + dd) * 64 + ((tk * 4) ^ flip));
-        const float ka[4] = {kv.x, kv.y, kv.z, kv.w};
-        const float* qsrc = q_s + (d0 + dd) * ROWS + (QT > 1 ? (tq * QT) ^ flip : tq);
-        float qa[QT];
+      for (int dd = 0; dd < 8; ++dd) {
+        const int flip = (dd >> 2) << 4;
+        uint4 kw[KG];
+#pragma unroll
+        for (int g = 0; g < KG; ++g)
+          kw[g] = *reinterpret_cast<const uint4*>(k_s + g * 64 * KD + (d0 + dd) * KD + ((tk * 4) ^ flip));
+        const uint32_t* qsrc = q_s + (d0 + dd) * ROWS + (QT > 1 ? (tq * QT) ^ flip : tq);
+        uint32_t qw[QT];
         if constexpr (QT == 4) {
-          const float4 qv = *reinterpret_cast<const float4*>(qsrc);
-          qa[0] = qv.x; qa[1] = qv.y; qa[2] = qv.z; qa[3] = qv.w;
+          const uint4 qv = *reinterpret_cast<const uint4*>(qsrc);
+          qw[0] = qv.x; qw[1] = qv.y; qw[2] = qv.z; qw[3] = qv.w;
         } else if constexpr (QT == 2) {
-          const float2 qv = *reinterpret_cast<const float2*>(qsrc);
-          qa[0] = qv.x; qa[1] = qv.y;
+          const uint2 qv = *reinterpret_cast<const uint2*>(qsrc);
+          qw[0] = qv.x; qw[1] = qv.y;
         } else {
-          qa[0] = *qsrc;
+          qw[0] = *qsrc;
         }
+        auto step = [&](auto which) {
+          constexpr int F = decltype(which)::value;
+          unsigned long long kp[2 * KG];
 #pragma unroll
-        for (int i = 0; i < QT; ++i)
+          for (int g = 0; g < KG; ++g) {
+            kp[2 * g] = f32x2_pack(feature<F>(kw[g].x), feature<F>(kw[g].y));
+            kp[2 * g + 1] = f32x2_pack(feature<F>(kw[g].z), feature<F>(kw[g].w));
+          }
 #pragma unroll
-          for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(qa[i], ka[j], acc[i][j]);
+          for (int i = 0; i < QT; ++i) {
+            const float q = feature<F>(qw[i]);
+            const unsigned long long qq = f32x2_pack(q, q);
+#pragma unroll
+            for (int j = 0; j < 2 * KG; ++j) acc[i][j] = f32x2_fma(qq, kp[j], acc[i][j]);
+          }
+        };
+        step(std::integral_constant<int, 0>{});
+        step(std::integral_constant<int, 1>{});
       }
     }
     // one score per (list, KV block): maximum over the list's rows and the block's R descriptors, then the scale. As in
     // the exact kernel the maximum starts at -inf: a NaN product never wins, and no score is NaN.
 #pragma unroll
-    for (int x = 0; x < LPT; ++x) {
-      float best[4];
+    for (int g = 0; g < KG; ++g) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        best[j] = -CUDART_INF_F;
+      for (int x = 0; x < LPT; ++x) {
+        float best[4];
 #pragma unroll
-        for (int i = 0; i < QT / LPT; ++i) best[j] = fmaxf(best[j], acc[x * (QT / LPT) + i][j]);
-      }
-      if (p.r > 1) { best[0] = fmaxf(best[0], best[1]); best[2] = fmaxf(best[2], best[3]); }
-      if (p.r > 2) best[0] = fmaxf(best[0], best[2]);
-      if (LPT == 1) {
-        for (int dlt = 1; dlt < (1 << p.mp_log2) / QT; dlt <<= 1) {
+        for (int j = 0; j < 4; ++j) best[j] = -CUDART_INF_F;
 #pragma unroll
-          for (int j = 0; j < 4; ++j) best[j] = fmaxf(best[j], __shfl_xor_sync(0xffffffffu, best[j], dlt));
+        for (int i = 0; i < QT / LPT; ++i) {
+          float s0, s1, s2, s3;
+          f32x2_unpack(acc[x * (QT / LPT) + i][2 * g], s0, s1);
+          f32x2_unpack(acc[x * (QT / LPT) + i][2 * g + 1], s2, s3);
+          best[0] = fmaxf(best[0], s0);
+          best[1] = fmaxf(best[1], s1);
+          best[2] = fmaxf(best[2], s2);
+          best[3] = fmaxf(best[3], s3);
         }
-      }
-      if (owner_scores[x]) {
-        const int first = base + tk * 4;       // a multiple of R
-        float* dst = owner_scores[x] + first / p.r;
-        if (first < n_keys) dst[0] = best[0] * scale;
-        if (p.r == 1) {
+        if (p.r > 1) { best[0] = fmaxf(best[0], best[1]); best[2] = fmaxf(best[2], best[3]); }
+        if (p.r > 2) best[0] = fmaxf(best[0], best[2]);
+        if (LPT == 1) {
+          for (int dlt = 1; dlt < (1 << p.mp_log2) / QT; dlt <<= 1) {
 #pragma unroll
-          for (int j = 1; j < 4; ++j)
-            if (first + j < n_keys) dst[j] = best[j] * scale;
-        } else if (p.r == 2) {
-          if (first + 2 < n_keys) dst[1] = best[2] * scale;
+            for (int j = 0; j < 4; ++j) best[j] = fmaxf(best[j], __shfl_xor_sync(0xffffffffu, best[j], dlt));
+          }
+        }
+        if (owner_scores[x]) {
+          const int first = base + g * KD + tk * 4;       // a multiple of R
+          float* dst = owner_scores[x] + first / p.r;
+          if (first < n_keys) dst[0] = best[0] * scale;
+          if (p.r == 1) {
+#pragma unroll
+            for (int j = 1; j < 4; ++j)
+              if (first + j < n_keys) dst[j] = best[j] * scale;
+          } else if (p.r == 2) {
+            if (first + 2 < n_keys) dst[1] = best[2] * scale;
+          }
         }
       }
     }
@@ -250,7 +292,7 @@ __global__ void __launch_bounds__(256) score_rows_kernel(const RowsParams p) {
   const int lane = tid & 31, warp = tid >> 5;
   if (p.topk <= 128) {
     // one warp per list: k-th largest score bit by bit, then ranks among the k that reach it
-    float* cand_s = q_s + warp * 256;
+    float* cand_s = smem + warp * 256;
     int* cand_i = reinterpret_cast<int*>(cand_s + 128);
     for (int l = warp; l < own; l += 8) {
       const float* s = scores + l * p.nt;
@@ -301,10 +343,10 @@ __global__ void __launch_bounds__(256) score_rows_kernel(const RowsParams p) {
   // inverted id, so that the order is score descending, id ascending; padding sorts last). Rounds of block-wide
   // arg-max, k per list and list after list, took 1320 us for 64 lists of 512 with k = 256, this 44 with 64 lists to a
   // tile and 20 with 14 (whole selector).
-  unsigned long long* keys = reinterpret_cast<unsigned long long*>(q_s);
+  unsigned long long* keys = reinterpret_cast<unsigned long long*>(smem);
   int p_log2 = 1;
   while ((1 << p_log2) < p.nt) ++p_log2;
-  const int batch = ((128 * ROWS + 128 * KD) / 2) >> p_log2, half = 1 << (p_log2 - 1);
+  const int batch = (p.tile_words / 2) >> p_log2, half = 1 << (p_log2 - 1);
   for (int l0 = 0; l0 < own; l0 += batch) {
     const int nl = min(batch, own - l0);
     for (int e = tid; e < nl << p_log2; e += blockDim.x) {
@@ -335,10 +377,10 @@ __global__ void __launch_bounds__(256) score_rows_kernel(const RowsParams p) {
   }
 }
 
-template <int QT, int LPT>
+template <int QT, int LPT, int KG>
 int launch_rows(const RowsParams& p, int grid, int csize, size_t smem, DeviceCtx* ctx, int slot, cudaStream_t stream) {
   if (!(ctx->small_attr & (1 << slot))) {
-    cudaError_t e = cudaFuncSetAttribute(score_rows_kernel<QT, LPT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(score_rows_kernel<QT, LPT, KG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (QT * 16 + KD) * 512 + SCORE_BYTES_MAX);
     if (e != cudaSuccess) return set_error(SB_ERR_CUDA, cudaGetErrorString(e));
     ctx->small_attr |= (1 << slot);
@@ -356,12 +398,13 @@ int launch_rows(const RowsParams& p, int grid, int csize, size_t smem, DeviceCtx
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, score_rows_kernel<QT, LPT>, p);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, score_rows_kernel<QT, LPT, KG>, p);
   return e == cudaSuccess ? SB_OK : set_error(SB_ERR_CUDA, cudaGetErrorString(e));
 }
 
 struct RowsPlan {
-  int lists, tiles, csize, qt;       // lists per row tile, row tiles per KV head, cluster size, rows per thread
+  int lists, tiles, csize, qt, kg;   // lists per row tile, row tiles per KV head, cluster size, rows per thread, key groups
+  int tile_words;                    // of shared memory, before the scores
   size_t smem;
 };
 
@@ -373,7 +416,6 @@ struct RowsPlan {
 // 1024 of 8 x 8192 2237 -> 1948. (A cluster of 8 CTAs per list and 16 descriptors, which was used for up to 148 lists before
 // the row tiles, took 15.1, 10.7 and 9.1 us for the first three; on a few lists of 65 to 128 keys it was 1 us faster.)
 RowsPlan plan_rows(long long heads, int qt, int nt, int r, int topk, int mp_log2, int sm_count) {
-  const int chunks = (nt * r + KD - 1) / KD;
   const float nf = static_cast<float>(nt);
   float sort_stage = 0.f, stages = 0.f;        // k > 128: cycles per list and stage beside others, number of stages
   int p_log2 = 1;
@@ -389,16 +431,22 @@ RowsPlan plan_rows(long long heads, int qt, int nt, int r, int topk, int mp_log2
     const int tiles = (qt + n - 1) / n, lists = (qt + tiles - 1) / tiles;
     const int rows = lists << mp_log2, per_thread = rows <= 16 ? 1 : rows <= 32 ? 2 : 4;
     for (int c = 8; c >= 1; c >>= 1) {
-      const int own = (lists + c - 1) / c;
+      const int kg = per_thread == 4 && nt * r > KD ? 2 : 1;           // no empty second half
+      const int own = (lists + c - 1) / c, chunks = (nt * r + KD * kg - 1) / (KD * kg);
       if ((c > 1 && c / 2 >= chunks) || own * nt * 4 > SCORE_BYTES_MAX) continue;
-      const size_t smem = static_cast<size_t>(16 * per_thread + KD) * 512 + static_cast<size_t>(own) * nt * 4;
+      // k > 128: room to sort as many lists at a time as fp32 tiles would leave
+      const int tile_words = topk > 128 ? (16 * per_thread + KD) * 128 : (16 * per_thread + KD * kg) * 64;
+      const size_t smem = (static_cast<size_t>(tile_words) + static_cast<size_t>(own) * nt) * 4;
       const long long ctas = heads * tiles * c;
-      const int resident = static_cast<int>(SMEM_PER_SM / (smem + 1024)) < 4 ? static_cast<int>(SMEM_PER_SM / (smem + 1024)) : 4;
+      const int most = per_thread < 4 ? 4 : kg == 1 ? 3 : 2;
+      const int resident = static_cast<int>(SMEM_PER_SM / (smem + 1024)) < most ? static_cast<int>(SMEM_PER_SM / (smem + 1024)) : most;
       const long long slots = static_cast<long long>(resident) * sm_count;
       const float waves = static_cast<float>((ctas + slots - 1) / slots);
       const float load = static_cast<float>((ctas + sm_count - 1) / sm_count);       // CTAs of an SM in all
-      // a chunk: bound by shared-memory reads, 8, 6 or 5 wavefronts per warp and feature; slower for a CTA by itself
-      float chunk = per_thread == 1 ? 5200.f : per_thread == 2 ? 6200.f : 8200.f;
+      // A chunk of 64 keys (128 with kg = 2), cycles of an SM; slower for a CTA by itself. A saturated SM takes 14000 for the
+      // last; the smaller figure chooses better among the plans of problems that do not saturate it (80 lists of 16 x 1024
+      // on four heads 39.3 us, 42.5 with 14000 and the fp32 tiles' 5200 and 6200; 64 of 16 x 512 25.9 and 28.1).
+      float chunk = per_thread == 1 ? 3200.f : per_thread == 2 ? 4200.f : kg == 1 ? 6000.f : 10500.f;
       if (ctas <= sm_count) chunk *= 1.17f;
       // clusters of a second wave wait until all their slots are free
       if (ctas > slots) chunk *= c == 8 ? 1.25f : c == 4 ? 1.2f : c == 2 ? 1.1f : 1.f;
@@ -417,7 +465,7 @@ RowsPlan plan_rows(long long heads, int qt, int nt, int r, int topk, int mp_log2
       const float ranking = alone > load * among ? alone : load * among;
       const float cost = waves * (c > 1 ? 3300.f : 2500.f) + load * chunk * static_cast<float>((chunks + c - 1) / c) + ranking;
       if (best.lists == 0 || cost < best_cost) {
-        best = RowsPlan{lists, tiles, c, per_thread, smem};
+        best = RowsPlan{lists, tiles, c, per_thread, kg, tile_words, smem};
         best_cost = cost;
       }
     }
@@ -451,7 +499,7 @@ int launch_pool_small_pair(const void* x, void* desc, long long num_desc, const 
 
 // Returns 1 when the problem is not a small one (the caller then takes the other kernels). force: whatever its size, up
 // to 2048 blocks (scores wanted, or problems the tensor-core forms do not take). Against score_topk_kernel, us, that one ->
-// this: 512 lists of 4 x 512 89 -> 69, 2048 of 1 x 2048 420 -> 161, 1024 of 64 x 8192 5370 -> 3790; behind it only on
+// this: 512 lists of 4 x 512 89 -> 66, 2048 of 1 x 2048 420 -> 161, 1024 of 64 x 8192 5370 -> 3370; behind it only on
 // problems of a few microseconds (262 of 4 x 136 with k = 1 16.8 -> 21.3, 202 of 16 x 342 55 -> 61 were the worst of 680).
 int launch_summary_small(const void* qd, const void* kd, float* scores, int32_t* ids, int32_t* fallback_counter,
                          int batch, int hq, int hkv, int qt, int nt, int r, int topk, cudaStream_t stream, bool force) {
@@ -484,13 +532,19 @@ int launch_summary_small(const void* qd, const void* kd, float* scores, int32_t*
   p.lists_per_cta = plan.lists;
   p.tiles_per_head = plan.tiles;
   p.mp_log2 = mp_log2;
+  p.tile_words = plan.tile_words;
   const int grid = static_cast<int>(heads) * plan.tiles * plan.csize;
-  if (plan.qt == 1) return launch_rows<1, 1>(p, grid, plan.csize, plan.smem, ctx, 0, stream);
-  if (plan.qt == 2 && mp_log2 == 0) return launch_rows<2, 2>(p, grid, plan.csize, plan.smem, ctx, 1, stream);
-  if (plan.qt == 2) return launch_rows<2, 1>(p, grid, plan.csize, plan.smem, ctx, 2, stream);
-  if (mp_log2 == 0) return launch_rows<4, 4>(p, grid, plan.csize, plan.smem, ctx, 3, stream);
-  if (mp_log2 == 1) return launch_rows<4, 2>(p, grid, plan.csize, plan.smem, ctx, 4, stream);
-  return launch_rows<4, 1>(p, grid, plan.csize, plan.smem, ctx, 5, stream);
+  if (plan.qt == 1) return launch_rows<1, 1, 1>(p, grid, plan.csize, plan.smem, ctx, 0, stream);
+  if (plan.qt == 2 && mp_log2 == 0) return launch_rows<2, 2, 1>(p, grid, plan.csize, plan.smem, ctx, 1, stream);
+  if (plan.qt == 2) return launch_rows<2, 1, 1>(p, grid, plan.csize, plan.smem, ctx, 2, stream);
+  if (plan.kg == 2) {
+    if (mp_log2 == 0) return launch_rows<4, 4, 2>(p, grid, plan.csize, plan.smem, ctx, 6, stream);
+    if (mp_log2 == 1) return launch_rows<4, 2, 2>(p, grid, plan.csize, plan.smem, ctx, 7, stream);
+    return launch_rows<4, 1, 2>(p, grid, plan.csize, plan.smem, ctx, 8, stream);
+  }
+  if (mp_log2 == 0) return launch_rows<4, 4, 1>(p, grid, plan.csize, plan.smem, ctx, 3, stream);
+  if (mp_log2 == 1) return launch_rows<4, 2, 1>(p, grid, plan.csize, plan.smem, ctx, 4, stream);
+  return launch_rows<4, 1, 1>(p, grid, plan.csize, plan.smem, ctx, 5, stream);
 }
 
 }  // namespace sb

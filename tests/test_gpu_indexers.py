@@ -391,6 +391,25 @@ def test_row_tile_selector_equals_the_exact_kernels(b, hkv, g, qb, nb, r, topk, 
     assert torch.equal(fast.ids, staged.ids)
 
 
+@pytest.mark.parametrize("keys", [64, 65, 127, 128, 129, 193])
+@pytest.mark.parametrize("g,qb", [(64, 20), (2, 700), (1, 1500)])     # one, 32 and 64 lists to a tile of 64 rows
+def test_row_tiles_at_the_edges_of_a_key_chunk(g, qb, keys):
+    """Two groups of 64 keys in a chunk, the second one full, ragged or empty; four, two and one rows of a thread to a
+    list: scores and ids bit for bit against the staged exact kernels."""
+    m = sp()
+    q, k, _ = gen.make_qkv(1, g, 1, qb * 128, keys * 128, seed=53, k_block_offset=0.5)
+    qc, kc = q.cuda(), k.cuda()
+    staged = m.SummarySelector(qc, kc, 1, topk=9, keep_scores=True)
+    staged.prepare()
+    staged.score()
+    fused = m.SummarySelector(qc, kc, 1, topk=9, keep_scores=True)
+    fused.run()
+    torch.cuda.synchronize()
+    m.device_status()
+    assert torch.equal(fused.scores, staged.scores)
+    assert torch.equal(fused.ids, staged.ids)
+
+
 @pytest.mark.parametrize("b,hkv,g,qb,nb,r,topk", [
     (1, 2, 1, 80, 33, 1, 33),        # 160 lists of one descriptor, every block selected
     (1, 1, 2, 150, 300, 2, 40),      # four descriptors, threshold search
