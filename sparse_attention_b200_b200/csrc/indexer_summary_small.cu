@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(256) pool_small_kernel(const __nv_bfloat16* __
 // is fmaf), the same sums with half the instructions; KG = 2 (64 rows x 128 keys, 4 x 8 per thread) shares the widened
 // queries among twice the keys. Now bound by the FMA pipe (60 % of its cycles busy, its throttle the largest stall; shared
 // memory 39 %). Whole selector, us, fp32 4 x 4 -> this: 1024 lists of 64 x 8192 3790 -> 3390, 128 of 64 x 2048 166 -> 152,
-// 64 of 64 x 512 29.6 -> 28.1. 4 x 8 with scalar FMAs took 3811; with fp32 keys 3309, but 96 KiB of shared memory: 512 lists
+// 64 of 64 x 512 29.6 -> 28.1. 4 x 8 with scalar FMAs took 3811; with fp32 keys 3309, but 96 KiB of shared memory: 4096 lists
 // of 1 x 2048 332 us instead of 310, and sorts of 1024 x 2048 361 instead of 243; 4 x 4 with packed FMAs 4062. QT, KG, L and
 // C are chosen by plan_rows().
 constexpr int KD = 64;
@@ -444,8 +444,8 @@ RowsPlan plan_rows(long long heads, int qt, int nt, int r, int topk, int mp_log2
       const float waves = static_cast<float>((ctas + slots - 1) / slots);
       const float load = static_cast<float>((ctas + sm_count - 1) / sm_count);       // CTAs of an SM in all
       // A chunk of 64 keys (128 with kg = 2), cycles of an SM; slower for a CTA by itself. A saturated SM takes 14000 for the
-      // last; the smaller figure chooses better among the plans of problems that do not saturate it (80 lists of 16 x 1024
-      // on four heads 39.3 us, 42.5 with 14000 and the fp32 tiles' 5200 and 6200; 64 of 16 x 512 25.9 and 28.1).
+      // last; the smaller figure chooses better among the plans of problems that do not saturate it (160 lists of 16 x 1024
+      // 39.3 us, 42.5 with 14000 and the fp32 tiles' 5200 and 6200; 64 of 16 x 512 25.9 and 28.1).
       float chunk = per_thread == 1 ? 3200.f : per_thread == 2 ? 4200.f : kg == 1 ? 6000.f : 10500.f;
       if (ctas <= sm_count) chunk *= 1.17f;
       // clusters of a second wave wait until all their slots are free
