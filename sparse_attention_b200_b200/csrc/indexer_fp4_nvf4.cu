@@ -615,9 +615,9 @@ fp4_nv_select_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
 // tensor cores give every dot within delta of its exact value, so only the elements whose
 // approximate value reaches (largest approximate value - 2 delta) can hold the exact maximum:
 // any other element is below the exact value of the approximate arg-max. Those few elements
-// (usually one) are queued with the other fifteen of their group of columns and evaluated at the end with the
-// canonical arithmetic (integer group sums, scaled and added in group order) straight from the codes in global
-// memory. Same scores, bit for bit, as fp4_score_mma_kernel, which evaluates all 16384 elements of a pair exactly.
+// (usually one) are queued with the other fifteen of their group of columns and evaluated, when the queue fills up and at
+// the end, with the canonical arithmetic (integer group sums, scaled and added in group order) straight from the codes in
+// global memory. Same scores, bit for bit, as fp4_score_mma_kernel, which evaluates all 16384 elements of a pair exactly.
 // The exact maximum of every evaluated group is also compared with its approximate one: a difference above delta is
 // counted and the pair is re-done by evaluating all of its elements.
 struct PruneParams {
@@ -678,16 +678,22 @@ __device__ __forceinline__ float fp4_exact_dot(const uint8_t* __restrict__ q_cod
 }
 
 constexpr int PR_QCAP = 2048;                // queued groups of elements per CTA
+// A queue that has grown beyond this is emptied at the next page's meeting: there always is room for all 1024 groups of a
+// page. (Emptied at the end only, every page behind two all-equal ones, or behind 2000 others, had to be evaluated in full.
+// Selection of 160 lists, us: 4096 pages 232000 -> 3150, 1024 pages, four of zeros, 113000 -> 1580.)
+constexpr int PR_DRAIN = PR_QCAP - 1024;
+constexpr int PR_PAGES_MAX = 3072;           // pages of a CTA: the results of more would leave one CTA to an SM
 constexpr int PR_OFF_AUX = OFF_CAND;         // barriers (128 bytes), misc (128 bytes)
 constexpr int PR_OFF_QUEUE = PR_OFF_AUX + 256;            // [PR_QCAP] groups waiting for their exact values
 constexpr int PR_OFF_APX = PR_OFF_QUEUE + PR_QCAP * 4;     // [PR_QCAP] their largest approximate values
 constexpr int PR_OFF_RES = PR_OFF_APX + PR_QCAP * 4;       // [pages per CTA] exact maxima as ordered ints
                                                            // then [pages per CTA] flags: pair to be re-done in full
+static_assert(2 * (PR_OFF_RES + PR_PAGES_MAX * 8 + 1024 + 1024) <= 228 * 1024, "two CTAs of the pruning scorer to an SM");
 
 // One CTA per (batch, index head, query tile, chunk of key pages), two CTAs per SM. Warps 0-7 epilogue (lane
 // quarter = warp & 3, query half = warp >> 2), warp 8 producer, warp 9 MMA issue. The epilogue
-// warps meet twice per page at a named barrier (largest approximate value of the page, then
-// largest exact value of the surviving elements); a warp whose bounded wait gave up keeps
+// warps meet once per page at a named barrier (largest approximate value of the page) and twice
+// more where they empty the queue; a warp whose bounded wait gave up keeps
 // taking part in those meetings, so nobody is left waiting for it.
 __global__ void __launch_bounds__(NUM_THREADS, 2)
 fp4_nv_prune_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
@@ -699,9 +705,13 @@ fp4_nv_prune_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
   const Geometry& g = p.g;
   unsigned char* aux = gbase + PR_OFF_AUX;
   const uint32_t bar0 = base + PR_OFF_AUX;
-  // tmem base, abort flag, L1 bits, largest key scale byte, largest approximate value of a page [3 slots], queue length,
-  // largest |approximate - exact| / delta (float bits)
+  // tmem base, abort flag, L1 bits, largest key scale byte, queue length, largest |approximate - exact| / delta (float bits)
   volatile int* misc = reinterpret_cast<volatile int*>(aux + 128);
+  // three slots for a page each: its largest approximate value, and whether the queue is to be emptied before the page
+  // queues anything (one word, so that everybody reads both at once)
+  volatile int* peak = misc + 6;
+  auto peak_word = [&](int slot) { return reinterpret_cast<volatile unsigned long long*>(peak + slot); };
+  constexpr unsigned long long NO_PEAK = 0x80000000ull;
   int* queue = reinterpret_cast<int*>(gbase + PR_OFF_QUEUE);
   float* queue_apx = reinterpret_cast<float*>(gbase + PR_OFF_APX);
   int* res = reinterpret_cast<int*>(gbase + PR_OFF_RES);
@@ -728,9 +738,9 @@ fp4_nv_prune_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
     misc[1] = 0;
     misc[2] = 0;
     misc[3] = 0;
-    for (int i = 4; i < 7; ++i) misc[i] = INT_MIN;
-    misc[7] = 0;
-    misc[8] = 0;
+    misc[4] = 0;
+    misc[5] = 0;
+    for (int i = 0; i < 3; ++i) *peak_word(2 * i) = NO_PEAK;
     for (int i = 0; i < A_STAGES; ++i) {
       mbar_init(bar(A_FULL + i), 2);
       mbar_init(bar(A_EMPTY + i), 1);
@@ -797,9 +807,37 @@ fp4_nv_prune_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const int half = warp >> 2;
     const int key_row = (warp & 3) * 32 + lane;
+    // the queued groups, sixteen threads each: exact values of the group's elements into the page's maximum
+    auto evaluate_queue = [&]() {
+      const int queued = misc[4];
+      for (int i = static_cast<int>(threadIdx.x) >> 4; i < ((queued + 15) & ~15); i += 16) {
+        const bool live = i < queued;
+        const int e = live ? queue[i] : 0, t = e >> 10, krow = (e >> 3) & 127;
+        float m = -INFINITY;
+        if (live) {
+          const long long page = (static_cast<long long>(b) * g.tiles + page0 + t) * g.hk + hk_idx;
+          const long long qrow = (q_row0 + (e & 7) * 16 + (threadIdx.x & 15)) * g.hidx + h;
+          const float x = fp4_exact_dot(g.qp + qrow * 64, g.qs + qrow * 8, g.kp + (page * 128 + krow) * 64,
+                                        g.ks + (page * 128 + krow) * 8);
+          if (x == x) m = x;
+        }
+#pragma unroll
+        for (int d = 8; d > 0; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
+        if (live && (threadIdx.x & 15) == 0 && m > -INFINITY) {
+          atomicMax(res + t, f2ord(m));
+          // the largest value of a group, exact and approximate, differ by at most delta, as its elements do
+          const float diff = fabsf(queue_apx[i] - m);
+          if (delta > 0.f) atomicMax(const_cast<int*>(misc + 5), __float_as_int(diff / delta));
+          if (!(diff <= delta)) {
+            redo[t] = 1;
+            atomicAdd(p.violations, 1);
+          }
+        }
+      }
+    };
     bool ok = true;
     for (int t = 0; t < num_tiles; ++t) {
-      const int st = t % ACC_STAGES, slot = 4 + t % 3;
+      const int st = t % ACC_STAGES, slot = 2 * (t % 3);
       if (ok) {
         bool w = mbar_wait(bar(ACC_FULL + st), (t / ACC_STAGES) & 1, guard, 0x5c0 + st);
         ok = __all_sync(0xffffffffu, w);
@@ -825,14 +863,21 @@ fp4_nv_prune_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
         }
         mine = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
         const float m = warp_max(mine);
-        if (lane == 0) atomicMax(const_cast<int*>(misc + slot), f2ord(m));
+        if (lane == 0) atomicMax(const_cast<int*>(peak + slot), f2ord(m));
       }
       meet();
+      const unsigned long long top = *peak_word(slot);
       // the slot of the page before is free now (everyone read it before this meeting); it is
       // next written for page t + 2, after the meeting of page t + 1
-      if (threadIdx.x == 0 && t > 0) misc[4 + (t - 1) % 3] = INT_MIN;
+      if (threadIdx.x == 0 && t > 0) *peak_word(2 * ((t - 1) % 3)) = NO_PEAK;
+      if ((top >> 32) != 0) {                  // everybody, and nobody queues anything until all are through
+        evaluate_queue();
+        meet();
+        if (threadIdx.x == 0) misc[4] = 0;
+        meet();
+      }
       if (ok) {
-        const float thr = ord2f(misc[slot]) - two;
+        const float thr = ord2f(static_cast<int>(top)) - two;
         // Groups of sixteen columns of this key row that hold an element that may be the maximum. Everyone waits for this
         // at the page's next meeting, and a lone lane does it: the column is left to the evaluation (looking for it here,
         // with its approximate value, took the lane longer than the page took everyone: 1070 cycles of an SM per page).
@@ -840,46 +885,18 @@ fp4_nv_prune_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
 #pragma unroll
           for (int c = 0; c < 4; ++c)
             if (!(m4[c] < thr)) {
-              const int at = atomicAdd(const_cast<int*>(misc + 7), 1);
-              if (at < PR_QCAP) {
-                queue[at] = (t << 10) | (key_row << 3) | (half * 4 + c);
-                queue_apx[at] = m4[c];
-              } else {
-                redo[t] = 1;                 // queue full (masses of ties): the page is re-done below
-              }
+              const int at = atomicAdd(const_cast<int*>(misc + 4), 1);
+              queue[at] = (t << 10) | (key_row << 3) | (half * 4 + c);
+              queue_apx[at] = m4[c];
+              if (at >= PR_DRAIN) peak[2 * ((t + 1) % 3) + 1] = 1;
             }
         }
       }
     }
     meet();
-    // the queued groups, sixteen threads each: exact values of the group's elements into the page's maximum
-    const int queued = min(misc[7], PR_QCAP);
-    for (int i = static_cast<int>(threadIdx.x) >> 4; i < ((queued + 15) & ~15); i += 16) {
-      const bool live = i < queued;
-      const int e = live ? queue[i] : 0, t = e >> 10, krow = (e >> 3) & 127;
-      float m = -INFINITY;
-      if (live) {
-        const long long page = (static_cast<long long>(b) * g.tiles + page0 + t) * g.hk + hk_idx;
-        const long long qrow = (q_row0 + (e & 7) * 16 + (threadIdx.x & 15)) * g.hidx + h;
-        const float x = fp4_exact_dot(g.qp + qrow * 64, g.qs + qrow * 8, g.kp + (page * 128 + krow) * 64,
-                                      g.ks + (page * 128 + krow) * 8);
-        if (x == x) m = x;
-      }
-#pragma unroll
-      for (int d = 8; d > 0; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
-      if (live && (threadIdx.x & 15) == 0 && m > -INFINITY) {
-        atomicMax(res + t, f2ord(m));
-        // the largest value of a group, exact and approximate, differ by at most delta, as its elements do
-        const float diff = fabsf(queue_apx[i] - m);
-        if (delta > 0.f) atomicMax(const_cast<int*>(misc + 8), __float_as_int(diff / delta));
-        if (!(diff <= delta)) {
-          redo[t] = 1;
-          atomicAdd(p.violations, 1);
-        }
-      }
-    }
+    evaluate_queue();
     meet();
-    if (threadIdx.x == 0 && misc[8] > 0) atomicMax(p.stats + 4, misc[8]);      // one global atomic per CTA
+    if (threadIdx.x == 0 && misc[5] > 0) atomicMax(p.stats + 4, misc[5]);      // one global atomic per CTA
     // a pair whose bound was violated: every one of its 16384 elements, exactly (256 threads)
     for (int t = 0; t < num_tiles; ++t) {
       if (!redo[t]) continue;
@@ -1477,7 +1494,7 @@ int launch_fp4_scores_prune(const void* qp, const void* qs, const void* kp, cons
   // CTAs as fit at once when the lists are few; a CTA keeps its query tile and takes a run of pages.
   long long chunks = (2LL * ctx->sm_count) / lists;
   if (chunks > tiles) chunks = tiles;
-  if (chunks < 1) chunks = 1;
+  if (chunks < (tiles + PR_PAGES_MAX - 1) / PR_PAGES_MAX) chunks = (tiles + PR_PAGES_MAX - 1) / PR_PAGES_MAX;
   p.pages_per_cta = static_cast<int>((tiles + chunks - 1) / chunks);
   p.chunks = (tiles + p.pages_per_cta - 1) / p.pages_per_cta;
   if (lists * p.chunks >= (1LL << 31)) return 1;

@@ -652,6 +652,68 @@ def test_fp4_pruned_tile_scores_bit_exact(case):
         assert torch.equal(ids.cpu(), ref)
 
 
+def _long_run_inputs(m, pages, zero, seed=21):
+    """160 lists of `pages` pages, one CTA of the pruning scorer per 3072 of them; pages `zero` all equal."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    choices = torch.tensor([0.25, 0.375, 0.5, 0.75, 1.0, 1.5, 2.0], device="cuda")
+
+    def scales(*shape):
+        return choices[torch.randint(7, shape, generator=g, device="cuda")].to(torch.float8_e4m3fn)
+    qp = torch.randint(256, (2048, 10, 64), dtype=torch.uint8, generator=g, device="cuda")
+    kp = torch.randint(256, (pages, 1, 128, 64), dtype=torch.uint8, generator=g, device="cuda")
+    kp[list(zero)] = 0
+    return m.prepare_fp4_inputs(qp, kp, scales(2048, 10, 8), scales(pages, 1, 128, 8), batch_size=1, len_q=2048,
+                                len_kv=pages * 128)
+
+
+@pytest.mark.parametrize("pages,topk,zero", [
+    (24, 8, (0, 1, 2, 3, 12, 13, 14)),    # each queues its 1024 groups; ordinary pages behind them
+    (40, 16, tuple(range(7, 40))),        # padding: only the first pages differ
+    (2500, 200, ()),                      # more pages than the queue has room for
+    (3100, 250, (1549, 1550, 3099)),      # more than one CTA takes
+    (18300, 200, ()),                     # the results of all of a list's pages would not fit a CTA's shared memory
+])
+def test_fp4_pruned_scores_of_long_runs(pages, topk, zero):
+    """The queue of the pruning scorer fills up, is emptied and fills up again: scores bit for bit those of the scorer that
+    evaluates every element, the same ids."""
+    m = sp()
+    inputs = _long_run_inputs(m, pages, zero)
+    ids, ws = m.fp4_indexer_fast(inputs, topk=topk)
+    exact_scores = torch.empty((1, 10, 16, pages), dtype=torch.float32, device="cuda")
+    exact_ids = m.fp4_indexer(inputs, topk=topk, tile_scores=exact_scores)
+    torch.cuda.synchronize()
+    m.device_status()
+    assert ws[:4].view(torch.int32).item() == 160 * ((pages + 3071) // 3072)      # CTAs of the pruning kernel
+    assert ws[12:16].view(torch.int32).item() == 0                                 # no bound was violated
+    pruned = _fast_path_tile_scores(ws, 1, 10, 1, 2048, pages * 128)
+    assert torch.equal(pruned.view(torch.int32), exact_scores.view(torch.int32))
+    assert torch.equal(ids, exact_ids)
+
+
+def test_fp4_pruning_full_queue_costs_little():
+    """Neither a long run nor pages of equal scores make the pages behind them dear. An ordinary page takes about 1 us of the
+    160 lists together, one that is evaluated in full 110 to 160 us: 2500 pages stay within twice the time per page of 1000
+    (500 pages in full would take 55 ms), and six all-equal pages among 1000, in full themselves, take about as long as the
+    other 994, which in full would take 100 times that."""
+    m = sp()
+
+    def us(pages, zero=()):
+        inputs = _long_run_inputs(m, pages, zero)
+        _, ws = m.fp4_indexer_fast(inputs, topk=160)
+        best = float("inf")
+        for _ in range(3):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            m.fp4_indexer_fast(inputs, topk=160, workspace=ws)
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b) * 1e3)
+        return best
+    plain = us(1000)
+    assert us(2500) < 2 * 2.5 * plain
+    assert us(1000, (0, 1, 2, 500, 501, 502)) < 4 * plain
+
+
 def _varlen_case(seed, hq, hk, q_lens, k_lens, shuffle_pages=True):
     g = torch.Generator().manual_seed(seed)
     total_q = sum(q_lens)
