@@ -977,11 +977,11 @@ constexpr int QS_STAGES = 8;           // pages in flight
 constexpr int QS_AHEAD = 4;            // pages whose scales are on their way to their staging ring
 constexpr int QS_OFF_Q = QS_STAGES * STAGE_BYTES;          // two query tiles: codes + scales
 constexpr int QS_OFF_RAW = QS_OFF_Q + 2 * STAGE_BYTES;     // staging ring: the scales of a page as they are in memory
-constexpr int QS_OFF_AUX = QS_OFF_RAW + QS_AHEAD * SF_BYTES;   // barriers, misc (64 bytes)
+constexpr int QS_OFF_AUX = QS_OFF_RAW + QS_AHEAD * SF_BYTES;   // barriers, misc (64 bytes), sums (64)
 enum { QS_K_FULL = 0, QS_K_EMPTY = QS_STAGES, QS_Q_FULL = 2 * QS_STAGES, QS_Q_EMPTY = QS_Q_FULL + 2,
        QS_ACC_FULL = QS_Q_EMPTY + 2, QS_ACC_EMPTY, QS_BARS };
 constexpr int QS_BAR_BYTES = (QS_BARS * 8 + 63) & ~63;
-constexpr int QS_SMEM = QS_OFF_AUX + QS_BAR_BYTES + 64 + 1024;
+constexpr int QS_SMEM = QS_OFF_AUX + QS_BAR_BYTES + 128 + 1024;
 // tensor memory: the accumulator, two slots of key scales, two of query scales
 constexpr int QS_SFK = 128, QS_SFQ = 144;
 static_assert(QS_SFQ + 16 <= TM_COLS, "tensor memory map");
@@ -1060,9 +1060,18 @@ struct ScoreWalk {
   }
 };
 
-// Where the run of this CTA begins: request, query tile, KV head, item of it, page; number of pages (0: nothing). One warp.
+// n / d, both positive; mostly by the short division
+__device__ __forceinline__ long long quotient(long long n, long long d) {
+  return ((n | d) >> 32) == 0 ? static_cast<long long>(static_cast<uint32_t>(n) / static_cast<uint32_t>(d)) : n / d;
+}
+
+// Where the run of this CTA begins: request, query tile, KV head, item of it, page; number of pages (0: nothing). All threads,
+// each with a slice of the requests, once; then the warp that has the run's request looks through its slice. (One warp, 32
+// requests to a step and up to twice over all of them, took 250 steps of dependent loads for 4096 requests while the others
+// waited. One-token requests of 100 to 400 keys in a graph, us: 256 15.0 -> 10.9, 1024 40.4 -> 19.5, 4096 160 -> 59, 16384 788 -> 231.)
 template <bool PACKED>
-__device__ __forceinline__ void find_run(const QueryScoreParams& p, volatile int* start, int lane) {
+__device__ __forceinline__ void find_run(const QueryScoreParams& p, volatile int* start, volatile long long* warp_sums, int warp,
+                                         int lane) {
   const int heads = p.hk * p.subs;
   auto scan = [&](long long v) {
 #pragma unroll
@@ -1072,48 +1081,62 @@ __device__ __forceinline__ void find_run(const QueryScoreParams& p, volatile int
     }
     return v;
   };
-  long long total = 0;
-  for (int b0 = 0; b0 < p.batch; b0 += 32) {
-    const int b = b0 + lane;
-    total += __shfl_sync(0xffffffffu, scan(b < p.batch ? heads * Request::load<PACKED>(p, b).total(p) : 0LL), 31);
+  const int slice = (p.batch + QS_THREADS - 1) / QS_THREADS;
+  const int lo = min(static_cast<int>(threadIdx.x) * slice, p.batch), hi = min(lo + slice, p.batch);
+  long long mine = 0;
+#pragma unroll 4
+  for (int b = lo; b < hi; ++b) mine += Request::load<PACKED>(p, b).total(p);
+  mine *= heads;
+  const long long sum = scan(mine);
+  if (lane == 31) warp_sums[warp] = sum;
+  if (threadIdx.x == 0) start[5] = 0;
+  __syncthreads();
+  long long total = 0, before = sum - mine;        // pages of all requests, pages before this thread's slice
+#pragma unroll
+  for (int w = 0; w < QS_THREADS / 32; ++w) {
+    const long long ws = warp_sums[w];
+    if (w < warp) before += ws;
+    total += ws;
   }
-  const long long per = max(2LL, (total + gridDim.x - 1) / gridDim.x), first = per * blockIdx.x;
-  if (first >= total) {
-    if (lane == 0) start[5] = 0;
-    return;
+  const long long per = max(2LL, quotient(total + gridDim.x - 1, gridDim.x)), first = per * blockIdx.x;
+  if (first >= total) return;
+  const unsigned owner = __ballot_sync(0xffffffffu, first >= before && first < before + mine);
+  if (owner == 0) return;
+  const int at = __ffs(owner) - 1, end = __shfl_sync(0xffffffffu, hi, at);
+  int begin = __shfl_sync(0xffffffffu, lo, at);
+  long long rest = first - __shfl_sync(0xffffffffu, before, at);
+  while (slice > 1) {                              // which request of the slice
+    if (begin >= end) return;
+    const int b = begin + lane;
+    const long long pages_b = b < end ? heads * Request::load<PACKED>(p, b).total(p) : 0LL, upto = scan(pages_b);
+    const unsigned hit = __ballot_sync(0xffffffffu, upto > rest);
+    if (hit != 0) {
+      const int in_slice = __ffs(hit) - 1;
+      begin += in_slice;
+      rest -= __shfl_sync(0xffffffffu, upto - pages_b, in_slice);
+      break;
+    }
+    rest -= __shfl_sync(0xffffffffu, upto, 31);
+    begin += 32;
   }
-  long long before = 0;                      // pages of the requests before the current ones
-  for (int b0 = 0; b0 < p.batch; b0 += 32) {
-    const int b = b0 + lane;
-    const long long mine = b < p.batch ? heads * Request::load<PACKED>(p, b).total(p) : 0LL;
-    const long long upto = before + scan(mine);
-    const unsigned hit = __ballot_sync(0xffffffffu, upto > first);
-    if (hit == 0) {
-      before = __shfl_sync(0xffffffffu, upto, 31);
+  const Request r = Request::load<PACKED>(p, begin);
+  for (int j0 = 0; j0 < r.qtiles; j0 += 32) {
+    const int j = j0 + lane;
+    const long long pages = j < r.qtiles ? r.visible(p, j) : 0, sum_j = scan(pages * heads);
+    const unsigned in = __ballot_sync(0xffffffffu, sum_j > rest);
+    if (in == 0) {
+      rest -= __shfl_sync(0xffffffffu, sum_j, 31);
       continue;
     }
-    const int at = __ffs(hit) - 1;
-    const Request r = Request::load<PACKED>(p, b0 + at);
-    long long rest = first - __shfl_sync(0xffffffffu, upto - mine, at);
-    for (int j0 = 0; j0 < r.qtiles; j0 += 32) {
-      const int j = j0 + lane;
-      const long long pages = j < r.qtiles ? r.visible(p, j) : 0, sum = scan(pages * heads);
-      const unsigned in = __ballot_sync(0xffffffffu, sum > rest);
-      if (in == 0) {
-        rest -= __shfl_sync(0xffffffffu, sum, 31);
-        continue;
-      }
-      if (lane == __ffs(in) - 1) {
-        const long long local = rest - (sum - pages * heads);
-        start[0] = b0 + at;
-        start[1] = j;
-        const int h = static_cast<int>(local / pages), kvh = h / p.subs;
-        start[2] = kvh;
-        start[3] = h - kvh * p.subs;
-        start[4] = static_cast<int>(local - h * pages);
-        start[5] = static_cast<int>(min(per, total - first));
-      }
-      return;
+    if (lane == __ffs(in) - 1) {
+      const long long local = rest - (sum_j - pages * heads);
+      start[0] = begin;
+      start[1] = j;
+      const int h = static_cast<int>(quotient(local, pages)), kvh = h / p.subs;
+      start[2] = kvh;
+      start[3] = h - kvh * p.subs;
+      start[4] = static_cast<int>(local - h * pages);
+      start[5] = static_cast<int>(min(per, total - first));
     }
     return;
   }
@@ -1147,11 +1170,11 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
     mbar_init(bar(QS_ACC_EMPTY), 4);
     fence_mbar_init();
   }
-  if (warp == 4) find_run<PACKED>(p, misc + 2, lane);
   if (warp == 5) {
     tmem_alloc(smem_u32(const_cast<int*>(misc)), TM_COLS);
     tmem_relinquish();
   }
+  find_run<PACKED>(p, misc + 2, reinterpret_cast<volatile long long*>(misc + 16), warp, lane);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();

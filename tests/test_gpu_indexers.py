@@ -916,6 +916,108 @@ def test_fp4_varlen_runs_of_pages(requests, hq, hk, q_hi, k_hi, causal, offsets)
         assert (exact[fin] - fast[fin]).abs().max().item() <= 128 * 36 * scale * 2.0 ** -18
 
 
+@pytest.mark.parametrize("requests,hq,hk,q_hi,causal", [
+    (224, 16, 1, 8, True),                     # one request to a thread of the CTA that looks for its run
+    (225, 4, 2, 150, True),                    # two
+    (1000, 16, 1, 1, False),
+    (7400, 2, 2, 3, True),                     # more than a warp has lanes
+])
+def test_fp4_varlen_runs_of_many_requests(requests, hq, hk, q_hi, causal):
+    """As test_fp4_varlen_runs_of_pages, by the number of requests; many of them empty or without a visible page."""
+    m = sp()
+    rng = np.random.RandomState(requests)
+    q_lens = [int(x) for x in rng.randint(0, q_hi + 1, requests)]
+    k_lens = [int(x) for x in rng.randint(0, 400, requests)]
+    q_lens[0] = q_lens[-1] = q_hi
+    k_lens[0] = k_lens[-1] = 390
+    qp, qs, kp, ks, cu_q, cu_k, cu_p, kv_idx = _varlen_case(requests, hq, hk, q_lens, k_lens)
+    dev = [t.cuda() for t in (qp, kp, qs, ks, cu_q, cu_k, cu_p)]
+    kw = dict(max_seqlen_q=max(q_lens), max_seqlen_k=max(k_lens), kv_indices=kv_idx.cuda(), causal=causal)
+    exact = m.fp4_block_scores_varlen(*dev, **kw)
+    fast = m.fp4_block_scores_varlen(*dev, exact=False, **kw)
+    torch.cuda.synchronize()
+    m.device_status()
+    assert torch.equal(torch.isinf(exact), torch.isinf(fast))
+    fin = torch.isfinite(exact)
+    scale = max(float(qs.float().max()) * float(ks.float().max()), 1.0)
+    assert fin.any() and (exact[fin] - fast[fin]).abs().max().item() <= 128 * 36 * scale * 2.0 ** -18
+
+
+def test_fp4_varlen_start_up_with_many_requests():
+    """A CTA finds its run of pages without a walk over all requests: 16384 requests of one page each take no more than six
+    times what the same pages take as 64 requests (2.6 measured, more than 10 with a walk over all requests by one warp)."""
+    m = sp()
+
+    def us(requests, pages):
+        q_lens, k_lens = [1] * requests, [128 * pages] * requests
+        qp, qs, kp, ks, cu_q, cu_k, cu_p, kv_idx = _varlen_case(3, 16, 1, q_lens, k_lens)
+        dev = [t.cuda() for t in (qp, kp, qs, ks, cu_q, cu_k, cu_p)]
+        kw = dict(max_seqlen_q=1, max_seqlen_k=128 * pages, kv_indices=kv_idx.cuda(), causal=True, exact=False)
+        best = float("inf")
+        for _ in range(6):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            m.fp4_block_scores_varlen(*dev, **kw)
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b) * 1e3)
+        return best
+    few, many = us(64, 256), us(16384, 1)
+    print(f"64 requests {few:.1f} us, 16384 requests {many:.1f} us")
+    assert many <= 6 * few
+
+
+@pytest.mark.parametrize("requests,hq,hk,q_hi,causal", [
+    (224, 16, 1, 8, True),                     # one request to a thread of the CTA that looks for its run
+    (225, 4, 2, 150, True),                    # two
+    (1000, 16, 1, 1, False),
+    (7400, 2, 2, 3, True),                     # more than a warp has lanes
+])
+def test_fp4_varlen_runs_of_many_requests(requests, hq, hk, q_hi, causal):
+    """As test_fp4_varlen_runs_of_pages, by the number of requests; many of them empty or without a visible page."""
+    m = sp()
+    rng = np.random.RandomState(requests)
+    q_lens = [int(x) for x in rng.randint(0, q_hi + 1, requests)]
+    k_lens = [int(x) for x in rng.randint(0, 400, requests)]
+    q_lens[0] = q_lens[-1] = q_hi
+    k_lens[0] = k_lens[-1] = 390
+    qp, qs, kp, ks, cu_q, cu_k, cu_p, kv_idx = _varlen_case(requests, hq, hk, q_lens, k_lens)
+    dev = [t.cuda() for t in (qp, kp, qs, ks, cu_q, cu_k, cu_p)]
+    kw = dict(max_seqlen_q=max(q_lens), max_seqlen_k=max(k_lens), kv_indices=kv_idx.cuda(), causal=causal)
+    exact = m.fp4_block_scores_varlen(*dev, **kw)
+    fast = m.fp4_block_scores_varlen(*dev, exact=False, **kw)
+    torch.cuda.synchronize()
+    m.device_status()
+    assert torch.equal(torch.isinf(exact), torch.isinf(fast))
+    fin = torch.isfinite(exact)
+    scale = max(float(qs.float().max()) * float(ks.float().max()), 1.0)
+    assert fin.any() and (exact[fin] - fast[fin]).abs().max().item() <= 128 * 36 * scale * 2.0 ** -18
+
+
+def test_fp4_varlen_start_up_with_many_requests():
+    """A CTA finds its run of pages without a walk over all requests: 16384 requests of one page each take no more than six
+    times what the same pages take as 64 requests (2.6 measured, more than 10 with a walk over all requests by one warp)."""
+    m = sp()
+
+    def us(requests, pages):
+        q_lens, k_lens = [1] * requests, [128 * pages] * requests
+        qp, qs, kp, ks, cu_q, cu_k, cu_p, kv_idx = _varlen_case(3, 16, 1, q_lens, k_lens)
+        dev = [t.cuda() for t in (qp, kp, qs, ks, cu_q, cu_k, cu_p)]
+        kw = dict(max_seqlen_q=1, max_seqlen_k=128 * pages, kv_indices=kv_idx.cuda(), causal=True, exact=False)
+        best = float("inf")
+        for _ in range(6):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            m.fp4_block_scores_varlen(*dev, **kw)
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b) * 1e3)
+        return best
+    few, many = us(64, 256), us(16384, 1)
+    print(f"64 requests {few:.1f} us, 16384 requests {many:.1f} us")
+    assert many <= 6 * few
+
+
 def test_fp4_scores_varlen_inconsistent_lengths_stay_in_bounds():
     """max_seqlen_k smaller than one request's key length, a page table shorter than the key
     length claims, and cu_seqlens_q that runs past total_q: the kernel must skip what does not fit.
