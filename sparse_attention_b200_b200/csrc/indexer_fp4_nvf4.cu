@@ -961,6 +961,8 @@ static bool aligned(const void* p, uintptr_t a) { return (reinterpret_cast<uintp
 // the other, are cut into equal runs, one per CTA: two CTAs per SM (160 tensor-memory columns each) stay for the whole
 // launch, whatever the lengths, which only the device knows. With a CTA per (item, 16 to 64 pages) the last round was
 // nearly empty and every CTA paid its start (descriptors, first loads: 4000 cycles) for 16 pages of 1000.
+// Launches of few CTAs give each a share of one item's pages instead, found by division (RUNS = false): there a run levels
+// nothing, and the way to its place is longer than the rest of the start (see the host side).
 // Warps 0-3 epilogue (lane quarter = warp), warp 4 copies the codes, warp 6 brings the scales, warp 5 issues the MMAs (its
 // elected lane).
 struct QueryScoreParams {
@@ -970,6 +972,7 @@ struct QueryScoreParams {
   int* status;
   int batch, hq, hk, total_q, total_pages, qt_max, tiles_out, causal;
   int group, subs;                     // query heads of a KV head; items of a KV head (heads, or blocks of 16 of them)
+  int share, shares;                   // launches without runs: pages of a CTA, CTAs of an item
 };
 constexpr int QS_THREADS = 224;
 constexpr int QS_PACK_Q = 8, QS_PACK_HEADS = 16;
@@ -1022,20 +1025,49 @@ struct Request {
 };
 
 // A role's place in the CTA's run of pages: the same items in the same order in every role.
-template <bool PACKED>
+template <bool PACKED, bool RUNS>
 struct ScoreWalk {
   int left;                      // pages of the run from the current item's `page` on
   int b, j, kvh, sub;            // item: request, query tile, KV head, query head or head block of it
   int page, end;                 // next page, visible pages of the item
   Request r;
-  __device__ __forceinline__ ScoreWalk(const QueryScoreParams& p, volatile const int* start)
-      : left(start[5]), b(start[0]), j(start[1]), kvh(start[2]), sub(start[3]), page(start[4]) {
-    r = Request::load<PACKED>(p, b);
-    end = r.visible(p, j);
+  ScoreWalk() = default;
+  __device__ __forceinline__ ScoreWalk(const QueryScoreParams& p, volatile const int* start) {
+    if constexpr (RUNS) {
+      left = start[5];
+      b = start[0];
+      j = start[1];
+      kvh = start[2];
+      sub = start[3];
+      page = start[4];
+      r = Request::load<PACKED>(p, b);
+      end = r.visible(p, j);
+    } else {                         // `left` is 0 where the share is empty
+      int rest = static_cast<int>(blockIdx.x) / p.shares;
+      page = (static_cast<int>(blockIdx.x) - rest * p.shares) * p.share;
+      const int items = p.hk * p.subs;               // of a query tile
+      b = rest / items;
+      rest -= b * items;
+      kvh = rest / p.subs;
+      sub = rest - kvh * p.subs;
+      j = 0;
+      if (!PACKED) {
+        rest = b;
+        b = rest / p.qt_max;
+        j = rest - b * p.qt_max;
+      }
+      r = Request::load<PACKED>(p, b);
+      end = j < r.qtiles ? r.visible(p, j) : 0;
+      left = max(0, min(p.share, end - page));
+    }
   }
   // pages of the run in the current item
   __device__ __forceinline__ int count() const { return min(left, end - page); }
   __device__ __forceinline__ void next(const QueryScoreParams& p) {
+    if constexpr (!RUNS) {
+      left = 0;
+      return;
+    }
     left -= count();
     page = 0;
     if (left <= 0 || ++sub < p.subs) return;
@@ -1142,7 +1174,7 @@ __device__ __forceinline__ void find_run(const QueryScoreParams& p, volatile int
   }
 }
 
-template <bool PACKED>
+template <bool PACKED, bool RUNS>
 __global__ void __launch_bounds__(QS_THREADS, 2)
 fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
                            const QueryScoreParams p) {
@@ -1174,17 +1206,23 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
     tmem_alloc(smem_u32(const_cast<int*>(misc)), TM_COLS);
     tmem_relinquish();
   }
-  find_run<PACKED>(p, misc + 2, reinterpret_cast<volatile long long*>(misc + 16), warp, lane);
+  ScoreWalk<PACKED, RUNS> place;
+  if constexpr (RUNS) find_run<PACKED>(p, misc + 2, reinterpret_cast<volatile long long*>(misc + 16), warp, lane);
+  else place = ScoreWalk<PACKED, RUNS>(p, nullptr);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = static_cast<uint32_t>(misc[0]);
-  const int total = misc[7];
+  const int total = RUNS ? misc[7] : place.left;
+  auto first_item = [&]() {
+    if constexpr (RUNS) return ScoreWalk<PACKED, RUNS>(p, misc + 2);
+    else return place;
+  };
 
   if (total > 0) {
   if (warp == 4) {
     // ----------------------------------------------------------- codes (TMA); page ids 32 at a time
-    ScoreWalk<PACKED> walk(p, misc + 2);
+    ScoreWalk<PACKED, RUNS> walk = first_item();
     int items = 0, left = 0, pg = 0, ids = 0;     // items begun, pages left in the current one
     int pushed = 0;
     bool ok = true;
@@ -1230,7 +1268,7 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
     // ----------------------------------------------------------- scales: staged QS_AHEAD pages ahead, then re-ordered
     // (asynchronous copies, not loads into registers: those need the loop unrolled over the pages in flight, and its
     // instructions alone, fetched for the first time, took 7000 cycles before the first page)
-    ScoreWalk<PACKED> ahead_walk(p, misc + 2), walk(p, misc + 2);
+    ScoreWalk<PACKED, RUNS> ahead_walk = first_item(), walk = first_item();
     int ids = 0, ahead_left = 0, ahead_pg = 0;    // of the walk ahead: 32 page ids, pages left in its item, next page
     auto raw = [&](int t) { return QS_OFF_RAW + (t % QS_AHEAD) * SF_BYTES + lane * 8; };
     auto fetch = [&](int t) {                     // rows lane, lane + 32, .. of page t; one group per page
@@ -1299,7 +1337,7 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
     // ----------------------------------------------------------- MMA issue (elected lane of a converged warp)
     constexpr uint32_t IDESC = idesc_nvf4(128, 128);
     const bool lead = elect_one();
-    ScoreWalk<PACKED> walk(p, misc + 2);
+    ScoreWalk<PACKED, RUNS> walk = first_item();
     bool ok = true;
     int items = 0, left = 0;
     for (int t = 0; t < total; ++t) {
@@ -1353,7 +1391,7 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
     const int row = warp * 32 + lane;
-    ScoreWalk<PACKED> walk(p, misc + 2);
+    ScoreWalk<PACKED, RUNS> walk = first_item();
     bool ok = true;
     int t = 0;
     while (ok && walk.left > 0) {
@@ -1570,7 +1608,24 @@ int launch_fp4_scores_varlen_nv(const void* qp, const void* qs, const void* kp, 
   if (items == 0 || p.tiles_out == 0) return SB_OK;
   // two CTAs per SM, at least two pages each
   const long long most = (items * p.tiles_out + 1) / 2;
-  const dim3 grid(static_cast<unsigned>(std::min<long long>(2LL * ctx->sm_count, most)));
+  long long ctas = std::min<long long>(2LL * ctx->sm_count, most);
+  // Up to four CTAs to an SM, the longest lengths taken for all, each gets a share of one item's pages instead of a run: the
+  // call has no last round to level, and a run's place costs 1.5 to 3 us to find. In a graph, us, runs -> shares (and before
+  // there were runs): one token of one request 6.9 -> 5.1 (5.5), of 64 requests of 100 to 400 keys 8.9 -> 5.3 (5.8), of 256 11.1 ->
+  // 9.0 (9.4), prefill of eight requests of up to 300 8.5 -> 6.3 (7.2). Beyond, runs are faster (64 requests of 1000 to 4000
+  // keys 11.1, shares 13.2) unless a request is one item of a few pages, where a run changes its item every other page: 600
+  // requests of 500 to 900 keys 18.9 -> 16.9 (16.2), 1024 of 100 to 400 20.1 -> 17.6 (16.0), 2048 32.6 -> 30.6 (26.3).
+  int share = 64;
+  while (share > 2 && items * ((p.tiles_out + share - 1) / share) < 4LL * ctx->sm_count) share >>= 1;
+  const long long shared = items * ((p.tiles_out + share - 1) / share);
+  const bool single = packed && items == batch;      // one item to a request
+  const bool runs = shared > (single && p.tiles_out <= 8 ? 16 : 4) * ctx->sm_count;
+  if (!runs) {
+    p.share = share;
+    p.shares = (p.tiles_out + share - 1) / share;
+    ctas = shared;
+  }
+  const dim3 grid(static_cast<unsigned>(ctas));
   CUtensorMap qm, km;
   {
     const cuuint64_t dims[3] = {64, static_cast<cuuint64_t>(hq), static_cast<cuuint64_t>(total_q)};
@@ -1591,10 +1646,11 @@ int launch_fp4_scores_varlen_nv(const void* qp, const void* qs, const void* kp, 
       return set_error(SB_ERR_CUDA, "cuTensorMapEncodeTiled failed for the key codes");
   }
   if (!(ctx->tc_attr & (1 << 12))) {
-    cudaError_t e = cudaFuncSetAttribute(fp4_nv_query_scores_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, QS_SMEM);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(fp4_nv_query_scores_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, QS_SMEM);
-    if (e != cudaSuccess) return set_error(SB_ERR_CUDA, cudaGetErrorString(e));
+    for (auto kernel : {fp4_nv_query_scores_kernel<false, false>, fp4_nv_query_scores_kernel<false, true>,
+                        fp4_nv_query_scores_kernel<true, false>, fp4_nv_query_scores_kernel<true, true>}) {
+      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, QS_SMEM);
+      if (e != cudaSuccess) return set_error(SB_ERR_CUDA, cudaGetErrorString(e));
+    }
     ctx->tc_attr |= (1 << 12);
   }
   cudaLaunchConfig_t cfg{};
@@ -1607,8 +1663,9 @@ int launch_fp4_scores_varlen_nv(const void* qp, const void* qs, const void* kp, 
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, packed ? fp4_nv_query_scores_kernel<true> : fp4_nv_query_scores_kernel<false>,
-                                     qm, km, p);
+  auto kernel = packed ? (runs ? fp4_nv_query_scores_kernel<true, true> : fp4_nv_query_scores_kernel<true, false>)
+                       : (runs ? fp4_nv_query_scores_kernel<false, true> : fp4_nv_query_scores_kernel<false, false>);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, qm, km, p);
   return e == cudaSuccess ? SB_OK : set_error(SB_ERR_CUDA, cudaGetErrorString(e));
 }
 

@@ -943,47 +943,26 @@ def test_fp4_varlen_runs_of_many_requests(requests, hq, hk, q_hi, causal):
     assert fin.any() and (exact[fin] - fast[fin]).abs().max().item() <= 128 * 36 * scale * 2.0 ** -18
 
 
-def test_fp4_varlen_start_up_with_many_requests():
-    """A CTA finds its run of pages without a walk over all requests: 16384 requests of one page each take no more than six
-    times what the same pages take as 64 requests (2.6 measured, more than 10 with a walk over all requests by one warp)."""
-    m = sp()
-
-    def us(requests, pages):
-        q_lens, k_lens = [1] * requests, [128 * pages] * requests
-        qp, qs, kp, ks, cu_q, cu_k, cu_p, kv_idx = _varlen_case(3, 16, 1, q_lens, k_lens)
-        dev = [t.cuda() for t in (qp, kp, qs, ks, cu_q, cu_k, cu_p)]
-        kw = dict(max_seqlen_q=1, max_seqlen_k=128 * pages, kv_indices=kv_idx.cuda(), causal=True, exact=False)
-        best = float("inf")
-        for _ in range(6):
-            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            a.record()
-            m.fp4_block_scores_varlen(*dev, **kw)
-            b.record()
-            torch.cuda.synchronize()
-            best = min(best, a.elapsed_time(b) * 1e3)
-        return best
-    few, many = us(64, 256), us(16384, 1)
-    print(f"64 requests {few:.1f} us, 16384 requests {many:.1f} us")
-    assert many <= 6 * few
-
-
-@pytest.mark.parametrize("requests,hq,hk,q_hi,causal", [
-    (224, 16, 1, 8, True),                     # one request to a thread of the CTA that looks for its run
-    (225, 4, 2, 150, True),                    # two
-    (1000, 16, 1, 1, False),
-    (7400, 2, 2, 3, True),                     # more than a warp has lanes
+@pytest.mark.parametrize("requests,hq,hk,q_hi,k_hi,causal", [
+    (1, 16, 1, 1, 200, True),                  # one CTA
+    (5, 40, 2, 8, 1500, True),                 # two blocks of heads to a KV head, shares of two pages, the last ones empty
+    (9, 6, 3, 300, 700, True),                 # query tiles and heads; requests shorter than the longest
+    (37, 16, 1, 1, 4000, False),               # 592 CTAs: the last size of a launch without runs
+    (38, 16, 1, 1, 4000, False),               # 608: the first with runs
+    (2368, 16, 1, 3, 500, True),               # one item to a request, few pages: as many CTAs as requests
+    (2369, 16, 1, 3, 500, True),               # and one more
 ])
-def test_fp4_varlen_runs_of_many_requests(requests, hq, hk, q_hi, causal):
-    """As test_fp4_varlen_runs_of_pages, by the number of requests; many of them empty or without a visible page."""
+def test_fp4_varlen_shares_of_an_item(requests, hq, hk, q_hi, k_hi, causal):
+    """Launches whose CTAs take shares of an item's pages, and those next to them that take runs, against the exact scorer
+    (bound as in test_fp4_varlen_runs_of_pages)."""
     m = sp()
     rng = np.random.RandomState(requests)
-    q_lens = [int(x) for x in rng.randint(0, q_hi + 1, requests)]
-    k_lens = [int(x) for x in rng.randint(0, 400, requests)]
-    q_lens[0] = q_lens[-1] = q_hi
-    k_lens[0] = k_lens[-1] = 390
-    qp, qs, kp, ks, cu_q, cu_k, cu_p, kv_idx = _varlen_case(requests, hq, hk, q_lens, k_lens)
+    q_lens = [int(x) for x in rng.randint(0 if requests > 4 else 1, q_hi + 1, requests)]
+    k_lens = [int(x) for x in rng.randint(1, k_hi + 1, requests)]
+    q_lens[-1], k_lens[-1] = q_hi, k_hi
+    qp, qs, kp, ks, cu_q, cu_k, cu_p, kv_idx = _varlen_case(requests + 1, hq, hk, q_lens, k_lens)
     dev = [t.cuda() for t in (qp, kp, qs, ks, cu_q, cu_k, cu_p)]
-    kw = dict(max_seqlen_q=max(q_lens), max_seqlen_k=max(k_lens), kv_indices=kv_idx.cuda(), causal=causal)
+    kw = dict(max_seqlen_q=q_hi, max_seqlen_k=k_hi, kv_indices=kv_idx.cuda(), causal=causal)
     exact = m.fp4_block_scores_varlen(*dev, **kw)
     fast = m.fp4_block_scores_varlen(*dev, exact=False, **kw)
     torch.cuda.synchronize()
