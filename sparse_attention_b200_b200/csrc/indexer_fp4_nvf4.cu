@@ -39,7 +39,7 @@ namespace fnv {
 constexpr int CODE_BYTES = 128 * 64;              // one operand tile: 128 rows of 64 bytes of codes
 constexpr int SF_BYTES = 1024;                    // its scales: two 512-byte chunks (features 0-63, 64-127)
 constexpr int STAGE_BYTES = CODE_BYTES + SF_BYTES;
-constexpr int A_STAGES = 6;
+constexpr int A_STAGES = 6;                       // at most (see Layout)
 constexpr int C_MAX = 192;
 constexpr int NUM_THREADS = 320;
 constexpr int TMA_WARP = 8, MMA_WARP = 9;
@@ -54,13 +54,19 @@ constexpr int MAX_TILES = 16384;                  // 64 KiB of scores
 constexpr int ACC_STAGES = 1;                     // accumulators of 128 columns (a whole query tile)
 
 constexpr int OFF_A = 0;
-constexpr int OFF_B = A_STAGES * STAGE_BYTES;     // query tile: codes + scales
-constexpr int RAW_STAGES = 4;                     // pages whose scales are on their way
-constexpr int OFF_RAW = OFF_B + STAGE_BYTES;      // staging ring: the scales of a page as they are in memory
-constexpr int OFF_CAND = OFF_RAW + RAW_STAGES * SF_BYTES;   // candidate arrays of the selection phase
-constexpr int OFF_SCORES = OFF_CAND + 4 * C_MAX * 4;
-// the selection phase re-uses [0, OFF_CAND) for int8 rows and fp32 scales of a query tile and a key page
-static_assert(2 * 128 * FP4_ROW_WORDS * 4 + 2 * 128 * 8 * 4 <= OFF_CAND, "staging area of the exact scorer does not fit");
+// Shared memory of the scorers by the number of pages in flight: six, or four where the selection kernel's scores (4 bytes a
+// page) leave no room for a second CTA on the SM beside six; the staging ring then shares the candidate arrays' place.
+template <int STAGES>
+struct Layout {
+  static constexpr int B = STAGES * STAGE_BYTES;            // query tile: codes + scales
+  static constexpr int RAW = B + STAGE_BYTES;               // staging ring: the scales of a page as they are in memory
+  static constexpr int RAW_STAGES = STAGES == A_STAGES ? 4 : 3;     // pages whose scales are on their way
+  static constexpr int CAND = STAGES == A_STAGES ? RAW + RAW_STAGES * SF_BYTES : RAW;     // arrays of the selection phase
+  static constexpr int SCORES = CAND + 4 * C_MAX * 4;
+  static_assert(STAGES == A_STAGES || RAW_STAGES * SF_BYTES <= SCORES - CAND, "staging ring");
+  // the selection phase re-uses [0, CAND) for int8 rows and fp32 scales of a query tile and a key page
+  static_assert(2 * 128 * FP4_ROW_WORDS * 4 + 2 * 128 * 8 * 4 <= CAND, "staging area of the exact scorer does not fit");
+};
 // tensor memory columns
 constexpr int TM_ACC = 0;
 constexpr int TM_SFA = ACC_STAGES * 128;           // 2 slots x 8 columns (two K halves of 4 columns)
@@ -221,27 +227,29 @@ struct Geometry {
 // warps (540 to 720), two or three producer warps per CTA here (450), three accumulators of 64 columns per CTA (450).
 // Producer warp: query tile once, then key pages page0 + (t + rot) % wrap for t = 0 .. num_tiles - 1 (num_tiles <= wrap,
 // rot < wrap).
+template <int STAGES>
 __device__ __forceinline__ void producer_role(const Geometry& g, const CUtensorMap* q_map, const CUtensorMap* k_map,
                                               uint32_t base, unsigned char* gbase, uint32_t bar0, const Guard& guard,
                                               int b, int h, int hk_idx, long long q_row0, int page0, int num_tiles,
                                               int rot, int wrap, int lane, int code0) {
+  using L = Layout<STAGES>;
   auto bar = [&](int i) { return bar0 + 8u * i; };
   auto page_of = [&](int t) { return page0 + (t + rot >= wrap ? t + rot - wrap : t + rot); };
   auto key_row = [&](int pg) { return ((static_cast<long long>(b) * g.tiles + pg) * g.hk + hk_idx) * 128; };
   if (lane == 0) {
     mbar_expect_tx(bar(B_FULL), CODE_BYTES);
-    tma_load_3d(base + OFF_B, q_map, 0, h, static_cast<int>(q_row0), bar(B_FULL));
+    tma_load_3d(base + L::B, q_map, 0, h, static_cast<int>(q_row0), bar(B_FULL));
   }
   {
     const ScaleRegs s = load_scales(g.qs + (q_row0 * g.hidx + h) * 8, static_cast<long long>(g.hidx) * 8, lane);
-    store_scale_chunks(gbase + OFF_B + CODE_BYTES, s, lane);
+    store_scale_chunks(gbase + L::B + CODE_BYTES, s, lane);
     fence_async_smem();
     __syncwarp();
     if (lane == 0) mbar_arrive(bar(B_FULL));
   }
   // The scales of a page are staged RAW_STAGES pages ahead by asynchronous copies, a lane its rows lane, lane + 32, .., and
   // re-ordered from there. (Loads into registers need the loop unrolled over the pages in flight.)
-  auto raw = [&](int t) { return OFF_RAW + (t % RAW_STAGES) * SF_BYTES + lane * 8; };
+  auto raw = [&](int t) { return L::RAW + (t % L::RAW_STAGES) * SF_BYTES + lane * 8; };
   auto fetch = [&](int t) {
     if (t < num_tiles) {
       const uint8_t* src = g.ks + key_row(page_of(t)) * 8 + lane * 8;
@@ -251,30 +259,30 @@ __device__ __forceinline__ void producer_role(const Geometry& g, const CUtensorM
     cp_async_commit();
   };
 #pragma unroll 1
-  for (int t = 0; t < RAW_STAGES; ++t) fetch(t);
+  for (int t = 0; t < L::RAW_STAGES; ++t) fetch(t);
   bool ok = true;
 #pragma unroll 1
   for (int t = 0; t < num_tiles; ++t) {
-    const int s = t % A_STAGES, use = t / A_STAGES;
+    const int s = t % STAGES, use = t / STAGES;
     if (use > 0) ok = mbar_wait_warp(bar(A_EMPTY + s), (use - 1) & 1, guard, code0 + s);
     if (!ok) break;
     if (lane == 0) {
       mbar_expect_tx(bar(A_FULL + s), CODE_BYTES);
       tma_load_2d(base + OFF_A + s * STAGE_BYTES, k_map, 0, static_cast<int>(key_row(page_of(t))), bar(A_FULL + s));
     }
-    cp_async_wait<RAW_STAGES - 1>();
+    cp_async_wait<L::RAW_STAGES - 1>();
     ScaleRegs regs;
 #pragma unroll
     for (int i = 0; i < 4; ++i) regs.r[i] = *reinterpret_cast<const uint2*>(gbase + raw(t) + i * 256);
     store_scale_chunks(gbase + OFF_A + s * STAGE_BYTES + CODE_BYTES, regs, lane);
     __syncwarp();
     if (lane == 0) mbar_arrive(bar(A_FULL + s));
-    fetch(t + RAW_STAGES);
+    fetch(t + L::RAW_STAGES);
   }
   cp_async_wait<0>();
   if (!ok)
-    for (int t = max(0, num_tiles - A_STAGES); t < num_tiles; ++t)
-      mbar_wait_drain(bar(A_FULL + t % A_STAGES), (t / A_STAGES) & 1);
+    for (int t = max(0, num_tiles - STAGES); t < num_tiles; ++t)
+      mbar_wait_drain(bar(A_FULL + t % STAGES), (t / STAGES) & 1);
 }
 
 // MMA warp: page t against the whole query tile into accumulator t % ACC_STAGES. The key scales of
@@ -282,6 +290,7 @@ __device__ __forceinline__ void producer_role(const Geometry& g, const CUtensorM
 // page t - 2, which had completed (their accumulator had been read out and released) before the MMAs
 // of page t - 1 were issued; this holds for one or two accumulators.
 static_assert(ACC_STAGES <= 2, "the two key-scale slots are protected by the accumulator hand-over only up to two accumulators");
+template <int STAGES>
 __device__ __forceinline__ void mma_role(uint32_t base, uint32_t bar0, uint32_t tmem, const Guard& guard, int num_tiles,
                                          int code0) {
   auto bar = [&](int i) { return bar0 + 8u * i; };
@@ -290,13 +299,13 @@ __device__ __forceinline__ void mma_role(uint32_t base, uint32_t bar0, uint32_t 
   if (!mbar_wait_warp(bar(B_FULL), 0, guard, code0)) return;
   tc_fence_after();
   if (lead) {
-    tmem_cp_scales(tmem + TM_SFB, desc_scale_chunk(base + OFF_B + CODE_BYTES));
-    tmem_cp_scales(tmem + TM_SFB + 4, desc_scale_chunk(base + OFF_B + CODE_BYTES + 512));
+    tmem_cp_scales(tmem + TM_SFB, desc_scale_chunk(base + Layout<STAGES>::B + CODE_BYTES));
+    tmem_cp_scales(tmem + TM_SFB + 4, desc_scale_chunk(base + Layout<STAGES>::B + CODE_BYTES + 512));
   }
-  const uint64_t b0 = desc_sw64_kmajor(base + OFF_B);
+  const uint64_t b0 = desc_sw64_kmajor(base + Layout<STAGES>::B);
   for (int t = 0; t < num_tiles; ++t) {
-    const int s = t % A_STAGES, st = t % ACC_STAGES;
-    if (!mbar_wait_warp(bar(A_FULL + s), (t / A_STAGES) & 1, guard, code0 + 1 + s)) return;
+    const int s = t % STAGES, st = t % ACC_STAGES;
+    if (!mbar_wait_warp(bar(A_FULL + s), (t / STAGES) & 1, guard, code0 + 1 + s)) return;
     fence_async_smem();              // the producer's scale stores, for the copies below
     tc_fence_after();
     // the scale copy does not touch the accumulator: it goes out before the accumulator hand-over is awaited
@@ -366,22 +375,24 @@ struct Params {
   int topk, cand;
 };
 
-// One CTA per (batch, index head, query tile), two CTAs per SM (the exact re-scoring of one
+// One CTA per (batch, index head, query tile), two CTAs per SM up to 16304 pages (the exact re-scoring of one
 // overlaps the tensor-core scoring of the other): approximate tile scores of every key
 // page on the tensor cores, then candidate selection and exact re-scoring.
 // Warps 0-7 epilogue (lane quarter = warp & 3, query half = warp >> 2), warp 8 producer,
 // warp 9 MMA issue (its elected lane).
+template <int STAGES>
 __global__ void __launch_bounds__(NUM_THREADS, 2)
 fp4_nv_select_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map, const Params p) {
+  using L = Layout<STAGES>;
   extern __shared__ unsigned char smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   unsigned char* gbase = smem_raw + (base - raw);
   const Geometry& g = p.g;
-  int* scores = reinterpret_cast<int*>(gbase + OFF_SCORES);
+  int* scores = reinterpret_cast<int*>(gbase + L::SCORES);
   const int score_bytes = (g.tiles * 4 + 15) & ~15;
-  unsigned char* aux = gbase + OFF_SCORES + score_bytes;
-  const uint32_t bar0 = base + OFF_SCORES + score_bytes;
+  unsigned char* aux = gbase + L::SCORES + score_bytes;
+  const uint32_t bar0 = base + L::SCORES + score_bytes;
   volatile int* misc = reinterpret_cast<volatile int*>(aux + 128);   // tmem base, abort, unsafe, l1q bits, l2q bits, k-th bound
   float* scratch_f = reinterpret_cast<float*>(aux + 192);            // [16]
   int* scratch_i = reinterpret_cast<int*>(aux + 256);                // [16]
@@ -400,7 +411,7 @@ fp4_nv_select_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
 
   if (threadIdx.x == 0) {
     misc[1] = 0;
-    for (int i = 0; i < A_STAGES; ++i) {
+    for (int i = 0; i < STAGES; ++i) {
       mbar_init(bar(A_FULL + i), 2);      // the TMA transaction of the codes + the producer warp's scale stores
       mbar_init(bar(A_EMPTY + i), 1);
     }
@@ -422,10 +433,10 @@ fp4_nv_select_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
   const uint32_t tmem = static_cast<uint32_t>(misc[0]);
 
   if (warp == TMA_WARP) {
-    producer_role(g, &q_map, &k_map, base, gbase, bar0, guard, b, h, hk_idx, q_row0, 0, num_tiles, rot, num_tiles, lane,
+    producer_role<STAGES>(g, &q_map, &k_map, base, gbase, bar0, guard, b, h, hk_idx, q_row0, 0, num_tiles, rot, num_tiles, lane,
                   0x500);
   } else if (warp == MMA_WARP) {
-    mma_role(base, bar0, tmem, guard, num_tiles, 0x510);
+    mma_role<STAGES>(base, bar0, tmem, guard, num_tiles, 0x510);
     __syncwarp();
   } else {
     // epilogue: thread = key row of the page, this warp's 64-query half of the tile
@@ -473,7 +484,7 @@ fp4_nv_select_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
   uint32_t* k_i8 = q_i8 + 128 * FP4_ROW_WORDS;
   float* q_sc = reinterpret_cast<float*>(k_i8 + 128 * FP4_ROW_WORDS);
   float* k_sc = q_sc + 128 * 8;
-  int32_t* cand_ids = reinterpret_cast<int32_t*>(gbase + OFF_CAND);
+  int32_t* cand_ids = reinterpret_cast<int32_t*>(gbase + L::CAND);
   int* cand_ex = reinterpret_cast<int*>(cand_ids + C_MAX);
   float* cand_apx = reinterpret_cast<float*>(cand_ex + C_MAX);     // approximate tile scores of the candidates
   int* near_s = reinterpret_cast<int*>(cand_apx + C_MAX);          // candidate needs its exact score
@@ -683,7 +694,7 @@ constexpr int PR_QCAP = 2048;                // queued groups of elements per CT
 // Selection of 160 lists, us: 4096 pages 232000 -> 3150, 1024 pages, four of zeros, 113000 -> 1580.)
 constexpr int PR_DRAIN = PR_QCAP - 1024;
 constexpr int PR_PAGES_MAX = 3072;           // pages of a CTA: the results of more would leave one CTA to an SM
-constexpr int PR_OFF_AUX = OFF_CAND;         // barriers (128 bytes), misc (128 bytes)
+constexpr int PR_OFF_AUX = Layout<A_STAGES>::CAND;         // barriers (128 bytes), misc (128 bytes)
 constexpr int PR_OFF_QUEUE = PR_OFF_AUX + 256;            // [PR_QCAP] groups waiting for their exact values
 constexpr int PR_OFF_APX = PR_OFF_QUEUE + PR_QCAP * 4;     // [PR_QCAP] their largest approximate values
 constexpr int PR_OFF_RES = PR_OFF_APX + PR_QCAP * 4;       // [pages per CTA] exact maxima as ordered ints
@@ -766,10 +777,10 @@ fp4_nv_prune_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
   const uint32_t tmem = static_cast<uint32_t>(misc[0]);
 
   if (warp == TMA_WARP) {
-    producer_role(g, &q_map, &k_map, base, gbase, bar0, guard, b, h, hk_idx, q_row0, page0, num_tiles, 0, num_tiles, lane,
+    producer_role<A_STAGES>(g, &q_map, &k_map, base, gbase, bar0, guard, b, h, hk_idx, q_row0, page0, num_tiles, 0, num_tiles, lane,
                   0x580);
   } else if (warp == MMA_WARP) {
-    mma_role(base, bar0, tmem, guard, num_tiles, 0x590);
+    mma_role<A_STAGES>(base, bar0, tmem, guard, num_tiles, 0x590);
     __syncwarp();
   } else {
     // epilogue: thread = key row of the page, this warp's 64-query half of the tile
@@ -1515,15 +1526,20 @@ int launch_fp4_indexer_tc(const void* qp, const void* qs, const void* kp, const 
   p.ids = ids;
   p.status = ctx->status;
   p.topk = topk; p.cand = cand;
-  const size_t smem = OFF_SCORES + ((static_cast<size_t>(tiles) * 4 + 15) & ~static_cast<size_t>(15)) + 320 + 1024;
-  if (!(ctx->tc_attr & (1 << 8))) {
-    cudaError_t e = cudaFuncSetAttribute(fp4_nv_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(fp4_nv_select_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+  // shared memory beside the layout's: scores, barriers and scratch, slack of the alignment
+  const size_t rest = ((static_cast<size_t>(tiles) * 4 + 15) & ~static_cast<size_t>(15)) + 320 + 1024;
+  // Two CTAs to an SM with 1 KiB of the system's each: with six stages up to 10672 pages, with four up to 16304. 1024 lists of
+  // 12000 pages, ms: six stages and one CTA 30.8, four and two 18.8; of 10000 pages six and two 15.6.
+  const bool six = 2 * (Layout<A_STAGES>::SCORES + rest + 1024) <= 228 * 1024;
+  auto kernel = six ? fp4_nv_select_kernel<A_STAGES> : fp4_nv_select_kernel<4>;
+  const int configured = six ? 1 << 8 : 1 << 21;
+  if (!(ctx->tc_attr & configured)) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     if (e != cudaSuccess) return set_error(SB_ERR_CUDA, cudaGetErrorString(e));
-    ctx->tc_attr |= (1 << 8);
+    ctx->tc_attr |= configured;
   }
-  fp4_nv_select_kernel<<<batch * hidx * qt, NUM_THREADS, smem, stream>>>(qm, km, p);
+  kernel<<<batch * hidx * qt, NUM_THREADS, (six ? Layout<A_STAGES>::SCORES : Layout<4>::SCORES) + rest, stream>>>(qm, km, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? SB_OK : set_error(SB_ERR_CUDA, cudaGetErrorString(e));
 }

@@ -611,6 +611,24 @@ def test_fp4_tensor_core_path_bit_exact():
     m.device_status()
 
 
+@pytest.mark.parametrize("pages", [10672, 10673, 12001, 16304, 16384])
+def test_fp4_selection_of_long_lists(pages):
+    """Six pages in flight up to 10672 pages, four beyond; one CTA to an SM again beyond 16304: ids of the exact scorer."""
+    m = sp()
+    g = torch.Generator(device="cuda").manual_seed(pages)
+    choices = torch.tensor([0.25, 0.375, 0.5, 0.75, 1.0, 1.5, 2.0], device="cuda")
+    qp = torch.randint(256, (256, 2, 64), dtype=torch.uint8, generator=g, device="cuda")
+    kp = torch.randint(256, (pages, 1, 128, 64), dtype=torch.uint8, generator=g, device="cuda")
+    qs = choices[torch.randint(7, (256, 2, 8), generator=g, device="cuda")].to(torch.float8_e4m3fn)
+    ks = choices[torch.randint(7, (pages, 1, 128, 8), generator=g, device="cuda")].to(torch.float8_e4m3fn)
+    inputs = m.prepare_fp4_inputs(qp, kp, qs, ks, batch_size=1, len_q=256, len_kv=pages * 128)
+    ids, ws = m.fp4_indexer_fast(inputs, topk=32)
+    torch.cuda.synchronize()
+    m.device_status()
+    assert ws[:4].view(torch.int32).item() == 4          # CTAs of the tensor-core kernel
+    assert torch.equal(ids, m.fp4_indexer(inputs, topk=32))
+
+
 def _fast_path_tile_scores(ws, b, hidx, hk, lq, lkv):
     """Tile scores the fast entry left in its workspace: 256 bytes of statistics, then the scores."""
     n = b * hidx * (lq // 128) * (lkv // 128)
