@@ -119,8 +119,9 @@ int sparse_b200_split_kv_segments(const int32_t* block_idx, const int32_t* block
                                   int topk, int kv_blocks, int nseg, void* stream);
 
 /* Main and merge of a KV-centric operator with a single KV range in one launch: its bf16 partial is the output. Lists
- * as sparse_b200_split_kv_segments writes them for nseg = 1. A row without any weight (an empty list, or only scores of
- * -inf) is 0 with LSE -inf, as sparse_b200_combine leaves it. lse may be NULL. */
+ * as sparse_b200_split_kv_segments writes them for nseg = 1. A row without any weight (an empty list, or no scores but
+ * -inf and NaN) is 0 with LSE -inf and a row with a NaN beside other scores or a score of +inf is NaN, as it is with several
+ * ranges where each has a finite score of the row. lse may be NULL. */
 int sparse_b200_kv_centric_single(const void* q, const void* k, const void* v, const int32_t* seg_block_idx,
                                   const int32_t* seg_block_count, void* out, float* lse, int batch, int hq, int hkv,
                                   int sq, int skv, int topk, void* stream);

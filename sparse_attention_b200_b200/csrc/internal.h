@@ -43,7 +43,9 @@ struct QCentricArgs {
   int owners = 1;
   void* const* owner_out = nullptr;
   float* const* owner_lse = nullptr;
-  bool dead_zero = false;       // bf16: a row without any weight is 0 with LSE -inf, as the merge of partials leaves it (not NaN)
+  // bf16: a row without any weight (scores of -inf or NaN only) is 0 with LSE -inf, as the merge of several ranges leaves it
+  // (not NaN)
+  bool dead_zero = false;
 };
 int launch_q_centric(const QCentricArgs& a, cudaStream_t stream);
 // scratch that a launch with these sizes splits its lists into (0: it does not)

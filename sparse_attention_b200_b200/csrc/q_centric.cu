@@ -110,7 +110,7 @@ struct Params {
   // num_virtual = items as the roles see them; without balancing tail_first = num_virtual = num_items.
   int tail_first, tail_parts, num_virtual;
   float* tail_lse;         // [pieces * 2 * 128]
-  int dead_zero;           // rows without any weight are 0 (see QCentricArgs)
+  int dead_zero;           // rows without any weight are 0 with LSE -inf (see QCentricArgs)
   FastDiv by_parts, by_seg, by_pairs, by_qt, by_hkv, by_qpairs, by_hq, by_group;
 };
 
@@ -774,7 +774,10 @@ q_centric_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
       }
       __syncwarp();
       if (lane == 0) *handed_ptr = handed + 1;
-      stats[q * TILE + row_in_tile] = p.dead_zero && row_sum == 0.f ? 0.f : 1.0f / row_sum;
+      // nothing but scores of -inf (sum 0) or NaN: weight 0, as a merge of ranges, which passes over LSEs of NaN, leaves it
+      const bool dead = p.dead_zero && row_max == -FLT_MAX && !(row_sum > 0.f);
+      if (dead) row_sum = 0.f;                   // LSE -inf
+      stats[q * TILE + row_in_tile] = dead ? 0.f : 1.0f / row_sum;
       if constexpr (SCATTER) {
         long long tile_row = s[q].out_row;
         const int slice = slice_of(sc, tile_row);

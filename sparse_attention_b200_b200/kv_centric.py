@@ -70,7 +70,7 @@ class Prepared:
         self.error = torch.zeros(1, dtype=torch.int32, device=dev)
         self.out = torch.empty((b, hq, sq, d), dtype=torch.bfloat16, device=dev)
         self.out_lse = torch.empty((b, hq, sq), dtype=torch.float32, device=dev)
-        # the bf16 partial of a single range is the output: same memory, and the merge leaves it as it is
+        # the bf16 partial of a single range is the output: main() writes it, combine() has nothing to do
         self.single = self.nseg == 1 and partial == "bf16"
         if self.single:
             self.partial, self.lses = self.out.unsqueeze(0), self.out_lse.unsqueeze(0)
@@ -91,18 +91,7 @@ class Prepared:
                 _lib.ptr(self.error), b, hkv, qb, self.topk, self.kv_blocks, self.nseg, _lib.current_stream()))
 
     def main(self):
-        from .q_centric import attention_partial_out
-        attention_partial_out(self.q, self.k, self.v, self.seg_ids, self.seg_counts, self.partial, self.lses)
-
-    def combine(self):
-        rows = self.out_lse.numel()
-        with torch.cuda.device(self.q.device):
-            _lib.check(_lib.lib().sparse_b200_combine(
-                _lib.ptr(self.partial), int(self.partial.dtype == torch.float32), _lib.ptr(self.lses),
-                _lib.ptr(self.out), _lib.ptr(self.out_lse), rows, self.nseg, 1, _lib.current_stream()))
-
-    def core(self):
-        if self.single:                          # main and merge in one launch
+        if self.single:
             (b, hq, sq, _), (hkv, skv) = self.q.shape, self.k.shape[1:3]
             with torch.cuda.device(self.q.device):
                 _lib.check(_lib.lib().sparse_b200_kv_centric_single(
@@ -110,6 +99,19 @@ class Prepared:
                     _lib.ptr(self.seg_counts), _lib.ptr(self.out), _lib.ptr(self.out_lse), b, hq, hkv, sq, skv, self.topk,
                     _lib.current_stream()))
             return
+        from .q_centric import attention_partial_out
+        attention_partial_out(self.q, self.k, self.v, self.seg_ids, self.seg_counts, self.partial, self.lses)
+
+    def combine(self):
+        if self.single:
+            return
+        rows = self.out_lse.numel()
+        with torch.cuda.device(self.q.device):
+            _lib.check(_lib.lib().sparse_b200_combine(
+                _lib.ptr(self.partial), int(self.partial.dtype == torch.float32), _lib.ptr(self.lses),
+                _lib.ptr(self.out), _lib.ptr(self.out_lse), rows, self.nseg, 1, _lib.current_stream()))
+
+    def core(self):
         self.main()
         self.combine()
 

@@ -244,3 +244,36 @@ def test_default_ranges(b, hkv, g, qb, nb, topk, with_counts, nseg):
         dead = m.Prepared(q.cuda(), k.cuda(), dev[2], dev[3], dev[4], nseg=n)
         out, lse = dead.run()
         assert (out == 0).all() and (lse == float("-inf")).all()
+
+
+def test_single_range_rows_of_nan_and_inf():
+    """One range against two, rows with scores of NaN and of +inf among them, every row with finite scores in both ranges
+    unless all of its scores are NaN: the same rows are 0 with LSE -inf and the same are NaN; the operator and its stages by
+    hand leave the same bits."""
+    m = sp()
+    q, k, v = gen.make_qkv(1, 4, 2, 512, 512, seed=71)
+    ids = gen.make_ids(1, 2, 4, 4, 4, 72, "unsorted")          # every list has all four blocks
+    q[0, 3, 200:333, :] = float("nan")                          # these rows: nothing but NaN
+    k[0, 1, 130, 7] = float("nan")                              # KV head 1: NaN in block 1 for every row
+    q[0, 0, :256, 9] = 1.0
+    q[0, 0, 256:, 9] = -1.0
+    k[0, 0, 300, 9] = float("inf")                              # head 0: +inf for half of the rows, -inf for the others
+    q[0, :, 100, 5] = float("nan")                              # nothing but NaN
+    dev = [t.cuda() for t in (q, k, v, ids)]
+    one, two = m.Prepared(*dev, nseg=1), m.Prepared(*dev, nseg=2)
+    (out, lse), (out2, lse2) = one.run(), two.run()
+    torch.cuda.synchronize()
+    m.device_status()
+    assert torch.equal(torch.isnan(out), torch.isnan(out2)) and torch.equal(torch.isnan(lse), torch.isnan(lse2))
+    assert torch.isnan(lse[0, 0, :256]).sum() == 255 and not torch.isnan(lse[0, 0, 256:]).any()
+    assert (out[0, :, 100] == 0).all() and (lse[0, :, 100] == float("-inf")).all() and (lse[0, 3, 200:333] == float("-inf")).all()
+    fin = torch.isfinite(lse)
+    assert torch.equal(fin, torch.isfinite(lse2)) and fin.any()
+    torch.testing.assert_close(out[fin].float(), out2[fin].float(), atol=0.02, rtol=0.02)
+    torch.testing.assert_close(lse[fin], lse2[fin], atol=0.002, rtol=0.0002)
+    bits, lse_bits = out.view(torch.int16).clone(), lse.view(torch.int32).clone()
+    one.poison()
+    one.metadata(), one.main(), one.combine()
+    assert torch.equal(one.out.view(torch.int16), bits) and torch.equal(one.out_lse.view(torch.int32), lse_bits)
+    fused, fused_lse = m.kv_centric_attention(*dev, nseg=1)
+    assert torch.equal(fused.view(torch.int16), bits) and torch.equal(fused_lse.view(torch.int32), lse_bits)
