@@ -131,7 +131,7 @@ int sparse_b200_kv_centric_single(const void* q, const void* k, const void* v, c
  * KV ranges are processed outer; each (query block, KV range) yields one partial
  * (O, LSE), merged per query. `workspace` (device, 256-byte aligned) must hold
  * sparse_b200_kv_centric_workspace_bytes(...) bytes; nothing is allocated. With nseg = 1 and bf16 partials the single
- * partial goes straight to out. */
+ * partial goes straight to out, and the workspace holds the lists only. */
 int64_t sparse_b200_kv_centric_workspace_bytes(int batch, int hq, int hkv, int sq, int topk, int nseg,
                                                int partial_is_f32);
 int sparse_b200_kv_centric(const void* q, const void* k, const void* v, const int32_t* block_idx,

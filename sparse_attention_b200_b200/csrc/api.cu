@@ -229,8 +229,10 @@ int64_t sparse_b200_kv_centric_workspace_bytes(int batch, int hq, int hkv, int s
   const size_t rows = static_cast<size_t>(batch) * hq * sq;
   size_t total = 256;                                                   // error word
   total += align256(lists * nseg * topk * 4) + align256(lists * nseg * 4);   // segment lists and counts
-  total += align256(rows * nseg * 128 * (partial_is_f32 ? 4 : 2));      // partial O
-  total += align256(rows * nseg * 4);                                   // partial LSE
+  if (nseg > 1 || partial_is_f32) {                                     // a single bf16 partial is the output
+    total += align256(rows * nseg * 128 * (partial_is_f32 ? 4 : 2));    // partial O
+    total += align256(rows * nseg * 4);                                 // partial LSE
+  }
   return static_cast<int64_t>(total);
 }
 
@@ -253,9 +255,6 @@ int sparse_b200_kv_centric(const void* q, const void* k, const void* v, const in
   w += align256(lists * nseg * topk * 4);
   int32_t* seg_counts = reinterpret_cast<int32_t*>(w);
   w += align256(lists * nseg * 4);
-  void* partial = w;
-  w += align256(rows * nseg * 128 * (partial_is_f32 ? 4 : 2));
-  float* plse = reinterpret_cast<float*>(w);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (cudaMemsetAsync(err, 0, 4, st) != cudaSuccess) return set_error(SB_ERR_CUDA, "memset failed");
   rc = launch_split_segments(block_idx, block_count, seg_ids, seg_counts, err, static_cast<long long>(lists), topk,
@@ -263,6 +262,9 @@ int sparse_b200_kv_centric(const void* q, const void* k, const void* v, const in
   if (rc) return rc;
   if (nseg == 1 && !partial_is_f32)      // one bf16 partial is the output
     return sparse_b200_kv_centric_single(q, k, v, seg_ids, seg_counts, out, lse, batch, hq, hkv, sq, skv, topk, stream);
+  void* partial = w;
+  w += align256(rows * nseg * 128 * (partial_is_f32 ? 4 : 2));
+  float* plse = reinterpret_cast<float*>(w);
   QCentricArgs a{q, k, v, seg_ids, seg_counts, partial, plse, batch, hq, hkv, sq, skv, topk, nseg,
                  partial_is_f32 ? 1 : 0};
   rc = launch_q_centric(a, st);

@@ -277,3 +277,29 @@ def test_single_range_rows_of_nan_and_inf():
     assert torch.equal(one.out.view(torch.int16), bits) and torch.equal(one.out_lse.view(torch.int32), lse_bits)
     fused, fused_lse = m.kv_centric_attention(*dev, nseg=1)
     assert torch.equal(fused.view(torch.int16), bits) and torch.equal(fused_lse.view(torch.int32), lse_bits)
+
+
+def test_workspace_of_a_single_range_holds_the_lists_only():
+    """A bf16 partial of a single range is the output: the fused entry asks for the lists' bytes, and writes nothing behind
+    them."""
+    import ctypes
+    m = sp()
+    b, hq, hkv, sq, nb, topk = 1, 4, 2, 1024, 12, 5
+    size = m.lib().sparse_b200_kv_centric_workspace_bytes
+    size.restype = ctypes.c_int64
+    lists, rows = b * hkv * sq // 128, b * hq * sq
+
+    def up(n):
+        return (n + 255) // 256 * 256
+    need = size(b, hq, hkv, sq, topk, 1, 0)
+    assert need == 256 + up(lists * topk * 4) + up(lists * 4)
+    assert size(b, hq, hkv, sq, topk, 1, 1) == need + up(rows * 128 * 4) + up(rows * 4)
+    assert size(b, hq, hkv, sq, topk, 3, 0) == 256 + up(3 * lists * topk * 4) + up(3 * lists * 4) + up(3 * rows * 256) + up(3 * rows * 4)
+    q, k, v = gen.make_qkv(b, hq, hkv, sq, nb * 128, seed=5)
+    ids = gen.make_ids(b, hkv, sq // 128, nb, topk, 6, "unsorted").cuda()
+    whole = torch.full((need + 4096,), 0xA5, dtype=torch.uint8, device="cuda")
+    out, lse = m.kv_centric_attention(q.cuda(), k.cuda(), v.cuda(), ids, nseg=1, workspace=whole[:need])
+    torch.cuda.synchronize()
+    m.device_status()
+    assert (whole[need:] == 0xA5).all()
+    close(out, lse, *oracle.gather_attention(q, k, v, ids.cpu()))
