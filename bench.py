@@ -308,7 +308,7 @@ class Workload:
             prep = sp.Prepared(self.q, self.k, self.v, self.ids, nseg=segments, partial="bf16")
             self.prepared = prep
             self.out, self.lse = prep.out, prep.out_lse
-            return prep.run, 3
+            return prep.run, 2 if prep.single else 3        # metadata, main and, with several ranges, their merge
         self.out = torch.empty_like(self.q)
         self.lse = torch.empty((self.ng, self.G, cfg["N"]), dtype=torch.float32, device=self.dev)
 
@@ -322,6 +322,9 @@ class Workload:
         prep, st = self.prepared, self.stages
         st["kv_metadata_ms"] = timed(prep.metadata, steps, warmup, barrier)
         st["kv_main_ms"] = timed(prep.main, steps, warmup, barrier)
+        st["kv_ranges"] = prep.nseg
+        if prep.single:                          # one range: main writes the output
+            return
         st["kv_combine_ms"] = timed(prep.combine, steps, warmup, barrier)
         rows = self.ng * self.G * self.cfg["N"]
         st["kv_combine_gbs"] = rows * (prep.nseg * (256 + 4) + 256 + 4) / st["kv_combine_ms"] / 1e6
@@ -820,7 +823,7 @@ def run_ours(args):
                              "algorithmic_bytes": attention_bytes(cfg, wl.ng), "algorithmic_flop": local_flops,
                              "peak_source": peaks["source"] + ", burst bf16",
                              "kernel": "q_centric_kernel" if cfg["op"] == "q_centric" else
-                                       "split_segments + q_centric_kernel (partials) + combine",
+                                       "split_segments + q_centric_kernel" + ("" if kernels == 2 else " (partials) + combine"),
                              "launches_timed": steps * kernels},
                 "indexer_ms": idx_ms if idx_ms else None,
                 "indexer": {"ms": idx_ms, "pool_ms": pool_ms, "select_ms": idx_ms - pool_ms,
@@ -1302,7 +1305,8 @@ def main():
     ap.add_argument("--no-configs", action="store_true", help="skip the c1..c4 sub-record of the headline run")
     ap.add_argument("--no-kv-split", action="store_true", help="skip the KV-split sub-record of multi-GPU runs")
     ap.add_argument("--n", type=int, default=0, help="override the token count of the workload (small profiler cases)")
-    ap.add_argument("--segments", type=int, default=4, help="KV-range segments of the KV-centric operator (c4)")
+    ap.add_argument("--segments", type=int, default=None,
+                    help="KV-range segments of the KV-centric operator (c4); its own choice where not given")
     args = ap.parse_args()
     if args.workload == "kvtoken":
         run_kv_token(args)
