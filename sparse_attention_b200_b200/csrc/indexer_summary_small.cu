@@ -415,6 +415,12 @@ struct RowsPlan {
 // 49.9 -> 11.5; 16 of 1 x 64 16.9 -> 9.6; 4 of 1 x 8 11.6 -> 8.1; 2048 of 1 x 2048, five lists to a tile, 662 -> 161;
 // 1024 of 8 x 8192 2237 -> 1948. (A cluster of 8 CTAs per list and 16 descriptors, which was used for up to 148 lists before
 // the row tiles, took 15.1, 10.7 and 9.1 us for the first three; on a few lists of 65 to 128 keys it was 1 us faster.)
+// The constants were fitted to the times of all plans of 673 problems (1 to 1448 lists of 1 to 64 x 8 to 8192, whole selector with
+// scores): the choice is 1.0 % behind the best plan (geometric mean) and 6.6 % ahead of fp32 tiles with a plan of their own. It is
+// more than 2 % behind those on 21 problems, more than 5 % on three (1204 lists of 3 x 291 64.5 -> 69.4 us, 744 of 4 x 1038 63.3 ->
+// 67.7, 171 of 16 x 1218 64.7 -> 68.2). With 128 keys to a chunk wherever there is a second half, and constants from fewer
+// problems, 82 were more than 2 % behind and 55 more than 5 (3 lists of 48 x 96 9.5 -> 11.8 us, now 8.9; 58 of 24 x 688 23.6 ->
+// 26.1, 21.9; 160 of 16 x 1024 71.3 -> 77.8, 71.3). On 200 further problems 6 and 1 are (23 and 13).
 RowsPlan plan_rows(long long heads, int qt, int nt, int r, int topk, int mp_log2, int sm_count) {
   const float nf = static_cast<float>(nt);
   float sort_stage = 0.f, stages = 0.f;        // k > 128: cycles per list and stage beside others, number of stages
@@ -430,8 +436,9 @@ RowsPlan plan_rows(long long heads, int qt, int nt, int r, int topk, int mp_log2
   for (int n = full;; n = (n + 1) / 2) {
     const int tiles = (qt + n - 1) / n, lists = (qt + tiles - 1) / tiles;
     const int rows = lists << mp_log2, per_thread = rows <= 16 ? 1 : rows <= 32 ? 2 : 4;
-    for (int c = 8; c >= 1; c >>= 1) {
-      const int kg = per_thread == 4 && nt * r > KD ? 2 : 1;           // no empty second half
+    for (int i = 0; i < 8; ++i) {
+      const int c = 8 >> (i >> 1), kg = 1 + (i & 1);
+      if (kg == 2 && (per_thread < 4 || nt * r <= KD)) continue;       // no empty second half
       const int own = (lists + c - 1) / c, chunks = (nt * r + KD * kg - 1) / (KD * kg);
       if ((c > 1 && c / 2 >= chunks) || own * nt * 4 > SCORE_BYTES_MAX) continue;
       // k > 128: room to sort as many lists at a time as fp32 tiles would leave
@@ -440,30 +447,27 @@ RowsPlan plan_rows(long long heads, int qt, int nt, int r, int topk, int mp_log2
       const long long ctas = heads * tiles * c;
       const int most = per_thread < 4 ? 4 : kg == 1 ? 3 : 2;
       const int resident = static_cast<int>(SMEM_PER_SM / (smem + 1024)) < most ? static_cast<int>(SMEM_PER_SM / (smem + 1024)) : most;
-      const long long slots = static_cast<long long>(resident) * sm_count;
-      const float waves = static_cast<float>((ctas + slots - 1) / slots);
       const float load = static_cast<float>((ctas + sm_count - 1) / sm_count);       // CTAs of an SM in all
-      // A chunk of 64 keys (128 with kg = 2), cycles of an SM; slower for a CTA by itself. A saturated SM takes 14000 for the
-      // last; the smaller figure chooses better among the plans of problems that do not saturate it (160 lists of 16 x 1024
-      // 39.3 us, 42.5 with 14000 and the fp32 tiles' 5200 and 6200; 64 of 16 x 512 25.9 and 28.1).
-      float chunk = per_thread == 1 ? 3200.f : per_thread == 2 ? 4200.f : kg == 1 ? 6000.f : 10500.f;
-      if (ctas <= sm_count) chunk *= 1.17f;
-      // clusters of a second wave wait until all their slots are free
-      if (ctas > slots) chunk *= c == 8 ? 1.25f : c == 4 ? 1.2f : c == 2 ? 1.1f : 1.f;
+      const float rounds = static_cast<float>(ctas) / static_cast<float>(resident * sm_count);
+      // a chunk of 64 keys (128 with kg = 2), cycles of an SM
+      float chunk = per_thread == 1 ? 2920.f : per_thread == 2 ? 3870.f : kg == 1 ? 5520.f : 10580.f;
+      // clusters of a second round wait until all their slots are free
+      if (c >= 4 && rounds > 1.f) chunk *= 1.f + (c == 8 ? 0.15f : 0.12f) * (rounds < 2.f ? rounds - 1.f : 1.f);
       const float share = static_cast<float>(lists) / static_cast<float>(c);
       float alone, among;                      // ranking: of the busiest CTA by itself, of the average one beside others
       if (nt <= 256 && ((own * nt + 255) >> 8) * nt <= 512 * ((own + 7) >> 3)) {
-        alone = static_cast<float>((own * nt + 255) >> 8) * nf * 10.f;
-        among = share * nf * nf * (10.f / 256.f);
+        alone = static_cast<float>((own * nt + 255) >> 8) * nf * 14.f;
+        among = share * nf * nf * (7.f / 256.f);
       } else if (topk <= 128) {
-        alone = search * (own > 5 ? 0.2f * static_cast<float>(own) : 1.f);
-        among = search * 0.2f * share;
+        alone = search * (own > 5 ? 0.34f * static_cast<float>(own) : 1.7f);
+        among = search * 0.28f * share;
       } else {
-        alone = stages * (own * sort_stage > 80.f ? own * sort_stage : 80.f);
-        among = stages * share * sort_stage;
+        alone = stages * (own * sort_stage > 80.f ? own * sort_stage : 80.f) * 7.3f;
+        among = stages * share * sort_stage * 1.3f;
       }
       const float ranking = alone > load * among ? alone : load * among;
-      const float cost = waves * (c > 1 ? 3300.f : 2500.f) + load * chunk * static_cast<float>((chunks + c - 1) / c) + ranking;
+      const float start = c == 1 ? 3240.f : c == 2 ? 4010.f : c == 4 ? 4910.f : 6690.f;
+      const float cost = (rounds > 1.f ? rounds : 1.f) * start + load * chunk * static_cast<float>((chunks + c - 1) / c) + ranking;
       if (best.lists == 0 || cost < best_cost) {
         best = RowsPlan{lists, tiles, c, per_thread, kg, tile_words, smem};
         best_cost = cost;

@@ -410,6 +410,31 @@ def test_row_tiles_at_the_edges_of_a_key_chunk(g, qb, keys):
     assert torch.equal(fused.ids, staged.ids)
 
 
+@pytest.mark.parametrize("hkv,g,qb,nb,r,topk", [
+    (1, 12, 3, 24, 4, 16),      # 64 rows, one list to a tile, two CTAs with a chunk of 64 keys each
+    (1, 32, 9, 75, 2, 75),      # four CTAs
+    (1, 6, 58, 172, 4, 16),     # two lists to a tile
+    (4, 8, 226, 41, 4, 41),     # more CTAs than fit at once
+    (1, 16, 160, 1024, 1, 16),  # clusters of eight, a little more than a round
+    (2, 1, 1131, 38, 4, 16),    # sixteen lists to a tile, one CTA each
+])
+def test_row_tiles_with_one_group_of_keys_to_a_chunk(hkv, g, qb, nb, r, topk):
+    """Problems whose 64-row tiles go through 64 keys at a time, or did with another estimate: scores and ids bit for bit
+    against the staged exact kernels."""
+    m = sp()
+    q, k, _ = gen.make_qkv(1, hkv * g, hkv, qb * 128, nb * 128, seed=59, k_block_offset=0.5)
+    qc, kc = q.cuda(), k.cuda()
+    staged = m.SummarySelector(qc, kc, r, topk=topk, keep_scores=True)
+    staged.prepare()
+    staged.score()
+    fused = m.SummarySelector(qc, kc, r, topk=topk, keep_scores=True)
+    fused.run()
+    torch.cuda.synchronize()
+    m.device_status()
+    assert torch.equal(fused.scores, staged.scores)
+    assert torch.equal(fused.ids, staged.ids)
+
+
 @pytest.mark.parametrize("b,hkv,g,qb,nb,r,topk", [
     (1, 2, 1, 80, 33, 1, 33),        # 160 lists of one descriptor, every block selected
     (1, 1, 2, 150, 300, 2, 40),      # four descriptors, threshold search
