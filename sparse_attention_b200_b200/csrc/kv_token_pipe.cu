@@ -39,8 +39,9 @@ constexpr int NUM_THREADS = 512;
 constexpr int EPI_WARP0 = 8;
 constexpr int MMA_WARP = 12;
 constexpr int LOAD_WARP = 13;
-// register budgets per thread after the setup barrier: 128 * (2 * 192 + 64 + 64) = 65536 (176 for the softmax warps
-// leave them 25 spilled words: main stage of eight 4 Ki sequences 718 -> 985 us)
+// register budgets per thread after the setup barrier: 128 * (2 * 192 + 64 + 64) = 65536. ptxas spills 28 bytes with bf16
+// partials and 20 with fp32 ones, 100 and 108 at 176 / 64 / 96 (main stage of eight 4 Ki sequences 718 -> 985 us); none did
+// before records and ids were fetched ahead.
 constexpr int SOFTMAX_REGS = 192;
 constexpr int EPI_REGS = 64;
 constexpr int CTRL_REGS = 64;

@@ -43,8 +43,8 @@ constexpr int NUM_THREADS = 512;     // four warpgroups: softmax 0, softmax 1, e
 constexpr int EPI_WARP0 = 8;         // warps 8..11: warp w serves tensor-memory lanes 32 * (w % 4) ..
 constexpr int MMA_WARP = 12;
 constexpr int LOAD_WARP = 13;
-// register budgets per thread after the setup barrier (setmaxnreg); 128 * (2 * 192 + 64 + 64) = 65536. At 176 / 64 / 96 the
-// softmax warps spill six words: 1 Mi-token group 34.2 -> 33.6 ms, KV-centric case 30.0 -> 29.7, 16 heads over 16 Ki keys
+// register budgets per thread after the setup barrier (setmaxnreg); 128 * (2 * 192 + 64 + 64) = 65536. bf16 output spills
+// nothing, fp32 output 44 bytes; at 176 / 64 / 96 they spill 24 and 60: 1 Mi-token group 34.2 -> 33.6 ms, KV-centric case 30.0 -> 29.7, 16 heads over 16 Ki keys
 // 124.6 -> 123.9 us, 32 heads at 32 Ki 1118 -> 1112 without (medians of three interleaved runs)
 constexpr int SOFTMAX_REGS = 192;
 constexpr int EPI_REGS = 64;
@@ -264,7 +264,7 @@ __device__ __forceinline__ int slice_of(const ScatterOff&, long long&) { return 
 // PAIR: pair mode (see the head of this file). An instantiation of its own for each mode: the roles' loops hold one mode's
 // code, and no branch on it (with a load of the parameter that the issuer has no register to keep) stands between a wait and
 // its MMAs. With FastDiv, which alone made the compiler reload more (all cases 3-12 % slower): 16 heads over 16 Ki keys
-// 126 -> 115.5 us, 32 heads at 32 Ki 1106 -> 1080 us, 1 Mi-token group 33.3 -> 32.7 ms, R1 selection + attention of a
+// 132.3 -> 123.4 us (four calls in a row), 32 heads at 32 Ki the same within 4 %, 1 Mi-token group 33.3 -> 32.7 ms, R1 selection + attention of a
 // 4 Ki prompt 35.1 -> 33.0 us.
 template <bool OUT_F32, bool PAIR, typename Scatter>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
