@@ -7,6 +7,7 @@ Differences the block-list contract brings: selections are per query BLOCK
 reverse index is by KV range (nseg ranges) instead of by single block, so the
 partial buffers are nseg x the output instead of TopK x (none with a single range)."""
 import functools
+import math
 
 import torch
 
@@ -22,15 +23,20 @@ def default_segments(kv_blocks, topk, items=None, rows=0, sm_count=148):
     One range has no partials to write and merge, and its K/V need not stay in L2 for that: 1 against 4 ranges, us: 64
     heads of 131072 tokens, 64 blocks 29100 and 33100; 8 heads over 8192 blocks (512 MB of K and V) 3570 and 4380; 8 heads
     of 256 query blocks, 16 blocks 510 and 775. More ranges are for launches whose work items leave SMs idle, in all or in
-    the last round. items: work items of one range (two 128-row tiles each), rows: output rows. An item takes 5.5 us + 1.7
-    us per block, a merge 6 us + 0.15 us per item and the partials' way through memory. On 110 random problems the choice is
-    1.47 times as fast as 4 ranges (geometric mean, 0.4 % behind the best of 1, 2 and 4)."""
+    the last round. items: work items of one range (two 128-row tiles each), rows: output rows. An item takes 3.8 us + 1.7
+    us per block, a merge 3.5 us + 0.04 us per item and the partials' way through L2 (10 TB/s); the longest lists of a range
+    hold topk / n blocks and a deviation that depends on the share of the blocks that a list takes. Fitted to 232 random
+    problems of up to 1300 items: 1.32 times as fast as 4 ranges (geometric mean, 0.1 % behind the best of 1, 2 and 4), on
+    none of them slower. (Without the deviation, and with other constants, 13 problems of 8 to 160 items were 5 to 29 %
+    slower: 32 items of 10 blocks 20.1 us with 4 ranges, 25.9 with one.)"""
     if items is None:
         return max(1, min(4, kv_blocks, topk))
 
     def cost(n):
-        merge = 6 + 0.15 * items + n * rows * 512 / 6e6 if n > 1 else 0
-        return -(-items * n // sm_count) * (5.5 + 1.7 * -(-topk // n)) + merge
+        deviation = 0.7 * (topk / n * (1 - 1 / n) * max(0, 1 - topk / kv_blocks)) ** 0.5
+        longest = min(topk, math.ceil(topk / n + deviation))
+        merge = 3.5 + 0.04 * items + n * rows * 512 / 1e7 if n > 1 else 0
+        return -(-items * n // sm_count) * (3.8 + 1.7 * longest) + merge
     return min((n for n in (1, 2, 4) if n <= min(kv_blocks, topk)), key=cost, default=1)
 
 
