@@ -1224,7 +1224,9 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = static_cast<uint32_t>(misc[0]);
-  const int total = RUNS ? misc[7] : place.left;
+  int total;
+  if constexpr (RUNS) total = misc[7];
+  else total = place.left;
   auto first_item = [&]() {
     if constexpr (RUNS) return ScoreWalk<PACKED, RUNS>(p, misc + 2);
     else return place;
