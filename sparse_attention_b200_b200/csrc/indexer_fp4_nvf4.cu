@@ -987,15 +987,24 @@ struct QueryScoreParams {
 };
 constexpr int QS_THREADS = 224;
 constexpr int QS_PACK_Q = 8, QS_PACK_HEADS = 16;
-constexpr int QS_STAGES = 8;           // pages in flight
 constexpr int QS_AHEAD = 4;            // pages whose scales are on their way to their staging ring
-constexpr int QS_OFF_Q = QS_STAGES * STAGE_BYTES;          // two query tiles: codes + scales
-constexpr int QS_OFF_RAW = QS_OFF_Q + 2 * STAGE_BYTES;     // staging ring: the scales of a page as they are in memory
-constexpr int QS_OFF_AUX = QS_OFF_RAW + QS_AHEAD * SF_BYTES;   // barriers, misc (64 bytes), sums (64)
-enum { QS_K_FULL = 0, QS_K_EMPTY = QS_STAGES, QS_Q_FULL = 2 * QS_STAGES, QS_Q_EMPTY = QS_Q_FULL + 2,
-       QS_ACC_FULL = QS_Q_EMPTY + 2, QS_ACC_EMPTY, QS_BARS };
-constexpr int QS_BAR_BYTES = (QS_BARS * 8 + 63) & ~63;
-constexpr int QS_SMEM = QS_OFF_AUX + QS_BAR_BYTES + 128 + 1024;
+// Shared memory and barriers: eight pages in flight and two query tiles. With shares of packed items (THREE) one query tile and
+// four pages (and 80 registers) leave room for a third CTA on the SM, which is set up by the time one of the other two gives up
+// its tensor memory: 1300 of the 4900 to 8600 cycles of a CTA. One-token requests in a graph, us: 1024 of 100 to 400 keys 17.6 ->
+// 16.6, 2048 30.6 -> 28.5, 1500 of 10 to 128 19.5 -> 17.2, 600 of 500 to 900 16.9 -> 17.5; six pages, which leave less L1, 17.2,
+// 29.3, 17.5 and 18.0. Not for query tiles of one head, whose launches of shares are one round: 16 requests 7.2 -> 8.8.
+template <bool THREE>
+struct QsMap {
+  static constexpr int STAGES = THREE ? 4 : 8, Q_TILES = THREE ? 1 : 2;
+  static constexpr int Q = STAGES * STAGE_BYTES;             // query tiles: codes + scales
+  static constexpr int RAW = Q + Q_TILES * STAGE_BYTES;      // staging ring: the scales of a page as they are in memory
+  static constexpr int AUX = RAW + QS_AHEAD * SF_BYTES;      // barriers, misc (64 bytes), sums (64)
+  enum { K_FULL = 0, K_EMPTY = STAGES, Q_FULL = 2 * STAGES, Q_EMPTY = Q_FULL + Q_TILES, BAR_ACC_FULL = Q_EMPTY + Q_TILES,
+         BAR_ACC_EMPTY, BARS };
+  static constexpr int BAR_BYTES = (BARS * 8 + 63) & ~63;
+  static constexpr int SMEM = AUX + BAR_BYTES + 128 + 1024;
+};
+static_assert(3 * (QsMap<true>::SMEM + 1024) <= 228 * 1024, "three CTAs to an SM");
 // tensor memory: the accumulator, two slots of key scales, two of query scales
 constexpr int QS_SFK = 128, QS_SFQ = 144;
 static_assert(QS_SFQ + 16 <= TM_COLS, "tensor memory map");
@@ -1186,31 +1195,32 @@ __device__ __forceinline__ void find_run(const QueryScoreParams& p, volatile int
 }
 
 template <bool PACKED, bool RUNS>
-__global__ void __launch_bounds__(QS_THREADS, 2)
+__global__ void __launch_bounds__(QS_THREADS, PACKED && !RUNS ? 3 : 2)
 fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
                            const QueryScoreParams p) {
+  using M = QsMap<PACKED && !RUNS>;
   extern __shared__ unsigned char smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   unsigned char* gbase = smem_raw + (base - raw);
-  const uint32_t bar0 = base + QS_OFF_AUX;
-  volatile int* misc = reinterpret_cast<volatile int*>(gbase + QS_OFF_AUX + QS_BAR_BYTES);   // tmem base, abort, start of the run
+  const uint32_t bar0 = base + M::AUX;
+  volatile int* misc = reinterpret_cast<volatile int*>(gbase + M::AUX + M::BAR_BYTES);   // tmem base, abort, start of the run
   auto bar = [&](int i) { return bar0 + 8u * i; };
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   Guard guard{misc + 1, p.status};
 
   if (threadIdx.x == 0) {
     misc[1] = 0;
-    for (int i = 0; i < QS_STAGES; ++i) {
-      mbar_init(bar(QS_K_FULL + i), 2);          // the TMA transaction of the codes + the producer warp's scale stores
-      mbar_init(bar(QS_K_EMPTY + i), 1);
+    for (int i = 0; i < M::STAGES; ++i) {
+      mbar_init(bar(M::K_FULL + i), 2);          // the TMA transaction of the codes + the producer warp's scale stores
+      mbar_init(bar(M::K_EMPTY + i), 1);
     }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(bar(QS_Q_FULL + i), 2);
-      mbar_init(bar(QS_Q_EMPTY + i), 1);
+    for (int i = 0; i < M::Q_TILES; ++i) {
+      mbar_init(bar(M::Q_FULL + i), 2);
+      mbar_init(bar(M::Q_EMPTY + i), 1);
     }
-    mbar_init(bar(QS_ACC_FULL), 1);
-    mbar_init(bar(QS_ACC_EMPTY), 4);
+    mbar_init(bar(M::BAR_ACC_FULL), 1);
+    mbar_init(bar(M::BAR_ACC_EMPTY), 4);
     fence_mbar_init();
   }
   if (warp == 5) {
@@ -1245,27 +1255,27 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
         ids = i < walk.r.pages ? __ldg(p.kv_indices + walk.r.page_begin + i) : 0;
       }
       if (left == 0) {
-        const int slot = items & 1;
-        if (items >= 2) ok = mbar_wait_warp(bar(QS_Q_EMPTY + slot), ((items >> 1) - 1) & 1, guard, 0x630 + slot);
+        const int slot = items & (M::Q_TILES - 1);
+        if (items >= 2) ok = mbar_wait_warp(bar(M::Q_EMPTY + slot), ((items >> 1) - 1) & 1, guard, 0x630 + slot);
         if (!ok) break;
         ++items;
         if (lane == 0) {
-          mbar_expect_tx(bar(QS_Q_FULL + slot), CODE_BYTES);
+          mbar_expect_tx(bar(M::Q_FULL + slot), CODE_BYTES);
           // packed: box {64 bytes, 16 heads, 8 queries}, row = query * 16 + head; else box {64 bytes, 1 head, 128 queries}
-          tma_load_3d(base + QS_OFF_Q + slot * STAGE_BYTES, &q_map, 0, walk.head0(p), walk.r.q_begin + walk.j * 128,
-                      bar(QS_Q_FULL + slot));
+          tma_load_3d(base + M::Q + slot * STAGE_BYTES, &q_map, 0, walk.head0(p), walk.r.q_begin + walk.j * 128,
+                      bar(M::Q_FULL + slot));
         }
         left = walk.count();
         pg = walk.page;
       }
-      const int s = t % QS_STAGES, use = t / QS_STAGES;
-      if (use > 0) ok = mbar_wait_warp(bar(QS_K_EMPTY + s), (use - 1) & 1, guard, 0x600 + s);
+      const int s = t % M::STAGES, use = t / M::STAGES;
+      if (use > 0) ok = mbar_wait_warp(bar(M::K_EMPTY + s), (use - 1) & 1, guard, 0x600 + s);
       if (!ok) break;
       const int ph = __shfl_sync(0xffffffffu, ids, pg & 31);
       if (lane == 0) {
-        mbar_expect_tx(bar(QS_K_FULL + s), CODE_BYTES);
+        mbar_expect_tx(bar(M::K_FULL + s), CODE_BYTES);
         tma_load_2d(base + OFF_A + s * STAGE_BYTES, &k_map, 0, ((ph < 0 || ph >= p.total_pages ? 0 : ph) * p.hk + walk.kvh) * 128,
-                    bar(QS_K_FULL + s));
+                    bar(M::K_FULL + s));
       }
       ++pushed;
       ++pg;
@@ -1273,9 +1283,9 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
     }
     if (!ok) {
       // let copies in flight land before the CTA gives up its shared memory
-      for (int t = max(0, pushed - QS_STAGES); t < pushed; ++t)
-        mbar_wait_drain(bar(QS_K_FULL + t % QS_STAGES), (t / QS_STAGES) & 1);
-      for (int i = max(0, items - 2); i < items; ++i) mbar_wait_drain(bar(QS_Q_FULL + (i & 1)), (i >> 1) & 1);
+      for (int t = max(0, pushed - M::STAGES); t < pushed; ++t)
+        mbar_wait_drain(bar(M::K_FULL + t % M::STAGES), (t / M::STAGES) & 1);
+      for (int i = max(0, items - 2); i < items; ++i) mbar_wait_drain(bar(M::Q_FULL + (i & 1)), (i >> 1) & 1);
     }
   } else if (warp == 6) {
     // ----------------------------------------------------------- scales: staged QS_AHEAD pages ahead, then re-ordered
@@ -1283,7 +1293,7 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
     // instructions alone, fetched for the first time, took 7000 cycles before the first page)
     ScoreWalk<PACKED, RUNS> ahead_walk = first_item(), walk = first_item();
     int ids = 0, ahead_left = 0, ahead_pg = 0;    // of the walk ahead: 32 page ids, pages left in its item, next page
-    auto raw = [&](int t) { return QS_OFF_RAW + (t % QS_AHEAD) * SF_BYTES + lane * 8; };
+    auto raw = [&](int t) { return M::RAW + (t % QS_AHEAD) * SF_BYTES + lane * 8; };
     auto fetch = [&](int t) {                     // rows lane, lane + 32, .. of page t; one group per page
       if (t < total) {
         const bool first = ahead_left == 0;
@@ -1312,7 +1322,7 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
 #pragma unroll 1
     for (int t = 0; t < total; ++t) {
       if (left == 0) {
-        const int slot = items & 1;
+        const int slot = items & (M::Q_TILES - 1);
         const int h0 = walk.head0(p), q0 = walk.j * 128;
         const int rows_live = walk.r.q_rows - q0, heads_here = PACKED ? p.group - walk.sub * QS_PACK_HEADS : 1;
         ScaleRegs s;
@@ -1324,16 +1334,16 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
             s.r[i] = __ldg(reinterpret_cast<const uint2*>(
                 p.qs + ((static_cast<long long>(walk.r.q_begin) + q0 + q) * p.hq + h0 + h) * 8));
         }
-        if (items >= 2) ok = mbar_wait_warp(bar(QS_Q_EMPTY + slot), ((items >> 1) - 1) & 1, guard, 0x634 + slot);
+        if (items >= 2) ok = mbar_wait_warp(bar(M::Q_EMPTY + slot), ((items >> 1) - 1) & 1, guard, 0x634 + slot);
         if (!ok) break;
         ++items;
-        store_scale_chunks(gbase + QS_OFF_Q + slot * STAGE_BYTES + CODE_BYTES, s, lane);
+        store_scale_chunks(gbase + M::Q + slot * STAGE_BYTES + CODE_BYTES, s, lane);
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar(QS_Q_FULL + slot));
+        if (lane == 0) mbar_arrive(bar(M::Q_FULL + slot));
         left = walk.count();
       }
-      const int s = t % QS_STAGES, use = t / QS_STAGES;
-      if (use > 0) ok = mbar_wait_warp(bar(QS_K_EMPTY + s), (use - 1) & 1, guard, 0x608 + s);
+      const int s = t % M::STAGES, use = t / M::STAGES;
+      if (use > 0) ok = mbar_wait_warp(bar(M::K_EMPTY + s), (use - 1) & 1, guard, 0x608 + s);
       if (!ok) break;
       cp_async_wait<QS_AHEAD - 1>();              // this lane's rows of page t have landed
       ScaleRegs regs;
@@ -1341,7 +1351,7 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
       for (int i = 0; i < 4; ++i) regs.r[i] = *reinterpret_cast<const uint2*>(gbase + raw(t) + i * 256);
       store_scale_chunks(gbase + OFF_A + s * STAGE_BYTES + CODE_BYTES, regs, lane);
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar(QS_K_FULL + s));
+      if (lane == 0) mbar_arrive(bar(M::K_FULL + s));
       fetch(t + QS_AHEAD);
       if (--left == 0) walk.next(p);
     }
@@ -1355,10 +1365,10 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
     int items = 0, left = 0;
     for (int t = 0; t < total; ++t) {
       const int slot = (items - (left ? 1 : 0)) & 1;       // of the current item's query tile
-      const uint32_t q_tile = base + QS_OFF_Q + slot * STAGE_BYTES;
+      const uint32_t q_tile = base + M::Q + slot * STAGE_BYTES;
       const uint32_t sfq = tmem + QS_SFQ + slot * 8;       // query scales: the A operand here
       if (left == 0) {
-        ok = mbar_wait_warp(bar(QS_Q_FULL + slot), (items >> 1) & 1, guard, 0x610 + slot);
+        ok = mbar_wait_warp(bar(M::Q_FULL + slot), (items >> 1) & 1, guard, 0x610 + slot);
         if (!ok) break;
         fence_async_smem();            // the producer's scale stores, for the copies below
         tc_fence_after();
@@ -1370,8 +1380,8 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
         left = walk.count();
         walk.next(p);
       }
-      const int s = t % QS_STAGES;
-      ok = mbar_wait_warp(bar(QS_K_FULL + s), (t / QS_STAGES) & 1, guard, 0x612 + s);
+      const int s = t % M::STAGES;
+      ok = mbar_wait_warp(bar(M::K_FULL + s), (t / M::STAGES) & 1, guard, 0x612 + s);
       if (!ok) break;
       fence_async_smem();              // the producer's scale stores, for the copies below
       tc_fence_after();
@@ -1382,7 +1392,7 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
         tmem_cp_scales(sfk + 4, desc_scale_chunk(base + OFF_A + s * STAGE_BYTES + CODE_BYTES + 512));
       }
       if (t >= 1) {
-        ok = mbar_wait_warp(bar(QS_ACC_EMPTY), (t - 1) & 1, guard, 0x61a);
+        ok = mbar_wait_warp(bar(M::BAR_ACC_EMPTY), (t - 1) & 1, guard, 0x61a);
         if (!ok) break;
         tc_fence_after();
       }
@@ -1391,9 +1401,9 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
 #pragma unroll
         for (int kh = 0; kh < 2; ++kh)
           mma_nvf4(tmem + TM_ACC, a0 + kh * 2, b0 + kh * 2, IDESC, sfq + kh * 4, sfk + kh * 4, kh);
-        tc_commit(bar(QS_ACC_FULL));
-        tc_commit(bar(QS_K_EMPTY + s));
-        if (left == 0) tc_commit(bar(QS_Q_EMPTY + slot));
+        tc_commit(bar(M::BAR_ACC_FULL));
+        tc_commit(bar(M::K_EMPTY + s));
+        if (left == 0) tc_commit(bar(M::Q_EMPTY + slot));
       }
     }
     __syncwarp();
@@ -1418,7 +1428,7 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
       const int stop = walk.page + walk.count();
       for (int pg = walk.page; pg < stop; ++pg, ++t) {
         const int ph = __ldg(p.kv_indices + walk.r.page_begin + pg);      // (the page stays -inf where it is out of range)
-        bool w = mbar_wait(bar(QS_ACC_FULL), t & 1, guard, 0x620);
+        bool w = mbar_wait(bar(M::BAR_ACC_FULL), t & 1, guard, 0x620);
         ok = __all_sync(0xffffffffu, w);
         if (!ok) break;
         tc_fence_after();
@@ -1433,7 +1443,7 @@ fp4_nv_query_scores_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
           if (half == 1) {
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar(QS_ACC_EMPTY));
+            if (lane == 0) mbar_arrive(bar(M::BAR_ACC_EMPTY));
           }
           if (visible >= (half + 1) * 64) {
 #pragma unroll
@@ -1632,7 +1642,7 @@ int launch_fp4_scores_varlen_nv(const void* qp, const void* qs, const void* kp, 
   // there were runs): one token of one request 6.9 -> 5.1 (5.5), of 64 requests of 100 to 400 keys 8.9 -> 5.3 (5.8), of 256 11.1 ->
   // 9.0 (9.4), prefill of eight requests of up to 300 8.5 -> 6.3 (7.2). Beyond, runs are faster (64 requests of 1000 to 4000
   // keys 11.1, shares 13.2) unless a request is one item of a few pages, where a run changes its item every other page: 600
-  // requests of 500 to 900 keys 18.9 -> 16.9 (16.2), 1024 of 100 to 400 20.1 -> 17.6 (16.0), 2048 32.6 -> 30.6 (26.3).
+  // requests of 500 to 900 keys 18.9 -> 17.5 (16.2), 1024 of 100 to 400 20.1 -> 16.6 (16.0), 2048 32.6 -> 28.5 (26.3).
   int share = 64;
   while (share > 2 && items * ((p.tiles_out + share - 1) / share) < 4LL * ctx->sm_count) share >>= 1;
   const long long shared = items * ((p.tiles_out + share - 1) / share);
@@ -1666,7 +1676,7 @@ int launch_fp4_scores_varlen_nv(const void* qp, const void* qs, const void* kp, 
   if (!(ctx->tc_attr & (1 << 12))) {
     for (auto kernel : {fp4_nv_query_scores_kernel<false, false>, fp4_nv_query_scores_kernel<false, true>,
                         fp4_nv_query_scores_kernel<true, false>, fp4_nv_query_scores_kernel<true, true>}) {
-      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, QS_SMEM);
+      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, QsMap<false>::SMEM);
       if (e != cudaSuccess) return set_error(SB_ERR_CUDA, cudaGetErrorString(e));
     }
     ctx->tc_attr |= (1 << 12);
@@ -1674,7 +1684,7 @@ int launch_fp4_scores_varlen_nv(const void* qp, const void* qs, const void* kp, 
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(QS_THREADS);
-  cfg.dynamicSmemBytes = QS_SMEM;
+  cfg.dynamicSmemBytes = packed && !runs ? QsMap<true>::SMEM : QsMap<false>::SMEM;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
